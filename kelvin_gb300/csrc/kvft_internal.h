@@ -42,6 +42,16 @@ struct KOut {
     long long bst;
 };
 
+// Products of one contraction that share their shapes and strides and differ
+// in where their operands start: C + oc[q] (+)= alpha (A + oa[q]) (B + ob[q]).
+// The spin blocks of a contraction are such a group; products with the same
+// oc add into the same block of C.
+constexpr int KV_MAXPROD = 24;
+struct KvProds {
+    int n = 0;
+    long long oa[KV_MAXPROD], ob[KV_MAXPROD], oc[KV_MAXPROD];   // element offsets
+};
+
 inline KIdx kidx1(int s0, long long t0) { return KIdx{{1, 1, s0}, {0, 0, t0}}; }
 inline KIdx kidx2(int s0, long long t0, int s1, long long t1) {
     return KIdx{{1, s0, s1}, {0, t0, t1}};
@@ -129,27 +139,10 @@ struct kvft_ctx {
     // bumped whenever a scratch or cached buffer is (re)allocated or freed:
     // a captured CUDA graph holds the addresses it saw
     uint64_t scratch_gen = 0;
-    // Packed operands shared by the products of one spin-blocked contraction
-    // (on inside KvTPackScope): key -> pool slot; the slots' buffers are
-    // scratch kept for the next contraction.
-    bool tpack_on = false;
-    std::map<std::string, int> tpack;
     // Pinned, device-mapped host staging of the amplitude read-back (two
     // halves), kept for the context's lifetime.
     void *hstage = nullptr;
     size_t hstage_bytes = 0;
-};
-struct KvTPackScope {
-    kvft_ctx *ctx;
-    bool prev;
-    explicit KvTPackScope(kvft_ctx *c) : ctx(c), prev(c->tpack_on) {
-        c->tpack_on = true;
-        if (!prev) c->tpack.clear();
-    }
-    ~KvTPackScope() {
-        ctx->tpack_on = prev;
-        if (!prev) ctx->tpack.clear();
-    }
 };
 // FP64 <-> FP32 by integer operations on the bit patterns, for values that
 // only steer the iteration (norms, the Anderson history): GB300's FP64 pipe
@@ -246,17 +239,42 @@ int kv_scratch(kvft_ctx *ctx, const char *key, size_t bytes, void **p);
 // C = alpha * A * B + beta * C, batched over `batch` tau points.
 int kv_gemm(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha,
             const KMat &A, const KMat &B, double beta, const KOut &C);
+// The same for a group of products in one launch; a block of C that several
+// products add into is scaled by beta once.
+int kv_gemm_group(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
+                  const KMat &B, double beta, const KOut &C, const KvProds &g);
 int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha,
-                const KMat &A, const KMat &B, double beta, const KOut &C);
+                const KMat &A, const KMat &B, double beta, const KOut &C, const KvProds &g);
 int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha,
-               const KMat &A, const KMat &B, double beta, const KOut &C,
-               int digits);
+               const KMat &A, const KMat &B, double beta, const KOut &C, int digits,
+               const KvProds &g);
+// The group of one product at the operands' own addresses.
+inline KvProds kv_one_prod() {
+    KvProds g;
+    g.n = 1;
+    g.oa[0] = g.ob[0] = g.oc[0] = 0;
+    return g;
+}
+// Host table of a group by block of C: blocks in order of falling source
+// count (the longest units first), source q of block c for
+// beg[c] <= q < beg[c + 1].  split: every product a block of its own (K
+// chunks that add into C by atomics).
+struct KvGroupTab {
+    int ncb = 0;
+    int beg[KV_MAXPROD + 1];
+    long long coff[KV_MAXPROD];
+    int prod[KV_MAXPROD];
+};
+KvGroupTab kv_group_tab(const KvProds &g, bool split);
 // Sets the profile category (n^6-class or not) and work (flops, or bytes
 // for the other class) of the next contraction launch.
 void kv_gemm_prof_set(kvft_ctx *ctx, int M, int N, int K, int batch, int nbA, int nbB,
                       double beta, bool tc);
 // C = beta * C over a strided output view (beta == 0 writes zeros).
 int kv_scale_view(kvft_ctx *ctx, int M, int N, int batch, double beta, const KOut &C);
+// The same over several blocks of C at the offsets off[0..n), in one launch.
+int kv_scale_blocks(kvft_ctx *ctx, int M, int N, int batch, double beta, const KOut &C, int n,
+                    const long long *off);
 // Reads (and clears) the device status word set by bounded waits; syncs.
 int kv_device_status(kvft_ctx *ctx);
 

@@ -163,20 +163,23 @@ int kv_einsum_desc(int nv, int no, const char *aix, const char *bix, const char 
 
 namespace {
 
-// One strided GEMM for a contraction already in GEMM form; a single row goes
-// as the transposed product C^T = B^T A^T, so that the long free dimension
-// is the GEMM's row dimension.
-int gemm_piece(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KvTen &A,
-               const KvTen &B, const KIdx &ar, const KIdx &ac, const KIdx &br, const KIdx &bc,
-               double beta, double *C, const KIdx &cr, const KIdx &cc, long long cbst) {
+// A group of strided GEMMs for a contraction already in GEMM form; a single
+// row goes as the transposed product C^T = B^T A^T, so that the long free
+// dimension is the GEMM's row dimension.
+int gemm_pieces(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KvTen &A,
+                const KvTen &B, const KIdx &ar, const KIdx &ac, const KIdx &br, const KIdx &bc,
+                double beta, double *C, const KIdx &cr, const KIdx &cc, long long cbst,
+                const KvProds &g) {
     if (M == 1 && N > 1) {
         KMat a{B.p, bc, br, B.bst, B.stable}, b{A.p, ac, ar, A.bst, A.stable};
         KOut c{C, cc, cr, cbst};
-        return kv_gemm(ctx, N, M, K, batch, alpha, a, b, beta, c);
+        KvProds t = g;
+        std::swap(t.oa, t.ob);
+        return kv_gemm_group(ctx, N, M, K, batch, alpha, a, b, beta, c, t);
     }
     KMat a{A.p, ar, ac, A.bst, A.stable}, b{B.p, br, bc, B.bst, B.stable};
     KOut c{C, cr, cc, cbst};
-    return kv_gemm(ctx, M, N, K, batch, alpha, a, b, beta, c);
+    return kv_gemm_group(ctx, M, N, K, batch, alpha, a, b, beta, c, g);
 }
 
 // true when the spin assignment (bit of each letter in `spins`) satisfies
@@ -213,12 +216,12 @@ int kv_einsum(kvft_ctx *ctx, int nv, int no, int batch, double alpha, const KvTe
         return kv_fail(ctx, KVFT_EINVAL, err);
     const int h = ctx->lam_spin;
     if (h <= 0 || nv != no || nv != 2 * h)
-        return gemm_piece(ctx, M, N, K, batch, alpha, A, B, ar, ac, br, bc, beta, C, cr, cc,
-                          cbst);
+        return gemm_pieces(ctx, M, N, K, batch, alpha, A, B, ar, ac, br, bc, beta, C, cr, cc,
+                           cbst, kv_one_prod());
     // Spin blocks: every letter runs over an alpha half and a beta half, and
-    // only the products whose operands satisfy their spin rules are nonzero.
-    // C is scaled by beta first; the products then add into it.
-    if (beta != 1.0) KV_TRY(kv_scale_view(ctx, M, N, batch, beta, KOut{C, cr, cc, cbst}));
+    // only the products whose operands satisfy their spin rules are nonzero:
+    // they run as one group.  The blocks of C that none of them writes are
+    // scaled by beta.
     std::string letters;
     for (const char *p : {A.ix, B.ix})
         for (const char *q = p; *q; q++)
@@ -229,18 +232,29 @@ int kv_einsum(kvft_ctx *ctx, int nv, int no, int batch, double alpha, const KvTe
                        &scc, &err, h) != KVFT_OK)
         return kv_fail(ctx, KVFT_EINVAL, err);
     unsigned char bit[128] = {0};
-    const int L = (int)letters.size();
+    const int L = (int)letters.size(), nc = (int)std::strlen(cix);
+    KvProds g;
+    std::vector<long long> written;
     for (unsigned m = 0; m < (1u << L); m++) {
         for (int k = 0; k < L; k++) bit[(unsigned char)letters[k]] = (m >> k) & 1;
         if (!spin_ok(A, bit) || !spin_ok(B, bit)) continue;
-        KvTen a = A, b = B;
-        a.p += spin_offset(A.ix, bit, h, nv, no);
-        b.p += spin_offset(B.ix, bit, h, nv, no);
-        double *c = C + spin_offset(cix, bit, h, nv, no);
-        KV_TRY(gemm_piece(ctx, sM, sN, sK, batch, alpha, a, b, sar, sac, sbr, sbc, 1.0, c, scr,
-                          scc, cbst));
+        if (g.n == KV_MAXPROD) return kv_fail(ctx, KVFT_EINVAL, "einsum: too many spin products");
+        g.oa[g.n] = spin_offset(A.ix, bit, h, nv, no);
+        g.ob[g.n] = spin_offset(B.ix, bit, h, nv, no);
+        g.oc[g.n] = spin_offset(cix, bit, h, nv, no);
+        written.push_back(g.oc[g.n++]);
     }
-    return KVFT_OK;
+    KV_TRY(gemm_pieces(ctx, sM, sN, sK, batch, alpha, A, B, sar, sac, sbr, sbc, beta, C, scr, scc,
+                       cbst, g));
+    if (beta == 1.0) return KVFT_OK;
+    std::vector<long long> rest;
+    for (unsigned m = 0; m < (1u << nc); m++) {
+        for (int k = 0; k < nc; k++) bit[(unsigned char)cix[k]] = (m >> k) & 1;
+        const long long o = spin_offset(cix, bit, h, nv, no);
+        if (std::find(written.begin(), written.end(), o) == written.end()) rest.push_back(o);
+    }
+    return kv_scale_blocks(ctx, sM, sN, batch, beta, KOut{C, scr, scc, cbst}, (int)rest.size(),
+                           rest.data());
 }
 
 int kv_add(kvft_ctx *ctx, int nv, int no, int batch, double alpha, const KvTen &src,

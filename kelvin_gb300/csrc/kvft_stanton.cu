@@ -56,14 +56,13 @@ void halve(KIdx &x, int comp, int h, int s, long long &off) {
 }
 
 // C = alpha A B + beta C over the block products that keep(spins) allows
-// (bit x of spins = spin of orbital index x, whose slots are idx[x]).  C
-// blocks that no product writes are scaled by beta (zeroed when C is the
-// whole contiguous buffer of `cwords` doubles and beta = 0), or left alone
-// with cwords = -1 (an intermediate whose readers skip those blocks too).
+// (bit x of spins = spin of orbital index x, whose slots are idx[x]), as one
+// group.  C blocks that no product writes are scaled by beta, or left alone
+// with rest = false (an intermediate whose readers skip those blocks too).
 template <class Keep>
 int spin_gemm(kvft_ctx *ctx, int h, int batch, double alpha, const KMat &A, const KMat &B,
               double beta, const KOut &C, const std::vector<std::vector<Slot>> &idx, Keep keep,
-              long long cwords = 0) {
+              bool rest = true) {
     const int nx = (int)idx.size();
     unsigned cmask = 0;
     for (int x = 0; x < nx; x++)
@@ -76,19 +75,11 @@ int spin_gemm(kvft_ctx *ctx, int h, int batch, double alpha, const KMat &A, cons
             if (v.size[s.comp] != 2 * h)
                 return kv_fail(ctx, KVFT_EINVAL, "spin blocks: index extent is not 2h");
         }
-    // products that share an operand sub-block share its digit planes
-    KvTPackScope tpack(ctx);
-    bool zeroed = false;
-    if (beta == 0.0 && cwords > 0) {
-        KV_CHECK(ctx, cudaMemsetAsync(C.p, 0, sizeof(double) * cwords, ctx->stream));
-        zeroed = true;
-    }
-    std::vector<char> written(1u << nx, 0);
-    for (unsigned m = 0; m < (1u << nx); m++) {
-        if (!keep(m)) continue;
-        KMat a = A, b = B;
-        KOut c = C;
-        long long oa = 0, ob = 0, oc = 0;
+    KMat a = A, b = B;
+    KOut c = C;
+    auto block = [&](unsigned m, long long &oa, long long &ob, long long &oc) {
+        a = A, b = B, c = C;
+        oa = ob = oc = 0;
         for (int x = 0; x < nx; x++) {
             const int sp = (m >> x) & 1;
             for (const Slot &s : idx[x]) {
@@ -97,26 +88,28 @@ int spin_gemm(kvft_ctx *ctx, int h, int batch, double alpha, const KMat &A, cons
                 else halve(s.dim ? c.c : c.r, s.comp, h, sp, oc);
             }
         }
-        a.p += oa;
-        b.p += ob;
-        c.p += oc;
-        const unsigned key = m & cmask;
-        const double be = written[key] ? 1.0 : beta;
-        written[key] = 1;
-        KV_TRY(kv_gemm(ctx, a.r.total(), b.c.total(), a.c.total(), batch, alpha, a, b, be, c));
+    };
+    KvProds g;
+    std::vector<char> written(1u << nx, 0);
+    for (unsigned m = 0; m < (1u << nx); m++) {
+        if (!keep(m)) continue;
+        if (g.n == KV_MAXPROD) return kv_fail(ctx, KVFT_EINVAL, "spin blocks: too many products");
+        block(m, g.oa[g.n], g.ob[g.n], g.oc[g.n]);
+        g.n++;
+        written[m & cmask] = 1;
     }
-    if (beta == 1.0 || zeroed || cwords < 0) return KVFT_OK;
+    KV_TRY(kv_gemm_group(ctx, a.r.total(), b.c.total(), a.c.total(), batch, alpha, a, b, beta, c,
+                         g));
+    if (beta == 1.0 || !rest) return KVFT_OK;
+    std::vector<long long> off;
     for (unsigned m = 0; m < (1u << nx); m++) {
         if ((m & ~cmask) || written[m]) continue;
-        KOut c = C;
-        long long oc = 0;
-        for (int x = 0; x < nx; x++)
-            for (const Slot &s : idx[x])
-                if (s.op == 2) halve(s.dim ? c.c : c.r, s.comp, h, (m >> x) & 1, oc);
-        c.p += oc;
-        KV_TRY(kv_scale_view(ctx, c.r.total(), c.c.total(), batch, beta, c));
+        long long oa, ob, oc;
+        block(m, oa, ob, oc);
+        off.push_back(oc);
     }
-    return KVFT_OK;
+    return kv_scale_blocks(ctx, c.r.total(), c.c.total(), batch, beta, c, (int)off.size(),
+                           off.data());
 }
 
 inline int sp(unsigned m, int x) { return (m >> x) & 1; }
@@ -204,8 +197,8 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
     typedef std::vector<std::vector<Slot>> Slots;
     auto sgemm = [&](int M, int N, int K, int batch, double alpha, const KMat &A,
                      const KMat &Bm, double beta, const KOut &C, const Slots &idx, auto keep,
-                     long long cwords) -> int {
-        if (sh) return spin_gemm(ctx, sh, batch, alpha, A, Bm, beta, C, idx, keep, cwords);
+                     bool rest = true) -> int {
+        if (sh) return spin_gemm(ctx, sh, batch, alpha, A, Bm, beta, C, idx, keep, rest);
         return kv_gemm(ctx, M, N, K, batch, alpha, A, Bm, beta, C);
     };
 
@@ -235,7 +228,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) &&
                             sp(m, 2) + sp(m, 3) == sp(m, 4) + sp(m, 1);
-                 }, 0));
+                 }));
 
     // ---- F_mi ------------------------------------------------------------
     KV_TRY(kv_bcast(ctx, B, oo, Foo, w.Fmi));
@@ -258,7 +251,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) &&
                             sp(m, 2) + sp(m, 3) == sp(m, 4) + sp(m, 1);
-                 }, 0));
+                 }));
 
     // ---- F_me ------------------------------------------------------------
     KV_TRY(kv_bcast(ctx, B, vo, Fov, w.Fme));
@@ -283,7 +276,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 3) == sp(m, 1) + sp(m, 2) && sp(m, 2) == sp(m, 3);
-                 }, 0));
+                 }));
     // - vovo[a,n,f,i] t1[f,n]   (M=(a,i), K=(n,f), N=tau)
     KV_TRY(kv_gemm(ctx, nv * no, B, no * nv, 1, -fac,
                    MAI(vovo, X2(nv, vo2, no, 1), X2(no, vo, nv, o)),
@@ -298,7 +291,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) &&
                             sp(m, 2) + sp(m, 3) == sp(m, 4) + sp(m, 1);
-                 }, 0));
+                 }));
     // +1/2 t2[a,e,m,n] ooov[n,m,i,e]; spins a e m n i
     KV_TRY(sgemm(nv, no, nv * no * no, B, 0.5 * fac,
                  MA(t2, X1(nv, vo2), X3(nv, oo, no, o, no, 1), v2o2),
@@ -308,7 +301,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) &&
                             sp(m, 3) + sp(m, 2) == sp(m, 4) + sp(m, 1);
-                 }, 0));
+                 }));
 
     // ---- ladder terms over antisymmetric pairs ---------------------------------
     // tau, W'_mnij, W'_abef and <mn||ef> are antisymmetric in each index pair,
@@ -350,7 +343,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                            {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                      [](unsigned m) {
                          return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) && sp(m, 3) == sp(m, 4);
-                     }, -1));
+                     }, false));
         // W'_c = oooo + Z - Z^(ij)
         const long long s4o[4] = {o * oo, oo, o, 1}, s4t[4] = {o * oo, oo, 1, o};
         KV_TRY(kv_pair_gather(ctx, B, no, no, oooo, s4o, 1.0, w.tmp4, s4o, 1.0, s4t, -1.0, o4,
@@ -378,7 +371,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                            {{1, 1, 1}, {2, 1, 1}}, {{1, 1, 2}, {2, 1, 2}}},
                      [](unsigned m) {
                          return sp(m, 0) == sp(m, 1) && sp(m, 2) + sp(m, 1) == sp(m, 3) + sp(m, 4);
-                     }, -1));
+                     }, false));
         // W'_abef_c = vvvv - Y + Y^(ab)
         const long long s4v[4] = {v * vv, vv, v, 1}, s4s[4] = {vv, v * vv, v, 1};
         KV_TRY(kv_pair_gather(ctx, B, nv, nv, vvvv, s4v, 1.0, w.tmp4, s4v, -1.0, s4s, 1.0, v4,
@@ -425,7 +418,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 1) + sp(m, 0) == sp(m, 2) + sp(m, 3) && sp(m, 3) == sp(m, 4);
-                 }, 0));
+                 }));
     // + t1[b,n] ooov[m,n,j,e]    (M=b, K=n, N=(m,e,j)); spins b n m e j
     KV_TRY(sgemm(nv, no * nv * no, no, B, 1.0,
                  MA(t1, X1(nv, o), X1(no, 1), vo),
@@ -435,7 +428,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{1, 1, 1}, {2, 1, 1}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) == sp(m, 1) && sp(m, 2) + sp(m, 1) == sp(m, 4) + sp(m, 3);
-                 }, 0));
+                 }));
     // - oovv[m,n,e,f] (t2[f,b,j,n]/2 + t1[f,j] t1[b,n])  (M=(m,e), K=(n,f), N=(tau,b,j))
     KV_TRY(kv_make_wmbej_tmp(ctx, B, nv, no, t1, t2, w.tmp4, sh));
     {
@@ -473,10 +466,12 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
             const std::vector<std::vector<Slot>> idx = {
                 {{0, 0, 1}, {2, 0, 1}}, {{0, 0, 2}, {2, 0, 2}}, {{0, 1, 1}, {1, 0, 1}},
                 {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 1}, {2, 1, 1}}, {{1, 1, 2}, {2, 1, 2}}};
+            // the seeded assembly reads Z's spin-conserving blocks only; the
+            // other one reads every element
             KV_TRY(spin_gemm(ctx, sh, B, 1.0, A, Bm, 0.0, C, idx, [](unsigned m) {
                 return sp(m, 0) + sp(m, 3) == sp(m, 1) + sp(m, 2) &&
                        sp(m, 2) + sp(m, 4) == sp(m, 3) + sp(m, 5);
-            }, (long long)B * v2o2));
+            }, seed_t2 == nullptr));
         } else {
             KV_TRY(kv_gemm(ctx, nv * no, nv * no, no * nv, B, 1.0, A, Bm, 0.0, C));
         }
@@ -492,7 +487,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 3) + sp(m, 2) && sp(m, 3) == sp(m, 4);
-                 }, -1));
+                 }, false));
     // Zabij += t1[a,m] Q[b,m,i,j]   (M=a, K=m, N=(b,i,j)); spins a m b i j
     KV_TRY(sgemm(nv, nv * no * no, no, B, 1.0,
                  MA(t1, X1(nv, o), X1(no, 1), vo),
@@ -502,7 +497,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{1, 1, 1}, {2, 1, 1}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) == sp(m, 1) && sp(m, 2) + sp(m, 1) == sp(m, 3) + sp(m, 4);
-                 }, 0));
+                 }));
 
     // ---- Z += Zab/2: t2 (F_be - 1/2 t1 F_me) and t1 vooo ----------------------
     KV_TRY(kv_bcast(ctx, 1, vv * B, w.Fae, w.Xbe));
@@ -518,7 +513,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 3) == sp(m, 1) + sp(m, 2) && sp(m, 4) == sp(m, 3);
-                 }, 0));
+                 }));
     // Zab += t1[a,m] vooo[b,m,i,j]   (M=a, K=m, N=(b,i,j)); spins a m b i j
     KV_TRY(sgemm(nv, nv * no * no, no, B, 0.5,
                  MA(t1, X1(nv, o), X1(no, 1), vo),
@@ -528,7 +523,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{1, 1, 1}, {2, 1, 1}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) == sp(m, 1) && sp(m, 2) + sp(m, 1) == sp(m, 3) + sp(m, 4);
-                 }, 0));
+                 }));
 
     // ---- Z += Zij/2: -t2 (F_mj + 1/2 t1 F_me) and vvvo t1 -----------------------
     KV_TRY(kv_bcast(ctx, 1, oo * B, w.Fmi, w.Xmj));
@@ -544,7 +539,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 2) + sp(m, 3) && sp(m, 3) == sp(m, 4);
-                 }, 0));
+                 }));
     // Zij += vvvo[a,b,e,j] t1[e,i]   (M=(a,b,j), K=e, N=i); spins a b j e i
     KV_TRY(sgemm(nv * nv * no, no, nv, B, 0.5,
                  MAI(vvvo, X3(nv, vv * o, nv, vo, no, 1), X1(nv, o)),
@@ -554,7 +549,7 @@ int kv_stanton(kvft_ctx *ctx, int nb, int nv, int no, const double *const F[4],
                        {{0, 1, 2}, {1, 0, 2}}, {{1, 1, 2}, {2, 1, 2}}},
                  [](unsigned m) {
                      return sp(m, 0) + sp(m, 1) == sp(m, 3) + sp(m, 2) && sp(m, 3) == sp(m, 4);
-                 }, 0));
+                 }));
 
     // ---- T2 += fac (1 - P(ab))(1 - P(ij)) (Z + ladders) -------------------------
     return kv_assemble_t2(ctx, B, nv, no, fac, w.Z, ladders ? w.Lc : nullptr, T2, seed_t2, sh);

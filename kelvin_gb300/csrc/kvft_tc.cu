@@ -75,7 +75,7 @@ inline FastDiv fastdiv(int d) {
 struct TcParams {
     int M, N;             // output extent
     int mt, nt;           // output tiles along M and N
-    int units;            // work units: mt * nt * batch * nsplit
+    int units;            // work units: C blocks * mt * nt * batch * nsplit
     int nsplit;           // >1: each K chunk is its own unit, added into C by FP64 atomics
     int chunk_kb;         // k-blocks per K chunk (exactness bound)
     int nkb_total;        // k-blocks of the padded K extent
@@ -84,32 +84,46 @@ struct TcParams {
     int a_batch_rows, b_batch_rows;   // row offset between batch entries (0: shared)
     const int *ea, *eb;   // row exponents of A / column exponents of B
     int ea_bst, eb_bst;
+    int batch;
+    // the group's products by block of C: block c starts at coff[c] and its
+    // sources are q = beg[c] .. beg[c + 1] - 1, each with the first plane row
+    // (arow, brow) and first exponent (aex, bex) of its operand sub-blocks
+    int beg[KV_MAXPROD + 1];
+    long long coff[KV_MAXPROD];
+    int arow[KV_MAXPROD], brow[KV_MAXPROD], aex[KV_MAXPROD], bex[KV_MAXPROD];
     double alpha, beta;
     int alpha_pow2;       // alpha = +-2^alpha_exp: folded into the exponent field
     int alpha_exp;
     unsigned alpha_sign;  // sign bit of alpha (bit 31 of the FP64 high word)
     KOut C;
     int *err;
-    FastDiv dv_split, dv_perb, dv_gsz;    // nsplit, mt nt, GROUP_M nt
+    FastDiv dv_split, dv_perb, dv_gsz, dv_batch;   // nsplit, mt nt, GROUP_M nt, batch
     FastDiv dv_cr2, dv_cr1;               // C's row index: sizes of its fast components
 };
 
-// A work unit: one output tile of one batch entry over a k-block range.
+// A work unit: one output tile of one batch entry of one block of C over a
+// k-block range, for every source of that block.  The sources run one after
+// the other through the pipeline, each with its own accumulation and its own
+// write to C (the first stores or scales, the others add): the same threads
+// write the same elements, so the order is the program's.
 struct Unit {
-    int b, m0, n0, kb0, kb1;
+    int b, cb, m0, n0, kb0, kb1;
 };
 
 // Units are numbered split-fastest, then in raster groups of GROUP_M m-tiles
-// (n-tiles walk inside a group), then by batch entry, so the CTAs that run
-// at the same time share a few A row panels and sweep B once per group.
+// (n-tiles walk inside a group), then by batch entry, then by block of C, so
+// the CTAs that run at the same time share a few A row panels and sweep B
+// once per group.
 __device__ __forceinline__ Unit unit_of(const TcParams &p, int u, int tn) {
     static_assert(GROUP_M == 8, "raster groups of 8 m-tiles (shift and mask below)");
     Unit w;
     const int t = p.dv_split.div(u);
     const int split = u - t * p.nsplit;
     const int per_b = p.mt * p.nt;
-    w.b = p.dv_perb.div(t);
-    const int r = t - w.b * per_b;
+    const int bc = p.dv_perb.div(t);
+    const int r = t - bc * per_b;
+    w.cb = p.dv_batch.div(bc);
+    w.b = bc - w.cb * p.batch;
     const int gsz = GROUP_M * p.nt;
     const int g = p.dv_gsz.div(r);
     const int first = g * GROUP_M;
@@ -399,27 +413,30 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bool ok = true;
             for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
                 const Unit w = unit_of(p, u, TN);
-                const int ya = w.b * p.a_batch_rows + w.m0, yb = w.b * p.b_batch_rows + w.n0;
-                for (int kb = w.kb0; kb < w.kb1; kb++) {
-                    if (!mbar_wait(smem_u32(&empty[st]), ph ^ 1) || *s_fail) {
-                        atomicExch(p.err, 1);
-                        *s_fail = 1;
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t fb = smem_u32(&full[st]);
-                    mbar_expect_tx(fb, bytes);
-                    const int x = kb * KBT;
-                    for (int s = 0; s < S; s++) {
-                        tma_load_2d(smem_u32(sA + st * stage_a + s * PLANE_BYTES), &tmA, x,
-                                    ya + s * p.Mp, fb);
-                        tma_load_2d(smem_u32(sB + st * stage_b + s * BPLANE), &tmB, x,
-                                    yb + s * p.Np, fb);
-                    }
-                    issued++;
-                    if (++st == NS) {
-                        st = 0;
-                        ph ^= 1;
+                for (int q = p.beg[w.cb]; q < p.beg[w.cb + 1] && ok; q++) {
+                    const int ya = p.arow[q] + w.b * p.a_batch_rows + w.m0;
+                    const int yb = p.brow[q] + w.b * p.b_batch_rows + w.n0;
+                    for (int kb = w.kb0; kb < w.kb1; kb++) {
+                        if (!mbar_wait(smem_u32(&empty[st]), ph ^ 1) || *s_fail) {
+                            atomicExch(p.err, 1);
+                            *s_fail = 1;
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t fb = smem_u32(&full[st]);
+                        mbar_expect_tx(fb, bytes);
+                        const int x = kb * KBT;
+                        for (int s = 0; s < S; s++) {
+                            tma_load_2d(smem_u32(sA + st * stage_a + s * PLANE_BYTES), &tmA, x,
+                                        ya + s * p.Mp, fb);
+                            tma_load_2d(smem_u32(sB + st * stage_b + s * BPLANE), &tmB, x,
+                                        yb + s * p.Np, fb);
+                        }
+                        issued++;
+                        if (++st == NS) {
+                            st = 0;
+                            ph ^= 1;
+                        }
                     }
                 }
             }
@@ -446,6 +463,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bool ok = true;
             for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
                 const Unit w = unit_of(p, u, TN);
+                const int nsrc = p.beg[w.cb + 1] - p.beg[w.cb];
+                for (int q = 0; q < nsrc && ok; q++)
                 for (int c0 = w.kb0; c0 < w.kb1 && ok; c0 += p.chunk_kb) {
                     const int c1 = min(c0 + p.chunk_kb, w.kb1);
                     const int set = gc % NSET;
@@ -516,196 +535,199 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         float rlo[FF ? WCOLS : 1];
         int gc = 0;
         bool ok = true;
-        int cached_n = -1, cached_b = -1;   // the columns coff / cexp hold (warp-uniform)
+        int cached_n = -1, cached_e = -1;   // the columns coff / cexp hold (warp-uniform)
         for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
             const Unit w = unit_of(p, u, TN);
             if (w.kb0 >= w.kb1) continue;
-            // C addresses of this unit; for the read-modify-write of a
-            // general beta the old values are prefetched into L2 now, while
-            // the MMAs run, so that it is not bound by the few loads a warp
-            // keeps in flight (the L2 reductions of beta = 1 fetch their lines
-            // at L2 themselves: prefetching them too cost 6 of 82 ms per
-            // 114-spin-orbital iteration in issue slots)
-            const int nw = w.n0 + h * WCOLS;          // first column of this warp
-            // column offsets and exponents: the same for every tile of this
-            // column range (and batch entry, when B is per batch)
-            const int bkey = p.eb_bst ? w.b : 0;
-            if (nw != cached_n || bkey != cached_b) {
-                __syncwarp();                            // the last tile's reads are done
-                for (int i = lane; i < WCOLS; i += 32) {
-                    const int n = nw + i;
-                    coff[i] = (n < p.N) ? p.C.c.off(n) : 0;
-                    cexp[i] = (n < p.N) ? exp_of(p.eb[(long long)bkey * p.eb_bst + n]) : 0;
-                }
-                cached_n = nw;
-                cached_b = bkey;
-            }
-            __syncwarp();
-            const int m = w.m0 + row;
-            const int nlim = p.N - nw;
-            long long roff = 0;
-            if (m < p.M) {                               // p.C.r.off(m), fast divisions
-                const int r1 = p.dv_cr2.div(m), i2 = m - r1 * p.C.r.size[2];
-                const int i0 = p.dv_cr1.div(r1), i1 = r1 - i0 * p.C.r.size[1];
-                roff = (long long)i0 * p.C.r.st[0] + (long long)i1 * p.C.r.st[1] +
-                       (long long)i2 * p.C.r.st[2];
-            }
-            double *Cr = p.C.p + (long long)w.b * p.C.bst + roff;
-            const int krow =
-                (m < p.M) ? exp_of(p.ea[(long long)w.b * p.ea_bst + m]) - 14 + p.alpha_exp : 0;
-            if (m < p.M && p.nsplit == 1 && p.beta != 0.0 && p.beta != 1.0) {
-                for (int i = 0; i < min(WCOLS, nlim); i++)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(Cr + coff[i]));
-            }
-            for (int c0 = w.kb0; c0 < w.kb1; c0 += p.chunk_kb) {
-                const int set = gc % NSET;
-                const bool got = mbar_wait(smem_u32(&accf[set]), (gc / NSET) & 1);
-                // one verdict per warp: tcgen05.ld below needs every lane
-                if (__any_sync(0xffffffffu, !got || *s_fail)) {
-                    if (lane == 0) {
-                        atomicExch(p.err, 6);
-                        *s_fail = 1;
+            const int q0 = p.beg[w.cb], q1 = p.beg[w.cb + 1];
+            for (int src = q0; src < q1 && ok; src++) {
+                const double beta = src == q0 ? p.beta : 1.0;
+                // C addresses of this unit; for the read-modify-write of a
+                // general beta the old values are prefetched into L2 now, while
+                // the MMAs run, so that it is not bound by the few loads a warp
+                // keeps in flight (the L2 reductions of beta = 1 fetch their lines
+                // at L2 themselves: prefetching them too cost 6 of 82 ms per
+                // 114-spin-orbital iteration in issue slots)
+                const int nw = w.n0 + h * WCOLS;          // first column of this warp
+                // column offsets and exponents: the same for every tile of this
+                // column range (and batch entry, when B is per batch)
+                const int ekey = p.bex[src] + w.b * p.eb_bst;
+                if (nw != cached_n || ekey != cached_e) {
+                    __syncwarp();                            // the last tile's reads are done
+                    for (int i = lane; i < WCOLS; i += 32) {
+                        const int n = nw + i;
+                        coff[i] = (n < p.N) ? p.C.c.off(n) : 0;
+                        cexp[i] = (n < p.N) ? exp_of(p.eb[ekey + n]) : 0;
                     }
-                    ok = false;
-                    break;
+                    cached_n = nw;
+                    cached_e = ekey;
                 }
-                fence_after();
-                const bool first = (c0 == w.kb0);
-                const uint32_t tb =
-                    tmem + ((uint32_t)(q * 32) << 16) + set * SET_COLS + h * WCOLS;
-#pragma unroll
-                for (int g = 0; g < NG; g++) {
-                    uint32_t r[MAXL][LW];
-#pragma unroll
-                    for (int l = 0; l < MAXL; l++)
-                        if (l < nl) tmem_ld<LW>(tb + l * TN + g * LW, r[l]);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int j = 0; j < LW; j++) {
-                        const int i = g * LW + j;
-                        float hi = __uint_as_float(r[0][j]);
-                        if constexpr (!FF) {
-                            if (nl > 1) hi += __uint_as_float(r[1][j]);
-                            rhi[i] = first ? hi : rhi[i] + hi;
-                        } else {
-                            // exact level sums, leading first: an FP32 pair
-                            float lo = 0.f, e;
-#pragma unroll
-                            for (int l = 1; l < MAXL; l++) {
-                                if (l < nl) {
-                                    two_sum(hi, __uint_as_float(r[l][j]), hi, e);
-                                    lo += e;
-                                }
-                            }
-                            if (first) {
-                                rhi[i] = hi;
-                                rlo[i] = lo;
+                __syncwarp();
+                const int m = w.m0 + row;
+                const int nlim = p.N - nw;
+                long long roff = 0;
+                if (m < p.M) {                               // p.C.r.off(m), fast divisions
+                    const int r1 = p.dv_cr2.div(m), i2 = m - r1 * p.C.r.size[2];
+                    const int i0 = p.dv_cr1.div(r1), i1 = r1 - i0 * p.C.r.size[1];
+                    roff = (long long)i0 * p.C.r.st[0] + (long long)i1 * p.C.r.st[1] +
+                           (long long)i2 * p.C.r.st[2];
+                }
+                double *Cr = p.C.p + (long long)w.b * p.C.bst + p.coff[w.cb] + roff;
+                const int krow =
+                    (m < p.M) ? exp_of(p.ea[p.aex[src] + w.b * p.ea_bst + m]) - 14 + p.alpha_exp : 0;
+                if (m < p.M && p.nsplit == 1 && beta != 0.0 && beta != 1.0) {
+                    for (int i = 0; i < min(WCOLS, nlim); i++)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(Cr + coff[i]));
+                }
+                for (int c0 = w.kb0; c0 < w.kb1; c0 += p.chunk_kb) {
+                    const int set = gc % NSET;
+                    const bool got = mbar_wait(smem_u32(&accf[set]), (gc / NSET) & 1);
+                    // one verdict per warp: tcgen05.ld below needs every lane
+                    if (__any_sync(0xffffffffu, !got || *s_fail)) {
+                        if (lane == 0) {
+                            atomicExch(p.err, 6);
+                            *s_fail = 1;
+                        }
+                        ok = false;
+                        break;
+                    }
+                    fence_after();
+                    const bool first = (c0 == w.kb0);
+                    const uint32_t tb =
+                        tmem + ((uint32_t)(q * 32) << 16) + set * SET_COLS + h * WCOLS;
+    #pragma unroll
+                    for (int g = 0; g < NG; g++) {
+                        uint32_t r[MAXL][LW];
+    #pragma unroll
+                        for (int l = 0; l < MAXL; l++)
+                            if (l < nl) tmem_ld<LW>(tb + l * TN + g * LW, r[l]);
+                        tmem_wait_ld();
+    #pragma unroll
+                        for (int j = 0; j < LW; j++) {
+                            const int i = g * LW + j;
+                            float hi = __uint_as_float(r[0][j]);
+                            if constexpr (!FF) {
+                                if (nl > 1) hi += __uint_as_float(r[1][j]);
+                                rhi[i] = first ? hi : rhi[i] + hi;
                             } else {
-                                float sm;
-                                two_sum(rhi[i], hi, sm, e);
-                                rlo[i] += lo + e;
-                                rhi[i] = sm;
+                                // exact level sums, leading first: an FP32 pair
+                                float lo = 0.f, e;
+    #pragma unroll
+                                for (int l = 1; l < MAXL; l++) {
+                                    if (l < nl) {
+                                        two_sum(hi, __uint_as_float(r[l][j]), hi, e);
+                                        lo += e;
+                                    }
+                                }
+                                if (first) {
+                                    rhi[i] = hi;
+                                    rlo[i] = lo;
+                                } else {
+                                    float sm;
+                                    two_sum(rhi[i], hi, sm, e);
+                                    rlo[i] += lo + e;
+                                    rhi[i] = sm;
+                                }
                             }
                         }
                     }
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&acce[set]));
+                    gc++;
                 }
-                fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&acce[set]));
-                gc++;
-            }
-            if (!ok) break;
-            // ---- the tile to C ----
-            if (m < p.M) {
-                // value of column i of this thread's row
-                auto value = [&](int i) -> double {
-                    const int k = krow + cexp[i];
-                    double v = f32_scaled(rhi[i], k, p.alpha_sign);
-                    if constexpr (FF) v += f32_scaled(rlo[i], k, p.alpha_sign);
-                    if (!p.alpha_pow2) v *= p.alpha;
-                    return v;
-                };
-                if (p.nsplit > 1 || p.beta == 1.0) {
-                    // C += value: each element gets exactly one addition in
-                    // this launch unless K chunks run as separate units, so a
-                    // fire-and-forget reduction at L2 gives old + value
-                    // rounded once, like a load-add-store, without the
-                    // thread waiting for the old value (measured on the
-                    // 114-spin-orbital n^5 class: 82 ms per iteration
-                    // against 120 ms for the load-add-store ring below)
-                    if constexpr (FF) {
-                        if (p.alpha_pow2) {
-                            // the FP32 pair as two reductions at L2: no FP64
-                            // add on the SM (GB300's FP64 pipe bounded this
-                            // write); C gets old + hi + lo in two roundings
-#pragma unroll
-                            for (int i = 0; i < WCOLS; i++) {
-                                if (i < nlim) {
-                                    const int k = krow + cexp[i];
-                                    atomicAdd(Cr + coff[i], f32_scaled(rhi[i], k, p.alpha_sign));
-                                    atomicAdd(Cr + coff[i], f32_scaled(rlo[i], k, p.alpha_sign));
+                if (!ok) break;
+                // ---- the tile to C ----
+                if (m < p.M) {
+                    // value of column i of this thread's row
+                    auto value = [&](int i) -> double {
+                        const int k = krow + cexp[i];
+                        double v = f32_scaled(rhi[i], k, p.alpha_sign);
+                        if constexpr (FF) v += f32_scaled(rlo[i], k, p.alpha_sign);
+                        if (!p.alpha_pow2) v *= p.alpha;
+                        return v;
+                    };
+                    if (p.nsplit > 1 || beta == 1.0) {
+                        // C += value: each element gets exactly one addition in
+                        // this launch unless K chunks run as separate units, so a
+                        // fire-and-forget reduction at L2 gives old + value
+                        // rounded once, like a load-add-store, without the
+                        // thread waiting for the old value (measured on the
+                        // 114-spin-orbital n^5 class: 82 ms per iteration
+                        // against 120 ms for the load-add-store ring below)
+                        if constexpr (FF) {
+                            if (p.alpha_pow2) {
+                                // the FP32 pair as two reductions at L2: no FP64
+                                // add on the SM (GB300's FP64 pipe bounded this
+                                // write); C gets old + hi + lo in two roundings
+    #pragma unroll
+                                for (int i = 0; i < WCOLS; i++) {
+                                    if (i < nlim) {
+                                        const int k = krow + cexp[i];
+                                        atomicAdd(Cr + coff[i], f32_scaled(rhi[i], k, p.alpha_sign));
+                                        atomicAdd(Cr + coff[i], f32_scaled(rlo[i], k, p.alpha_sign));
+                                    }
                                 }
+                            } else {
+    #pragma unroll
+                                for (int i = 0; i < WCOLS; i++)
+                                    if (i < nlim) atomicAdd(Cr + coff[i], value(i));
                             }
                         } else {
-#pragma unroll
+    #pragma unroll
                             for (int i = 0; i < WCOLS; i++)
                                 if (i < nlim) atomicAdd(Cr + coff[i], value(i));
                         }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < WCOLS; i++)
-                            if (i < nlim) atomicAdd(Cr + coff[i], value(i));
-                    }
-                } else if (p.beta == 0.0) {
-                    if (FF && p.alpha_pow2) {
-                        // hi stored, lo added at L2: hi + lo rounded once,
-                        // as the FP64 add gave, without it on the SM
-#pragma unroll
-                        for (int i = 0; i < WCOLS; i++) {
-                            if (i < nlim) {
-                                const int k = krow + cexp[i];
-                                Cr[coff[i]] = f32_scaled(rhi[i], k, p.alpha_sign);
-                                if constexpr (FF)
-                                    atomicAdd(Cr + coff[i], f32_scaled(rlo[i], k, p.alpha_sign));
+                    } else if (beta == 0.0) {
+                        if (FF && p.alpha_pow2) {
+                            // hi stored, lo added at L2: hi + lo rounded once,
+                            // as the FP64 add gave, without it on the SM
+    #pragma unroll
+                            for (int i = 0; i < WCOLS; i++) {
+                                if (i < nlim) {
+                                    const int k = krow + cexp[i];
+                                    Cr[coff[i]] = f32_scaled(rhi[i], k, p.alpha_sign);
+                                    if constexpr (FF)
+                                        atomicAdd(Cr + coff[i], f32_scaled(rlo[i], k, p.alpha_sign));
+                                }
                             }
+                        } else {
+    #pragma unroll
+                            for (int i = 0; i < WCOLS; i++)
+                                if (i < nlim) Cr[coff[i]] = value(i);
                         }
                     } else {
-#pragma unroll
-                        for (int i = 0; i < WCOLS; i++)
-                            if (i < nlim) Cr[coff[i]] = value(i);
-                    }
-                } else {
-                    // read-modify-write: the old values of the next RING
-                    // groups of WG columns are in flight while one group is
-                    // combined and stored
-                    constexpr int NGW = WCOLS / WG, RING = FF ? 3 : 2;
-                    double old[RING][WG];
-#pragma unroll
-                    for (int q = 0; q < RING; q++)
-#pragma unroll
-                        for (int j = 0; j < WG; j++)
-                            old[q][j] = (q < NGW && q * WG + j < nlim) ? Cr[coff[q * WG + j]] : 0.0;
-#pragma unroll
-                    for (int g = 0; g < NGW; g++) {
-                        const int q = g % RING;
-#pragma unroll
-                        for (int j = 0; j < WG; j++) {
-                            const int i = g * WG + j;
-                            const double v = (p.beta == 1.0) ? old[q][j] + value(i)
-                                                             : fma(p.beta, old[q][j], value(i));
-                            if (i < nlim) Cr[coff[i]] = v;
-                        }
-                        if (g + RING < NGW) {
-#pragma unroll
+                        // read-modify-write: the old values of the next RING
+                        // groups of WG columns are in flight while one group is
+                        // combined and stored
+                        constexpr int NGW = WCOLS / WG, RING = FF ? 3 : 2;
+                        double old[RING][WG];
+    #pragma unroll
+                        for (int q = 0; q < RING; q++)
+    #pragma unroll
+                            for (int j = 0; j < WG; j++)
+                                old[q][j] = (q < NGW && q * WG + j < nlim) ? Cr[coff[q * WG + j]] : 0.0;
+    #pragma unroll
+                        for (int g = 0; g < NGW; g++) {
+                            const int q = g % RING;
+    #pragma unroll
                             for (int j = 0; j < WG; j++) {
-                                const int i = (g + RING) * WG + j;
-                                old[q][j] = (i < nlim) ? Cr[coff[i]] : 0.0;
+                                const int i = g * WG + j;
+                                const double v = fma(beta, old[q][j], value(i));
+                                if (i < nlim) Cr[coff[i]] = v;
+                            }
+                            if (g + RING < NGW) {
+    #pragma unroll
+                                for (int j = 0; j < WG; j++) {
+                                    const int i = (g + RING) * WG + j;
+                                    old[q][j] = (i < nlim) ? Cr[coff[i]] : 0.0;
+                                }
                             }
                         }
                     }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
     }
     fence_before();
@@ -728,6 +750,14 @@ struct PackView {
     KIdx r, c;
     long long bst;
     int stable;         // contents fixed while the pack cache is on
+    int nb;             // batch entries of one sub-block
+    int nsub;           // sub-blocks of the view (the group's distinct operands) and
+    long long sub[KV_MAXPROD];   // where they start
+    // batch entry b of the packed form: sub-block b / nb, its entry b % nb
+    __device__ __forceinline__ const double *base(int b) const {
+        const int q = b / nb;
+        return p + sub[q] + (long long)(b - q * nb) * bst;
+    }
 };
 
 // Operand tiles of 32 rows x 64 k go through shared memory so that global
@@ -791,12 +821,12 @@ __device__ __forceinline__ int raw_exp(unsigned long long bits) {
 // are taken in registers from each thread's 8 values, and the next tile's
 // loads are issued before the current tile's values are used.
 __global__ void __launch_bounds__(256)
-pack_exp_kernel(PackView v, int R, int K, int rows_fast, int ktiles, int *__restrict__ ex) {
+pack_exp_kernel(const __grid_constant__ PackView v, int R, int K, int rows_fast, int ktiles, int *__restrict__ ex) {
     __shared__ long long off[PT_R + PT_K];
     __shared__ int rmax[8][PT_R];
     const int b = blockIdx.z, r0 = blockIdx.y * PT_R;
     const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    const double *base = v.p + (long long)b * v.bst;
+    const double *base = v.base(b);
     const int kt0 = blockIdx.x * ktiles;
     const int nkt = min(ktiles, (K + PT_K - 1) / PT_K - kt0);
     // rows_fast: one row per thread (lane); otherwise four rows (w + 8 i)
@@ -934,7 +964,7 @@ __device__ __forceinline__ void store_digits(__nv_bfloat16 *ob, size_t plane,
 // flight in registers while the current one is converted.
 template <int S>
 __global__ void __launch_bounds__(256)
-pack_digits_kernel(PackView v, int R, int K, int ld, int rows_fast, int ktn, int rtn,
+pack_digits_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int ktn, int rtn,
                    int ntiles, const int *__restrict__ ex, __nv_bfloat16 *__restrict__ out) {
     __shared__ unsigned long long val[PT_R][PT_K + 1];
     __shared__ long long off[PT_R + PT_K];
@@ -953,7 +983,7 @@ pack_digits_kernel(PackView v, int R, int K, int ld, int rows_fast, int ktn, int
         decode(t, b, r0, k0);
         tile_offsets(v, r0, k0, R, K, off);
         __syncthreads();
-        tile_fetch(v.p + (long long)b * v.bst, off, rows_fast, pre);
+        tile_fetch(v.base(b), off, rows_fast, pre);
     }
     for (; t < ntiles; t += gridDim.x) {
         const long long tn = (long long)t + gridDim.x;
@@ -976,7 +1006,7 @@ pack_digits_kernel(PackView v, int R, int K, int ld, int rows_fast, int ktn, int
             tile_offsets(v, rn, kn, R, K, off);
         }
         __syncthreads();
-        if (tn < ntiles) tile_fetch(v.p + (long long)bn * v.bst, off, rows_fast, pre);
+        if (tn < ntiles) tile_fetch(v.base(bn), off, rows_fast, pre);
         const int k = k0 + 2 * lane;
         if (k < K) {
             for (int rr = w; rr < PT_R; rr += 8) {
@@ -1007,7 +1037,7 @@ __host__ __device__ constexpr size_t pack_rows_smem(int kt) {
 
 template <int S, int KT>
 __global__ void __launch_bounds__(256, 2)
-pack_rows_kernel(PackView v, int R, int K, int ld, int rows_fast, int rtiles, int ntiles,
+pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int rtiles, int ntiles,
                  int *__restrict__ ex, __nv_bfloat16 *__restrict__ out) {
     constexpr int NK = KT * PT_K, LDV = NK + 1, PER = NK / 8;   // values per thread
     extern __shared__ unsigned long long prs[];
@@ -1022,7 +1052,7 @@ pack_rows_kernel(PackView v, int R, int K, int ld, int rows_fast, int rtiles, in
     unsigned long long pre[PER];
     auto fetch = [&](int t) {
         const int b = t / rtiles, r0 = (t - b * rtiles) * PT_R;
-        const double *base = v.p + (long long)b * v.bst;
+        const double *base = v.base(b);
         if (rows_fast) {
             const long long ro = (r0 + lane < R) ? v.r.off(r0 + lane) : -1;
 #pragma unroll
@@ -1151,12 +1181,14 @@ struct Packed {
 // and only reach output rows/columns that the epilogue discards.
 // Identity of a packed operand: address, view, extents and digit count.
 std::string pack_key(const PackView &v, int R, int K, int nb, int S) {
-    char b[320];
+    char b[400];
     snprintf(b, sizeof b, "%p|%d,%d,%d:%lld,%lld,%lld|%d,%d,%d:%lld,%lld,%lld|%lld|%d,%d,%d,%d",
              (const void *)v.p, v.r.size[0], v.r.size[1], v.r.size[2], v.r.st[0], v.r.st[1],
              v.r.st[2], v.c.size[0], v.c.size[1], v.c.size[2], v.c.st[0], v.c.st[1], v.c.st[2],
              v.bst, R, K, nb, S);
-    return b;
+    std::string key = b;
+    for (int q = 0; q < v.nsub; q++) key += "," + std::to_string(v.sub[q]);
+    return key;
 }
 
 // persistent digit pass: as many blocks as fit on the SMs at once
@@ -1250,20 +1282,6 @@ int pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb
             buf = nullptr;
         }
     }
-    if (!buf && !v.stable && ctx->tpack_on) {
-        // an operand sub-block already packed for an earlier product of the
-        // same spin-blocked contraction
-        ckey = pack_key(v, R, K, nb, S);
-        auto it = ctx->tpack.find(ckey);
-        const int slot = (it != ctx->tpack.end()) ? it->second : (int)ctx->tpack.size();
-        char sk[32];
-        snprintf(sk, sizeof sk, "tpack%d", slot);
-        KV_TRY(kv_scratch(ctx, sk, bytes, &buf));
-        out->planes = (__nv_bfloat16 *)buf;
-        out->ex = (int *)((uint8_t *)buf + pbytes);
-        if (it != ctx->tpack.end()) return KVFT_OK;
-        ctx->tpack[ckey] = slot;
-    }
     if (!buf) KV_TRY(kv_scratch(ctx, key, bytes, &buf));
     out->planes = (__nv_bfloat16 *)buf;
     out->ex = (int *)((uint8_t *)buf + pbytes);
@@ -1331,8 +1349,20 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
     return kv_launch_check(ctx, "tc_gemm");
 }
 
+// The distinct operand sub-blocks of a group: sub[q] of them at offsets
+// v.sub, which[q] the one product q uses.
+PackView group_view(const double *p, const KIdx &r, const KIdx &c, long long bst, int stable,
+                    int nb, int n, const long long *off, int *which) {
+    PackView v{p, r, c, bst, stable, nb, 0, {}};
+    for (int q = 0; q < n; q++) {
+        which[q] = (int)(std::find(v.sub, v.sub + v.nsub, off[q]) - v.sub);
+        if (which[q] == v.nsub) v.sub[v.nsub++] = off[q];
+    }
+    return v;
+}
+
 int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
-                const KMat &B, double beta, const KOut &C, int D) {
+                const KMat &B, double beta, const KOut &C, int D, const KvProds &g) {
     const int S = std::min(D - 1, MAXS);
     // D >= 4: three to six levels, FP32 pairs, TN = 64, and 32-deep k-blocks
     // (six digit planes per stage); D <= 3: 64-deep k-blocks, so that every
@@ -1342,26 +1372,44 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const int tn = (ff || N <= 64) ? 64 : 128;
     const int kb = ff ? 32 : 64;
     const int nbA = A.bst ? batch : 1, nbB = B.bst ? batch : 1;
-    Packed pa, pb;
-    KV_TRY(pack(ctx, "tc_pack_a", PackView{A.p, A.r, A.c, A.bst, A.stable}, M, K, nbA, S, &pa));
+    int wa[KV_MAXPROD], wb[KV_MAXPROD];
     // B is K x N; its K-major form has rows = N (B's column index), cols = K
-    KV_TRY(pack(ctx, "tc_pack_b", PackView{B.p, B.c, B.r, B.bst, B.stable}, N, K, nbB, S, &pb));
+    const PackView va = group_view(A.p, A.r, A.c, A.bst, A.stable, nbA, g.n, g.oa, wa);
+    const PackView vb = group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
+    Packed pa, pb;
+    KV_TRY(pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, S, &pa));
+    KV_TRY(pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, S, &pb));
+    const long long rows_a = (long long)va.nsub * nbA * S * M, rows_b = (long long)vb.nsub * nbB * S * N;
+    if (rows_a > 0x7FFFFFFFLL || rows_b > 0x7FFFFFFFLL)
+        return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: operand too large");
     CUtensorMap ma, mb;
-    KV_TRY(make_map(ctx, &ma, pa.planes, pa.K, pa.ld, (long long)nbA * S * pa.R, kb, TM));
-    KV_TRY(make_map(ctx, &mb, pb.planes, pb.K, pb.ld, (long long)nbB * S * pb.R, kb, tn));
+    KV_TRY(make_map(ctx, &ma, pa.planes, pa.K, pa.ld, rows_a, kb, TM));
+    KV_TRY(make_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
     const int mt = (M + TM - 1) / TM, nt = (N + tn - 1) / tn;
     const int nkb_total = (K + kb - 1) / kb;
     const int nchunks = (nkb_total + KCHUNK / kb - 1) / (KCHUNK / kb);
     const int chunk_kb = (nkb_total + nchunks - 1) / nchunks;     // balanced chunks
     const long long tiles = (long long)mt * nt * batch;
     // fewer output tiles than two waves of SMs and several K chunks: every
-    // chunk becomes a unit of its own and adds into C with FP64 atomics
-    // (C pre-scaled by beta)
+    // chunk of every product becomes a unit of its own and adds into C with
+    // FP64 atomics (C pre-scaled by beta)
     const bool par = nchunks > 1 && tiles < 2LL * ctx->sm_count;
-    const long long units = tiles * (par ? nchunks : 1);
+    const KvGroupTab tab = kv_group_tab(g, par);
+    const long long units = tiles * (par ? nchunks : 1) * tab.ncb;
     if (units > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: too many tiles");
-    if (par && beta != 1.0) KV_TRY(kv_scale_view(ctx, M, N, batch, beta, C));
+    if (par && beta != 1.0) {
+        const KvGroupTab t = kv_group_tab(g, false);
+        KV_TRY(kv_scale_blocks(ctx, M, N, batch, beta, C, t.ncb, t.coff));
+    }
     TcParams p;
+    p.batch = batch;
+    for (int c = 0; c <= tab.ncb; c++) p.beg[c] = tab.beg[c];
+    for (int c = 0; c < tab.ncb; c++) p.coff[c] = tab.coff[c];
+    for (int q = 0; q < g.n; q++) {
+        const int x = wa[tab.prod[q]], y = wb[tab.prod[q]];
+        p.arow[q] = x * nbA * S * M, p.aex[q] = x * nbA * M;
+        p.brow[q] = y * nbB * S * N, p.bex[q] = y * nbB * N;
+    }
     p.M = M;
     p.N = N;
     p.mt = mt;
@@ -1395,6 +1443,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     p.dv_split = fastdiv(p.nsplit);
     p.dv_perb = fastdiv(p.mt * p.nt);
     p.dv_gsz = fastdiv(GROUP_M * p.nt);
+    p.dv_batch = fastdiv(batch);
     p.dv_cr2 = fastdiv(C.r.size[2]);
     p.dv_cr1 = fastdiv(C.r.size[1]);
     switch (D) {
@@ -1414,11 +1463,11 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
 }  // namespace
 
 int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
-               const KMat &B, double beta, const KOut &C, int digits) {
+               const KMat &B, double beta, const KOut &C, int digits, const KvProds &g) {
     const int D = digits;
     if (D < 2 || D > MAXS + 1) return kv_fail(ctx, KVFT_EINVAL, "tensor-core digits out of range");
     if (M <= 0 || N <= 0 || batch <= 0) return KVFT_OK;
-    if (K <= 0) return kv_gemm_f64(ctx, M, N, K, batch, alpha, A, B, beta, C);
+    if (K <= 0) return kv_gemm_f64(ctx, M, N, K, batch, alpha, A, B, beta, C, g);
     // C^T = B^T A^T costs nothing but the operand roles.  The epilogue's lanes
     // are the tile rows, so the stride-1 index of C goes to the rows (each
     // store then covers 32 consecutive doubles) unless that extent is short
@@ -1434,9 +1483,11 @@ int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, cons
         const KMat At{B.p, B.c, B.r, B.bst, B.stable};
         const KMat Bt{A.p, A.c, A.r, A.bst, A.stable};
         const KOut Ct{C.p, C.c, C.r, C.bst};
-        return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D);
+        KvProds t = g;
+        std::swap(t.oa, t.ob);
+        return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, t);
     }
-    return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D);
+    return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g);
 }
 
 // Device status word written by bounded waits (0 = fine).
@@ -1468,9 +1519,9 @@ extern "C" int kvft_gemm(kvft_ctx *ctx, int M, int N, int K, int batch, int prec
     kv_gemm_prof_set(ctx, M, N, K, batch, batch, batch, 0.0, precision != KVFT_PREC_FP64);
     int st;
     if (precision == KVFT_PREC_FP64)
-        st = kv_gemm_f64(ctx, M, N, K, batch, 1.0, a, b, 0.0, c);
+        st = kv_gemm_f64(ctx, M, N, K, batch, 1.0, a, b, 0.0, c, kv_one_prod());
     else
-        st = kv_gemm_tc(ctx, M, N, K, batch, 1.0, a, b, 0.0, c, digits);
+        st = kv_gemm_tc(ctx, M, N, K, batch, 1.0, a, b, 0.0, c, digits, kv_one_prod());
     if (st != KVFT_OK) return st;
     return kv_device_status(ctx);
 }

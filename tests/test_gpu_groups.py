@@ -1,0 +1,85 @@
+"""Products that share one launch (the spin blocks of a contraction), and the
+FP64 kernel's free tile extents."""
+import numpy
+import pytest
+
+from kelvin_gb300 import _lib, ft_cc_equations, systems
+from kelvin_gb300.cc_utils import DeviceSolver
+from kelvin_gb300.quadrature import ft_quad
+from oracle import ft_ccsd as oft
+from oracle import ft_utils
+
+pytestmark = pytest.mark.gpu
+
+
+# One output, single rows and columns, extents around the 64 and 128 tile
+# limits and around each thread's output counts, one k and k around the block
+# of 16, K split over blocks (few outputs, long K), odd batches.
+@pytest.mark.parametrize("M,N,K,batch", [
+    (1, 1, 1, 1), (1, 129, 3, 2), (129, 1, 17, 1), (13, 2197, 13, 3), (2197, 13, 13, 3),
+    (19, 19, 6859, 2), (8, 8, 512, 10), (64, 65, 16, 1), (65, 64, 15, 1), (127, 33, 33, 5),
+    (361, 361, 361, 1), (57, 4000, 57, 1), (2, 300, 1000, 1)])
+def test_gemm_fp64_tiles(ctx, M, N, K, batch):
+    rng = numpy.random.default_rng(M + 3 * N + 7 * K + batch)
+    A = rng.standard_normal((batch, M, K))
+    B = rng.standard_normal((batch, K, N))
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, (batch, M, N))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, N, K, batch, _lib.PREC_FP64, 7, dA.ptr, dB.ptr, dC.ptr),
+              "kvft_gemm")
+    # each of the two sums (numpy's and the kernel's) is within K units of
+    # roundoff of the exact one, relative to the sum of magnitudes
+    bound = 2.0 * (K + 2) * 2.0 ** -53 * (abs(A) @ abs(B))
+    assert (abs(dC.to_host() - A @ B) <= bound).all()
+
+
+# Odd alpha halves, so that every block's offset is odd: 3 (all products on
+# the FP64 pipe), 13 and 17 (both engines), against the oracle's full sums.
+@pytest.mark.parametrize("pw,prec,digits,tol", [
+    (3, _lib.PREC_FP64, 7, 1e-12), (3, _lib.PREC_FP64_TC, 7, 1e-12),
+    (13, _lib.PREC_FP64, 7, 1e-12), (17, _lib.PREC_FP64_TC, 7, 1e-10)])
+def test_grouped_update_vs_oracle(ctx, pw, prec, digits, tol):
+    s = systems.ueg_recipe(2, 2.0, pw, 0.5)
+    beta, ng = 1.0 / s.T, 4
+    en = s.g_energies_tot()
+    n = en.shape[0]
+    ti, g, G = ft_quad(ng, beta, "lin")
+    F, I = oft.ft_integrals(s.g_fock_tot(), s.g_aint_tot(), en, beta, s.mu)
+    D1, D2 = ft_utils.D1(en, en), ft_utils.D2(en, en)
+    rng = numpy.random.default_rng(pw)
+    sp = numpy.arange(n) >= n // 2
+    t1 = rng.standard_normal((ng, n, n)) * 0.05 * (sp[:, None] == sp)
+    t2 = rng.standard_normal((ng, n, n, n, n)) * 0.05
+    t2 = t2 - t2.transpose(0, 2, 1, 3, 4)
+    t2 = (t2 - t2.transpose(0, 1, 2, 4, 3)) * (
+        sp[:, None, None, None].astype(int) + sp[None, :, None, None]
+        == sp[None, None, :, None].astype(int) + sp)
+    r1, r2 = oft.ccsd_stanton(F, I, t1, t2, D1, D2, ti, ng, G)
+    ctx.set_precision(prec, digits)
+    try:
+        o1, o2 = ft_cc_equations.ccsd_stanton(F, I, t1, t2, D1, D2, ti, ng, G, ctx=ctx)
+    finally:
+        ctx.set_precision(_lib.PREC_FP64, 7)
+    assert abs(o1 - r1).max() <= tol * max(1.0, abs(r1).max())
+    assert abs(o2 - r2).max() <= tol * max(1.0, abs(r2).max())
+
+
+# The Lambda path's groups write beta = 0 outputs without a separate pass over
+# them; a device buffer that held NaN before must come out clean.
+def test_grouped_lambda_leaves_no_stale_blocks(ctx):
+    s = systems.ueg_recipe(2, 2.0, 7, 0.5)
+    beta = 1.0 / s.T
+    ti, g, G = ft_quad(4, beta, "lin")
+    sv = DeviceSolver.from_system(ctx, s.g_energies_tot(), s.g_fock_tot(), s.g_aint_tot(), beta,
+                                  s.mu, ti, g, G)
+    try:
+        sv.guess(1)
+        conv = {"max_iter": 2, "damp": 0.2, "tconv": 1e-14}
+        on = sv.lambda_solve(conv)
+        sv.spin_blocks(False)
+        off = sv.lambda_solve(conv)
+    finally:
+        sv.close()
+    for a, b in zip(on, off):
+        assert numpy.isfinite(a).all()
+        assert abs(a - b).max() <= 1e-12 * max(1.0, abs(b).max())
