@@ -32,10 +32,7 @@
 // TMA (64-byte swizzle, 32-element k-blocks, every digit plane of a k-block
 // per pipeline stage).  Every mbarrier wait is bounded by %globaltimer; on
 // expiry the kernel records an error word and unwinds.
-#include "kvft_internal.h"
-
-#include <cuda.h>
-#include <cuda_bf16.h>
+#include "kvft_tc.h"
 
 #include <cmath>
 #include <cstdio>
@@ -44,33 +41,11 @@
 
 namespace {
 
-constexpr int TM = 128;
-constexpr int MAXS = 6;
 constexpr int KCHUNK = 2048;                  // exactness bound of the level-3 sum
 constexpr int NEPI = 8;                       // epilogue warps: two per TMEM lane quadrant
 constexpr int NTHREADS = 64 + 32 * NEPI;      // + TMA producer warp + MMA warp
 constexpr int TMEM_COLS = 512;               // all of an SM's TMEM (one CTA per SM)
 constexpr int GROUP_M = 8;                    // m-tiles per raster group (L2 reuse)
-constexpr unsigned long long WAIT_NS = 2000000000ull;   // 2 s per wait
-
-// x / d for 0 <= x < 2^31 by a multiply and a shift (Granlund-Montgomery:
-// m = ceil(2^(31+l) / d) with 2^l >= d), in place of the ~20 instructions of
-// an integer division by a run-time divisor in the per-tile index arithmetic.
-struct FastDiv {
-    unsigned long long m;
-    int s;
-    __device__ __forceinline__ int div(int x) const {
-        return (int)(((unsigned long long)(unsigned)x * m) >> s);
-    }
-};
-inline FastDiv fastdiv(int d) {
-    int l = 0;
-    while ((1LL << l) < d) l++;
-    FastDiv f;
-    f.s = 31 + l;
-    f.m = ((1ULL << f.s) + (unsigned long long)d - 1) / (unsigned long long)d;
-    return f;
-}
 
 struct TcParams {
     int M, N;             // output extent
@@ -144,169 +119,6 @@ __device__ __forceinline__ Unit unit_of(const TcParams &p, int u, int tn) {
         w.kb1 = p.nkb_total;
     }
     return w;
-}
-
-// Knuth's error-free sum: s + e == a + b exactly (round-to-nearest FP32)
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
-}
-
-// FP64 value of x 2^k with sign flipped by `sgn` (0 or 0x80000000), built
-// from the FP32 bit pattern in 32-bit halves: high word = sign | exponent
-// E - 127 + 1023 + k | top 20 mantissa bits, low word = the other 3 mantissa
-// bits at the top (exact; FP32 subnormals, below 2^-126 of the accumulator,
-// give 0)
-__device__ __forceinline__ double f32_scaled(float x, int k, unsigned sgn) {
-    const uint32_t u = __float_as_uint(x);
-    const int E = (int)((u >> 23) & 0xFF);
-    const int e64 = E + (1023 - 127) + k;
-    if (E == 0 || e64 <= 0) return 0.0;
-    const uint32_t hi = ((u & 0x80000000u) ^ sgn) | ((uint32_t)e64 << 20) | ((u >> 3) & 0xFFFFFu);
-    return __hiloint2double((int)hi, (int)(u << 29));
-}
-
-// Raw row exponents are reduced with atomicMax into an array preset to
-// 0x80808080 (below any binary exponent); exp_of turns a raw maximum into the
-// packing exponent e_r = max + 2 (|x| 2^-e_r < 1/2), or 0 for an all-zero row.
-constexpr int EXP_RAW_FLOOR = -1100;
-__host__ __device__ __forceinline__ int exp_of(int raw) {
-    return raw < EXP_RAW_FLOOR ? 0 : raw + 2;
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ unsigned long long gtime() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// bounded wait: false after WAIT_NS of wall time
-__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity) {
-    if (mbar_try(a, parity)) return true;
-    const unsigned long long t0 = gtime();
-    while (true) {
-        if (mbar_try(a, parity)) return true;
-        if (gtime() - t0 > WAIT_NS) return false;
-    }
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
-                                            uint32_t mbar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
-        : "memory");
-}
-
-// UMMA shared-memory descriptor of a K-major operand tile whose rows are one
-// k-block of KBT BF16 values: KBT = 32 -> 64-byte swizzle (8-row groups 512 B
-// apart), KBT = 64 -> 128-byte swizzle (8-row groups 1024 B apart)
-template <int KBT>
-__device__ __forceinline__ uint64_t desc_of(uint32_t saddr) {
-    static_assert(KBT == 32 || KBT == 64, "k-block of 32 or 64");
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-    d |= (uint64_t)1 << 16;                         // leading byte offset (unused)
-    d |= (uint64_t)((8 * KBT * 2) >> 4) << 32;      // stride byte offset
-    d |= (uint64_t)1 << 46;                         // descriptor version
-    d |= (uint64_t)(KBT == 32 ? 4 : 2) << 61;       // SWIZZLE_64B / SWIZZLE_128B
-    return d;
-}
-
-// kind::f16 instruction descriptor: BF16 x BF16 -> FP32, K-major A and B,
-// M = 128, N = tn
-__host__ __device__ constexpr uint32_t idesc_of(int tn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) |
-           ((uint32_t)(TM >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
-                                     uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t a) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t mbar) {
-    asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
-        : "memory");
-}
-
-__device__ __forceinline__ void fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-#define TMEM_LD16(taddr, r)                                                                   \
-    asm volatile(                                                                             \
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13," \
-        "%14,%15}, [%16];"                                                                    \
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),              \
-          "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),           \
-          "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                                  \
-        : "r"(taddr))
-
-#define TMEM_LD8(taddr, r)                                                                    \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"     \
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),     \
-                   "=r"(r[6]), "=r"(r[7])                                                     \
-                 : "r"(taddr))
-
-#define TMEM_LD4(taddr, r)                                                                    \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"                 \
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])                             \
-                 : "r"(taddr))
-
-// 32 lanes x LW consecutive columns of TMEM
-template <int LW>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t *r) {
-    static_assert(LW == 16 || LW == 8 || LW == 4, "TMEM load width");
-    if constexpr (LW == 16) {
-        TMEM_LD16(taddr, r);
-    } else if constexpr (LW == 8) {
-        TMEM_LD8(taddr, r);
-    } else {
-        TMEM_LD4(taddr, r);
-    }
-}
-
-__device__ __forceinline__ void tmem_wait_ld() {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // Shared-memory bytes of the kernel: 1 KB alignment slack, NS pipeline stages
@@ -745,21 +557,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // Digit packing: FP64 strided view (rows x K) -> S BF16 planes [b][s][Rp][Kp]
 // and row exponents [b][Rp].
 // ---------------------------------------------------------------------------
-struct PackView {
-    const double *p;
-    KIdx r, c;
-    long long bst;
-    int stable;         // contents fixed while the pack cache is on
-    int nb;             // batch entries of one sub-block
-    int nsub;           // sub-blocks of the view (the group's distinct operands) and
-    long long sub[KV_MAXPROD];   // where they start
-    // batch entry b of the packed form: sub-block b / nb, its entry b % nb
-    __device__ __forceinline__ const double *base(int b) const {
-        const int q = b / nb;
-        return p + sub[q] + (long long)(b - q * nb) * bst;
-    }
-};
-
 // Operand tiles of 32 rows x 64 k go through shared memory so that global
 // reads are coalesced along whichever operand index is contiguous in memory
 // (the row index for some permuted views, k for others) and plane writes are
@@ -810,10 +607,6 @@ __device__ __forceinline__ void tile_fetch(const double *base, const long long *
                                  : 0ull;
         }
     }
-}
-
-__device__ __forceinline__ int raw_exp(unsigned long long bits) {
-    return (bits & 0x7FFFFFFFFFFFFFFFull) ? (int)((bits >> 52) & 0x7FF) - 1023 : -2000;
 }
 
 // raw row exponents: max binary exponent over each row of `ktiles`
@@ -1149,10 +942,10 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2D map over digit planes (K x rows, row stride ld elements); one box is a
-// k-block of kb values (swizzled by its 2 kb bytes) by box_rows rows
-int make_map(kvft_ctx *ctx, CUtensorMap *map, void *base, int K, int ld, long long rows, int kb,
-             int box_rows) {
+}  // namespace
+
+int kv_tc_map(kvft_ctx *ctx, CUtensorMap *map, void *base, int K, int ld, long long rows, int kb,
+              int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return kv_fail(ctx, KVFT_EDEVICE, "cuTensorMapEncodeTiled unavailable");
     cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
@@ -1167,11 +960,7 @@ int make_map(kvft_ctx *ctx, CUtensorMap *map, void *base, int K, int ld, long lo
     return KVFT_OK;
 }
 
-struct Packed {
-    __nv_bfloat16 *planes;
-    int *ex;
-    int R, ld, K, nb;
-};
+namespace {
 
 // Digit planes [nb][S][R][ld] and exponents [nb][R].  ld = K rounded up to 64
 // elements, so that every row starts on a 128-byte line and a TMA box row
@@ -1249,8 +1038,10 @@ int pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, in
     }
 }
 
-int pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int S,
-         Packed *out) {
+}  // namespace
+
+int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int S,
+               Packed *out) {
     const int ld = (K + 63) / 64 * 64;
     const size_t plane_bytes = (size_t)R * ld * 2;
     const size_t pbytes = ((size_t)nb * S * plane_bytes + 1023) / 1024 * 1024;
@@ -1315,6 +1106,26 @@ int pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb
     return KVFT_OK;
 }
 
+PackView kv_tc_group_view(const double *p, const KIdx &r, const KIdx &c, long long bst, int stable,
+                          int nb, int n, const long long *off, int *which) {
+    PackView v{p, r, c, bst, stable, nb, 0, {}};
+    for (int q = 0; q < n; q++) {
+        which[q] = (int)(std::find(v.sub, v.sub + v.nsub, off[q]) - v.sub);
+        if (which[q] == v.nsub) v.sub[v.nsub++] = off[q];
+    }
+    return v;
+}
+
+bool kv_tc_pow2(double alpha, int *exp, unsigned *sign) {
+    int ex = 0;
+    const bool yes = std::fabs(std::frexp(alpha, &ex)) == 0.5;
+    *exp = yes ? ex - 1 : 0;
+    *sign = yes && alpha < 0 ? 0x80000000u : 0u;
+    return yes;
+}
+
+namespace {
+
 // The stride-1 index of a view: its fastest dimension of extent > 1 has
 // element stride 1 (or the index has a single value).
 bool unit_stride(const KIdx &x) {
@@ -1349,18 +1160,6 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
     return kv_launch_check(ctx, "tc_gemm");
 }
 
-// The distinct operand sub-blocks of a group: sub[q] of them at offsets
-// v.sub, which[q] the one product q uses.
-PackView group_view(const double *p, const KIdx &r, const KIdx &c, long long bst, int stable,
-                    int nb, int n, const long long *off, int *which) {
-    PackView v{p, r, c, bst, stable, nb, 0, {}};
-    for (int q = 0; q < n; q++) {
-        which[q] = (int)(std::find(v.sub, v.sub + v.nsub, off[q]) - v.sub);
-        if (which[q] == v.nsub) v.sub[v.nsub++] = off[q];
-    }
-    return v;
-}
-
 int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
                 const KMat &B, double beta, const KOut &C, int D, const KvProds &g) {
     const int S = std::min(D - 1, MAXS);
@@ -1374,17 +1173,17 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const int nbA = A.bst ? batch : 1, nbB = B.bst ? batch : 1;
     int wa[KV_MAXPROD], wb[KV_MAXPROD];
     // B is K x N; its K-major form has rows = N (B's column index), cols = K
-    const PackView va = group_view(A.p, A.r, A.c, A.bst, A.stable, nbA, g.n, g.oa, wa);
-    const PackView vb = group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
+    const PackView va = kv_tc_group_view(A.p, A.r, A.c, A.bst, A.stable, nbA, g.n, g.oa, wa);
+    const PackView vb = kv_tc_group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
     Packed pa, pb;
-    KV_TRY(pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, S, &pa));
-    KV_TRY(pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, S, &pb));
+    KV_TRY(kv_tc_pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, S, &pa));
+    KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, S, &pb));
     const long long rows_a = (long long)va.nsub * nbA * S * M, rows_b = (long long)vb.nsub * nbB * S * N;
     if (rows_a > 0x7FFFFFFFLL || rows_b > 0x7FFFFFFFLL)
         return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: operand too large");
     CUtensorMap ma, mb;
-    KV_TRY(make_map(ctx, &ma, pa.planes, pa.K, pa.ld, rows_a, kb, TM));
-    KV_TRY(make_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
+    KV_TRY(kv_tc_map(ctx, &ma, pa.planes, pa.K, pa.ld, rows_a, kb, TM));
+    KV_TRY(kv_tc_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
     const int mt = (M + TM - 1) / TM, nt = (N + tn - 1) / tn;
     const int nkb_total = (K + kb - 1) / kb;
     const int nchunks = (nkb_total + KCHUNK / kb - 1) / (KCHUNK / kb);
@@ -1431,13 +1230,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     p.eb_bst = (nbB > 1) ? pb.R : 0;
     p.alpha = alpha;
     p.beta = par ? 1.0 : beta;
-    {
-        int ex2 = 0;
-        const double fr = std::frexp(alpha, &ex2);
-        p.alpha_pow2 = (std::fabs(fr) == 0.5) ? 1 : 0;
-        p.alpha_exp = p.alpha_pow2 ? ex2 - 1 : 0;
-        p.alpha_sign = (p.alpha_pow2 && alpha < 0) ? 0x80000000u : 0u;
-    }
+    p.alpha_pow2 = kv_tc_pow2(alpha, &p.alpha_exp, &p.alpha_sign);
     p.C = C;
     p.err = ctx->dflag;
     p.dv_split = fastdiv(p.nsplit);
@@ -1468,7 +1261,17 @@ int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, cons
     if (D < 2 || D > MAXS + 1) return kv_fail(ctx, KVFT_EINVAL, "tensor-core digits out of range");
     if (M <= 0 || N <= 0 || batch <= 0) return KVFT_OK;
     if (K <= 0) return kv_gemm_f64(ctx, M, N, K, batch, alpha, A, B, beta, C, g);
-    // C^T = B^T A^T costs nothing but the operand roles.  The epilogue's lanes
+    // C^T = B^T A^T, the same products
+    const KMat At{B.p, B.c, B.r, B.bst, B.stable};
+    const KMat Bt{A.p, A.c, A.r, A.bst, A.stable};
+    const KOut Ct{C.p, C.c, C.r, C.bst};
+    KvProds gt = g;
+    std::swap(gt.oa, gt.ob);
+    if (kv_thin_fits(M, N, K, batch, A, B, C))
+        return kv_gemm_thin(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g);
+    if (kv_thin_fits(N, M, K, batch, At, Bt, Ct))
+        return kv_gemm_thin(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt);
+    // The transpose costs nothing but the operand roles.  The epilogue's lanes
     // are the tile rows, so the stride-1 index of C goes to the rows (each
     // store then covers 32 consecutive doubles) unless that extent is short
     // and K long (the unused TMEM lanes would cost MMA time); otherwise the
@@ -1479,14 +1282,7 @@ int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, cons
         const int ext = cc ? N : M;
         if (ext >= 64 || K <= 512) swap = cc;
     }
-    if (swap) {
-        const KMat At{B.p, B.c, B.r, B.bst, B.stable};
-        const KMat Bt{A.p, A.c, A.r, A.bst, A.stable};
-        const KOut Ct{C.p, C.c, C.r, C.bst};
-        KvProds t = g;
-        std::swap(t.oa, t.ob);
-        return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, t);
-    }
+    if (swap) return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt);
     return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g);
 }
 

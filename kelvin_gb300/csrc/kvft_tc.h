@@ -1,0 +1,252 @@
+// Device helpers and host entry points shared by the tensor-core contraction
+// kernels (kvft_tc.cu: the general tiles; kvft_tc_thin.cu: a big tensor with a
+// small matrix).
+#pragma once
+
+#include "kvft_internal.h"
+
+#include <cuda.h>
+#include <cuda_bf16.h>
+
+namespace {
+
+constexpr int TM = 128;
+constexpr int MAXS = 6;
+constexpr unsigned long long WAIT_NS = 2000000000ull;   // 2 s per wait
+
+// x / d for 0 <= x < 2^31 by a multiply and a shift (Granlund-Montgomery:
+// m = ceil(2^(31+l) / d) with 2^l >= d), in place of the ~20 instructions of
+// an integer division by a run-time divisor in the per-tile index arithmetic.
+struct FastDiv {
+    unsigned long long m;
+    int s;
+    __device__ __forceinline__ int div(int x) const {
+        return (int)(((unsigned long long)(unsigned)x * m) >> s);
+    }
+};
+inline FastDiv fastdiv(int d) {
+    int l = 0;
+    while ((1LL << l) < d) l++;
+    FastDiv f;
+    f.s = 31 + l;
+    f.m = ((1ULL << f.s) + (unsigned long long)d - 1) / (unsigned long long)d;
+    return f;
+}
+
+// Knuth's error-free sum: s + e == a + b exactly (round-to-nearest FP32)
+__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
+    s = a + b;
+    const float bb = s - a;
+    e = (a - (s - bb)) + (b - bb);
+}
+
+// FP64 value of x 2^k with sign flipped by `sgn` (0 or 0x80000000), built
+// from the FP32 bit pattern in 32-bit halves: high word = sign | exponent
+// E - 127 + 1023 + k | top 20 mantissa bits, low word = the other 3 mantissa
+// bits at the top (exact; FP32 subnormals, below 2^-126 of the accumulator,
+// give 0)
+__device__ __forceinline__ double f32_scaled(float x, int k, unsigned sgn) {
+    const uint32_t u = __float_as_uint(x);
+    const int E = (int)((u >> 23) & 0xFF);
+    const int e64 = E + (1023 - 127) + k;
+    if (E == 0 || e64 <= 0) return 0.0;
+    const uint32_t hi = ((u & 0x80000000u) ^ sgn) | ((uint32_t)e64 << 20) | ((u >> 3) & 0xFFFFFu);
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// Raw row exponents are reduced with atomicMax into an array preset to
+// 0x80808080 (below any binary exponent); exp_of turns a raw maximum into the
+// packing exponent e_r = max + 2 (|x| 2^-e_r < 1/2), or 0 for an all-zero row.
+constexpr int EXP_RAW_FLOOR = -1100;
+__host__ __device__ __forceinline__ int exp_of(int raw) {
+    return raw < EXP_RAW_FLOOR ? 0 : raw + 2;
+}
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ unsigned long long gtime() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect_tx(uint32_t a, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(a), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// bounded wait: false after WAIT_NS of wall time
+__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity) {
+    if (mbar_try(a, parity)) return true;
+    const unsigned long long t0 = gtime();
+    while (true) {
+        if (mbar_try(a, parity)) return true;
+        if (gtime() - t0 > WAIT_NS) return false;
+    }
+}
+
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
+                                            uint32_t mbar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
+        : "memory");
+}
+
+// UMMA shared-memory descriptor of a K-major operand tile whose rows are one
+// k-block of KBT BF16 values: KBT = 32 -> 64-byte swizzle (8-row groups 512 B
+// apart), KBT = 64 -> 128-byte swizzle (8-row groups 1024 B apart)
+template <int KBT>
+__device__ __forceinline__ uint64_t desc_of(uint32_t saddr) {
+    static_assert(KBT == 32 || KBT == 64, "k-block of 32 or 64");
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;                         // leading byte offset (unused)
+    d |= (uint64_t)((8 * KBT * 2) >> 4) << 32;      // stride byte offset
+    d |= (uint64_t)1 << 46;                         // descriptor version
+    d |= (uint64_t)(KBT == 32 ? 4 : 2) << 61;       // SWIZZLE_64B / SWIZZLE_128B
+    return d;
+}
+
+// kind::f16 instruction descriptor: BF16 x BF16 -> FP32, K-major A and B,
+// M = 128, N = tn
+__host__ __device__ constexpr uint32_t idesc_of(int tn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) |
+           ((uint32_t)(TM >> 4) << 24);
+}
+
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
+                                     uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t a) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t mbar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+        : "memory");
+}
+
+__device__ __forceinline__ void fence_before() {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void fence_after() {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+#define TMEM_LD16(taddr, r)                                                                   \
+    asm volatile(                                                                             \
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13," \
+        "%14,%15}, [%16];"                                                                    \
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),              \
+          "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),           \
+          "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                                  \
+        : "r"(taddr))
+
+#define TMEM_LD8(taddr, r)                                                                    \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"     \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),     \
+                   "=r"(r[6]), "=r"(r[7])                                                     \
+                 : "r"(taddr))
+
+#define TMEM_LD4(taddr, r)                                                                    \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"                 \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])                             \
+                 : "r"(taddr))
+
+// 32 lanes x LW consecutive columns of TMEM
+template <int LW>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t *r) {
+    static_assert(LW == 16 || LW == 8 || LW == 4, "TMEM load width");
+    if constexpr (LW == 16) {
+        TMEM_LD16(taddr, r);
+    } else if constexpr (LW == 8) {
+        TMEM_LD8(taddr, r);
+    } else {
+        TMEM_LD4(taddr, r);
+    }
+}
+
+__device__ __forceinline__ void tmem_wait_ld() {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ int raw_exp(unsigned long long bits) {
+    return (bits & 0x7FFFFFFFFFFFFFFFull) ? (int)((bits >> 52) & 0x7FF) - 1023 : -2000;
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Digit packing (kvft_tc.cu): FP64 strided view (rows x K) -> S BF16 planes
+// [b][s][R][ld] and row exponents [b][R].
+// ---------------------------------------------------------------------------
+struct PackView {
+    const double *p;
+    KIdx r, c;
+    long long bst;
+    int stable;         // contents fixed while the pack cache is on
+    int nb;             // batch entries of one sub-block
+    int nsub;           // sub-blocks of the view (the group's distinct operands) and
+    long long sub[KV_MAXPROD];   // where they start
+    // batch entry b of the packed form: sub-block b / nb, its entry b % nb
+    __device__ __forceinline__ const double *base(int b) const {
+        const int q = b / nb;
+        return p + sub[q] + (long long)(b - q * nb) * bst;
+    }
+};
+
+struct Packed {
+    __nv_bfloat16 *planes;
+    int *ex;
+    int R, ld, K, nb;
+};
+
+
+// Packs v (R rows x K, nb packed batch entries, S planes) into the scratch
+// buffer `key`, or into the cache of stable operands.
+int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int S,
+               Packed *out);
+// 2D tensor map over digit planes (K x rows, row stride ld elements); one box
+// is a k-block of kb values (swizzled by its 2 kb bytes) by box_rows rows.
+int kv_tc_map(kvft_ctx *ctx, CUtensorMap *map, void *base, int K, int ld, long long rows, int kb,
+              int box_rows);
+// The view of a group's distinct operand sub-blocks; which[q]: the one product
+// q uses.
+PackView kv_tc_group_view(const double *p, const KIdx &r, const KIdx &c, long long bst, int stable,
+                          int nb, int n, const long long *off, int *which);
+// alpha = +-2^exp: exp and the sign bit of its high word; false otherwise
+// (exp = sign = 0).
+bool kv_tc_pow2(double alpha, int *exp, unsigned *sign);
+
+// The contraction of a big tensor with a small matrix (K and one free extent
+// at most 64, each a single tensor index): kvft_tc_thin.cu.  kv_thin_fits says
+// whether the shape is one it takes, with the big operand as A.
+bool kv_thin_fits(int M, int N, int K, int batch, const KMat &A, const KMat &B, const KOut &C);
+int kv_gemm_thin(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
+                 const KMat &B, double beta, const KOut &C, int D, const KvProds &g);

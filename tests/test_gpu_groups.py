@@ -83,3 +83,29 @@ def test_grouped_lambda_leaves_no_stale_blocks(ctx):
     for a, b in zip(on, off):
         assert numpy.isfinite(a).all()
         assert abs(a - b).max() <= 1e-12 * max(1.0, abs(b).max())
+
+
+# A big tensor with a small matrix (K, N <= 64): k and column edges of the 32-
+# and 64-deep tiles and of the 16-column MMA steps, one column, partial row
+# tiles, the big operand on either side (its rows or k contiguous), every
+# digit count.  Norm-wise bounds by digit count as for the general kernel.
+@pytest.mark.parametrize("M,N,K,batch", [(2049, 1, 16, 1), (700, 16, 17, 3), (1100, 33, 32, 2),
+                                         (1025, 64, 33, 2), (2100, 57, 57, 1), (900, 31, 64, 4)])
+@pytest.mark.parametrize("digits", [2, 3, 4, 5, 6, 7])
+@pytest.mark.parametrize("big_left", [True, False])
+def test_thin_contraction(ctx, M, N, K, batch, digits, big_left):
+    rng = numpy.random.default_rng(M + 3 * N + 7 * K + digits)
+    A = rng.standard_normal((batch, M, K)) * numpy.exp(rng.standard_normal((batch, M, 1)) * 3)
+    B = rng.standard_normal((batch, K, N)) * numpy.exp(rng.standard_normal((batch, 1, N)) * 3)
+    A[:, 5] = 0.0
+    if not big_left:
+        A, B = (numpy.ascontiguousarray(x.transpose(0, 2, 1)) for x in (B, A))
+    m, n = A.shape[1], B.shape[2]
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, (batch, m, n))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, m, n, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    C = dC.to_host()
+    tol = {2: 2e-3, 3: 5e-5, 4: 5e-7, 5: 5e-9, 6: 5e-11, 7: 5e-12}[digits]
+    bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
+    assert (abs(C - A @ B) <= tol * (256 / K) ** 0.5 * bound).all()
