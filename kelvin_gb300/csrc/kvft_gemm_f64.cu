@@ -11,20 +11,23 @@ namespace {
 
 // GB300 issues about 2 FP64 FMAs per clock per SM: a warp's FMA occupies the
 // pipe for 16 clocks, in which the SM can issue 64 other instructions and
-// serve 16 shared-memory wavefronts.  So FMAs spent on padding are the only
-// cost that counts, and operand reuse in registers buys nothing.  The tile
-// is BM x BN for any extents (chosen by the host to divide M and N, whatever
-// the orbital count), its outputs are laid out flat over the threads -- o =
-// t + 128 i, i < T, along C's contiguous index, so stores coalesce -- and
-// every FMA takes its two operands from shared memory (2 LDS against 16 pipe
-// clocks).  Blocks are small (128 threads, under 30 KB), so several per SM
-// overlap one's loads with another's FMAs.
+// serve 16 shared-memory wavefronts.  So FMAs spent on padding are what costs,
+// and operand reuse in registers buys little.  Two layouts:
+//   rows   a big tensor times a small matrix (N columns at a time, N <= 24): a
+//          thread owns one row and all N columns, its A value comes from shared
+//          memory once per k and B's by broadcast; no FMA is padding but those
+//          of the last, partial row block.
+//   flat   everything else: a BM x BN tile of any extents (chosen by the host
+//          to divide M and N), its outputs flat over the threads -- o = t + 128
+//          i, i < T, along C's contiguous index -- and both operands of every
+//          FMA from shared memory (2 LDS against 16 pipe clocks).
+// Blocks are small, so several per SM overlap one's loads with another's FMAs.
 // Measured, the whole update of 19 plane waves (38 spin orbitals, ng = 10,
 // 26.4 GFLOP; 21 ms at the FP64 peak): 64.7 ms with 64 x 64 tiles (19-wide
-// outputs padded to 64) and one launch per product, 29.1 ms with these tiles
+// outputs padded to 64) and one launch per product, 29.1 ms with flat tiles
 // and one launch per group; an 8-site ring's iteration (8-wide outputs)
 // 4.5 -> 0.6 ms.
-constexpr int NT = 128, BK = 16, TMAX = 16, BDIM_MAX = 128;
+constexpr int NT = 128, TMAX = 16, BDIM_MAX = 128;
 
 struct F64Params {
     int M, N, K;
@@ -32,21 +35,50 @@ struct F64Params {
     int batch, nsplit, klen;     // K range of one block: klen (a multiple of BK)
     int a_kfast, b_kfast;        // K contiguous in A / B
     int cm_fast;                 // outputs of a tile flat along m (else along n)
-    int atomic;                  // add into C by atomics (K split over blocks)
+    int store;                   // 0 add by atomics (K split), 1 store, 2 add, 3 general beta
+    int unit;                    // alpha = 1 (1) or -1 (2): no multiplication by it
+    int c_trans;                 // rows layout: C contiguous along its columns
     double alpha, beta;
     const double *A, *B;
     KIdx Ar, Ac, Br, Bc;
+    KIdxDiv dar, dac, dbr, dbc, dcr, dcc;
+    FastDiv dnt, dmt, dks, dbatch, dflat;
     long long a_bst, b_bst;
     KOut C;
     int beg[KV_MAXPROD + 1];     // sources of each block of C
     long long oa[KV_MAXPROD], ob[KV_MAXPROD], oc[KV_MAXPROD];
 };
 
-__host__ __device__ constexpr size_t f64_smem(int BM, int BN) {
+// block -> (C block, batch, K split, tile), tiles along n fastest
+struct F64Tile {
+    int tn, tm, ks, b, cb;
+    __device__ __forceinline__ F64Tile(const F64Params &p, int u) {
+        int q = p.dnt.div(u);
+        tn = u - q * p.nt;
+        u = q, q = p.dmt.div(u);
+        tm = u - q * p.mt;
+        u = q, q = p.dks.div(u);
+        ks = u - q * p.nsplit;
+        cb = p.dbatch.div(q);
+        b = q - cb * p.batch;
+    }
+};
+
+__device__ __forceinline__ void f64_out(const F64Params &p, double *dst, double acc) {
+    const double v = p.unit ? (p.unit == 2 ? -acc : acc) : p.alpha * acc;
+    if (p.store == 1) *dst = v;
+    else if (p.store == 2) *dst += v;
+    else if (p.store == 0) atomicAdd(dst, v);
+    else *dst = fma(p.beta, *dst, v);
+}
+
+__host__ __device__ constexpr size_t f64_smem(int BM, int BN, int BK) {
     return 8 * (size_t)(BK * ((BM | 1) + (BN | 1)) + 2 * (BM + BN) + 2 * BK);
 }
 
-template <int T>
+// BK: k values per shared-memory block; 32 where few outputs per thread make
+// the loads' latency the chain
+template <int T, int BK>
 __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F64Params p) {
     extern __shared__ double sm[];
     const int lda = p.BM | 1, ldb = p.BN | 1;
@@ -56,48 +88,42 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F6
     long long *bc = ar + p.BM, *cr = bc + p.BN, *cc = cr + p.BM;
     long long *ak = cc + p.BN, *bk = ak + BK;          // K offsets of the current k block
     const int tid = threadIdx.x;
-    // block -> (C block, batch, K split, tile), tiles along n fastest
-    int u = blockIdx.x;
-    const int tn = u % p.nt;
-    u /= p.nt;
-    const int tm = u % p.mt;
-    u /= p.mt;
-    const int ks = u % p.nsplit;
-    u /= p.nsplit;
-    const int b = u % p.batch, cb = u / p.batch;
-    const int m0 = tm * p.BM, n0 = tn * p.BN;
+    const F64Tile t(p, blockIdx.x);
+    const int m0 = t.tm * p.BM, n0 = t.tn * p.BN;
     const int bm = min(p.BM, p.M - m0), bn = min(p.BN, p.N - n0);
-    const int kbeg = ks * p.klen, kend = min(p.K, kbeg + p.klen);
+    const int kbeg = t.ks * p.klen, kend = min(p.K, kbeg + p.klen);
     for (int x = tid; x < bm; x += NT) {
-        ar[x] = p.Ar.off(m0 + x);
-        cr[x] = p.C.r.off(m0 + x);
+        ar[x] = p.dar.off(p.Ar, m0 + x);
+        cr[x] = p.dcr.off(p.C.r, m0 + x);
     }
     for (int x = tid; x < bn; x += NT) {
-        bc[x] = p.Bc.off(n0 + x);
-        cc[x] = p.C.c.off(n0 + x);
+        bc[x] = p.dbc.off(p.Bc, n0 + x);
+        cc[x] = p.dcc.off(p.C.c, n0 + x);
     }
-    // this thread's outputs; one past the tile repeats the last output and is
-    // not stored, and costs FMAs only in a warp that has others
-    const int cnt = bm * bn, wbase = tid & ~31;
-    short im[T], in[T];
+    // this thread's outputs as shared-memory offsets m | n << 16; one past the
+    // tile (not in `ok`) repeats element 0 and is not stored
+    const int cnt = p.BM * p.BN, wbase = tid & ~31;
+    int mn[T];
+    unsigned ok = 0;
     double acc[T];
 #pragma unroll
     for (int i = 0; i < T; i++) {
-        const int o = min(tid + NT * i, cnt - 1);
-        const int q = p.cm_fast ? o / bm : o / bn;
-        const int r = o - q * (p.cm_fast ? bm : bn);
-        im[i] = (short)(p.cm_fast ? r : q);
-        in[i] = (short)(p.cm_fast ? q : r);
+        const int o = tid + NT * i;
+        const int q = p.dflat.div(o), r = o - q * (p.cm_fast ? p.BM : p.BN);
+        const int m = p.cm_fast ? r : q, n = p.cm_fast ? q : r;
+        const bool in = o < cnt && m < bm && n < bn;
+        mn[i] = in ? m | n << 16 : 0;
+        ok |= (unsigned)in << i;
         acc[i] = 0.0;
     }
-    for (int s = p.beg[cb]; s < p.beg[cb + 1]; s++) {
-        const double *A = p.A + (long long)b * p.a_bst + p.oa[s];
-        const double *B = p.B + (long long)b * p.b_bst + p.ob[s];
+    for (int s = p.beg[t.cb]; s < p.beg[t.cb + 1]; s++) {
+        const double *A = p.A + (long long)t.b * p.a_bst + p.oa[s];
+        const double *B = p.B + (long long)t.b * p.b_bst + p.ob[s];
         for (int k0 = kbeg; k0 < kend; k0 += BK) {
             const int kn = min(BK, kend - k0);
             __syncthreads();                           // the last k block is used up
-            if (tid < kn) ak[tid] = p.Ac.off(k0 + tid);
-            else if (tid >= 32 && tid < 32 + kn) bk[tid - 32] = p.Br.off(k0 + tid - 32);
+            if (tid < kn) ak[tid] = p.dac.off(p.Ac, k0 + tid);
+            else if (tid >= 64 && tid < 64 + kn) bk[tid - 64] = p.dbr.off(p.Br, k0 + tid - 64);
             __syncthreads();
             if (p.a_kfast) {
                 const int k = tid % BK;
@@ -124,19 +150,115 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F6
             for (int k = 0; k < kn; k++, as += lda, bs += ldb) {
 #pragma unroll
                 for (int i = 0; i < T; i++)
-                    if (wbase + NT * i < cnt) acc[i] = fma(as[im[i]], bs[in[i]], acc[i]);
+                    if (wbase + NT * i < cnt)
+                        acc[i] = fma(as[mn[i] & 0xFFFF], bs[mn[i] >> 16], acc[i]);
             }
         }
     }
-    double *C = p.C.p + (long long)b * p.C.bst + p.oc[cb];
+    double *C = p.C.p + (long long)t.b * p.C.bst + p.oc[t.cb];
 #pragma unroll
-    for (int i = 0; i < T; i++) {
-        if (tid + NT * i >= cnt) break;
-        double *dst = C + cr[im[i]] + cc[in[i]];
-        const double v = p.alpha * acc[i];
-        if (p.atomic) atomicAdd(dst, v);
-        else *dst = (p.beta != 0.0) ? v + p.beta * (*dst) : v;
+    for (int i = 0; i < T; i++)
+        if (ok >> i & 1) f64_out(p, C + cr[mn[i] & 0xFFFF] + cc[mn[i] >> 16], acc[i]);
+}
+
+constexpr int RK = 16;           // k values per shared-memory block of the rows layout
+
+// doubles of the operand blocks, or of the transposed result
+__host__ __device__ constexpr int rows_work(int nthr, int T) {
+    return RK * (nthr | 1) + RK * T > nthr * (T | 1) ? RK * (nthr | 1) + RK * T : nthr * (T | 1);
+}
+__host__ __device__ constexpr size_t rows_smem(int nthr, int T) {
+    return 8 * (size_t)(rows_work(nthr, T) + nthr + 2 * RK + 2 * T);
+}
+
+// the rows layout: blockDim.x rows, columns n0 .. n0 + T - 1
+template <int T>
+__global__ void __launch_bounds__(NT) gemm_f64_rows_kernel(const __grid_constant__ F64Params p) {
+    extern __shared__ __align__(16) double sm[];
+    const int nthr = blockDim.x, lda = nthr | 1, tid = threadIdx.x;
+    double *Bs = sm;                                   // [RK][T]
+    double *As = Bs + RK * T;                          // [RK][lda]
+    long long *ar = (long long *)(sm + rows_work(nthr, T));   // A row offsets
+    long long *ak = ar + nthr, *bk = ak + RK;          // K offsets of the current k block
+    long long *bc = bk + RK, *cc = bc + T;
+    const F64Tile t(p, blockIdx.x);
+    const int m0 = t.tm * p.BM, n0 = t.tn * p.BN;
+    const int bm = min(p.BM, p.M - m0), bn = min(p.BN, p.N - n0);
+    const bool live = tid < bm;
+    const long long aro = live ? p.dar.off(p.Ar, m0 + tid) : 0;
+    ar[tid] = aro;
+    if (tid < bn) {
+        bc[tid] = p.dbc.off(p.Bc, n0 + tid);
+        cc[tid] = p.dcc.off(p.C.c, n0 + tid);
     }
+    double acc[T];
+#pragma unroll
+    for (int i = 0; i < T; i++) acc[i] = 0.0;
+    for (int s = p.beg[t.cb]; s < p.beg[t.cb + 1]; s++) {
+        const double *A = p.A + (long long)t.b * p.a_bst + p.oa[s];
+        const double *B = p.B + (long long)t.b * p.b_bst + p.ob[s];
+        for (int k0 = 0; k0 < p.K; k0 += RK) {
+            const int kn = min(RK, p.K - k0);
+            __syncthreads();                           // the last k block is used up
+            if (tid < kn) {
+                ak[tid] = p.dac.off(p.Ac, k0 + tid);
+                bk[tid] = p.dbr.off(p.Br, k0 + tid);
+            }
+            __syncthreads();
+            if (p.a_kfast) {
+                const int k = tid % RK;
+                if (k < kn)
+                    for (int m = tid / RK; m < bm; m += nthr / RK)
+                        As[k * lda + m] = A[ar[m] + ak[k]];
+            } else if (live) {
+                double v[RK];
+#pragma unroll
+                for (int k = 0; k < RK; k++) v[k] = k < kn ? A[aro + ak[k]] : 0.0;
+#pragma unroll
+                for (int k = 0; k < RK; k++) As[k * lda + tid] = v[k];
+            }
+            for (int x = tid; x < kn * T; x += nthr) {
+                const int k = x / T, n = x - k * T;
+                Bs[x] = n < bn ? B[bc[n] + bk[k]] : 0.0;
+            }
+            __syncthreads();
+            if (live)
+                for (int k = 0; k < kn; k++) {
+                    const double a = As[k * lda + tid];
+                    const double2 *bs = reinterpret_cast<const double2 *>(Bs + k * T);
+#pragma unroll
+                    for (int i = 0; i < T; i += 2) {
+                        if (i < bn) {
+                            const double2 b = bs[i / 2];
+                            acc[i] = fma(a, b.x, acc[i]);
+                            if (i + 1 < bn) acc[i + 1] = fma(a, b.y, acc[i + 1]);
+                        }
+                    }
+                }
+        }
+    }
+    double *C = p.C.p + (long long)t.b * p.C.bst + p.oc[t.cb] +
+                (live ? p.dcr.off(p.C.r, m0 + tid) : 0);
+    if (p.c_trans) {
+        // C contiguous along its columns: the block's rows go through shared
+        // memory so that neighbouring threads write neighbouring columns
+        __syncthreads();
+        double *Cs = sm;                               // [nthr][T | 1], in As and Bs
+        long long *cr = ar;
+        cr[tid] = C - p.C.p;
+#pragma unroll
+        for (int i = 0; i < T; i++) Cs[tid * (T | 1) + i] = acc[i];
+        __syncthreads();
+        for (int x = tid; x < bm * bn; x += nthr) {
+            const int m = x / bn, n = x - m * bn;
+            f64_out(p, p.C.p + cr[m] + cc[n], Cs[m * (T | 1) + n]);
+        }
+        return;
+    }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < T; i++)
+        if (i < bn) f64_out(p, C + cc[i], acc[i]);
 }
 
 struct ScaleBlocks {
@@ -183,11 +305,17 @@ void f64_tile(int M, int N, int cap, int *BM, int *BN) {
     *BN = M <= N ? bl : bs;
 }
 
-template <int T>
+template <int T, int BK>
 int launch_f64_t(kvft_ctx *ctx, const F64Params &p, int grid) {
-    const size_t smem = f64_smem(p.BM, p.BN);
-    gemm_f64_kernel<T><<<grid, NT, smem, ctx->stream>>>(p);
+    const size_t smem = f64_smem(p.BM, p.BN, BK);
+    gemm_f64_kernel<T, BK><<<grid, NT, smem, ctx->stream>>>(p);
     return kv_launch_check(ctx, "gemm_f64");
+}
+
+template <int T>
+int launch_rows_t(kvft_ctx *ctx, const F64Params &p, int grid) {
+    gemm_f64_rows_kernel<T><<<grid, p.BM, rows_smem(p.BM, T), ctx->stream>>>(p);
+    return kv_launch_check(ctx, "gemm_f64_rows");
 }
 
 }  // namespace
@@ -254,39 +382,74 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     if (M <= 0 || N <= 0 || batch <= 0) return KVFT_OK;
     KvGroupTab tab = kv_group_tab(g, false);
     if (K <= 0) return kv_scale_blocks(ctx, M, N, batch, beta, C, tab.ncb, tab.coff);
+    if (N > 64 && M <= 64) {
+        // C^T = B^T A^T: the big operand goes to the rows
+        const KMat At{B.p, B.c, B.r, B.bst, B.stable}, Bt{A.p, A.c, A.r, A.bst, A.stable};
+        KvProds gt = g;
+        std::swap(gt.oa, gt.ob);
+        return kv_gemm_f64(ctx, N, M, K, batch, alpha, At, Bt, beta, KOut{C.p, C.c, C.r, C.bst},
+                           gt);
+    }
     F64Params p;
     p.M = M, p.N = N, p.K = K, p.batch = batch;
-    // The largest tile (16 outputs per thread) that leaves four blocks per
-    // SM to balance the SMs, down to two outputs per thread; then K is split
-    // into chunks of at least 64 while fewer than two blocks per SM remain.
-    int T = TMAX;
-    long long tiles = 0;
-    for (;; T /= 2) {
-        f64_tile(M, N, NT * T, &p.BM, &p.BN);
-        p.mt = ceil_div(M, p.BM);
-        p.nt = ceil_div(N, p.BN);
-        tiles = (long long)p.mt * p.nt * batch;
-        if (T == 2 || tiles * tab.ncb >= 4LL * ctx->sm_count) break;
+    p.nsplit = 1, p.klen = K;
+    const long long want = 2LL * ctx->sm_count, nprod = (long long)batch * tab.ncb;
+    // The rows layout for a big tensor times a small matrix, with the widest
+    // blocks (128, 64 or 32 rows) that leave four per SM; when even 32 rows
+    // leave less than two per SM the flat layout balances better (and splits K).
+    p.nt = ceil_div(N, 24);
+    p.BN = ceil_div(N, p.nt);
+    bool rows = N <= 64 && M >= 4 * N;
+    for (p.BM = 128; rows; p.BM /= 2) {
+        const long long blocks = ceil_div(M, p.BM) * (long long)p.nt * nprod;
+        if (blocks >= 2 * want) break;
+        if (p.BM == 32) {
+            rows = blocks >= want;
+            break;
+        }
     }
-    const long long want = 2LL * ctx->sm_count;
-    p.nsplit = 1;
-    if (tiles * tab.ncb < want && K > 64)
-        p.nsplit = (int)std::min<long long>(ceil_div(want, tiles * tab.ncb), ceil_div(K, 64));
-    p.klen = ceil_div(ceil_div(K, p.nsplit), BK) * BK;
-    p.nsplit = ceil_div(K, p.klen);
-    p.atomic = p.nsplit > 1;
-    if (p.atomic) {
+    p.mt = rows ? ceil_div(M, p.BM) : 0;
+    int T = TMAX;
+    long long tiles = (long long)p.mt * p.nt * batch;
+    if (!rows) {
+        // The largest tile (16 outputs per thread) that leaves four blocks per
+        // SM to balance the SMs, down to two outputs per thread; then K is
+        // split into chunks of at least 32 while fewer than two blocks per SM
+        // remain.
+        for (;; T /= 2) {
+            f64_tile(M, N, NT * T, &p.BM, &p.BN);
+            p.mt = ceil_div(M, p.BM);
+            p.nt = ceil_div(N, p.BN);
+            tiles = (long long)p.mt * p.nt * batch;
+            if (T == 2 || tiles * tab.ncb >= 2 * want) break;
+        }
+        const int bk = T <= 4 ? 32 : 16;
+        if (tiles * tab.ncb < want && K > 32)
+            p.nsplit = (int)std::min<long long>(ceil_div(want, tiles * tab.ncb), ceil_div(K, 32));
+        p.klen = ceil_div(ceil_div(K, p.nsplit), bk) * bk;
+        p.nsplit = ceil_div(K, p.klen);
+    }
+    p.store = beta == 0.0 ? 1 : beta == 1.0 ? 2 : 3;
+    if (p.nsplit > 1) {
         KV_TRY(kv_scale_blocks(ctx, M, N, batch, beta, C, tab.ncb, tab.coff));
         tab = kv_group_tab(g, true);
+        p.store = 0;
     }
     const long long grid = tiles * p.nsplit * tab.ncb;
     if (grid > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "gemm: too many tiles");
-    p.a_kfast = kidx_fast_stride(A.c) == 1;
+    p.a_kfast = kidx_fast_stride(A.c) == 1 && kidx_fast_stride(A.r) != 1;
     p.b_kfast = kidx_fast_stride(B.r) == 1;
     p.cm_fast = kidx_fast_stride(C.r) == 1 && kidx_fast_stride(C.c) != 1;
+    p.c_trans = kidx_fast_stride(C.c) == 1 && kidx_fast_stride(C.r) != 1;
+    p.unit = alpha == 1.0 ? 1 : alpha == -1.0 ? 2 : 0;
     p.alpha = alpha, p.beta = beta;
     p.A = A.p, p.B = B.p, p.C = C;
     p.Ar = A.r, p.Ac = A.c, p.Br = B.r, p.Bc = B.c;
+    p.dar = kidx_div(A.r), p.dac = kidx_div(A.c), p.dbr = kidx_div(B.r), p.dbc = kidx_div(B.c);
+    p.dcr = kidx_div(C.r), p.dcc = kidx_div(C.c);
+    p.dnt = fastdiv(p.nt), p.dmt = fastdiv(p.mt), p.dks = fastdiv(p.nsplit);
+    p.dbatch = fastdiv(batch);
+    p.dflat = fastdiv(p.cm_fast ? p.BM : p.BN);
     p.a_bst = A.bst, p.b_bst = B.bst;
     for (int c = 0; c < tab.ncb; c++) p.oc[c] = tab.coff[c];
     for (int c = 0; c <= tab.ncb; c++) p.beg[c] = tab.beg[c];
@@ -295,11 +458,16 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         p.ob[q] = g.ob[tab.prod[q]];
     }
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
+    if (rows) {
+        if (p.BN <= 8) return launch_rows_t<8>(ctx, p, (int)grid);
+        if (p.BN <= 16) return launch_rows_t<16>(ctx, p, (int)grid);
+        return launch_rows_t<24>(ctx, p, (int)grid);
+    }
     switch (T) {
-    case 16: return launch_f64_t<16>(ctx, p, (int)grid);
-    case 8: return launch_f64_t<8>(ctx, p, (int)grid);
-    case 4: return launch_f64_t<4>(ctx, p, (int)grid);
-    default: return launch_f64_t<2>(ctx, p, (int)grid);
+    case 16: return launch_f64_t<16, 16>(ctx, p, (int)grid);
+    case 8: return launch_f64_t<8, 16>(ctx, p, (int)grid);
+    case 4: return launch_f64_t<4, 32>(ctx, p, (int)grid);
+    default: return launch_f64_t<2, 32>(ctx, p, (int)grid);
     }
 }
 

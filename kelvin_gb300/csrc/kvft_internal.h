@@ -67,6 +67,36 @@ inline long long kidx_fast_stride(const KIdx &x) {
     return 0;
 }
 
+// x / d for 0 <= x < 2^31 by a multiply and a shift (Granlund-Montgomery:
+// m = ceil(2^(31+l) / d) with 2^l >= d), in place of the ~20 instructions of
+// an integer division by a run-time divisor in the index arithmetic of tiles.
+struct FastDiv {
+    unsigned long long m;
+    int s;
+    __device__ __forceinline__ int div(int x) const {
+        return (int)(((unsigned long long)(unsigned)x * m) >> s);
+    }
+};
+inline FastDiv fastdiv(int d) {
+    int l = 0;
+    while ((1LL << l) < d) l++;
+    FastDiv f;
+    f.s = 31 + l;
+    f.m = ((1ULL << f.s) + (unsigned long long)d - 1) / (unsigned long long)d;
+    return f;
+}
+
+// KIdx::off with its two divisions precomputed.
+struct KIdxDiv {
+    FastDiv d2, d1;
+    __device__ __forceinline__ long long off(const KIdx &x, int m) const {
+        const int r1 = d2.div(m), i2 = m - r1 * x.size[2];
+        const int i0 = d1.div(r1), i1 = r1 - i0 * x.size[1];
+        return (long long)i0 * x.st[0] + (long long)i1 * x.st[1] + (long long)i2 * x.st[2];
+    }
+};
+inline KIdxDiv kidx_div(const KIdx &x) { return KIdxDiv{fastdiv(x.size[2]), fastdiv(x.size[1])}; }
+
 // Profile categories (kvft_profile_stats order): work in flops for
 // KV_CAT_GEMM6, in bytes for the others.
 enum KvCat { KV_CAT_GEMM6 = 0, KV_CAT_GEMM = 1, KV_CAT_QUAD = 2, KV_CAT_ENERGY = 3,

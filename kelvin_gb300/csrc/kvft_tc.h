@@ -14,25 +14,6 @@ constexpr int TM = 128;
 constexpr int MAXS = 6;
 constexpr unsigned long long WAIT_NS = 2000000000ull;   // 2 s per wait
 
-// x / d for 0 <= x < 2^31 by a multiply and a shift (Granlund-Montgomery:
-// m = ceil(2^(31+l) / d) with 2^l >= d), in place of the ~20 instructions of
-// an integer division by a run-time divisor in the per-tile index arithmetic.
-struct FastDiv {
-    unsigned long long m;
-    int s;
-    __device__ __forceinline__ int div(int x) const {
-        return (int)(((unsigned long long)(unsigned)x * m) >> s);
-    }
-};
-inline FastDiv fastdiv(int d) {
-    int l = 0;
-    while ((1LL << l) < d) l++;
-    FastDiv f;
-    f.s = 31 + l;
-    f.m = ((1ULL << f.s) + (unsigned long long)d - 1) / (unsigned long long)d;
-    return f;
-}
-
 // Knuth's error-free sum: s + e == a + b exactly (round-to-nearest FP32)
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
     s = a + b;

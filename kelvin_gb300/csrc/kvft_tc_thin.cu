@@ -69,18 +69,12 @@ struct ThinParams {
     const int *eb;               // exponents of the small matrices' rows
     int eb_bst, b_batch_rows, b_plane_rows;
     int *err;
-    FastDiv dv_mt, dv_batch, dv_ar2, dv_ar1, dv_cr2, dv_cr1;
+    FastDiv dv_mt, dv_batch;
+    KIdxDiv dv_ar, dv_cr;
     int beg[KV_MAXPROD + 1];
     long long coff[KV_MAXPROD], oa[KV_MAXPROD];
     int brow[KV_MAXPROD], bex[KV_MAXPROD];
 };
-
-__device__ __forceinline__ long long kidx_off(const KIdx &x, const FastDiv &d2, const FastDiv &d1,
-                                              int m) {
-    const int r1 = d2.div(m), i2 = m - r1 * x.size[2];
-    const int i0 = d1.div(r1), i1 = r1 - i0 * x.size[1];
-    return (long long)i0 * x.st[0] + (long long)i1 * x.st[1] + (long long)i2 * x.st[2];
-}
 
 // High word of x 2^k (x a finite FP32 value, its low word is the bits << 29):
 // the exponent and top mantissa bits of x moved to their FP64 place plus kk =
@@ -271,7 +265,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
         if (p.a_rows_fast) {
             const int m = m0 + row;
             const bool ok = m < p.M;
-            const double *q0 = base + (ok ? kidx_off(p.Ar, p.dv_ar2, p.dv_ar1, m) : 0);
+            const double *q0 = base + (ok ? p.dv_ar.off(p.Ar, m) : 0);
             const int kn = ok ? p.K : 0;
 #pragma unroll
             for (int c = 0; c < VP / 8; c++) {
@@ -286,7 +280,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
             }
         } else {
             const int r = m0 + warp * RW + (lane % RW);
-            const long long ro = r < p.M ? kidx_off(p.Ar, p.dv_ar2, p.dv_ar1, r) : -1;
+            const long long ro = r < p.M ? p.dv_ar.off(p.Ar, r) : -1;
             const int k = 2 * (KBT == 64 ? lane : lane % 16);
             const long long ko = (long long)k * p.ks;
 #pragma unroll
@@ -428,7 +422,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
         if (newA) fetch(n);
         // ---- C ----
         const int m = s.mt * TM + row;
-        const long long roff = m < p.M ? kidx_off(p.Cr, p.dv_cr2, p.dv_cr1, m) : -1;
+        const long long roff = m < p.M ? p.dv_cr.off(p.Cr, m) : -1;
         double *Cb = p.C + p.coff[s.cb] + (long long)s.b * p.c_bst;
         const int store = s.src == p.beg[s.cb] ? p.store : 0;
         const int krow = rexp[row];
@@ -619,8 +613,7 @@ int kv_gemm_thin(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, co
     p.err = ctx->dflag;
     p.dv_mt = fastdiv(p.mt);
     p.dv_batch = fastdiv(batch);
-    p.dv_ar2 = fastdiv(A.r.size[2]), p.dv_ar1 = fastdiv(A.r.size[1]);
-    p.dv_cr2 = fastdiv(C.r.size[2]), p.dv_cr1 = fastdiv(C.r.size[1]);
+    p.dv_ar = kidx_div(A.r), p.dv_cr = kidx_div(C.r);
     for (int c = 0; c <= tab.ncb; c++) p.beg[c] = tab.beg[c];
     for (int c = 0; c < tab.ncb; c++) p.coff[c] = tab.coff[c];
     for (int q = 0; q < g.n; q++) {

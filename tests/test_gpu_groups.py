@@ -18,7 +18,11 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,batch", [
     (1, 1, 1, 1), (1, 129, 3, 2), (129, 1, 17, 1), (13, 2197, 13, 3), (2197, 13, 13, 3),
     (19, 19, 6859, 2), (8, 8, 512, 10), (64, 65, 16, 1), (65, 64, 15, 1), (127, 33, 33, 5),
-    (361, 361, 361, 1), (57, 4000, 57, 1), (2, 300, 1000, 1)])
+    (361, 361, 361, 1), (57, 4000, 57, 1), (2, 300, 1000, 1),
+    # a row per thread: 128-, 64- and 32-row blocks, 1 to 24 columns, several
+    # column tiles (25, 49, 64), K around its block of 16, either side big
+    (40000, 1, 16, 2), (33000, 24, 17, 4), (20011, 25, 15, 3), (9000, 49, 31, 3),
+    (64, 7777, 9, 5), (8, 512, 8, 60), (5000, 13, 13, 20)])
 def test_gemm_fp64_tiles(ctx, M, N, K, batch):
     rng = numpy.random.default_rng(M + 3 * N + 7 * K + batch)
     A = rng.standard_normal((batch, M, K))
