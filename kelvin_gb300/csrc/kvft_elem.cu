@@ -279,18 +279,59 @@ assemble_t2_kernel(int nv, int no, int sh, double fac, const double *__restrict_
     }
 }
 
-// The same with spin blocks (nv = no = n = 2h): for each (b, j) only the
-// (f, n) with s_f - s_n = s_j - s_b are written -- the alpha-alpha and
-// beta-beta quadrants, or the one mixed quadrant -- in 32 x 32 tiles laid out
-// from each quadrant's origin (no tile straddles the spin boundary; block x
-// = quadrant and tile).
-__global__ void __launch_bounds__(256)
-wmbej_tmp_spin_kernel(int n, int h, const double *__restrict__ t1,
+// ---- spin blocks: square tiles of a quadrant ----------------------------------
+// A quadrant of h x h elements is cut into nt x nt square tiles of edge te =
+// ceil(h / nt), nt = ceil(h / 64): one tile for h <= 64.  A block walks a
+// tile's elements flat, so only its last pass has idle threads, whatever h
+// is.  (32 x 32 tiles with a thread per column took 3.8x the passes at h = 33:
+// helper 1.62 -> 0.48, assembly 1.88 -> 0.85 ms per 66-spin-orbital iteration
+// of 16 tau points.)
+constexpr int ST_T = 256;
+
+struct SpinTiles {
+    int h, nt, te;
+    __host__ __device__ explicit SpinTiles(int h_)
+        : h(h_), nt((h_ + 63) / 64), te((h_ + (h_ + 63) / 64 - 1) / ((h_ + 63) / 64)) {}
+};
+
+// f(r, c) over a rows x cols tile, flat over the block's threads (c fastest)
+template <class F>
+__device__ __forceinline__ void tile_walk(int rows, int cols, F f) {
+    const int dr = ST_T / cols, dc = ST_T - dr * cols;
+    int r = threadIdx.x / cols, c = threadIdx.x - r * cols;
+#pragma unroll 4
+    while (r < rows) {
+        f(r, c);
+        r += dr;
+        c += dc;
+        if (c >= cols) {
+            c -= cols;
+            r++;
+        }
+    }
+}
+
+// x / 2 by integer arithmetic (exact, as the multiplication; the FP64 pipe
+// only takes values with the smallest exponents)
+__device__ __forceinline__ double half_of(double x) {
+    const int hi = __double2hiint(x);
+    if ((hi & 0x7FE00000) == 0 || (hi & 0x7FF00000) == 0x7FF00000) return 0.5 * x;
+    return __hiloint2double(hi - 0x00100000, __double2loint(x));
+}
+
+// out[y][b][j][n][f] = 0.5 t2[y][f][b][j][n] + t1[y][f][j] t1[y][b][n] (nv = no =
+// n = 2h): for each (b, j) only the (f, n) with s_f - s_n = s_j - s_b are
+// written -- the alpha-alpha and beta-beta quadrants, or the one mixed
+// quadrant.  The t1 t1 term vanishes unless s_f = s_j (and s_b = s_n).  Block x:
+// quadrant and tile.
+__global__ void __launch_bounds__(ST_T)
+wmbej_tmp_spin_kernel(int n, SpinTiles g, const double *__restrict__ t1,
                       const double *__restrict__ t2, double *__restrict__ out) {
-    __shared__ double tile[32][33];
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    const int nth = (h + 31) / 32, nt2 = nth * nth;
+    extern __shared__ double tile[];
+    const int h = g.h, ld = g.te | 1, nt2 = g.nt * g.nt;
     const int q = blockIdx.x / nt2, tt = blockIdx.x % nt2;
+    const int fo = tt / g.nt * g.te, mo = tt % g.nt * g.te;
+    const int rows = min(g.te, h - fo), cols = min(g.te, h - mo);
     const long long y = blockIdx.z;
     const long long oo = (long long)n * n;
     const double *u = t1 + y * oo;
@@ -299,43 +340,38 @@ wmbej_tmp_spin_kernel(int n, int h, const double *__restrict__ t1,
         const int d = (j >= h) - (b >= h);          // s_f - s_n
         if (d != 0 && q) continue;                  // block-uniform
         const int sf = d == 0 ? q : (d > 0), sn = d == 0 ? q : (d < 0);
-        const int f0 = sf * h + 32 * (tt / nth), n0 = sn * h + 32 * (tt % nth);
-        const int fhi = sf * h + h, nhi = sn * h + h;
+        const int f0 = sf * h + fo, m0 = sn * h + mo;
+        const bool tt1 = sf == (j >= h);
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int f = f0 + ty + 8 * i, m = n0 + tx;
-            if (f < fhi && m < nhi)
-                tile[ty + 8 * i][tx] = t2[((y * n + f) * n + b) * oo + (long long)j * n + m];
-        }
+        const double *src = t2 + ((y * n + f0) * n + b) * oo + (long long)j * n + m0;
+        tile_walk(rows, cols, [&](int r, int c) { tile[r * ld + c] = src[r * n * oo + c]; });
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int m = n0 + ty + 8 * i, f = f0 + tx;
-            if (f < fhi && m < nhi)
-                out[(((y * n + b) * n + j) * n + m) * n + f] =
-                    0.5 * tile[tx][ty + 8 * i] + u[f * n + j] * u[b * n + m];
-        }
+        double *dst = out + (((y * n + b) * n + j) * n + m0) * n + f0;
+        tile_walk(cols, rows, [&](int c, int r) {
+            const double x = half_of(tile[r * ld + c]);
+            dst[(long long)c * n + r] =
+                tt1 ? fma(u[(f0 + r) * n + j], u[b * n + m0 + c], x) : x;
+        });
     }
 }
 
 // The seeded assembly with spin blocks (nv = no = n = 2h): for the pair
 // (a < b) of spin sum t = s_a + s_b only the (i, j) with s_i + s_j = t are
 // written -- the alpha-alpha quadrant (t = 0), the beta-beta one (t = 2), or
-// the alpha-beta quadrant with its mirror beta-alpha (t = 1).  Tiles are laid
-// out from each quadrant's origin, so no tile straddles the spin boundary:
-// tile pairs (it <= jt) of a diagonal quadrant, every (it, jt) of the
-// alpha-beta one with its mirror tile in the beta-alpha one.  The other
-// elements of T2 are left as they are (zero: nothing writes or reads them).
+// the alpha-beta quadrant with its mirror beta-alpha (t = 1): tile pairs (it
+// <= jt) of a diagonal quadrant, every (it, jt) of the alpha-beta one with its
+// mirror tile in the beta-alpha one.  The other elements of T2 are left as
+// they are (zero: nothing writes or reads them).  Bound by the FP64 pipe (five
+// operations per pair of outputs) as much as by memory.
 template <int FS>
-__global__ void __launch_bounds__(256, 3)
-assemble_t2_spin_kernel(int n, int h, double fac, const double *__restrict__ Z,
+__global__ void __launch_bounds__(ST_T)
+assemble_t2_spin_kernel(int n, SpinTiles g, double fac, const double *__restrict__ Z,
                         const double *__restrict__ Lc, const double *__restrict__ seed,
                         double *__restrict__ T2) {
+    extern __shared__ double tile[];
+    const int h = g.h, ld = g.te | 1;
     const PairOrder ov{n, h};
-    __shared__ double qa[32][33], qb[32][33];
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
-    const int nth = (h + 31) / 32;
+    double *qa = tile, *qb = tile + g.te * ld;      // Z[a,b] - Z[b,a]: the tile, its mirror
     const long long y = blockIdx.z;
     const int pv = n * (n - 1) / 2;
     const long long oo = (long long)n * n, s4 = oo * oo;
@@ -345,36 +381,37 @@ assemble_t2_spin_kernel(int n, int h, double fac, const double *__restrict__ Z,
         const int tab = (a >= h) + (b >= h);
         int it, jt;
         if (tab == 1) {
-            if ((int)blockIdx.x >= nth * nth) continue;              // block-uniform
-            it = blockIdx.x / nth;
-            jt = blockIdx.x % nth;
+            if ((int)blockIdx.x >= g.nt * g.nt) continue;            // block-uniform
+            it = blockIdx.x / g.nt;
+            jt = blockIdx.x % g.nt;
         } else {
-            if ((int)blockIdx.x >= nth * (nth + 1) / 2) continue;
+            if ((int)blockIdx.x >= g.nt * (g.nt + 1) / 2) continue;
             it = 0;
             int rem = blockIdx.x;
-            while (rem >= nth - it) {
-                rem -= nth - it;
+            while (rem >= g.nt - it) {
+                rem -= g.nt - it;
                 it++;
             }
             jt = it + rem;
         }
         const int ilo = tab == 2 ? h : 0, jlo = tab == 0 ? 0 : h;   // quadrant origins
-        const int ihi = ilo + h, jhi = jlo + h;
-        const int i0 = ilo + 32 * it, j0 = jlo + 32 * jt;
+        const int i0 = ilo + g.te * it, j0 = jlo + g.te * jt;
+        const int ni = min(g.te, ilo + h - i0), nj = min(g.te, jlo + h - j0);
         const bool mirror = tab == 1 || it != jt;
+        const double *qt = mirror ? qb : qa;
         const long long oab = y * s4 + ((long long)a * n + b) * oo;
         const long long oba = y * s4 + ((long long)b * n + a) * oo;
         const double *L = Lc ? Lc + (y * pv + pab) * (long long)pv : nullptr;
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int r = ty + 8 * k;
-            int i = i0 + r, j = j0 + tx;
-            qa[r][tx] = (i < ihi && j < jhi) ? Z[oab + i * n + j] - Z[oba + i * n + j] : 0.0;
-            i = j0 + r;
-            j = i0 + tx;
-            qb[r][tx] = (i < jhi && j < ihi) ? Z[oab + i * n + j] - Z[oba + i * n + j] : 0.0;
-        }
+        tile_walk(ni, nj, [&](int r, int c) {
+            const int x = (i0 + r) * n + j0 + c;
+            qa[r * ld + c] = Z[oab + x] - Z[oba + x];
+        });
+        if (mirror)
+            tile_walk(nj, ni, [&](int r, int c) {
+                const int x = (j0 + r) * n + i0 + c;
+                qb[r * ld + c] = Z[oab + x] - Z[oba + x];
+            });
         __syncthreads();
         // L over (i < j); both indices of a written element have the pair's type
         auto ladder = [&](int i, int j) -> double {
@@ -382,25 +419,19 @@ assemble_t2_spin_kernel(int n, int h, double fac, const double *__restrict__ Z,
             return i < j ? L[ov.index(i, j)] : -L[ov.index(j, i)];
         };
         const long long sab = ((long long)a * n + b) * oo, sba = ((long long)b * n + a) * oo;
-        auto put = [&](int x, double R) {
+        auto put = [&](int i, int j, double R0) {
+            const int x = i * n + j;
+            const double R = FS == 0 ? fac * R0 : (FS == 1 ? R0 : -R0);
             T2[oab + x] = R - seed[sab + x];
             T2[oba + x] = -R - seed[sba + x];
         };
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int r = ty + 8 * k;
-            int i = i0 + r, j = j0 + tx;
-            if (i < ihi && j < jhi) {
-                const double R0 = qa[r][tx] - qb[tx][r] + ladder(i, j);
-                put(i * n + j, FS == 0 ? fac * R0 : (FS == 1 ? R0 : -R0));
-            }
-            i = j0 + r;
-            j = i0 + tx;
-            if (mirror && i < jhi && j < ihi) {
-                const double R0 = qb[r][tx] - qa[tx][r] + ladder(i, j);
-                put(i * n + j, FS == 0 ? fac * R0 : (FS == 1 ? R0 : -R0));
-            }
-        }
+        tile_walk(ni, nj, [&](int r, int c) {
+            put(i0 + r, j0 + c, qa[r * ld + c] - qt[c * ld + r] + ladder(i0 + r, j0 + c));
+        });
+        if (mirror)
+            tile_walk(nj, ni, [&](int r, int c) {
+                put(j0 + r, i0 + c, qb[r * ld + c] - qa[c * ld + r] + ladder(j0 + r, i0 + c));
+            });
     }
 }
 
@@ -536,9 +567,10 @@ int kv_make_wmbej_tmp(kvft_ctx *ctx, int batch, int nv, int no,
     if (batch > 65535) return kv_fail(ctx, KVFT_EINVAL, "wmbej_tmp: batch too large");
     KvProfScope prof(ctx, KV_CAT_ELEM, 16.0 * total * kv_spin_frac(nv, no, spin_half));
     if (spin_half > 0 && nv == no && nv == 2 * spin_half) {
-        const int nth = (spin_half + 31) / 32;
-        const dim3 gs(2 * nth * nth, std::min(nv * no, 2048), batch);
-        wmbej_tmp_spin_kernel<<<gs, 256, 0, ctx->stream>>>(nv, spin_half, t1, t2, out);
+        const SpinTiles st(spin_half);
+        const size_t smem = sizeof(double) * st.te * (st.te | 1);
+        const dim3 gs(2 * st.nt * st.nt, std::min(nv * no, 2048), batch);
+        wmbej_tmp_spin_kernel<<<gs, ST_T, smem, ctx->stream>>>(nv, st, t1, t2, out);
         return kv_launch_check(ctx, "wmbej_tmp_spin");
     }
     // each block walks several (b, j): short-lived blocks would leave the SMs
@@ -571,14 +603,25 @@ int kv_assemble_t2(kvft_ctx *ctx, int batch, int nv, int no, double fac, const d
                                                                   T2)
     const int fs = fac == 1.0 ? 1 : (fac == -1.0 ? 2 : 0);
     if (seed && sh) {
-        const int nth = (sh + 31) / 32;
-        const dim3 gs(nth * nth, std::min(pv, 65535), batch);
+        const SpinTiles st(sh);
+        const size_t smem = 2 * sizeof(double) * st.te * (st.te | 1);
+        const dim3 gs(st.nt * st.nt, std::min(pv, 65535), batch);
+        static bool attr = false;
+        if (!attr) {
+            const void *k[3] = {(const void *)assemble_t2_spin_kernel<0>,
+                                (const void *)assemble_t2_spin_kernel<1>,
+                                (const void *)assemble_t2_spin_kernel<2>};
+            for (const void *f : k)
+                KV_CHECK(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   2 * 8 * 64 * 65));
+            attr = true;
+        }
         if (fs == 1)
-            assemble_t2_spin_kernel<1><<<gs, 256, 0, ctx->stream>>>(nv, sh, fac, Z, Lc, seed, T2);
+            assemble_t2_spin_kernel<1><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
         else if (fs == 2)
-            assemble_t2_spin_kernel<2><<<gs, 256, 0, ctx->stream>>>(nv, sh, fac, Z, Lc, seed, T2);
+            assemble_t2_spin_kernel<2><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
         else
-            assemble_t2_spin_kernel<0><<<gs, 256, 0, ctx->stream>>>(nv, sh, fac, Z, Lc, seed, T2);
+            assemble_t2_spin_kernel<0><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
         return kv_launch_check(ctx, "assemble_t2_spin");
     }
     if (seed) {

@@ -201,6 +201,33 @@ __device__ __forceinline__ double kv_f2d(float f) {
                             (int)(u << 29));
 }
 
+// The six spin patterns (sa, sb, si, sj) of a T2-shaped tensor with sa + sb =
+// si + sj (0 = alpha, 1 = beta), four bits each: sa | sb << 1 | si << 2 | sj
+// << 3.
+constexpr unsigned KV_SPIN_PATTERNS = 0u | 15u << 4 | 10u << 8 | 6u << 12 | 9u << 16 | 5u << 20;
+
+// The spin-conserving elements of one tau point (nv = no = n = 2h) in units of
+// 32 for a warp: unit u covers 32 consecutive positions of one (pattern, a, b)
+// quadrant of h x h elements (i, j), so that lanes stay full whatever h is (a
+// row of h = 33 as one unit and a half left 31 of 64 lanes idle).
+struct KvSpinUnits {
+    int h, n, hh, nch;
+    __device__ __forceinline__ KvSpinUnits(int h_) : h(h_), n(2 * h_), hh(h_ * h_), nch((h_ * h_ + 31) / 32) {}
+    __device__ __forceinline__ long long count() const { return 6LL * hh * nch; }
+    // l = a n + b and r = i n + j of a lane's element; false past the quadrant
+    __device__ __forceinline__ bool at(long long u, int lane, int &l, int &r) const {
+        const int item = (int)(u / nch), e = (int)(u - (long long)item * nch) * 32 + lane;
+        if (e >= hh) return false;
+        const int pat = item / hh, ab = item - pat * hh, a1 = ab / h, i1 = e / h;
+        const unsigned c = KV_SPIN_PATTERNS >> (4 * pat);
+        const int a = a1 + (int)(c & 1u) * h, b = ab - a1 * h + (int)((c >> 1) & 1u) * h;
+        const int i = i1 + (int)((c >> 2) & 1u) * h, j = e - i1 * h + (int)((c >> 3) & 1u) * h;
+        l = a * n + b;
+        r = i * n + j;
+        return true;
+    }
+};
+
 // Fraction of a T2-shaped tensor (nv nv no no) that the spin-conserving
 // blocks hold: 6 of the 16 spin blocks when nv = no = 2 sh, else all.  The
 // profiled algorithmic bytes of a pass that touches only those elements are

@@ -33,26 +33,90 @@ struct QuadParams {
     int step;                // recurrence step (0: general path)
     int uniform;             // all ti[k+1]-ti[k] equal
     int full;
+    int same;                // first chained row from which gd, g1 and cs are constant
     int symmetric;           // ti[x] + ti[ng-1-x] the same for every x
+    int mirror;              // the same to the last bits
     double alpha;            // damping (fused update only)
     int spin_half;           // fused update over the spin-conserving elements only (0: all)
 };
 
-__device__ __forceinline__ double denom(const QuadParams &q, long long p,
-                                        const double *D, const double *ev,
-                                        const double *eo) {
+// d of element p = l NR + r (rank 1: l = a, r = i; rank 2: l = a nv + b, r = i
+// no + j)
+__device__ __forceinline__ double denom(const QuadParams &q, long long p, int l, int r,
+                                        const double *D, const double *ev, const double *eo) {
     if (D) return D[p];
-    if (q.rank == 1) {
-        int i = (int)(p % q.no);
-        int a = (int)(p / q.no);
-        return ev[a] - eo[i];
+    if (q.rank == 1) return ev[l] - eo[r];
+    const int a = l / q.nv, i = r / q.no;
+    return ev[a] + ev[l - a * q.nv] - eo[i] - eo[r - i * q.no];
+}
+
+// e^x by table lookup (P. T. P. Tang, ACM TOMS 15, 144 (1989)): x = n ln2/64 +
+// r, |r| <= ln2/128, e^x = 2^(n / 64) (1 + (e^r - 1)) with the 64 values of
+// 2^(j/64) in shared memory and a fifth-order Taylor polynomial (its remainder
+// is below 4e-17): ten FP64 operations, and two of them more for e^-x, where
+// the library function takes about 17 and the reciprocal ten -- the FP64 pipe
+// is what these kernels wait for.  Within one unit in the last place of the
+// exact value; |x| >= 700 and NaN go to the library function.
+constexpr int ETAB = 64;
+__device__ __forceinline__ void exp_table(double *T) {       // caller synchronises
+    for (int j = threadIdx.x; j < ETAB; j += blockDim.x) T[j] = exp2(j * (1.0 / ETAB));
+}
+__device__ __forceinline__ double exp_scaled(const double *T, int n, double p) {
+    const double t = T[n & (ETAB - 1)], y = fma(t, p, t);
+    return __hiloint2double(__double2hiint(y) + (n >> 6) * (1 << 20), __double2loint(y));
+}
+__device__ __forceinline__ bool exp_reduce(double x, int &n, double &r) {
+    if ((__double2hiint(x) & 0x7FFFFFFF) >= 0x4085E000) return false;       // |x| >= 700, NaN
+    const double t = fma(x, 92.332482616893656877, 6755399441055744.0);     // 64 / ln 2
+    n = __double2loint(t);
+    const double nd = t - 6755399441055744.0;
+    r = fma(nd, -0.010830424696223417, x);               // ln2/64, 36 bits, and the rest
+    r = fma(nd, -2.5728046223276688e-14, r);
+    return true;
+}
+__device__ __forceinline__ double exp_tab(double x, const double *T) {
+    int n;
+    double r;
+    if (!exp_reduce(x, n, r)) return exp(x);
+    const double q = fma(fma(fma(r, 1.0 / 120.0, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+    return exp_scaled(T, n, fma(q * r, r, r));
+}
+// e^x and e^-x: the polynomial's even and odd parts
+__device__ __forceinline__ void exp_tab2(double x, const double *T, double &ep, double &em) {
+    int n;
+    double r;
+    if (!exp_reduce(x, n, r)) {
+        ep = exp(x);
+        em = exp(-x);
+        return;
     }
-    long long r = p;
-    int j = (int)(r % q.no); r /= q.no;
-    int i = (int)(r % q.no); r /= q.no;
-    int b = (int)(r % q.nv);
-    int a = (int)(r / q.nv);
-    return ev[a] + ev[b] - eo[i] - eo[j];
+    const double r2 = r * r;
+    const double ev = r2 * fma(r2, 1.0 / 24.0, 0.5);
+    const double od = fma(r * r2, fma(r2, 1.0 / 120.0, 1.0 / 6.0), r);
+    ep = exp_scaled(T, n, ev + od);
+    em = exp_scaled(T, -n, ev - od);
+}
+
+// f(p, l, r) for this thread's elements: every one, or with spin blocks the
+// spin-conserving ones (the others are zero and stay zero)
+template <class F>
+__device__ __forceinline__ void quad_visit(const QuadParams &q, F f) {
+    if (q.spin_half > 0) {
+        const KvSpinUnits su(q.spin_half);
+        const long long n2 = (long long)q.no * q.no, units = su.count();
+        for (long long u = blockIdx.x * (long long)(QT / 32) + threadIdx.x / 32; u < units;
+             u += (long long)gridDim.x * (QT / 32)) {
+            int l, r;
+            if (su.at(u, threadIdx.x % 32, l, r)) f(l * n2 + r, l, r);
+        }
+        return;
+    }
+    const int NR = q.rank == 2 ? q.no * q.no : q.no;
+    for (long long p = blockIdx.x * (long long)QT + threadIdx.x; p < q.P;
+         p += (long long)gridDim.x * QT) {
+        const int l = (int)(p / NR);
+        f(p, l, (int)(p - (long long)l * NR));
+    }
 }
 
 // Shared memory: ti[ng], G[ng*ng], the chained-row coefficients cs[ng]
@@ -90,7 +154,8 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
     double *ti = sm;
     double *G = ti + ng;
     double *cs = G + ng * ng, *g1 = cs + ng, *gd = g1 + ng;
-    double *rk = gd + ng;                                  // [ng][QT]
+    double *et = gd + ng;                                  // 2^(j/64)
+    double *rk = et + ETAB;                                // [ng][QT]
     double *tb = rk + (q.uniform ? 0 : ng * QT);           // [ng][QT]
     for (int k = threadIdx.x; k < ng; k += QT) ti[k] = ti_g[k];
     for (int k = threadIdx.x; k < ng * ng; k += QT) G[k] = G_g[k];
@@ -100,19 +165,20 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
         g1[y] = (y >= 1) ? G_g[y * ng + y - 1] : 0.0;
         gd[y] = G_g[y * ng + y];
     }
+    exp_table(et);
     __syncthreads();
     const double oma = 1.0 - q.alpha;
 
     double s_diff = 0.0, s_norm = 0.0;
     const int t = threadIdx.x;
-    auto element = [&](long long p) {
-        const double d = denom(q, p, D, ev, eo);
+    auto element = [&](long long p, int l, int r) {
+        const double d = denom(q, p, l, r, D, ev, eo);
         // step factors r_k = exp((ti[k]-ti[k+1]) d)
         double r0 = 1.0;
         if (UNI) {
-            r0 = (ng > 1) ? exp((ti[0] - ti[1]) * d) : 1.0;
+            r0 = (ng > 1) ? exp_tab((ti[0] - ti[1]) * d, et) : 1.0;
         } else {
-            for (int k = 0; k + 1 < ng; k++) rk[k * QT + t] = exp((ti[k] - ti[k + 1]) * d);
+            for (int k = 0; k + 1 < ng; k++) rk[k * QT + t] = exp_tab((ti[k] - ti[k + 1]) * d, et);
         }
         const double r02 = r0 * r0;
         float f_diff = 0.f, f_norm = 0.f;
@@ -120,8 +186,26 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
         if (q.step > 0) {
             // chained rows; keep the last `step` outputs and inputs in registers
             double Tm1 = 0.0, Tm2 = 0.0, tbm1 = 0.0, tbm2 = 0.0;
-            for (int y = 0; y < ng; y++) {
-                const double tby = tbar[(long long)y * q.P + p];
+            const double *tp = tbar + p;
+            double *op = out + p;
+            auto emit = [&](double *o, double told, double Ty, double tby) {
+                if (MODE == 0) {
+                    *o = Ty;
+                } else {
+                    // damped update Told + (1 - alpha)(T - Told) and the norms
+                    const double df = Ty - told;
+                    const double nt = fma(oma, df, told);
+                    const float fd = abs_to_f32(df), fn = abs_to_f32(nt);
+                    f_diff = fmaf(fd, fd, f_diff);
+                    f_norm = fmaf(fn, fn, f_norm);
+                    *o = nt;
+                }
+                Tm2 = Tm1; Tm1 = Ty;
+                tbm2 = tbm1; tbm1 = tby;
+            };
+            const int same = UNI ? q.same : ng;
+            for (int y = 0; y < same; y++, tp += q.P, op += q.P) {
+                const double tby = *tp;
                 double Ty;
                 if (y < q.step) {
                     // direct: x in [0, y]
@@ -136,26 +220,34 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
                     // T_y = w (T_{y-1} - G[y-1,y-1] tb_{y-1}) + G[y,y-1] w tb_{y-1}
                     //       + G[y,y] tb_y
                     Ty = fma(gd[y], tby, RK(y - 1) * fma(cs[y], tbm1, Tm1));
-                } else {  // step 2
-                    const double w1 = RK(y - 1);
-                    const double w2 = UNI ? r02 : w1 * RK(y - 2);
-                    Ty = fma(gd[y], tby, fma(g1[y] * w1, tbm1, w2 * fma(cs[y], tbm2, Tm2)));
+                } else {  // step 2: r_{y-1} (r_{y-2} (T + cs tb)_{y-2} + g1 tb_{y-1}) + gd tb_y
+                    const double z = fma(RK(y - 2), fma(cs[y], tbm2, Tm2), g1[y] * tbm1);
+                    Ty = fma(RK(y - 1), z, gd[y] * tby);
                 }
-                if (MODE == 0) {
-                    out[(long long)y * q.P + p] = Ty;
-                } else {
-                    // damped update Told + (1 - alpha)(T - Told) and the norms
-                    double *o = out + (long long)y * q.P + p;
-                    const double told = *o;
-                    const double df = Ty - told;
-                    const double nt = fma(oma, df, told);
-                    const float fd = abs_to_f32(df), fn = abs_to_f32(nt);
-                    f_diff = fmaf(fd, fd, f_diff);
-                    f_norm = fmaf(fn, fn, f_norm);
-                    *o = nt;
+                emit(op, MODE == 1 ? *op : 0.0, Ty, tby);
+            }
+            if (UNI && same < ng) {
+                // rows that share their coefficients (Simpson's rule on a
+                // uniform grid): the products with the step factors are formed
+                // once, four FP64 operations per row instead of five; the
+                // loads of four rows are issued together
+                const double cd = gd[same], c1 = g1[same] * r0, c2 = cs[same] * r02;
+                for (int y = same; y < ng; y += 4) {
+                    double tv[4], ov[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        tv[k] = y + k < ng ? tp[k * q.P] : 0.0;
+                        ov[k] = MODE == 1 && y + k < ng ? op[k * q.P] : 0.0;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (y + k >= ng) break;
+                        const double Ty = fma(cd, tv[k], fma(c1, tbm1, fma(c2, tbm2, r02 * Tm2)));
+                        emit(op + k * q.P, ov[k], Ty, tv[k]);
+                    }
+                    tp += 4 * q.P;
+                    op += 4 * q.P;
                 }
-                Tm2 = Tm1; Tm1 = Ty;
-                tbm2 = tbm1; tbm1 = tby;
             }
         } else {
             for (int x = 0; x < ng; x++) tb[x * QT + t] = tbar[(long long)x * q.P + p];
@@ -194,28 +286,7 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
             s_norm += (double)f_norm;
         }
     };
-    if (q.spin_half > 0) {
-        // spin blocks: only the spin-conserving elements move (the others
-        // are zero and stay zero); each (a, b, i) row holds them as one run
-        // of h consecutive j or none, and one warp takes one run
-        const int h = q.spin_half, n = q.no;
-        const long long rows = q.P / n;
-        const int lane = t % 32;
-        const long long tw = (long long)gridDim.x * (QT / 32);
-        for (long long u = blockIdx.x * (long long)(QT / 32) + t / 32; u < 2 * rows; u += tw) {
-            const long long r = u >> 1;
-            const int jh = (int)(u & 1);
-            const int i = (int)(r % n);
-            const long long ab = r / n;
-            const int b = (int)(ab % n), a = (int)(ab / n);
-            if ((a >= h) + (b >= h) != (i >= h) + jh) continue;
-            for (int jj = lane; jj < h; jj += 32) element(r * n + (long long)jh * h + jj);
-        }
-    } else {
-        for (long long p = blockIdx.x * (long long)QT + t; p < q.P;
-             p += (long long)gridDim.x * QT)
-            element(p);
-    }
+    quad_visit(q, element);
     if (MODE == 1) {
         // block reduction of the two sums (fixed order: deterministic)
         __shared__ double red[2][QT];
@@ -252,8 +323,8 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
 //     (relative error ~1e-14 of sum |G u|, far inside the parity bounds).
 // An element whose factors leave the safe range (non-finite u, or a bound on
 // |T_y| near the FP64 limit), and every element when D is given explicitly,
-// takes the FP64 path: exps, E_{ng-1-x} = 1/E_x on a grid symmetric about tc,
-// and FP64 FMAs.
+// takes the FP64 path: table exponentials, E_{ng-1-x} = 1/E_x on a grid
+// symmetric about tc, and FP64 FMAs.
 // ---------------------------------------------------------------------------
 struct DenseTabs {
     const double *v, *vi, *o, *oi;   // [ng][NL] / [ng][NR]: E and 1/E factors
@@ -347,7 +418,8 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
     double *G = ti + ng;                                   // [ng][ng] FP64
     float *Gh = reinterpret_cast<float *>(G + ng * ng);    // [ng][ng] FP32 high part
     float *Gl = Gh + ng * ng;                              //          low part
-    double *c0 = G + ng * ng + ng * ng;                    // [ng][QT]: u (FP64 or FP32 pair)
+    double *et = G + ng * ng + ng * ng;                    // 2^(j/64)
+    double *c0 = et + ETAB;                                // [ng][QT]: u (FP64 or FP32 pair)
     double *c1 = c0 + ng * QT;                             // [ng][QT]: E (FP64 path)
     for (int k = threadIdx.x; k < ng; k += QT) ti[k] = ti_g[k];
     for (int k = threadIdx.x; k < ng * ng; k += QT) {
@@ -357,6 +429,7 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
         Gh[k] = h;
         Gl[k] = (float)(g - (double)h);
     }
+    exp_table(et);
     __syncthreads();
     const double oma = 1.0 - q.alpha;
     const double tc = 0.5 * (ti[0] + ti[ng - 1]);
@@ -379,12 +452,10 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
         }
     };
 
-    auto element = [&](long long p) {
+    auto element = [&](long long p, int l, int r) {
         float f_diff = 0.f, f_norm = 0.f;
         bool table = tb_.v != nullptr;
         if (table) {
-            const long long l = p / tb_.NR;
-            const long long r = p - l * tb_.NR;
             // u_x = E_x tbar_x and the largest binary exponent among them.
             // Range tests and the scale are integer operations on exponent
             // fields: the FP64 pipe, GB300's scarce unit here, only takes the
@@ -395,8 +466,12 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
                 const double u = E * tbar[(long long)x * q.P + p];
                 c0[x * QT + t] = u;
                 umax_e = max(umax_e, dexp(u));        // inf / NaN: 0x7FF, refused below
+                if (q.mirror) {                       // 1 / E_{ng-1-x} = E_x
+                    c1[(ng - 1 - x) * QT + t] = E;
+                    eimax_e = max(eimax_e, dexp(E));
+                }
             }
-            for (int y = 0; y < ng; y++) {
+            for (int y = 0; y < ng && !q.mirror; y++) {
                 const double Ei = __ldg(tb_.vi + y * tb_.NL + l) * __ldg(tb_.oi + y * tb_.NR + r);
                 c1[y * QT + t] = Ei;
                 eimax_e = max(eimax_e, dexp(Ei));
@@ -435,15 +510,15 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
         }
         if (!table) {
             // FP64 path
-            const double d = denom(q, p, D, ev, eo);
+            const double d = denom(q, p, l, r, D, ev, eo);
             const int nx = q.symmetric ? (ng + 1) / 2 : ng;
             for (int x = 0; x < nx; x++) {
-                const double E = exp((ti[x] - tc) * d);
-                c1[x * QT + t] = E;
+                double E, Ei;
+                exp_tab2((ti[x] - tc) * d, et, E, Ei);
+                c1[x * QT + t] = q.symmetric ? E : Ei;
                 c0[x * QT + t] = E * tbar[(long long)x * q.P + p];
                 const int xm = ng - 1 - x;
                 if (q.symmetric && xm != x) {
-                    const double Ei = 1.0 / E;
                     c1[xm * QT + t] = Ei;
                     c0[xm * QT + t] = Ei * tbar[(long long)xm * q.P + p];
                 }
@@ -451,8 +526,7 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
             for (int y = 0; y < ng; y++) {
                 double acc = 0.0;
                 for (int x = 0; x < ng; x++) acc = fma(G[y * ng + x], c0[x * QT + t], acc);
-                const double Ty = q.symmetric ? acc * c1[(ng - 1 - y) * QT + t]
-                                              : acc / c1[y * QT + t];
+                const double Ty = acc * c1[(q.symmetric ? ng - 1 - y : y) * QT + t];
                 emit(p, y, Ty, f_diff, f_norm);
             }
         }
@@ -461,25 +535,7 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
             s_norm += (double)f_norm;
         }
     };
-    if (q.spin_half > 0) {
-        const int h = q.spin_half, n = q.no;
-        const long long rows = q.P / n;
-        const int lane = t % 32;
-        const long long tw = (long long)gridDim.x * (QT / 32);
-        for (long long u = blockIdx.x * (long long)(QT / 32) + t / 32; u < 2 * rows; u += tw) {
-            const long long rr = u >> 1;
-            const int jh = (int)(u & 1);
-            const int i = (int)(rr % n);
-            const long long ab = rr / n;
-            const int b = (int)(ab % n), a = (int)(ab / n);
-            if ((a >= h) + (b >= h) != (i >= h) + jh) continue;
-            for (int jj = lane; jj < h; jj += 32) element(rr * n + (long long)jh * h + jj);
-        }
-    } else {
-        for (long long p = blockIdx.x * (long long)QT + t; p < q.P;
-             p += (long long)gridDim.x * QT)
-            element(p);
-    }
+    quad_visit(q, element);
     if (MODE == 1) {
         __shared__ double red[2][QT];
         red[0][t] = s_diff;
@@ -509,7 +565,9 @@ __global__ void quad_single_kernel(QuadParams q, int ig, const double *__restric
                                    double *__restrict__ out) {
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < q.P;
          p += (long long)gridDim.x * blockDim.x) {
-        const double d = denom(q, p, D, ev, eo);
+        const int NR = q.rank == 2 ? q.no * q.no : q.no;
+        const int l = (int)(p / NR);
+        const double d = denom(q, p, l, (int)(p - (long long)l * NR), D, ev, eo);
         double acc = 0.0;
         for (int x = 0; x < q.ng; x++) {
             const double g = G[ig * q.ng + x];
@@ -545,9 +603,11 @@ __global__ void reduce_pairs_kernel(const double *__restrict__ partial, int n,
     }
 }
 
-// Host-side analysis of the grid: recurrence step and uniform spacing.
+// Host-side analysis of the grid: recurrence step, uniform spacing, and (step
+// 2) the first row from which the chained rows' coefficients are the same.
 void analyse_grid(int ng, const double *ti, const double *G, int full, int *step,
-                  int *uniform) {
+                  int *uniform, int *same) {
+    *same = ng;
     *uniform = 1;
     for (int k = 1; k + 1 < ng; k++) {
         double d0 = ti[1] - ti[0], dk = ti[k + 1] - ti[k];
@@ -563,22 +623,35 @@ void analyse_grid(int ng, const double *ti, const double *G, int full, int *step
         for (int y = s; y < ng && ok; y++)
             for (int x = 0; x < y - s && ok; x++)
                 if (G[y * ng + x] != G[(y - s) * ng + x]) ok = false;
-        if (ok) { *step = s; return; }
+        if (!ok) continue;
+        *step = s;
+        if (s == 2) {
+            auto row = [&](int y, int k) {
+                return k == 0 ? G[y * ng + y] : k == 1 ? G[y * ng + y - 1]
+                              : G[y * ng + y - 2] - G[(y - 2) * ng + y - 2];
+            };
+            int y = ng - 1;
+            while (y > 2 && row(y - 1, 0) == row(ng - 1, 0) && row(y - 1, 1) == row(ng - 1, 1) &&
+                   row(y - 1, 2) == row(ng - 1, 2))
+                y--;
+            *same = std::max(2, y);
+        }
+        return;
     }
 }
 
-// ti, G, cs, g1, gd; then the per-thread columns: step factors (general
+// ti, G, cs, g1, gd, the exponential's table; then the per-thread columns: step factors (general
 // lower-triangular path on a non-uniform grid), inputs (general and dense
 // paths), and the dense path's scale factors
 size_t quad_smem(int ng, int uniform, int step, int full) {
-    return sizeof(double) * (4 * ng + ng * ng + ((uniform || full) ? 0 : ng * QT) +
+    return sizeof(double) * (4 * ng + ng * ng + ETAB + ((uniform || full) ? 0 : ng * QT) +
                              (step > 0 ? 0 : ng * QT) + (full ? ng * QT : 0));
 }
 
-// ti[x] + ti[ng-1-x] equal for every x (to rounding)
-int grid_symmetric(int ng, const double *ti) {
+// ti[x] + ti[ng-1-x] equal for every x (to `rel` of the range)
+int grid_symmetric(int ng, const double *ti, double rel) {
     const double c = ti[0] + ti[ng - 1];
-    const double tol = 1e-13 * std::max(std::fabs(ti[ng - 1] - ti[0]), 1e-300);
+    const double tol = rel * std::max(std::fabs(ti[ng - 1] - ti[0]), 1e-300);
     for (int x = 0; x < ng; x++)
         if (std::fabs(ti[x] + ti[ng - 1 - x] - c) > tol) return 0;
     return 1;
@@ -589,7 +662,7 @@ int grid_symmetric(int ng, const double *ti) {
 namespace {
 
 size_t dense_smem(int ng) {
-    return sizeof(double) * ((size_t)ng + 2 * (size_t)ng * ng + 2 * (size_t)ng * QT);
+    return sizeof(double) * ((size_t)ng + 2 * (size_t)ng * ng + ETAB + 2 * (size_t)ng * QT);
 }
 
 // The dense-G integral: pair tables of the orbital energies (when given),
@@ -680,8 +753,9 @@ int kv_quad_launch(kvft_ctx *ctx, int mode, int ng, long long P, int rank, int n
     // spin blocks: only the spin-conserving elements are integrated (the
     // solver's passes, which read no other; callers pass 0 otherwise)
     q.spin_half = (rank == 2 && nv == no && nv == 2 * spin_half) ? spin_half : 0;
-    analyse_grid(ng, hti, hG, full, &q.step, &q.uniform);
-    q.symmetric = grid_symmetric(ng, hti);
+    analyse_grid(ng, hti, hG, full, &q.step, &q.uniform, &q.same);
+    q.symmetric = grid_symmetric(ng, hti, 1e-13);
+    q.mirror = grid_symmetric(ng, hti, 1e-15);
     if (full) return quad_dense_launch(ctx, mode, q, tbar, ti, hti, G, D, ev, eo, out, res);
     size_t smem = quad_smem(ng, q.uniform, q.step, q.full);
     long long blocks = (P + QT - 1) / QT;

@@ -450,10 +450,6 @@ constexpr int AA_T = 256;
 constexpr int AA_U = 4;     // elements per thread per batch (all loads before any store)
 constexpr int AA_BLOCKS = 3; // resident blocks per SM (at most 85 registers a thread)
 
-// The six spin patterns (sa, sb, si, sj) with sa + sb = si + sj (0 = alpha,
-// 1 = beta), four bits each: sa | sb << 1 | si << 2 | sj << 3.
-constexpr unsigned AA_PATTERNS = 0u | 15u << 4 | 10u << 8 | 6u << 12 | 9u << 16 | 5u << 20;
-
 // Calls f(base, o, cb, cs, cnt) with batches of up to AA_U elements: the
 // amplitude index base + o[u] and the compact index cb + u cs (the position
 // in the visit order, which the FP32 history uses), u < cnt valid.  T2 with
@@ -474,7 +470,7 @@ __device__ __forceinline__ void aa_visit(const AaSeg &g, F f) {
             const int rem = (int)(it - y * 6 * hh);
             const int pat = rem / hh, ab = rem - pat * hh;
             const int a1 = ab / h, b1 = ab - a1 * h;
-            const unsigned c = AA_PATTERNS >> (4 * pat);
+            const unsigned c = KV_SPIN_PATTERNS >> (4 * pat);
             const int a = a1 + (int)(c & 1u) * h, b = b1 + (int)((c >> 1) & 1u) * h;
             const long long base = y * g.P + (((long long)a * n + b) * n + (long long)((c >> 2) & 1u) * h) * n +
                                    (long long)((c >> 3) & 1u) * h;
@@ -659,7 +655,7 @@ __host__ __device__ __forceinline__ long long spin_item_base(long long it, long 
     const int rem = (int)(it - y * 6 * hh);
     const int pat = rem / hh, ab = rem - pat * hh;
     const int a1 = ab / h, b1 = ab - a1 * h;
-    const unsigned c = AA_PATTERNS >> (4 * pat);
+    const unsigned c = KV_SPIN_PATTERNS >> (4 * pat);
     const long long a = a1 + (long long)(c & 1u) * h, b = b1 + (long long)((c >> 1) & 1u) * h;
     return y * P + ((a * n + b) * n + (long long)((c >> 2) & 1u) * h) * n +
            (long long)((c >> 3) & 1u) * h;

@@ -1,0 +1,78 @@
+"""The tau integral's exponentials and its walk over the spin-conserving
+elements."""
+import numpy
+import pytest
+
+from kelvin_gb300 import quadrature, systems
+from kelvin_gb300.cc_utils import DeviceSolver
+from kelvin_gb300.quadrature import ft_quad
+from oracle import ft_ccsd as oft
+from oracle import ft_utils
+from oracle import quadrature as oq
+
+pytestmark = pytest.mark.gpu
+
+
+def test_exponential_range(ctx):
+    """One weight per element: T[1] = G[1,0] exp(-delta d) tbar[0].  Arguments
+    over the table's range, at its edges (|x| = 700, where the library function
+    takes over), large ones that overflow or vanish, zero, and n ln2/128 (the
+    largest remainders).  Tolerance: one unit in the last place for each of the
+    two exponentials and half for each of the two products."""
+    x = numpy.concatenate((numpy.linspace(-720.0, 720.0, 4001),
+                           numpy.arange(-64, 65) * numpy.log(2.0) / 128.0,
+                           [700.0, -700.0, numpy.nextafter(700.0, 0.0), 0.0, -0.0, 800.0, -800.0]))
+    n = x.shape[0]
+    ti, g, G = quadrature.ft_quad(2, 1.0, "lin")
+    t = numpy.zeros((2, 1, n))
+    t[0] = 1.0
+    out = quadrature.int_tbar1(2, t, ti, -x.reshape(1, n), G)
+    with numpy.errstate(over="ignore"):
+        ref = 0.5 * numpy.exp(x)
+    fin = numpy.isfinite(ref)
+    assert numpy.array_equal(numpy.isfinite(out[1, 0]), fin)
+    assert (abs(out[1, 0][fin] - ref[fin]) <= 3.0 * 2.0 ** -52 * ref[fin] + 5e-324).all()
+
+
+@pytest.mark.parametrize("quad,ng,tol", [("lin", 2, 1e-13), ("lin", 3, 1e-13), ("lin", 5, 1e-13),
+                                         ("lin", 8, 1e-13), ("lin", 17, 1e-13), ("mid", 9, 1e-13),
+                                         ("ln", 6, 1e-13), ("gl", 7, 1e-12), ("gl", 8, 1e-12)])
+def test_int_tbar_rectangular(ctx, quad, ng, tol):
+    """Rows with shared coefficients (and the ones before them), the mapped
+    grid, dense grids with and without a middle node; nv != no."""
+    rng = numpy.random.default_rng(ng)
+    nv, no = 5, 3
+    ti, g, G = ft_quad(ng, 2.0, quad)
+    D = rng.standard_normal((nv, nv, no, no)) * 2.0
+    t = rng.standard_normal((ng, nv, nv, no, no))
+    full = quad == "gl"
+    ref = oq.int_tbar2(ng, t, ti, D, G, full=full)
+    out = quadrature.int_tbar2(ng, t, ti, D, G, full=full)
+    assert abs(out - ref).max() <= tol * max(1.0, abs(ref).max())
+
+
+# alpha halves of one, several and partial units of 32 elements per quadrant,
+# and of several assembly tiles (h > 64 would need 130 spin orbitals: the tile
+# arithmetic is the same for every quadrant)
+@pytest.mark.parametrize("pw,quad", [(1, "lin"), (3, "gl"), (6, "lin"), (11, "gl")])
+def test_spin_blocked_step_vs_oracle(ctx, pw, quad):
+    s = systems.ueg_recipe(1.0 if pw == 1 else 2, 2.0, pw, 0.5)
+    beta, ng = 1.0 / s.T, 5
+    en = s.g_energies_tot()
+    ti, g, G = ft_quad(ng, beta, quad)
+    sv = DeviceSolver.from_system(ctx, en, s.g_fock_tot(), s.g_aint_tot(), beta, s.mu, ti, g, G)
+    try:
+        sv.full = quad == "gl"
+        assert sv.spin_blocks() == pw
+        sv.guess(1)
+        x1, x2 = sv.amplitudes()
+        E, _ = sv.step(0.3)
+        T1, T2 = sv.amplitudes()
+    finally:
+        sv.close()
+    F, I = oft.ft_integrals(s.g_fock_tot(), s.g_aint_tot(), en, beta, s.mu)
+    D1, D2 = ft_utils.D1(en, en), ft_utils.D2(en, en)
+    r1, r2 = oft.ccsd_stanton(F, I, x1, x2, D1, D2, ti, ng, G, full=quad == "gl")
+    assert abs(T1 - (0.3 * x1 + 0.7 * r1)).max() <= 1e-12 * max(1.0, abs(r1).max())
+    assert abs(T2 - (0.3 * x2 + 0.7 * r2)).max() <= 1e-12 * max(1.0, abs(r2).max())
+    assert abs(E - oft.ft_cc_energy(T1, T2, F.ov, I.oovv, g, beta)) <= 1e-12
