@@ -9,112 +9,174 @@
 namespace {
 
 constexpr int TILE = 32;
+constexpr int EN_T = 256;
 
-// One block per 32 x 32 tile of (a,b) x (i,j); thread (tx, ty) takes i,j =
-// ij0 + tx and the four (a,b) rows ty + 8k.  Per element and tau point two
-// FP64 FMAs: s1 += g_y T2_y and s2 += (g_y T1_y[a,i]) T1_y[b,j], the first
-// factor of the second from a shared table over the few (a, i) values of the
-// tile, filled for a chunk of tau points at a time; the element's weight is
-// then s1/4 + s2/2.
-constexpr int WTAB = 1024;                  // doubles of the (y, a, i) table
-
-__global__ void __launch_bounds__(256, 2)
-energy2_kernel(int ng, int nv, int no, const double *__restrict__ T1,
-               const double *__restrict__ T2, const double *__restrict__ eri,
-               const double *__restrict__ g, int qterm, int sh, double *__restrict__ partial) {
-    __shared__ double E[TILE][TILE + 1];     // [ij][ab]
-    __shared__ double red[256];
-    __shared__ double gs[WTAB / 4];          // g_y of the chunk
-    __shared__ double wt[WTAB];              // [y][a - a_lo][i - i_lo]: g_y T1_y[a,i]
-    const long long V2 = (long long)nv * nv, O2 = (long long)no * no;
-    const long long ab0 = (long long)blockIdx.y * TILE, ij0 = (long long)blockIdx.x * TILE;
-    const int t = threadIdx.x, tx = t % TILE, ty = t / TILE;   // ty in [0, 8)
-    if (sh > 0) {
-        // spin blocks: a tile whose (a,b) spin sums and (i,j) spin sums never
-        // meet holds only zero amplitudes and adds nothing
-        __shared__ int live;
-        if (t < 32) {
-            const long long ab = ab0 + t, ij = ij0 + t;
-            unsigned sab = 0, sij = 0;
-            if (ab < V2) sab = 1u << ((int)(ab / nv >= sh) + (int)(ab % nv >= sh));
-            if (ij < O2) sij = 1u << ((int)(ij / no >= sh) + (int)(ij % no >= sh));
-            sab = __reduce_or_sync(0xffffffffu, sab);
-            sij = __reduce_or_sync(0xffffffffu, sij);
-            if (t == 0) live = (sab & sij) != 0;
-        }
-        __syncthreads();
-        if (!live) {
-            if (t == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = 0.0;
-            return;
-        }
-    }
-    for (int r = ty; r < TILE; r += 8) {
-        long long ij = ij0 + r, ab = ab0 + tx;
-        E[r][tx] = (ij < O2 && ab < V2) ? eri[ij * V2 + ab] : 0.0;
-    }
-    const long long ab_hi = min(ab0 + TILE, V2) - 1, ij_hi = min(ij0 + TILE, O2) - 1;
-    const int a_lo = (int)(ab0 / nv), na = (int)(ab_hi / nv) - a_lo + 1;
-    const int i_lo = (int)(ij0 / no), ni = (int)(ij_hi / no) - i_lo + 1;
-    const int yc = qterm ? max(1, min(WTAB / 4, WTAB / (na * ni))) : WTAB / 4;
-    const long long ij = ij0 + tx;
-    const bool live = ij < O2;
-    const int i = live ? (int)(ij / no) : 0, j = live ? (int)(ij % no) : 0;
-    int ka[4], kb[4];
-    long long kab[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const long long ab = min(ab0 + ty + 8 * k, ab_hi);
-        kab[k] = ab;
-        ka[k] = (int)(ab / nv);
-        kb[k] = (int)(ab % nv);
-    }
-    double s1[4] = {0.0, 0.0, 0.0, 0.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};
-    const long long sy = (long long)nv * no;
-    for (int y0 = 0; y0 < ng; y0 += yc) {
-        const int ny = min(yc, ng - y0);
-        __syncthreads();
-        for (int x = t; x < ny; x += 256) gs[x] = g[y0 + x];
-        if (qterm)
-            for (int x = t; x < ny * na * ni; x += 256) {
-                const int yy = x / (na * ni), r = x % (na * ni);
-                const int a = a_lo + r / ni, ii = i_lo + r % ni;
-                wt[x] = g[y0 + yy] * T1[(y0 + yy) * sy + (long long)a * no + ii];
-            }
-        __syncthreads();
-        if (!live) continue;
-        const double *t2 = T2 + (long long)y0 * V2 * O2 + ij;
-        for (int yy = 0; yy < ny; yy++) {
-            const double gy = gs[yy];
-#pragma unroll
-            for (int k = 0; k < 4; k++) s1[k] = fma(gy, t2[kab[k] * O2], s1[k]);
-            t2 += V2 * O2;
-        }
-        if (qterm) {
-            const double *u = T1 + (long long)y0 * sy + j;
-            const double *w = wt + (i - i_lo);
-            for (int yy = 0; yy < ny; yy++) {
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    s2[k] = fma(w[(ka[k] - a_lo) * ni], u[(long long)kb[k] * no], s2[k]);
-                u += sy;
-                w += na * ni;
-            }
-        }
-    }
-    double acc = 0.0;
-    if (live)
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int r = ty + 8 * k;
-            if (ab0 + r < V2) acc = fma(fma(0.25, s1[k], 0.5 * s2[k]), E[tx][r], acc);
-        }
+// Block sum of acc (fixed order) into partial[blockIdx.x]; the last block to
+// arrive adds the partials in index order and writes (sum) inv_beta to *res, so
+// one launch gives a deterministic total.  *count is zero before the launch
+// and zero again after it.
+__device__ __forceinline__ void finish_sum(double acc, double *red, double *partial,
+                                           unsigned *count, double inv_beta, double *res) {
+    __shared__ bool last;
+    const int t = threadIdx.x;
     red[t] = acc;
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
+    for (int s = EN_T / 2; s > 0; s >>= 1) {
         if (t < s) red[t] += red[t + s];
         __syncthreads();
     }
-    if (t == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+    if (t == 0) {
+        partial[blockIdx.x] = red[0];
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0.0;
+    for (int k = t; k < (int)gridDim.x; k += EN_T) a += __ldcg(partial + k);
+    red[t] = a;
+    __syncthreads();
+    for (int s = EN_T / 2; s > 0; s >>= 1) {
+        if (t < s) red[t] += red[t + s];
+        __syncthreads();
+    }
+    if (t == 0) {
+        *res = red[0] * inv_beta;
+        *count = 0;
+    }
+}
+
+// This thread's share of sum_y g_y sum_ai T1_y[a,i] f[i,a]
+__device__ __forceinline__ double energy1(int ng, int nv, int no, const double *T1,
+                                          const double *f, const double *g) {
+    double acc = 0.0;
+    for (int k = blockIdx.x * EN_T + threadIdx.x; k < nv * no; k += gridDim.x * EN_T) {
+        const int a = k / no, i = k - a * no;
+        double s = 0.0;
+        for (int y = 0; y < ng; y++) s = fma(g[y], T1[(long long)y * nv * no + k], s);
+        acc = fma(s, f[i * nv + a], acc);
+    }
+    return acc;
+}
+
+// Blocks walk 32 x 32 tiles of (a,b) x (i,j); thread (tx, ty) takes i,j = ij0 +
+// tx and the four (a,b) rows ty + 8k.  Per element and tau point one FP64 FMA,
+// s1 += g_y T2_y, and on half of the elements a second: M[ai,bj] = sum_y (g_y
+// T1_y[a,i]) T1_y[b,j] is symmetric in its two pairs, so only the rows a <= b
+// form it, and those with a < b take it against eri[ij,ab] + eri[ji,ba] (66
+// spin orbitals, 16 points: 1.43 -> 1.16 ms; the FP64 pipe's floor is 1.0, the
+// memory's 0.38).  The first factors come from a shared table over the few
+// (a, i) of the tile, filled for a chunk of tau points at a time.
+constexpr int WTAB = 1024;                  // doubles of the (y, a, i) table
+
+__global__ void __launch_bounds__(EN_T, 3)
+energy2_kernel(int ng, int nv, int no, const double *__restrict__ T1,
+               const double *__restrict__ T2, const double *__restrict__ f,
+               const double *__restrict__ eri, const double *__restrict__ g, int qterm, int sh,
+               int gx, int tiles, double *partial, unsigned *count, double inv_beta,
+               double *res) {
+    __shared__ double E[TILE][TILE + 1];     // [ij][ab]
+    __shared__ double red[EN_T];
+    __shared__ double gs[WTAB / 4];          // g_y of the chunk
+    __shared__ double wt[WTAB];              // [y][a - a_lo][i - i_lo]: g_y T1_y[a,i]
+    __shared__ int tile_live;
+    const long long V2 = (long long)nv * nv, O2 = (long long)no * no;
+    const int t = threadIdx.x, tx = t % TILE, ty = t / TILE;   // ty in [0, 8)
+    double acc = energy1(ng, nv, no, T1, f, g);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const long long ab0 = (long long)(tile / gx) * TILE, ij0 = (long long)(tile % gx) * TILE;
+        __syncthreads();                     // the last tile's tables are used up
+        if (sh > 0) {
+            // spin blocks: a tile whose (a,b) spin sums and (i,j) spin sums never
+            // meet holds only zero amplitudes and adds nothing
+            if (t < 32) {
+                const long long ab = ab0 + t, ij = ij0 + t;
+                unsigned sab = 0, sij = 0;
+                if (ab < V2) sab = 1u << ((int)(ab / nv >= sh) + (int)(ab % nv >= sh));
+                if (ij < O2) sij = 1u << ((int)(ij / no >= sh) + (int)(ij % no >= sh));
+                sab = __reduce_or_sync(0xffffffffu, sab);
+                sij = __reduce_or_sync(0xffffffffu, sij);
+                if (t == 0) tile_live = (sab & sij) != 0;
+            }
+            __syncthreads();
+            if (!tile_live) continue;
+        }
+        for (int r = ty; r < TILE; r += 8) {
+            const long long ij = ij0 + r, ab = ab0 + tx;
+            E[r][tx] = (ij < O2 && ab < V2) ? eri[ij * V2 + ab] : 0.0;
+        }
+        const long long ab_hi = min(ab0 + TILE, V2) - 1, ij_hi = min(ij0 + TILE, O2) - 1;
+        const int a_lo = (int)(ab0 / nv), na = (int)(ab_hi / nv) - a_lo + 1;
+        const int i_lo = (int)(ij0 / no), ni = (int)(ij_hi / no) - i_lo + 1;
+        const int yc = qterm ? max(1, min(WTAB / 4, WTAB / (na * ni))) : WTAB / 4;
+        const long long ij = ij0 + tx;
+        const bool live = ij < O2;
+        const int i = live ? (int)(ij / no) : 0, j = live ? (int)(ij - (long long)i * no) : 0;
+        // row k of this thread: ab0 + ty + 8 k, the last row again past the end
+        const int row0 = ty, rows = (int)(ab_hi - ab0);
+        auto row = [&](int k) { return (long long)min(row0 + 8 * k, rows); };
+        double s1[4] = {0.0, 0.0, 0.0, 0.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};
+        const long long sy = (long long)nv * no;
+        for (int y0 = 0; y0 < ng; y0 += yc) {
+            const int ny = min(yc, ng - y0);
+            __syncthreads();
+            for (int x = t; x < ny; x += EN_T) gs[x] = g[y0 + x];
+            if (qterm)
+                for (int x = t; x < ny * na * ni; x += EN_T) {
+                    const int yy = x / (na * ni), r = x % (na * ni);
+                    const int a = a_lo + r / ni, ii = i_lo + r % ni;
+                    wt[x] = g[y0 + yy] * T1[(y0 + yy) * sy + (long long)a * no + ii];
+                }
+            __syncthreads();
+            if (!live) continue;
+            const double *t2 = T2 + (long long)y0 * V2 * O2 + ab0 * O2 + ij;
+            // four tau points of loads in flight
+            int yy = 0;
+            for (; yy + 4 <= ny; yy += 4) {
+                double v[4][4];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) v[q][k] = t2[q * V2 * O2 + row(k) * O2];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+#pragma unroll
+                    for (int k = 0; k < 4; k++) s1[k] = fma(gs[yy + q], v[q][k], s1[k]);
+                t2 += 4 * V2 * O2;
+            }
+            for (; yy < ny; yy++) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) s1[k] = fma(gs[yy], t2[row(k) * O2], s1[k]);
+                t2 += V2 * O2;
+            }
+            if (qterm) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int ab = (int)(ab0 + row(k)), a = ab / nv, b = ab - a * nv;
+                    if (a > b) continue;                       // warp-uniform
+                    const double *u = T1 + (long long)y0 * sy + (long long)b * no + j;
+                    const double *w = wt + (a - a_lo) * ni + (i - i_lo);
+#pragma unroll 8
+                    for (int z = 0; z < ny; z++) s2[k] = fma(w[z * na * ni], u[z * sy], s2[k]);
+                }
+            }
+        }
+        if (live)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int r = ty + 8 * k;
+                if (ab0 + r >= V2) continue;
+                const double e = E[tx][r];
+                acc = fma(0.25 * s1[k], e, acc);
+                const int ab = (int)(ab0 + r), a = ab / nv, b = ab - a * nv;
+                if (!qterm || a > b) continue;
+                const double e2 = a < b ? eri[((long long)j * no + i) * V2 + (long long)b * nv + a]
+                                        : 0.0;
+                acc = fma(0.5 * s2[k], e + e2, acc);
+            }
+    }
+    finish_sum(acc, red, partial, count, inv_beta, res);
 }
 
 // Spin blocks (nv = no = 2h): only the spin-conserving (a, b, i, j) carry
@@ -124,95 +186,60 @@ energy2_kernel(int ng, int nv, int no, const double *__restrict__ T1,
 // eri[i][j][a][b] are read along b into shared memory and its amplitudes
 // T2_y[a][b][i][j] along j, so both streams are coalesced and no element
 // outside the conserving blocks is read.  The T1 T1 term vanishes unless s_b
-// = s_j (T1 is spin-diagonal), i.e. on the s_a = s_i items.  One partial sum
-// per item, reduced in a fixed order.
+// = s_j (T1 is spin-diagonal), i.e. on the s_a = s_i items.
 constexpr int ESP_HMAX = 96;                 // h x (h + 1) doubles of shared memory
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(EN_T)
 energy2_spin_kernel(int ng, int n, int h, const double *__restrict__ T1,
-                    const double *__restrict__ T2, const double *__restrict__ eri,
-                    const double *__restrict__ g, int qterm, long long items,
-                    double *__restrict__ partial) {
+                    const double *__restrict__ T2, const double *__restrict__ f,
+                    const double *__restrict__ eri, const double *__restrict__ g, int qterm,
+                    long long items, double *partial, unsigned *count, double inv_beta,
+                    double *res) {
     extern __shared__ double E[];            // [h][h + 1]: E[j1][b1]
-    __shared__ double red[256];
+    __shared__ double red[EN_T];
     __shared__ double gs[64], w[64];         // g_y and g_y T1_y[a][i]
     const int t = threadIdx.x, hh = h * h, ld = h + 1;
     const long long n2 = (long long)n * n, P = n2 * n2;
+    double acc = energy1(ng, n, n, T1, f, g);
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
         const int q = (int)(it & 1);
         const long long ai = it >> 1;
         const int a = (int)(ai / n), i = (int)(ai - (long long)a * n);
         const int sa = a >= h, si = i >= h;
-        double acc = 0.0;
-        if (sa == si || q == 0) {            // block-uniform
-            const int sb = sa == si ? q : si, sj = sa == si ? q : sa;
-            const bool tt = qterm && sa == si;
-            __syncthreads();                 // E, gs, w of the last item are used up
-            for (int x = t; x < ng; x += 256) {
-                gs[x] = g[x];
-                w[x] = tt ? g[x] * T1[(long long)x * n2 + (long long)a * n + i] : 0.0;
-            }
-            for (int x = t; x < hh; x += 256) {
-                const int j1 = x / h, b1 = x - j1 * h;
-                E[j1 * ld + b1] = eri[(((long long)i * n + sj * h + j1) * n + a) * n + sb * h + b1];
-            }
-            __syncthreads();
-            const long long base = ((long long)a * n + sb * h) * n2 + (long long)i * n + sj * h;
-            for (int x = t; x < hh; x += 256) {
-                const int b1 = x / h, j1 = x - b1 * h;
-                const double *t2 = T2 + base + (long long)b1 * n2 + j1;
-                double s1 = 0.0, s2 = 0.0;
-                for (int y = 0; y < ng; y++) s1 = fma(gs[y], t2[(long long)y * P], s1);
-                if (tt) {
-                    const double *u = T1 + (long long)(sb * h + b1) * n + sj * h + j1;
-                    for (int y = 0; y < ng; y++) s2 = fma(w[y], u[(long long)y * n2], s2);
-                }
-                acc = fma(fma(0.25, s1, 0.5 * s2), E[j1 * ld + b1], acc);
-            }
+        if (sa != si && q) continue;         // block-uniform
+        const int sb = sa == si ? q : si, sj = sa == si ? q : sa;
+        const bool tt = qterm && sa == si;
+        __syncthreads();                     // E, gs, w of the last item are used up
+        for (int x = t; x < ng; x += EN_T) {
+            gs[x] = g[x];
+            w[x] = tt ? g[x] * T1[(long long)x * n2 + (long long)a * n + i] : 0.0;
         }
-        red[t] = acc;
+        for (int x = t; x < hh; x += EN_T) {
+            const int j1 = x / h, b1 = x - j1 * h;
+            E[j1 * ld + b1] = eri[(((long long)i * n + sj * h + j1) * n + a) * n + sb * h + b1];
+        }
         __syncthreads();
-        for (int st = 128; st > 0; st >>= 1) {
-            if (t < st) red[t] += red[t + st];
-            __syncthreads();
+        const long long base = ((long long)a * n + sb * h) * n2 + (long long)i * n + sj * h;
+        for (int x = t; x < hh; x += EN_T) {
+            const int b1 = x / h, j1 = x - b1 * h;
+            const double *t2 = T2 + base + (long long)b1 * n2 + j1;
+            double s1 = 0.0, s2 = 0.0;
+#pragma unroll 4
+            for (int y = 0; y < ng; y++) s1 = fma(gs[y], t2[(long long)y * P], s1);
+            if (tt) {
+                const double *u = T1 + (long long)(sb * h + b1) * n + sj * h + j1;
+#pragma unroll 4
+                for (int y = 0; y < ng; y++) s2 = fma(w[y], u[(long long)y * n2], s2);
+            }
+            acc = fma(fma(0.25, s1, 0.5 * s2), E[j1 * ld + b1], acc);
         }
-        if (t == 0) partial[it] = red[0];
     }
+    finish_sum(acc, red, partial, count, inv_beta, res);
 }
 
-__global__ void energy1_kernel(int ng, int nv, int no, const double *__restrict__ T1,
-                               const double *__restrict__ f, const double *__restrict__ g,
-                               double *__restrict__ out) {
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int k = threadIdx.x; k < nv * no; k += 256) {
-        const int a = k / no, i = k % no;
-        double s = 0.0;
-        for (int y = 0; y < ng; y++) s = fma(g[y], T1[(long long)y * nv * no + k], s);
-        acc = fma(s, f[i * nv + a], acc);
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = red[0];
-}
-
-__global__ void energy_final_kernel(const double *__restrict__ partial, int n,
-                                    const double *__restrict__ e1, double inv_beta,
-                                    double *__restrict__ res) {
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int k = threadIdx.x; k < n; k += 256) acc += partial[k];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *res = (e1[0] + red[0]) * inv_beta;
+// Blocks of the dense form: two per SM resident, eight waves of them at most
+int energy_grid(int sm_count, long long tiles) {
+    return (int)std::max(1LL, std::min(tiles, (long long)sm_count * 16));
 }
 
 }  // namespace
@@ -222,14 +249,18 @@ int kv_energy(kvft_ctx *ctx, int ng, int nv, int no, const double *T1, const dou
               const double *f, const double *eri, const double *g, double beta, int qterm,
               double *dres, int spin_half) {
     const long long V2 = (long long)nv * nv, O2 = (long long)no * no;
-    dim3 grid((unsigned)((O2 + TILE - 1) / TILE), (unsigned)((V2 + TILE - 1) / TILE));
+    const long long gx = (O2 + TILE - 1) / TILE, gy = (V2 + TILE - 1) / TILE;
     const int sh = (nv == no && nv == 2 * spin_half) ? spin_half : 0;
     const bool spin = sh > 0 && sh <= ESP_HMAX && ng <= 64;
     // spin items (a, i, q), or the 32 x 32 tiles of the dense kernel
-    const long long nblk = spin ? 2LL * nv * nv : (long long)grid.x * grid.y;
+    const long long work = spin ? 2LL * nv * nv : gx * gy;
+    if (work > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "energy: too many tiles");
+    const int grid = spin ? (int)std::min<long long>(work, (long long)ctx->sm_count * 8)
+                          : energy_grid(ctx->sm_count, work);
     void *part = nullptr;
-    KV_TRY(kv_scratch(ctx, "energy_partial", sizeof(double) * (nblk + 1), &part));
+    KV_TRY(kv_scratch(ctx, "energy_partial", sizeof(double) * grid, &part));
     double *pp = (double *)part;
+    unsigned *count = (unsigned *)ctx->dflag + KV_FLAG_ENERGY;
     // algorithmic bytes: T2 (all tau points) + eri + T1; with spin blocks the
     // spin-conserving elements of T2 and eri
     KvProfScope prof(ctx, KV_CAT_ENERGY,
@@ -244,18 +275,13 @@ int kv_energy(kvft_ctx *ctx, int ng, int nv, int no, const double *T1, const dou
                                                (int)(sizeof(double) * ESP_HMAX * (ESP_HMAX + 1))));
             attr = true;
         }
-        const int gb = (int)std::min<long long>(nblk, (long long)ctx->sm_count * 8);
-        energy2_spin_kernel<<<gb, 256, smem, ctx->stream>>>(ng, nv, sh, T1, T2, eri, g, qterm,
-                                                           nblk, pp);
-        KV_TRY(kv_launch_check(ctx, "energy2_spin"));
-    } else {
-        energy2_kernel<<<grid, 256, 0, ctx->stream>>>(ng, nv, no, T1, T2, eri, g, qterm, sh, pp);
-        KV_TRY(kv_launch_check(ctx, "energy2"));
+        energy2_spin_kernel<<<grid, EN_T, smem, ctx->stream>>>(ng, nv, sh, T1, T2, f, eri, g, qterm,
+                                                              work, pp, count, 1.0 / beta, dres);
+        return kv_launch_check(ctx, "energy2_spin");
     }
-    energy1_kernel<<<1, 256, 0, ctx->stream>>>(ng, nv, no, T1, f, g, pp + nblk);
-    KV_TRY(kv_launch_check(ctx, "energy1"));
-    energy_final_kernel<<<1, 256, 0, ctx->stream>>>(pp, (int)nblk, pp + nblk, 1.0 / beta, dres);
-    return kv_launch_check(ctx, "energy_final");
+    energy2_kernel<<<grid, EN_T, 0, ctx->stream>>>(ng, nv, no, T1, T2, f, eri, g, qterm, sh, (int)gx,
+                                                   (int)work, pp, count, 1.0 / beta, dres);
+    return kv_launch_check(ctx, "energy2");
 }
 
 extern "C" int kvft_ft_cc_energy(kvft_ctx *ctx, int ng, int nv, int no, const double *T1,
@@ -297,6 +323,7 @@ extern "C" int kvft_ft_cc_energy(kvft_ctx *ctx, int ng, int nv, int no, const do
 
 namespace {
 constexpr int NOALLOC_MAX_TILES = 32767;   // 32 x 32 tiles of (a,b) x (i,j)
+// partial sums of the blocks, and the arrival count in the last word
 __device__ __align__(256) double g_energy_scratch[NOALLOC_MAX_TILES + 1];
 std::mutex g_energy_scratch_mu;
 double *g_energy_scratch_ptr[64] = {};     // device address of the array, per device
@@ -327,24 +354,21 @@ extern "C" int kvft_ft_cc_energy_noalloc(void *stream, int ng, int nv, int no,
         scratch = g_energy_scratch_ptr[dev];
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const int nblk = (int)(gx * gy);
-    // each launch's own status (cudaLaunchKernel reports that launch), so
-    // that an earlier unrelated error left on the thread is not returned as
-    // this call's
-    int sh = 0;
-    double *part1 = scratch + nblk;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return KVFT_EDEVICE;
+    // the launch's own status (cudaLaunchKernel reports that launch), so that
+    // an earlier unrelated error left on the thread is not returned as this
+    // call's
+    int sh = 0, igx = (int)gx, tiles = (int)(gx * gy);
+    unsigned *count = (unsigned *)(scratch + NOALLOC_MAX_TILES);
     double inv_beta = 1.0 / beta;
-    void *a2[] = {&ng, &nv, &no, (void *)&T1, (void *)&T2, (void *)&eri, (void *)&g, &qterm,
-                  &sh, &scratch};
-    void *a1[] = {&ng, &nv, &no, (void *)&T1, (void *)&f, (void *)&g, &part1};
-    int nb = nblk;
-    void *af[] = {&scratch, &nb, &part1, &inv_beta, &omega_dev};
-    if (cudaLaunchKernel((const void *)energy2_kernel, dim3((unsigned)gx, (unsigned)gy),
-                         dim3(256), a2, 0, st) != cudaSuccess ||
-        cudaLaunchKernel((const void *)energy1_kernel, dim3(1), dim3(256), a1, 0, st) !=
-            cudaSuccess ||
-        cudaLaunchKernel((const void *)energy_final_kernel, dim3(1), dim3(256), af, 0, st) !=
-            cudaSuccess)
+    void *a2[] = {&ng, &nv, &no, (void *)&T1, (void *)&T2, (void *)&f, (void *)&eri, (void *)&g,
+                  &qterm, &sh, &igx, &tiles, &scratch, &count, &inv_beta, &omega_dev};
+    // the count starts from zero whatever an overlapping (racing) call left
+    if (cudaMemsetAsync(count, 0, sizeof(unsigned), st) != cudaSuccess ||
+        cudaLaunchKernel((const void *)energy2_kernel, dim3((unsigned)energy_grid(sms, tiles)),
+                         dim3(EN_T), a2, 0, st) != cudaSuccess)
         return KVFT_EDEVICE;
     return KVFT_OK;
 }

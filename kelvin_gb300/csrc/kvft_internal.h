@@ -127,6 +127,7 @@ struct KvDryOp {
 // ---------------------------------------------------------------------------
 // Context
 // ---------------------------------------------------------------------------
+constexpr int KV_FLAG_ENERGY = 16;
 struct kvft_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -140,7 +141,8 @@ struct kvft_ctx {
     void *l2buf = nullptr;
     // cached scratch buffers keyed by purpose
     std::map<std::string, std::pair<void *, size_t>> scratch;
-    int *dflag = nullptr;            // device status word for bounded waits
+    int *dflag = nullptr;            // device words, zero at rest: [0] status of bounded
+                                     // waits, [KV_FLAG_ENERGY] the energy's arrival count
     struct KvProf *prof = nullptr;
     // Digit planes of stable operands (the integral blocks), kept across the
     // residual evaluations of one solver: on only inside solver-driven

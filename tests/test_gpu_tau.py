@@ -76,3 +76,23 @@ def test_spin_blocked_step_vs_oracle(ctx, pw, quad):
     assert abs(T1 - (0.3 * x1 + 0.7 * r1)).max() <= 1e-12 * max(1.0, abs(r1).max())
     assert abs(T2 - (0.3 * x2 + 0.7 * r2)).max() <= 1e-12 * max(1.0, abs(r2).max())
     assert abs(E - oft.ft_cc_energy(T1, T2, F.ov, I.oovv, g, beta)) <= 1e-12
+
+
+# The symmetric T1 T1 half (rows a < b, a = b, a > b in one tile, a tile that
+# spans three values of a), rectangular extents, one tile and several waves of
+# them, T1's share on more and fewer blocks than elements; both Q terms.
+@pytest.mark.parametrize("nv,no,ng", [(1, 1, 1), (1, 40, 3), (11, 2, 4), (13, 7, 20), (34, 33, 5),
+                                      (60, 21, 2)])
+@pytest.mark.parametrize("qterm", [True, False])
+def test_energy_rectangular(ctx, nv, no, ng, qterm):
+    from kelvin_gb300 import ft_cc_energy
+    rng = numpy.random.default_rng(nv + no)
+    T1 = rng.standard_normal((ng, nv, no))
+    T2 = rng.standard_normal((ng, nv, nv, no, no))
+    f, eri = rng.standard_normal((no, nv)), rng.standard_normal((no, no, nv, nv))
+    g = rng.random(ng)
+    E = ft_cc_energy.ft_cc_energy(T1, T2, f, eri, g, 2.0, qterm, ctx=ctx)
+    ref = oft.ft_cc_energy(T1, T2, f, eri, g, 2.0, qterm)
+    # both sums lie within a roundoff per term of the sum of magnitudes
+    mag = oft.ft_cc_energy(abs(T1), abs(T2), abs(f), abs(eri), g, 2.0, qterm)
+    assert abs(E - ref) <= 4.0 * 2.0 ** -53 * (ng + 4) * mag + 1e-15 * mag
