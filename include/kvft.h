@@ -63,7 +63,12 @@ int kvft_event_record(kvft_ctx *ctx, int slot);            /* slot < 64 */
 int kvft_event_elapsed_ms(kvft_ctx *ctx, int s0, int s1, float *ms);
 int kvft_launch_count(kvft_ctx *ctx, uint64_t *count);     /* own kernels */
 int kvft_flush_l2(kvft_ctx *ctx);                          /* writes 256 MB */
-/* Free and total device memory of the context's device (cudaMemGetInfo). */
+/* Memory from kvft_alloc comes with arbitrary contents.  kvft_free waits for the
+ * whole device, as cudaFree does, and keeps the block for a later kvft_alloc of
+ * the process: at most a 32nd of the device in all, returned to the driver
+ * when an allocation fails and when the device's last context is destroyed. */
+/* Free (the driver's and the kept blocks) and total memory of the context's
+ * device. */
 int kvft_mem_info(kvft_ctx *ctx, size_t *free_bytes, size_t *total_bytes);
 /* Cap on the tau-chunk workspace of solvers on this context (bytes; 0: the
  * default, 60% of the free device memory), so that several resident solvers

@@ -289,6 +289,14 @@ int kv_cuda(kvft_ctx *ctx, cudaError_t e, const char *what);
     } while (0)
 int kv_launch_check(kvft_ctx *ctx, const char *what);
 
+// Device memory of the library.  kv_dev_free keeps a block for the next
+// kv_dev_alloc of about its size instead of returning it to the driver, up to
+// a 32nd of the device per process (kvft_ctx.cu).  kv_mem_info: free bytes
+// (the driver's and those kept) and total bytes.
+int kv_dev_alloc(kvft_ctx *ctx, size_t bytes, void **p);
+int kv_dev_free(kvft_ctx *ctx, void *p);
+int kv_mem_info(kvft_ctx *ctx, size_t *free_bytes, size_t *total_bytes);
+
 // scratch memory owned by the context (grows, never shrinks until destroy)
 int kv_scratch(kvft_ctx *ctx, const char *key, size_t bytes, void **p);
 

@@ -744,7 +744,7 @@ extern "C" int kvft_ccsd_lambda(kvft_ctx *ctx, int ng, int nv, int no,
     int nb = ng;
     if (!ctx->dry) {
         size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
+        if (kv_mem_info(ctx, &fr, &tot) == KVFT_OK) {
             const double per = (double)kv_lambda_workspace(1, nv, no) + 8.0 * (vo + v2o2);
             nb = (int)std::max(1.0, std::min((double)ng, 0.7 * (double)fr / per));
         }

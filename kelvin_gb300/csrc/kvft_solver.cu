@@ -245,7 +245,7 @@ namespace {
 
 int salloc(kvft_solver *s, size_t bytes, double **p) {
     void *q = nullptr;
-    KV_CHECK(s->ctx, cudaMalloc(&q, bytes ? bytes : 16));
+    KV_TRY(kv_dev_alloc(s->ctx, bytes, &q));
     s->allocs.push_back(q);
     *p = (double *)q;
     return KVFT_OK;
@@ -291,7 +291,7 @@ int upload_grid(kvft_solver *s, const double *ti, const double *g, const double 
 // planes of two operands must fit in 60% of the memory not held by the solver
 int pick_chunk(kvft_solver *s) {
     size_t fr = 0, tot = 0;
-    KV_CHECK(s->ctx, cudaMemGetInfo(&fr, &tot));
+    KV_TRY(kv_mem_info(s->ctx, &fr, &tot));
     size_t held = 0;
     for (auto &kv : s->ctx->scratch) held += kv.second.second;
     size_t per = kv_chunk_bytes_per_tau(s->ctx, s->nv, s->no);
@@ -688,7 +688,7 @@ void host_parallel(long long n, F f) {
 
 void destroy(kvft_solver *s) {
     if (s->gexec) cudaGraphExecDestroy(s->gexec);
-    for (void *p : s->allocs) cudaFree(p);
+    for (void *p : s->allocs) kv_dev_free(s->ctx, p);
     if (s->hsc) cudaFreeHost(s->hsc);
     if (s->done) cudaEventDestroy(s->done);
     if (s->aa_ev) cudaEventDestroy(s->aa_ev);
@@ -728,8 +728,8 @@ int kvft_solver_create(kvft_ctx *ctx, int n, int ng, const double *eps, const do
     if (st == KVFT_OK) st = salloc(s, sizeof(double) * n, &s->sfo);
     if (st == KVFT_OK) st = salloc(s, sizeof(double) * n, &s->sfv);
     if (st == KVFT_OK) st = upload_grid(s, ti, g, G);
-    if (st == KVFT_OK && (cudaMalloc(&dfock, sizeof(double) * n2) != cudaSuccess ||
-                          cudaMalloc(&deri, sizeof(double) * n4) != cudaSuccess))
+    if (st == KVFT_OK && (kv_dev_alloc(ctx, sizeof(double) * n2, (void **)&dfock) != KVFT_OK ||
+                          kv_dev_alloc(ctx, sizeof(double) * n4, (void **)&deri) != KVFT_OK))
         st = kv_fail(ctx, KVFT_ENOMEM, "solver_create: no room for the raw integrals");
     if (st == KVFT_OK) {
         cudaStream_t str = ctx->stream;
@@ -758,8 +758,8 @@ int kvft_solver_create(kvft_ctx *ctx, int n, int ng, const double *eps, const do
     }
     if (st == KVFT_OK) st = finish_create(s, out);
     cudaStreamSynchronize(ctx->stream);
-    if (dfock) cudaFree(dfock);
-    if (deri) cudaFree(deri);
+    if (dfock) kv_dev_free(ctx, dfock);
+    if (deri) kv_dev_free(ctx, deri);
     if (st != KVFT_OK) destroy(s);
     return st;
 }
@@ -890,7 +890,7 @@ int aa_alloc(kvft_solver *s, int m) {
                     s->allocs.erase(s->allocs.begin() + i);
                     break;
                 }
-            cudaFree(*p);
+            kv_dev_free(s->ctx, *p);
             *p = nullptr;
         }
         s->aa_h = h;
@@ -901,8 +901,7 @@ int aa_alloc(kvft_solver *s, int m) {
     for (int i = 0; i < 1 + 2 * m; i++) {
         if (*arr[i]) continue;
         void *q = nullptr;
-        if (cudaMalloc(&q, sizeof(float) * words) != cudaSuccess) {
-            cudaGetLastError();
+        if (kv_dev_alloc(s->ctx, sizeof(float) * words, &q) != KVFT_OK) {
             return kv_fail(s->ctx, KVFT_ENOMEM, "solver_set_acceleration: no room for the history");
         }
         s->allocs.push_back(q);
@@ -1672,7 +1671,7 @@ int kvft_ccsd_stanton(kvft_ctx *ctx, int ng, int nv, int no, const double *const
     KvSpinScope spins(ctx, sh);
     KV_TRY(seed_neg(ctx, ng, s1, F[2], T1b));
     size_t fr = 0, tot = 0;
-    KV_CHECK(ctx, cudaMemGetInfo(&fr, &tot));
+    KV_TRY(kv_mem_info(ctx, &fr, &tot));
     size_t held = 0;
     for (auto &kv : ctx->scratch) held += kv.second.second;
     size_t per = kv_chunk_bytes_per_tau(ctx, nv, no);

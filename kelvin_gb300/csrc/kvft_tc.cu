@@ -1064,8 +1064,8 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
         }
         // keep it only while a tenth of the device stays free
         size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr > bytes + tot / 10 &&
-            cudaMalloc(&buf, bytes) == cudaSuccess) {
+        if (kv_mem_info(ctx, &fr, &tot) == KVFT_OK && fr > bytes + tot / 10 &&
+            kv_dev_alloc(ctx, bytes, &buf) == KVFT_OK) {
             ctx->pack_cache[ckey] = {buf, bytes};
             ctx->scratch_gen++;
         } else {
