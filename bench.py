@@ -86,6 +86,13 @@ TRAFFIC_FILE = os.path.join(ROOT, "profiles", "traffic.json")
 STEP_EVENTS = 8     # first event slot of the per-step timings (at most 50 steps)
 
 
+def digit_pairs(digits):
+    """Digit-pair products of the tensor-core contraction: levels 2 .. digits
+    of seven-bit digits; seven levels of accuracy take nine-bit digits and
+    levels 2 .. 6."""
+    return sum(l - 1 for l in range(2, min(digits, 6) + 1))
+
+
 def load_peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -468,7 +475,7 @@ def run_gpu(args, w):
                 peak = 1.25
                 psrc = "nominal GB300 FP64 1.25 TFLOP/s (no measured FP64 figure)"
             else:
-                pairs = sum(l - 1 for l in range(2, digits + 1))
+                pairs = digit_pairs(digits)
                 achieved *= pairs      # BF16 tensor flops issued per FP64-equivalent flop
                 peak = peaks["bf16_tflops_sustained"]
                 psrc = "bf16_tflops_sustained of %s peaks; achieved = the spin-blocked " \
@@ -713,7 +720,7 @@ def run_gemm(args):
     prof = ctx.profile_end()
     ms = ctx.elapsed_ms(0, 1) / args.steps
     flops = 2.0 * M * N * K * B
-    pairs = sum(l - 1 for l in range(2, digits + 1)) if args.precision != "fp64" else 1
+    pairs = digit_pairs(digits) if args.precision != "fp64" else 1
     print(json.dumps({"gemm": [M, N, K, B], "precision": args.precision, "digits": digits,
                       "ms": ms, "fp64_equiv_tflops": flops / ms / 1e9,
                       "bf16_tflops_issued": flops * pairs / ms / 1e9 if pairs > 1 else None,

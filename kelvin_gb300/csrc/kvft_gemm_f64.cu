@@ -528,7 +528,7 @@ void kv_gemm_prof_set(kvft_ctx *ctx, int M, int N, int K, int batch, int nbA, in
     if (ctx->gemm_cat == KV_CAT_GEMM6) {
         ctx->gemm_work = 2.0 * M * N * (double)K * batch;
     } else {
-        const double el = tc ? 2.0 * std::min(ctx->digits - 1, 6) : 8.0;
+        const double el = tc ? 2.0 * kv_tc_planes(ctx->digits) : 8.0;
         ctx->gemm_work = el * K * ((double)M * nbA + (double)N * nbB) +
                          8.0 * M * (double)N * batch * (beta != 0.0 ? 2 : 1);
     }

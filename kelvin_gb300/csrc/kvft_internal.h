@@ -315,6 +315,8 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha,
 int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha,
                const KMat &A, const KMat &B, double beta, const KOut &C, int digits,
                const KvProds &g);
+// Digit planes of an operand at the given digit count (kvft_tc.h).
+int kv_tc_planes(int digits);
 // The group of one product at the operands' own addresses.
 inline KvProds kv_one_prod() {
     KvProds g;

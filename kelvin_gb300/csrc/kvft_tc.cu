@@ -5,24 +5,26 @@
 // splitting):
 //
 //   * packing: every row r of A (and every column of B) is scaled by 2^-e_r
-//     so that |y| < 1/2, then y = 2^-7 sum_{s=1..S} P_s with balanced base-128
-//     digits P_s = d_s 2^-7(s-1), d_s in [-64, 64] -- exact in BF16.  The
-//     digits are extracted with integer arithmetic from the FP64 bit pattern.
-//   * products: A B = 2^(e_m + e_n - 14) sum_{s,t} P_s^A P_t^B.  Pair (s,t)
-//     carries the weight 2^-7(s+t-2); pairs with s + t <= D are kept.  Each
-//     digit product is an integer below 2^12 (times a power of two), so an
-//     FP32 accumulator over K <= 2048 terms and two pairs is exact.
+//     so that |y| < 1/2, then y = 2^-C sum_{s=1..S} P_s with balanced digits
+//     P_s = d_s 2^(C - pos(s)), exact in BF16 (kvft_tc.h: digit schemes; base
+//     128 up to D = 6, nine-bit digits at D = 7).  The digits are extracted
+//     with integer arithmetic from the FP64 bit pattern.
+//   * products: A B = 2^(e_m + e_n - 2 C) sum_{s,t} P_s^A P_t^B.  Pairs of one
+//     level s + t have one weight; levels up to NL + 1 are kept.  A base-128
+//     product is an integer below 2^12 (times a power of two), so an FP32
+//     accumulator over K <= 2048 terms and two pairs is exact; nine-bit digits
+//     are read out after 512 terms.
 //     Every level l = s + t has its own TMEM accumulator, at column
 //     (l - 2) TN of the set, and the digit planes of a B tile lie one after
 //     another in shared memory, so a single tcgen05.mma of A plane s against
 //     B planes t0..t0+k-1 (N = k TN <= 256) adds each product into its own
-//     level: 8 MMAs per 16-deep k-step for D = 7 instead of 21 pair MMAs,
+//     level: 5 MMAs per 16-deep k-step for D = 7 instead of 15 pair MMAs,
 //     which keeps the tensor core's shared-memory reads of A below the SM's
 //     shared-memory bandwidth.
 //   * epilogue: the accumulators are read from TMEM (tcgen05.ld), the K
-//     chunks (K > 2048) are summed in registers, and the tile is scaled by
-//     2^(e_m + e_n - 14) alpha and written to the FP64 output view once.
-// With D = 7 (21 pair products, six digits) the norm-wise relative error is
+//     chunks (K > KCHUNK) are summed in registers, and the tile is scaled by
+//     2^(e_m + e_n - 2 C) alpha and written to the FP64 output view once.
+// With D = 7 (15 pair products, five digits) the norm-wise relative error is
 // ~1e-11, far inside the 1e-8 amplitude / 1e-10 Ha parity bounds; D = 3..5 is
 // the mixed-precision form.
 //
@@ -41,17 +43,18 @@
 
 namespace {
 
-constexpr int KCHUNK = 2048;                  // exactness bound of the level-3 sum
 constexpr int NEPI = 8;                       // epilogue warps: two per TMEM lane quadrant
 constexpr int NTHREADS = 64 + 32 * NEPI;      // + TMA producer warp + MMA warp
 constexpr int TMEM_COLS = 512;               // all of an SM's TMEM (one CTA per SM)
+constexpr int KRANGE = 2048;                  // K range of a unit that adds by atomics
 constexpr int GROUP_M = 8;                    // m-tiles per raster group (L2 reuse)
 
 struct TcParams {
     int M, N;             // output extent
     int mt, nt;           // output tiles along M and N
     int units;            // work units: C blocks * mt * nt * batch * nsplit
-    int nsplit;           // >1: each K chunk is its own unit, added into C by FP64 atomics
+    int nsplit;           // >1: each K range is its own unit, added into C by FP64 atomics
+    int split_kb;         // k-blocks per K range
     int chunk_kb;         // k-blocks per K chunk (exactness bound)
     int nkb_total;        // k-blocks of the padded K extent
     int S, D, NS;         // digit planes, levels, pipeline stages
@@ -112,8 +115,8 @@ __device__ __forceinline__ Unit unit_of(const TcParams &p, int u, int tn) {
         w.n0 = (rr / gm) * tn;
     }
     if (p.nsplit > 1) {
-        w.kb0 = split * p.chunk_kb;
-        w.kb1 = min(w.kb0 + p.chunk_kb, p.nkb_total);
+        w.kb0 = split * p.split_kb;
+        w.kb1 = min(w.kb0 + p.split_kb, p.nkb_total);
     } else {
         w.kb0 = 0;
         w.kb1 = p.nkb_total;
@@ -144,14 +147,20 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb) {
 //               when D <= 3 (the few-digit form), an unevaluated FP32 pair
 //               (error-free two-sums) otherwise.  After the last chunk the
 //               tile goes to C once: FP64 built from bit patterns with the
-//               scale 2^(e_m + e_n - 14) (and a power-of-two alpha) in the
+//               scale 2^(e_m + e_n - 2 C) (and a power-of-two alpha) in the
 //               exponent field, old values of C loaded 8 at a time.
 //
 // D <= 3: TN = 128, two levels (256 columns) per set, two sets, so the MMAs
-// of one chunk run while the epilogue drains the other.  D >= 4: TN = 64, up
-// to six levels (384 columns), one set; the epilogue frees it as soon as the
-// levels are in registers (a few percent of a chunk's MMA time), and writes
-// the tile while the next chunk accumulates.
+// of one chunk run while the epilogue drains the other.  D >= 4: TN = 64, three
+// to five levels, two sets up to D = 5; at D = 6 there is room for one, which
+// the epilogue frees as soon as the levels are in registers (a few percent of
+// a 2048-deep chunk's MMA time).  D = 7 reads out four times as often and so
+// takes TN = 48, where two sets of five levels fit (against 64 columns and one
+// set: 1 % of an update of 54 spin orbitals and 10 tau points, 5 % of a
+// residual of 21 occupied and 37 virtual spin orbitals; at D = 6 the narrower
+// tile costs 4.5 % of a sweep of 114 spin orbitals and 3 tau points instead).
+// Seven levels in whole: 12.4 -> 11.2 ms for that update (nine-bit digits, 15
+// products for 21), 34.2 -> 32.2 ms for a Lambda sweep of 38 and 8 points.
 //
 // DL (the digit levels D) is a template parameter: the MMA issue loop is then
 // straight-line code whose descriptors are per-stage bases plus constant
@@ -160,19 +169,18 @@ template <int TN, bool FF, int KBT, int DL>
 __global__ void __launch_bounds__(NTHREADS, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                TcParams p) {
-    constexpr int SD = DL - 1 < MAXS ? DL - 1 : MAXS;   // digit planes
+    using G = Dig<DL>;
+    constexpr int SD = G::S, nl = G::NL;     // digit planes and levels
     constexpr int PLANE_BYTES = TM * KBT * 2;    // one digit plane of an A k-block
     constexpr int BPLANE = TN * KBT * 2;         // one digit plane of a B k-block
     constexpr int WCOLS = TN / 2;            // columns per epilogue warp
     constexpr int LW = FF ? 4 : 16;          // columns per TMEM load (<= 32 registers in flight)
     constexpr int NG = WCOLS / LW;           // TMEM loads per level
     constexpr int WG = 8;                    // columns per store group
-    constexpr int MAXL = FF ? 6 : 2;         // levels per set
-    constexpr int NSET = FF ? 1 : 2;         // accumulator sets
-    constexpr int SET_COLS = MAXL * TN;      // 384 or 256 TMEM columns
+    constexpr int SET_COLS = nl * TN;        // TMEM columns of a set
+    constexpr int NSET = 2 * SET_COLS <= TMEM_COLS ? 2 : 1;   // accumulator sets
     constexpr int PMAX = 256 / TN;           // B planes per MMA (N <= 256)
     static_assert(NSET * SET_COLS <= TMEM_COLS, "accumulator sets exceed TMEM");
-    constexpr uint32_t IDESC = idesc_of(TN);
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int S = SD;
@@ -307,8 +315,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         for (int kk = 0; kk < KBT / 16; kk++) {
 #pragma unroll
                             for (int s = 1; s <= S; s++) {
-                                if (s >= DL) continue;
-                                const int tmax = min(S, DL - s);
+                                const int tmax = nl + 1 - s;
                                 const uint32_t acc = (kk > 0 || s > 1) ? 1u : later;
                                 const uint64_t da = dA + (((s - 1) * PLANE_BYTES + kk * 32) >> 4);
 #pragma unroll
@@ -316,8 +323,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                     const int np = min(PMAX, tmax - t0 + 1);
                                     const uint64_t db =
                                         dB + (((t0 - 1) * BPLANE + kk * 32) >> 4);
-                                    umma(tacc + (s + t0 - 2) * TN, da, db, idesc_of(np * TN),
-                                         acc);
+                                    umma(tacc + (s + t0 - 2) * TN, da, db,
+                                         idesc_of(np * TN), acc);
                                 }
                             }
                         }
@@ -340,7 +347,6 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // ---- epilogue ----
         const int ew = warp - 2, q = warp & 3, h = ew >> 2;
         const int row = q * 32 + lane;
-        constexpr int nl = DL - 1;                  // levels 2..D
         long long *coff = s_coff + ew * WCOLS;
         int *cexp = s_cexp + ew * WCOLS;
         float rhi[WCOLS];
@@ -385,8 +391,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                            (long long)i2 * p.C.r.st[2];
                 }
                 double *Cr = p.C.p + (long long)w.b * p.C.bst + p.coff[w.cb] + roff;
-                const int krow =
-                    (m < p.M) ? exp_of(p.ea[p.aex[src] + w.b * p.ea_bst + m]) - 14 + p.alpha_exp : 0;
+                const int krow = (m < p.M) ? exp_of(p.ea[p.aex[src] + w.b * p.ea_bst + m]) -
+                                                 2 * G::C + p.alpha_exp
+                                           : 0;
                 if (m < p.M && p.nsplit == 1 && beta != 0.0 && beta != 1.0) {
                     for (int i = 0; i < min(WCOLS, nlim); i++)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(Cr + coff[i]));
@@ -409,27 +416,25 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         tmem + ((uint32_t)(q * 32) << 16) + set * SET_COLS + h * WCOLS;
     #pragma unroll
                     for (int g = 0; g < NG; g++) {
-                        uint32_t r[MAXL][LW];
+                        uint32_t r[nl][LW];
     #pragma unroll
-                        for (int l = 0; l < MAXL; l++)
-                            if (l < nl) tmem_ld<LW>(tb + l * TN + g * LW, r[l]);
+                        for (int l = 0; l < nl; l++)
+                            tmem_ld<LW>(tb + l * TN + g * LW, r[l]);
                         tmem_wait_ld();
     #pragma unroll
                         for (int j = 0; j < LW; j++) {
                             const int i = g * LW + j;
                             float hi = __uint_as_float(r[0][j]);
                             if constexpr (!FF) {
-                                if (nl > 1) hi += __uint_as_float(r[1][j]);
+                                if (nl > 1) hi += __uint_as_float(r[nl > 1 ? 1 : 0][j]);
                                 rhi[i] = first ? hi : rhi[i] + hi;
                             } else {
                                 // exact level sums, leading first: an FP32 pair
                                 float lo = 0.f, e;
     #pragma unroll
-                                for (int l = 1; l < MAXL; l++) {
-                                    if (l < nl) {
-                                        two_sum(hi, __uint_as_float(r[l][j]), hi, e);
-                                        lo += e;
-                                    }
+                                for (int l = 1; l < nl; l++) {
+                                    two_sum(hi, __uint_as_float(r[l][j]), hi, e);
+                                    lo += e;
                                 }
                                 if (first) {
                                     rhi[i] = hi;
@@ -671,7 +676,7 @@ pack_exp_kernel(const __grid_constant__ PackView v, int R, int K, int rows_fast,
 // Balanced base-128 digits of x 2^-e (|x 2^-e| < 1/2), most significant
 // first, from the FP64 bit pattern with integer arithmetic only.
 __device__ __forceinline__ void digits_of(unsigned long long bits, int e, int S, int *d) {
-    for (int s = 0; s < MAXS; s++) d[s] = 0;
+    for (int s = 0; s < S; s++) d[s] = 0;
     const int be = (int)((bits >> 52) & 0x7FF);
     if (be == 0) return;                        // zero / subnormal (< 2^-1022): zero
     const long long mant = (long long)((bits & 0xFFFFFFFFFFFFFull) | (1ull << 52));
@@ -736,29 +741,41 @@ __device__ __forceinline__ __nv_bfloat162 digit_pair(int d0, int d1) {
     return __floats2bfloat162_rn(f0, f1);
 }
 
-template <int S>
-__device__ __forceinline__ void store_digits(__nv_bfloat16 *ob, size_t plane,
-                                             unsigned long long x0, unsigned long long x1,
-                                             int e) {
-    int d0[MAXS], d1[MAXS];
-    digits_of_s<S>(x0, e, d0);
-    digits_of_s<S>(x1, e, d1);
-    *reinterpret_cast<__nv_bfloat162 *>(ob) = digit_pair<0>(d0[0], d1[0]);
-    if (S > 1) *reinterpret_cast<__nv_bfloat162 *>(ob + plane) = digit_pair<1>(d0[1], d1[1]);
-    if (S > 2) *reinterpret_cast<__nv_bfloat162 *>(ob + 2 * plane) = digit_pair<2>(d0[2], d1[2]);
-    if (S > 3) *reinterpret_cast<__nv_bfloat162 *>(ob + 3 * plane) = digit_pair<3>(d0[3], d1[3]);
-    if (S > 4) *reinterpret_cast<__nv_bfloat162 *>(ob + 4 * plane) = digit_pair<4>(d0[4], d1[4]);
-    if (S > 5) *reinterpret_cast<__nv_bfloat162 *>(ob + 5 * plane) = digit_pair<5>(d0[5], d1[5]);
+// Base-128 digits here come from the loop above: digit_words, the same values,
+// costs these kernels 1.5 % of a step of 114 spin orbitals.
+template <int D>
+__device__ __forceinline__ void store_digits(uint16_t *ob, size_t plane, unsigned long long x0,
+                                             unsigned long long x1, int e) {
+    constexpr int S = Dig<D>::S;
+    if constexpr (Dig<D>::WIDE) {
+        uint32_t w[S];
+        digit_words<D>(x0, x1, e, w);
+#pragma unroll
+        for (int s = 0; s < S; s++) *reinterpret_cast<uint32_t *>(ob + s * plane) = w[s];
+    } else {
+        int d0[S], d1[S];
+        digits_of_s<S>(x0, e, d0);
+        digits_of_s<S>(x1, e, d1);
+        *reinterpret_cast<__nv_bfloat162 *>(ob) = digit_pair<0>(d0[0], d1[0]);
+        if constexpr (S > 1)
+            *reinterpret_cast<__nv_bfloat162 *>(ob + plane) = digit_pair<1>(d0[1], d1[1]);
+        if constexpr (S > 2)
+            *reinterpret_cast<__nv_bfloat162 *>(ob + 2 * plane) = digit_pair<2>(d0[2], d1[2]);
+        if constexpr (S > 3)
+            *reinterpret_cast<__nv_bfloat162 *>(ob + 3 * plane) = digit_pair<3>(d0[3], d1[3]);
+        if constexpr (S > 4)
+            *reinterpret_cast<__nv_bfloat162 *>(ob + 4 * plane) = digit_pair<4>(d0[4], d1[4]);
+    }
 }
 
-// planes[b][s][row][k] (row stride ld) = d_s 2^-7s; each thread packs two k.
+// planes[b][s][row][k] (row stride ld); each thread packs two k.
 // Persistent blocks walk the 32 x 64 tiles t = blockIdx.x, + gridDim.x, ...
 // (k tile fastest, then row tile, then batch); the next tile's loads are in
 // flight in registers while the current one is converted.
-template <int S>
+template <int D>
 __global__ void __launch_bounds__(256)
 pack_digits_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int ktn, int rtn,
-                   int ntiles, const int *__restrict__ ex, __nv_bfloat16 *__restrict__ out) {
+                   int ntiles, const int *__restrict__ ex, uint16_t *__restrict__ out) {
     __shared__ unsigned long long val[PT_R][PT_K + 1];
     __shared__ long long off[PT_R + PT_K];
     const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
@@ -807,7 +824,7 @@ pack_digits_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int
                 if (row >= R) break;
                 const int e = exp_of(ex[(long long)b * R + row]);
                 // the second value is zero beyond K (tile fill)
-                store_digits<S>(out + (size_t)b * S * plane + (size_t)row * ld + k, plane,
+                store_digits<D>(out + (size_t)b * Dig<D>::S * plane + (size_t)row * ld + k, plane,
                                 val[rr][2 * lane], val[rr][2 * lane + 1], e);
             }
         }
@@ -828,10 +845,10 @@ __host__ __device__ constexpr size_t pack_rows_smem(int kt) {
     return (size_t)PT_R * (kt * PT_K + 1) * 8 + (size_t)(kt * PT_K) * 8;
 }
 
-template <int S, int KT>
+template <int D, int KT>
 __global__ void __launch_bounds__(256, 2)
 pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int rtiles, int ntiles,
-                 int *__restrict__ ex, __nv_bfloat16 *__restrict__ out) {
+                 int *__restrict__ ex, uint16_t *__restrict__ out) {
     constexpr int NK = KT * PT_K, LDV = NK + 1, PER = NK / 8;   // values per thread
     extern __shared__ unsigned long long prs[];
     unsigned long long *val = prs;                                      // [PT_R][LDV]
@@ -911,13 +928,13 @@ pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int r
             const int row = r0 + rr;
             if (row >= R) break;
             const int e = exp_of(rexp[rr]);
-            __nv_bfloat16 *ob = out + (size_t)b * S * plane + (size_t)row * ld;
+            uint16_t *ob = out + (size_t)b * Dig<D>::S * plane + (size_t)row * ld;
 #pragma unroll
             for (int j = 0; j < KT; j++) {
                 const int k = 2 * lane + 64 * j;
                 if (k >= K) break;
                 // the second value is zero beyond K
-                store_digits<S>(ob + k, plane, val[rr * LDV + k], val[rr * LDV + k + 1], e);
+                store_digits<D>(ob + k, plane, val[rr * LDV + k], val[rr * LDV + k + 1], e);
             }
         }
     }
@@ -969,79 +986,80 @@ namespace {
 // boxes with zeros; rows past R inside a 128-row box belong to the next plane
 // and only reach output rows/columns that the epilogue discards.
 // Identity of a packed operand: address, view, extents and digit count.
-std::string pack_key(const PackView &v, int R, int K, int nb, int S) {
+std::string pack_key(const PackView &v, int R, int K, int nb, int D) {
     char b[400];
     snprintf(b, sizeof b, "%p|%d,%d,%d:%lld,%lld,%lld|%d,%d,%d:%lld,%lld,%lld|%lld|%d,%d,%d,%d",
              (const void *)v.p, v.r.size[0], v.r.size[1], v.r.size[2], v.r.st[0], v.r.st[1],
              v.r.st[2], v.c.size[0], v.c.size[1], v.c.size[2], v.c.st[0], v.c.st[1], v.c.st[2],
-             v.bst, R, K, nb, S);
+             v.bst, R, K, nb, D);
     std::string key = b;
     for (int q = 0; q < v.nsub; q++) key += "," + std::to_string(v.sub[q]);
     return key;
 }
 
 // persistent digit pass: as many blocks as fit on the SMs at once
-template <int S>
+template <int D>
 int launch_pack_digits(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int rows_fast,
                        int ktn, int rtn, long long tiles, Packed *out) {
     static int per_sm = 0;
     if (!per_sm) {
         KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                          &per_sm, pack_digits_kernel<S>, 256, 0));
+                          &per_sm, pack_digits_kernel<D>, 256, 0));
         per_sm = std::max(per_sm, 1);
     }
     const int grid = (int)std::min(tiles, (long long)per_sm * ctx->sm_count);
-    pack_digits_kernel<S><<<grid, 256, 0, ctx->stream>>>(v, R, K, ld, rows_fast, ktn, rtn,
+    pack_digits_kernel<D><<<grid, 256, 0, ctx->stream>>>(v, R, K, ld, rows_fast, ktn, rtn,
                                                         (int)tiles, out->ex, out->planes);
     return KVFT_OK;
 }
 
-template <int S, int KT>
+template <int D, int KT>
 int launch_pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb,
                      int rows_fast, int rtiles, Packed *out) {
     constexpr size_t smem = pack_rows_smem(KT);
     static int per_sm = 0;
     if (!per_sm) {
-        KV_CHECK(ctx, cudaFuncSetAttribute(pack_rows_kernel<S, KT>,
+        KV_CHECK(ctx, cudaFuncSetAttribute(pack_rows_kernel<D, KT>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                          &per_sm, pack_rows_kernel<S, KT>, 256, smem));
+                          &per_sm, pack_rows_kernel<D, KT>, 256, smem));
         per_sm = std::max(per_sm, 1);
     }
     const long long ntiles = (long long)rtiles * nb;
     if (ntiles > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many row tiles");
     const int grid = (int)std::min(ntiles, (long long)per_sm * ctx->sm_count);
-    pack_rows_kernel<S, KT><<<grid, 256, smem, ctx->stream>>>(
+    pack_rows_kernel<D, KT><<<grid, 256, smem, ctx->stream>>>(
         v, R, K, ld, rows_fast, rtiles, (int)ntiles, out->ex, out->planes);
     return kv_launch_check(ctx, "pack_rows");
 }
 
-template <int S>
+template <int D>
 int pack_rows_s(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, int rows_fast,
                 int rtiles, Packed *out) {
-    if (K <= PT_K) return launch_pack_rows<S, 1>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+    if (K <= PT_K) return launch_pack_rows<D, 1>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     if (K <= 2 * PT_K)
-        return launch_pack_rows<S, 2>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
-    return launch_pack_rows<S, 4>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+        return launch_pack_rows<D, 2>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+    return launch_pack_rows<D, 4>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
 }
 
-int pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, int S,
+int pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, int D,
               int rows_fast, int rtiles, Packed *out) {
-    switch (S) {
-    case 1: return pack_rows_s<1>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+    switch (D) {
     case 2: return pack_rows_s<2>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     case 3: return pack_rows_s<3>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     case 4: return pack_rows_s<4>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     case 5: return pack_rows_s<5>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     case 6: return pack_rows_s<6>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+    case 7: return pack_rows_s<7>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     default: return kv_fail(ctx, KVFT_EINVAL, "pack: digit count out of range");
     }
 }
 
 }  // namespace
 
-int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int S,
+int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int D,
                Packed *out) {
+    const int S = dig_planes(D);
     const int ld = (K + 63) / 64 * 64;
     const size_t plane_bytes = (size_t)R * ld * 2;
     const size_t pbytes = ((size_t)nb * S * plane_bytes + 1023) / 1024 * 1024;
@@ -1055,10 +1073,10 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     std::string ckey;
     if (v.stable && ctx->pack_cache_on) {
         // an integral block packed during an earlier residual evaluation
-        ckey = pack_key(v, R, K, nb, S);
+        ckey = pack_key(v, R, K, nb, D);
         auto it = ctx->pack_cache.find(ckey);
         if (it != ctx->pack_cache.end()) {
-            out->planes = (__nv_bfloat16 *)it->second.first;
+            out->planes = (uint16_t *)it->second.first;
             out->ex = (int *)((uint8_t *)it->second.first + pbytes);
             return KVFT_OK;
         }
@@ -1074,14 +1092,14 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
         }
     }
     if (!buf) KV_TRY(kv_scratch(ctx, key, bytes, &buf));
-    out->planes = (__nv_bfloat16 *)buf;
+    out->planes = (uint16_t *)buf;
     out->ex = (int *)((uint8_t *)buf + pbytes);
     KvProfScope prof(ctx, KV_CAT_PACK, 8.0 * nb * (double)R * K + (double)nb * S * plane_bytes);
     // coalesce global reads along the contiguous index
     const int rows_fast = (kidx_fast_stride(v.r) == 1 && kidx_fast_stride(v.c) != 1) ? 1 : 0;
     const long long rtiles = (R + PT_R - 1) / PT_R;
     if (rtiles > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: too many rows");
-    if (K <= PR_KMAX) return pack_rows(ctx, v, R, K, ld, nb, S, rows_fast, (int)rtiles, out);
+    if (K <= PR_KMAX) return pack_rows(ctx, v, R, K, ld, nb, D, rows_fast, (int)rtiles, out);
     KV_CHECK(ctx, cudaMemsetAsync(out->ex, 0x80, (size_t)nb * R * sizeof(int), ctx->stream));
     const dim3 g((K + PT_K - 1) / PT_K, (unsigned)rtiles, nb);
     // long rows: each exponent block walks up to 16 k tiles, so that about
@@ -1092,13 +1110,13 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     pack_exp_kernel<<<ge, 256, 0, ctx->stream>>>(v, R, K, rows_fast, ktiles, out->ex);
     KV_TRY(kv_launch_check(ctx, "pack_exp"));
     if (tiles > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many tiles");
-    switch (S) {
+    switch (D) {
 #define KV_PACK_CASE(s_)                                                                   \
     case s_:                                                                               \
         KV_TRY(launch_pack_digits<s_>(ctx, v, R, K, ld, rows_fast, g.x, g.y, tiles, out)); \
         break;
-        KV_PACK_CASE(1) KV_PACK_CASE(2) KV_PACK_CASE(3) KV_PACK_CASE(4) KV_PACK_CASE(5)
-        KV_PACK_CASE(6)
+        KV_PACK_CASE(2) KV_PACK_CASE(3) KV_PACK_CASE(4) KV_PACK_CASE(5) KV_PACK_CASE(6)
+        KV_PACK_CASE(7)
 #undef KV_PACK_CASE
     default: return kv_fail(ctx, KVFT_EINVAL, "pack: digit count out of range");
     }
@@ -1162,13 +1180,15 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
 
 int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
                 const KMat &B, double beta, const KOut &C, int D, const KvProds &g) {
-    const int S = std::min(D - 1, MAXS);
-    // D >= 4: three to six levels, FP32 pairs, TN = 64, and 32-deep k-blocks
-    // (six digit planes per stage); D <= 3: 64-deep k-blocks, so that every
-    // TMA box row is a full 128-byte line, and TN = 128 unless C has at most
-    // 64 columns (then 64-wide tiles keep all eight epilogue warps busy)
+    const int S = dig_planes(D);
+    // D >= 4: three to five levels, FP32 pairs, TN = 64 (48 at D = 7, see the
+    // kernel) and 32-deep k-blocks (up to five digit
+    // planes per stage); D <= 3: 64-deep k-blocks, so that every TMA box row is
+    // a full 128-byte line, and TN = 128 unless C has at most 64 columns (then
+    // 64-wide tiles keep all eight epilogue warps busy)
     const bool ff = D >= 4;
-    const int tn = (ff || N <= 64) ? 64 : 128;
+    const int tn = D == 7 ? 48 : (ff || N <= 64) ? 64 : 128;
+    const int kchunk = D == 7 ? Dig<7>::KCHUNK : Dig<6>::KCHUNK;
     const int kb = ff ? 32 : 64;
     const int nbA = A.bst ? batch : 1, nbB = B.bst ? batch : 1;
     int wa[KV_MAXPROD], wb[KV_MAXPROD];
@@ -1176,8 +1196,8 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const PackView va = kv_tc_group_view(A.p, A.r, A.c, A.bst, A.stable, nbA, g.n, g.oa, wa);
     const PackView vb = kv_tc_group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
     Packed pa, pb;
-    KV_TRY(kv_tc_pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, S, &pa));
-    KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, S, &pb));
+    KV_TRY(kv_tc_pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, D, &pa));
+    KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, D, &pb));
     const long long rows_a = (long long)va.nsub * nbA * S * M, rows_b = (long long)vb.nsub * nbB * S * N;
     if (rows_a > 0x7FFFFFFFLL || rows_b > 0x7FFFFFFFLL)
         return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: operand too large");
@@ -1186,15 +1206,17 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     KV_TRY(kv_tc_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
     const int mt = (M + TM - 1) / TM, nt = (N + tn - 1) / tn;
     const int nkb_total = (K + kb - 1) / kb;
-    const int nchunks = (nkb_total + KCHUNK / kb - 1) / (KCHUNK / kb);
-    const int chunk_kb = (nkb_total + nchunks - 1) / nchunks;     // balanced chunks
+    const int nranges = (nkb_total + KRANGE / kb - 1) / (KRANGE / kb);
+    const int split_kb = (nkb_total + nranges - 1) / nranges;     // balanced ranges
+    const int nchunks = (split_kb + kchunk / kb - 1) / (kchunk / kb);
+    const int chunk_kb = (split_kb + nchunks - 1) / nchunks;      // balanced chunks
     const long long tiles = (long long)mt * nt * batch;
-    // fewer output tiles than two waves of SMs and several K chunks: every
-    // chunk of every product becomes a unit of its own and adds into C with
+    // fewer output tiles than two waves of SMs and several K ranges: every
+    // range of every product becomes a unit of its own and adds into C with
     // FP64 atomics (C pre-scaled by beta)
-    const bool par = nchunks > 1 && tiles < 2LL * ctx->sm_count;
+    const bool par = nranges > 1 && tiles < 2LL * ctx->sm_count;
     const KvGroupTab tab = kv_group_tab(g, par);
-    const long long units = tiles * (par ? nchunks : 1) * tab.ncb;
+    const long long units = tiles * (par ? nranges : 1) * tab.ncb;
     if (units > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: too many tiles");
     if (par && beta != 1.0) {
         const KvGroupTab t = kv_group_tab(g, false);
@@ -1214,7 +1236,8 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     p.mt = mt;
     p.nt = nt;
     p.units = (int)units;
-    p.nsplit = par ? nchunks : 1;
+    p.nsplit = par ? nranges : 1;
+    p.split_kb = split_kb;
     p.chunk_kb = chunk_kb;
     p.nkb_total = nkb_total;
     p.S = S;
@@ -1249,7 +1272,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     case 4: return launch_tc<64, true, 32, 4>(ctx, ma, mb, p);
     case 5: return launch_tc<64, true, 32, 5>(ctx, ma, mb, p);
     case 6: return launch_tc<64, true, 32, 6>(ctx, ma, mb, p);
-    default: return launch_tc<64, true, 32, 7>(ctx, ma, mb, p);
+    default: return launch_tc<48, true, 32, 7>(ctx, ma, mb, p);
     }
 }
 
@@ -1258,7 +1281,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
 int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
                const KMat &B, double beta, const KOut &C, int digits, const KvProds &g) {
     const int D = digits;
-    if (D < 2 || D > MAXS + 1) return kv_fail(ctx, KVFT_EINVAL, "tensor-core digits out of range");
+    if (D < 2 || D > 7) return kv_fail(ctx, KVFT_EINVAL, "tensor-core digits out of range");
     if (M <= 0 || N <= 0 || batch <= 0) return KVFT_OK;
     if (K <= 0) return kv_gemm_f64(ctx, M, N, K, batch, alpha, A, B, beta, C, g);
     // C^T = B^T A^T, the same products
@@ -1285,6 +1308,8 @@ int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, cons
     if (swap) return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt);
     return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g);
 }
+
+int kv_tc_planes(int digits) { return dig_planes(std::min(digits, 7)); }
 
 // Device status word written by bounded waits (0 = fine).
 int kv_device_status(kvft_ctx *ctx) {

@@ -11,7 +11,40 @@
 namespace {
 
 constexpr int TM = 128;
-constexpr int MAXS = 6;
+
+// ---- digit schemes -------------------------------------------------------------
+// The digit count D = 2..7 of the interface names an accuracy.  A scheme writes
+// y, |y| < 1/2, as sum_s d_s 2^-pos(s) with S digits of bits(s) bits (balanced:
+// |d_s| <= 2^(bits(s) - 1)), stored as P_s = d_s 2^(C - pos(s)), exact in
+// BF16; products P_s P_t of one level s + t add up in one FP32
+// accumulator, the levels 2 .. NL + 1 are kept, and a sum runs over at most
+// KCHUNK terms before it is read out.
+//   D <= 6  seven-bit digits, S = NL = D - 1.
+//   D = 7   digits of 8, 9, 9, 9 and 9 bits, five levels: 15 products; seven-bit
+//           digits need 21 for six planes.
+// BF16 holds balanced nine-bit digits, so the wide ones spend no product on
+// bits that the type leaves empty.  What bounds the width is the rounding of
+// the FP32 sums, hence the narrower leading digit and the shorter KCHUNK.
+// Error against seven-bit digits in an exact emulation with round-to-nearest
+// and with truncating FP32 sums (K = 57 to 3249; normal, uniform, constant,
+// few-valued and wide-range operands, A A^T): 0.1 to 0.8 of it, in the 2-norm
+// and for the largest element.  At D = 6 the digits stay as they are: results
+// there are only good to ~1e-9, and any other digits would move them by that.
+template <int D>
+struct Dig {
+    static_assert(D >= 2 && D <= 7, "digit count");
+    static constexpr bool WIDE = D == 7;
+    static constexpr int S = WIDE ? 5 : D - 1;
+    static constexpr int NL = S;                       // levels (accumulators)
+    static constexpr int KCHUNK = WIDE ? 512 : 2048;
+    static constexpr int C = WIDE ? 8 : 7;
+    // bits after the point down to and including digit s = 1 .. S
+    __host__ __device__ static constexpr int pos(int s) { return WIDE ? 9 * s - 1 : 7 * s; }
+    __host__ __device__ static constexpr int bits(int s) {
+        return s == 1 ? pos(1) : pos(s) - pos(s - 1);
+    }
+};
+inline int dig_planes(int D) { return D == 7 ? Dig<7>::S : D - 1; }
 constexpr unsigned long long WAIT_NS = 2000000000ull;   // 2 s per wait
 
 // Knuth's error-free sum: s + e == a + b exactly (round-to-nearest FP32)
@@ -181,6 +214,70 @@ __device__ __forceinline__ int raw_exp(unsigned long long bits) {
     return (bits & 0x7FFFFFFFFFFFFFFFull) ? (int)((bits >> 52) & 0x7FF) - 1023 : -2000;
 }
 
+// Digit planes of the pair (x0, x1) of a row with packing exponent e: word s -
+// 1 holds the two BF16 values P_s.  The balanced digits of the rounded |x|
+// 2^(pos(S) - e) are its bit fields once half a digit has been added at every
+// place but the top one, so no digit waits for another's carry; a field
+// becomes a float by its place in the significand of 1.5 2^23, and the sign is
+// set on the packed word.  Integer operations on the FP64 bit pattern
+// otherwise; subnormals count as zero.
+template <int D>
+__device__ __forceinline__ void digit_words(unsigned long long x0, unsigned long long x1, int e,
+                                            uint32_t (&w)[Dig<D>::S]) {
+    using G = Dig<D>;
+    constexpr int S = G::S, T = G::pos(S);
+    uint32_t sg = 0;
+    float f[2][S];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const unsigned long long x = h ? x1 : x0;
+        const uint32_t hi = (uint32_t)(x >> 32);
+        const int be = (int)((hi >> 20) & 0x7FF);
+        sg |= h ? (hi & 0x80000000u) : (hi >> 31) << 15;
+        uint32_t fld[S];
+        if constexpr (T <= 21) {
+            // the T bits and the rounding bit lie in the significand's high
+            // word (|x| 2^-e < 1/2: the shift of the whole is at least 33)
+            uint32_t bias = 0;
+#pragma unroll
+            for (int s = 2; s <= S; s++) bias |= 1u << (T - G::pos(s) + G::bits(s) - 1);
+            const int n = 52 + e - (be - 1023) - T - 32;
+            uint32_t Y = n < 22 && be != 0 ? (((hi & 0xFFFFFu) | 0x100000u) + (1u << (n - 1))) >> n
+                                           : 0u;
+            Y += bias;
+#pragma unroll
+            for (int s = 1; s <= S; s++) {
+                const uint32_t q = Y >> (T - G::pos(s));
+                fld[s - 1] = s == 1 ? q : q & ((1u << G::bits(s)) - 1);
+            }
+        } else {
+            unsigned long long bias = 0;
+#pragma unroll
+            for (int s = 2; s <= S; s++) bias |= 1ull << (T - G::pos(s) + G::bits(s) - 1);
+            const int n = 1023 + 52 + e - T - be;             // at least 54 - T
+            const unsigned long long mant = (x & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+            unsigned long long Y = n < 55 && be != 0 ? (mant + (1ull << (n - 1))) >> n : 0ull;
+            Y += bias;
+#pragma unroll
+            for (int s = 1; s <= S; s++) {
+                const uint32_t q = (uint32_t)(Y >> (T - G::pos(s)));
+                fld[s - 1] = s == 1 ? q : q & ((1u << G::bits(s)) - 1);
+            }
+        }
+#pragma unroll
+        for (int s = 1; s <= S; s++) {
+            const float sc = 1.0f / (float)(1ull << (G::pos(s) - G::C));   // P_s = d_s sc, exact
+            const float off = s == 1 ? 12582912.0f : 12582912.0f + (float)(1 << (G::bits(s) - 1));
+            f[h][s - 1] = fmaf(__uint_as_float(0x4B400000u | fld[s - 1]), sc, -off * sc);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(f[0][s], f[1][s]);
+        w[s] = *reinterpret_cast<const uint32_t *>(&v) ^ sg;
+    }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -203,15 +300,15 @@ struct PackView {
 };
 
 struct Packed {
-    __nv_bfloat16 *planes;
+    uint16_t *planes;
     int *ex;
     int R, ld, K, nb;
 };
 
 
-// Packs v (R rows x K, nb packed batch entries, S planes) into the scratch
-// buffer `key`, or into the cache of stable operands.
-int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int S,
+// Packs v (R rows x K, nb packed batch entries, the digits of scheme D) into
+// the scratch buffer `key`, or into the cache of stable operands.
+int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int D,
                Packed *out);
 // 2D tensor map over digit planes (K x rows, row stride ld elements); one box
 // is a k-block of kb values (swizzled by its 2 kb bytes) by box_rows rows.

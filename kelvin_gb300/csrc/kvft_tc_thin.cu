@@ -47,7 +47,7 @@
 namespace {
 
 constexpr int KMAX = 64, NMAX = 64;
-constexpr int MMAS = 2 * MAXS;               // MMAs of a k-step (at most two per A plane)
+constexpr int MMAS = 10;                     // MMAs of a k-step (at most two per A plane)
 
 struct ThinParams {
     int M, N, K, TN;             // TN: N rounded up to 16 (columns of one level)
@@ -110,60 +110,6 @@ struct Step {
     }
 };
 
-// Digit planes of the pair (x0, x1) of a row with packing exponent e: word s
-// holds the two BF16 values d_s 2^-7s (kvft_tc.cu: digits_of).  The balanced
-// digits of the rounded |x| 2^(7S - e) are its base-128 fields once 64 has
-// been added at every digit but the top one, so no digit waits for another's
-// carry; a field becomes a float by its place in the significand of 1.5 2^23.
-template <int S>
-__device__ __forceinline__ void digit_words(unsigned long long x0, unsigned long long x1, int e,
-                                            uint32_t (&w)[S]) {
-    uint32_t sg = 0;
-    float f[2][S];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const unsigned long long x = h ? x1 : x0;
-        const uint32_t hi = (uint32_t)(x >> 32);
-        const int be = (int)((hi >> 20) & 0x7FF);
-        sg |= h ? (hi & 0x80000000u) : (hi >> 31) << 15;
-        uint32_t fld[S];
-        if constexpr (S <= 3) {
-            constexpr uint32_t BIAS = S == 1 ? 0u : S == 2 ? 64u : 64u + (64u << 7);
-            const int n = 52 + e - (be - 1023) - 7 * S - 32;
-            uint32_t Y = n < 22 && be != 0 ? (((hi & 0xFFFFFu) | 0x100000u) + (1u << (n - 1))) >> n
-                                           : 0u;
-            Y += BIAS;
-#pragma unroll
-            for (int s = 0; s < S; s++)
-                fld[s] = s ? (Y >> (7 * (S - 1 - s))) & 127u : Y >> (7 * (S - 1));
-        } else {
-            unsigned long long bias = 0;
-#pragma unroll
-            for (int s = 0; s < S - 1; s++) bias |= 64ull << (7 * s);
-            // |x| 2^-e < 1/2: the shift right is at least 54 - 7 S
-            const int n = 1023 + 52 + e - 7 * S - be;
-            const unsigned long long mant = (x & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-            unsigned long long Y = n < 55 && be != 0 ? (mant + (1ull << (n - 1))) >> n : 0ull;
-            Y += bias;
-#pragma unroll
-            for (int s = 0; s < S; s++)
-                fld[s] = s ? (uint32_t)(Y >> (7 * (S - 1 - s))) & 127u
-                           : (uint32_t)(Y >> (7 * (S - 1)));
-        }
-#pragma unroll
-        for (int s = 0; s < S; s++) {
-            const float sc = 1.0f / (float)(1ull << (7 * s));
-            f[h][s] = fmaf(__uint_as_float(0x4B400000u | fld[s]), sc,
-                           (s ? -12582976.0f : -12582912.0f) * sc);
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(f[0][s], f[1][s]);
-        w[s] = *reinterpret_cast<const uint32_t *>(&v) ^ sg;
-    }
-}
-
 __device__ __forceinline__ void sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w)
                  : "memory");
@@ -188,7 +134,8 @@ template <int KBT, int DL>
 __global__ void __launch_bounds__(thin_threads(KBT, DL), thin_threads(KBT, DL) == 512 ? 1 : 2)
 tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ThinParams p) {
     constexpr int NT = thin_threads(KBT, DL);
-    constexpr int S = DL - 1 < MAXS ? DL - 1 : MAXS, nl = DL - 1;
+    using G = Dig<DL>;
+    constexpr int S = G::S, nl = G::NL;
     constexpr int PLANE = TM * KBT * 2;
     constexpr int NKP = NT / TM;                 // threads per row (a_rows_fast)
     constexpr int VP = KBT / NKP;                // values of A per thread
@@ -217,7 +164,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
     int nmma = 0;
 #pragma unroll
     for (int q = 1; q <= S; q++) {
-        const int tmax = min(S, DL - q);
+        const int tmax = nl + 1 - q;
         for (int t0 = 1; t0 <= tmax; t0 += pmax, nmma++)
             if (tid == 0)
                 mma[nmma] = make_uint4((q + t0 - 2) * p.TN, ((q - 1) * PLANE) >> 4,
@@ -351,7 +298,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
                     uint32_t w[4][S];
 #pragma unroll
                     for (int j = 0; j < 4; j++)
-                        digit_words<S>(pre[8 * c + 2 * j], pre[8 * c + 2 * j + 1], e, w[j]);
+                        digit_words<DL>(pre[8 * c + 2 * j], pre[8 * c + 2 * j + 1], e, w[j]);
                     const uint32_t a = sA32 + chunk(row, c * NKP + part);
 #pragma unroll
                     for (int t = 0; t < S; t++)
@@ -374,7 +321,7 @@ tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ 
                     if (kp == 0) rexp[r] = p.krow0 + e * (1 << 20);
                     if (2 * kp < kpad) {
                         uint32_t w[S];
-                        digit_words<S>(pre[2 * v], pre[2 * v + 1], e, w);
+                        digit_words<DL>(pre[2 * v], pre[2 * v + 1], e, w);
                         const uint32_t a = sA32 + chunk(r, kp >> 2) + (kp & 3) * 4;
 #pragma unroll
                         for (int t = 0; t < S; t++) sts32(a + t * PLANE, w[t]);
@@ -535,13 +482,13 @@ constexpr size_t THIN_SMEM_CAP = 226 * 1024;
 
 template <int KBT, int DL>
 int launch_thin(kvft_ctx *ctx, const CUtensorMap &mb, ThinParams &p) {
-    constexpr int S = DL - 1 < MAXS ? DL - 1 : MAXS, NT = thin_threads(KBT, DL);
+    constexpr int S = Dig<DL>::S, NT = thin_threads(KBT, DL);
     auto kern = tc_thin_kernel<KBT, DL>;
     p.nbuf = 2;
     if (thin_smem(KBT, S, NT, p.TN, 2) > THIN_SMEM_CAP) p.nbuf = 1;
     size_t smem = thin_smem(KBT, S, NT, p.TN, p.nbuf);
     // CTAs that share an SM must fit its TMEM together
-    const int cols = (DL - 1) * p.TN;
+    const int cols = Dig<DL>::NL * p.TN;
     int per = NT == 512 || cols > 256 ? 1 : 2;
     if (per == 1) smem = std::max(smem, (size_t)118 * 1024);
     else if (2 * smem > THIN_SMEM_CAP) per = 1;
@@ -576,13 +523,13 @@ bool kv_thin_fits(int M, int N, int K, int batch, const KMat &A, const KMat &B, 
 
 int kv_gemm_thin(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
                  const KMat &B, double beta, const KOut &C, int D, const KvProds &g) {
-    const int S = std::min(D - 1, MAXS);
+    const int S = dig_planes(D);
     const int kbt = K <= 32 ? 32 : 64;
     const int nbB = B.bst ? batch : 1;
     int wb[KV_MAXPROD];
     const PackView vb = kv_tc_group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
     Packed pb;
-    KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, S, &pb));
+    KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, D, &pb));
     const long long rows = (long long)vb.nsub * nbB * S * N;
     const KvGroupTab tab = kv_group_tab(g, false);
     ThinParams p;
@@ -605,7 +552,8 @@ int kv_gemm_thin(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, co
     p.store = beta == 1.0 ? 0 : beta == 0.0 ? 1 : 2;
     int alpha_exp = 0;
     p.alpha_pow2 = kv_tc_pow2(alpha, &alpha_exp, &p.alpha_sign);
-    p.krow0 = (1023 - 127 - 14 + alpha_exp) * (1 << 20);
+    const int c2 = 2 * (D == 7 ? Dig<7>::C : Dig<6>::C);
+    p.krow0 = (1023 - 127 - c2 + alpha_exp) * (1 << 20);
     p.eb = pb.ex;
     p.eb_bst = nbB > 1 ? N : 0;
     p.b_batch_rows = nbB > 1 ? S * N : 0;

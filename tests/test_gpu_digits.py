@@ -1,0 +1,60 @@
+"""The wide digits of seven levels (nine-bit, read out every 512 terms) are at
+least as accurate as seven-bit digits of the same level count: the error of the device product is at most that of seven-bit
+digits with exact sums, computed here, in the 2-norm and for the largest
+element.  Operands: normal, A A^T (equal signs in every square), few-valued,
+constant, wide-range; K below, at and above the read-out length and the
+kernels' k-blocks."""
+import numpy
+import pytest
+
+from kelvin_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(kind, K, M=48):
+    rng = numpy.random.default_rng(K)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((K, M))
+    if kind == "aat":
+        B = A.T.copy()
+    elif kind == "few":
+        A, B = 1.0 / rng.integers(1, 12, (M, K)), 1.0 / rng.integers(1, 9, (K, M))
+    elif kind == "const":
+        A, B = numpy.full((M, K), 0.3), numpy.full((K, M), 0.7)
+    elif kind == "wide":
+        A, B = A * numpy.exp(3 * A), B * numpy.exp(3 * B)
+    return A, B
+
+
+def seven_bit(A, D):
+    """Balanced base-128 digits (D - 1 of them) of the rows of A, as FP64
+    values, and the row exponents."""
+    S = D - 1
+    e = numpy.floor(numpy.log2(abs(A).max(1))) + 2
+    Y = numpy.floor(abs(A) * 2.0 ** (7 * S - e)[:, None] + 0.5).astype(numpy.int64)
+    d = []
+    for s in range(S, 1, -1):
+        low = ((Y + 64) & 127) - 64
+        d.insert(0, low * 2.0 ** (-7 * s))
+        Y = (Y - low) >> 7
+    d.insert(0, Y * 2.0 ** -7)
+    return [x * numpy.sign(A) for x in d], e
+
+
+@pytest.mark.parametrize("kind", ["normal", "aat", "few", "const", "wide"])
+@pytest.mark.parametrize("K", [33, 57, 64, 300, 512, 545, 3249])
+def test_wide_digits_no_less_accurate_than_seven_bit(ctx, K, kind, digits=7):
+    A, B = operands(kind, K)
+    ref = A.astype(numpy.longdouble) @ B.astype(numpy.longdouble)
+    (a, ea), (b, eb) = seven_bit(A, digits), seven_bit(B.T, digits)
+    old = sum((a[s - 1] @ b[t - 1].T).astype(numpy.longdouble)
+              for s in range(1, digits) for t in range(1, digits) if s + t <= digits)
+    old = old * numpy.longdouble(2) ** (ea[:, None] + eb[None, :])
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, ref.shape)
+    ctx.check(ctx.L.kvft_gemm(ctx.h, A.shape[0], B.shape[1], K, 1, _lib.PREC_FP64_TC, digits,
+                              dA.ptr, dB.ptr, dC.ptr), "kvft_gemm")
+    bound = abs(A).max(1)[:, None] * abs(B).max(0)[None, :]
+    err, err7 = abs(dC.to_host() - ref) / bound, abs(old - ref) / bound
+    assert (err ** 2).sum() <= (err7 ** 2).sum()
+    assert err.max() <= err7.max()
