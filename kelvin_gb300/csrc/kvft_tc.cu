@@ -1206,15 +1206,28 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     KV_TRY(kv_tc_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
     const int mt = (M + TM - 1) / TM, nt = (N + tn - 1) / tn;
     const int nkb_total = (K + kb - 1) / kb;
-    const int nranges = (nkb_total + KRANGE / kb - 1) / (KRANGE / kb);
+    const long long tiles = (long long)mt * nt * batch;
+    // K ranges.  Fewer output tiles than two waves of SMs and several ranges of
+    // 2048: every range of every product becomes a unit of its own and adds
+    // into C with FP64 atomics (C pre-scaled by beta).  With error-free level
+    // sums (D >= 4) the ranges may be shorter: while there are fewer units than
+    // SMs, down to 256 deep (below that the pipeline's start and the atomics
+    // cost what the other SMs would save).  D <= 3 keeps 2048, which is part
+    // of its rounding.  37 x 37 outputs against K = 16317, one product, seven
+    // levels: 40 us on 8 SMs; the residual of 37 virtual and 21 occupied spin
+    // orbitals 1067 -> 962 us, a solve of 38 and 10 points 53.6 -> 52.8 ms.
+    int nranges = (nkb_total + KRANGE / kb - 1) / (KRANGE / kb);
+    bool par = nranges > 1 && tiles < 2LL * ctx->sm_count;
+    const long long now = tiles * (par ? (long long)nranges * g.n : kv_group_tab(g, false).ncb);
+    if (ff && now < ctx->sm_count) {
+        const long long want = (ctx->sm_count + tiles * g.n - 1) / (tiles * g.n);
+        nranges = (int)std::max<long long>(nranges, std::min<long long>(want, K / 256));
+        par = nranges > 1;
+    }
     const int split_kb = (nkb_total + nranges - 1) / nranges;     // balanced ranges
+    nranges = (nkb_total + split_kb - 1) / split_kb;
     const int nchunks = (split_kb + kchunk / kb - 1) / (kchunk / kb);
     const int chunk_kb = (split_kb + nchunks - 1) / nchunks;      // balanced chunks
-    const long long tiles = (long long)mt * nt * batch;
-    // fewer output tiles than two waves of SMs and several K ranges: every
-    // range of every product becomes a unit of its own and adds into C with
-    // FP64 atomics (C pre-scaled by beta)
-    const bool par = nranges > 1 && tiles < 2LL * ctx->sm_count;
     const KvGroupTab tab = kv_group_tab(g, par);
     const long long units = tiles * (par ? nranges : 1) * tab.ncb;
     if (units > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: too many tiles");

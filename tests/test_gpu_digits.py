@@ -58,3 +58,22 @@ def test_wide_digits_no_less_accurate_than_seven_bit(ctx, K, kind, digits=7):
     err, err7 = abs(dC.to_host() - ref) / bound, abs(old - ref) / bound
     assert (err ** 2).sum() <= (err7 ** 2).sum()
     assert err.max() <= err7.max()
+
+
+# Few output tiles: with four or more levels K is cut into ranges of 256 and
+# more that add into C.  Either side of the first cut (512), one k-block more,
+# a long K with one, several and enough tiles, a batch.  Tolerances: those of
+# the digit counts (norm-wise), which do not depend on how K is cut.
+@pytest.mark.parametrize("digits,tol", [(4, 5e-7), (5, 5e-9), (6, 5e-11), (7, 5e-12)])
+@pytest.mark.parametrize("M,N,K,batch", [(70, 40, 511, 1), (70, 40, 512, 1), (70, 40, 545, 1),
+                                         (37, 21, 16317, 1), (130, 100, 2049, 3),
+                                         (600, 1, 700, 1), (2000, 700, 600, 1)])
+def test_split_k_with_few_tiles(ctx, M, N, K, batch, digits, tol):
+    rng = numpy.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((batch, M, K)), rng.standard_normal((batch, K, N))
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray.from_host(ctx, numpy.full((batch, M, N), numpy.nan))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, N, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
+    assert (abs(dC.to_host() - A @ B) <= tol * bound).all()
