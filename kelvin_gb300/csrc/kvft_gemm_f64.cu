@@ -73,18 +73,20 @@ __device__ __forceinline__ void f64_out(const F64Params &p, double *dst, double 
 }
 
 __host__ __device__ constexpr size_t f64_smem(int BM, int BN, int BK) {
-    return 8 * (size_t)(BK * ((BM | 1) + (BN | 1)) + 2 * (BM + BN) + 2 * BK);
+    const int work = BK * ((BM | 1) + (BN | 1));       // and one sum per thread
+    return 8 * (size_t)((work > NT ? work : NT) + 2 * (BM + BN) + 2 * BK);
 }
 
 // BK: k values per shared-memory block; 32 where few outputs per thread make
-// the loads' latency the chain
-template <int T, int BK>
+// the loads' latency the chain.  SL > 1: a tile of at most NT / SL outputs,
+// whose threads take K in SL interleaved slices.
+template <int T, int BK, int SL>
 __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F64Params p) {
     extern __shared__ double sm[];
     const int lda = p.BM | 1, ldb = p.BN | 1;
     double *As = sm;                                   // [BK][lda]
     double *Bs = As + BK * lda;                        // [BK][ldb]
-    long long *ar = (long long *)(Bs + BK * ldb);      // A row, B column, C row, C column
+    long long *ar = (long long *)(sm + max(BK * (lda + ldb), NT));   // A row, B column, C row, C column
     long long *bc = ar + p.BM, *cr = bc + p.BN, *cc = cr + p.BM;
     long long *ak = cc + p.BN, *bk = ak + BK;          // K offsets of the current k block
     const int tid = threadIdx.x;
@@ -102,13 +104,14 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F6
     }
     // this thread's outputs as shared-memory offsets m | n << 16; one past the
     // tile (not in `ok`) repeats element 0 and is not stored
-    const int cnt = p.BM * p.BN, wbase = tid & ~31;
+    constexpr int CS = NT / SL;                        // threads of a K slice
+    const int cnt = p.BM * p.BN, ot = tid % CS, ks = tid / CS, wbase = ot & ~31;
     int mn[T];
     unsigned ok = 0;
     double acc[T];
 #pragma unroll
     for (int i = 0; i < T; i++) {
-        const int o = tid + NT * i;
+        const int o = ot + NT * i;
         const int q = p.dflat.div(o), r = o - q * (p.cm_fast ? p.BM : p.BN);
         const int m = p.cm_fast ? r : q, n = p.cm_fast ? q : r;
         const bool in = o < cnt && m < bm && n < bn;
@@ -146,14 +149,22 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F6
                 }
             }
             __syncthreads();
-            const double *as = As, *bs = Bs;
-            for (int k = 0; k < kn; k++, as += lda, bs += ldb) {
+            const double *as = As + ks * lda, *bs = Bs + ks * ldb;
+            for (int k = ks; k < kn; k += SL, as += SL * lda, bs += SL * ldb) {
 #pragma unroll
                 for (int i = 0; i < T; i++)
                     if (wbase + NT * i < cnt)
                         acc[i] = fma(as[mn[i] & 0xFFFF], bs[mn[i] >> 16], acc[i]);
             }
         }
+    }
+    if constexpr (SL > 1) {                            // the slices' sums, in order
+        __syncthreads();
+        As[tid] = acc[0];
+        __syncthreads();
+        if (ks > 0) return;
+#pragma unroll
+        for (int q = 1; q < SL; q++) acc[0] += As[ot + q * CS];
     }
     double *C = p.C.p + (long long)t.b * p.C.bst + p.oc[t.cb];
 #pragma unroll
@@ -305,10 +316,10 @@ void f64_tile(int M, int N, int cap, int *BM, int *BN) {
     *BN = M <= N ? bl : bs;
 }
 
-template <int T, int BK>
+template <int T, int BK, int SL = 1>
 int launch_f64_t(kvft_ctx *ctx, const F64Params &p, int grid) {
     const size_t smem = f64_smem(p.BM, p.BN, BK);
-    gemm_f64_kernel<T, BK><<<grid, NT, smem, ctx->stream>>>(p);
+    gemm_f64_kernel<T, BK, SL><<<grid, NT, smem, ctx->stream>>>(p);
     return kv_launch_check(ctx, "gemm_f64");
 }
 
@@ -467,7 +478,14 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     case 16: return launch_f64_t<16, 16>(ctx, p, (int)grid);
     case 8: return launch_f64_t<8, 16>(ctx, p, (int)grid);
     case 4: return launch_f64_t<4, 32>(ctx, p, (int)grid);
-    default: return launch_f64_t<2, 32>(ctx, p, (int)grid);
+    default:
+        // At most 64 outputs a tile leave half or more of a block's warps
+        // without one, always the same warps and so the same FP64 pipes of the
+        // SM; they take slices of K instead (60 products of 8 x 8 outputs, K =
+        // 512: 20 -> 12.5 us; an 8-site ring's iteration 503 -> 471 us).
+        if (p.BM * p.BN <= 32) return launch_f64_t<2, 32, 4>(ctx, p, (int)grid);
+        if (p.BM * p.BN <= 64) return launch_f64_t<2, 32, 2>(ctx, p, (int)grid);
+        return launch_f64_t<2, 32>(ctx, p, (int)grid);
     }
 }
 

@@ -22,7 +22,11 @@ pytestmark = pytest.mark.gpu
     # a row per thread: 128-, 64- and 32-row blocks, 1 to 24 columns, several
     # column tiles (25, 49, 64), K around its block of 16, either side big
     (40000, 1, 16, 2), (33000, 24, 17, 4), (20011, 25, 15, 3), (9000, 49, 31, 3),
-    (64, 7777, 9, 5), (8, 512, 8, 60), (5000, 13, 13, 20)])
+    (64, 7777, 9, 5), (8, 512, 8, 60), (5000, 13, 13, 20),
+    # K in two or four slices of a block: 32, 33, 64 and 65 outputs a tile, K
+    # below the slice count and around the block of 32
+    (4, 8, 1, 2), (4, 8, 3, 2), (8, 4, 33, 2), (3, 11, 31, 1), (8, 8, 5, 3), (8, 8, 65, 3),
+    (5, 13, 34, 1)])
 def test_gemm_fp64_tiles(ctx, M, N, K, batch):
     rng = numpy.random.default_rng(M + 3 * N + 7 * K + batch)
     A = rng.standard_normal((batch, M, K))
