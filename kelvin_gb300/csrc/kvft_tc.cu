@@ -940,6 +940,113 @@ pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int r
     }
 }
 
+// Longer rows (up to 8 x 512): one pass by clusters.  A cluster's CTAs hold 16
+// whole rows in their shared memory, a slab of K each; row maxima meet through
+// distributed shared memory, and every CTA writes the digits of its slab.  The
+// operand is read once and in one launch, where the general path below reads
+// it twice in two and clears the exponents in a third.  The loads are
+// asynchronous copies to shared memory, so a block's whole slab is in flight
+// at once, and three or more blocks an SM overlap loads and conversion (16 rows
+// keep a slab of 416, K = 3249, at 53 KB; 32 rows leave two blocks and cost 15 %).
+// Bound by the copies' issue and the conversion: 3.3 to 3.7 TB/s of 8 + 2 S
+// bytes an element.  Three levels, before and now: 3249 x 3249
+// 2.8 -> 3.3 TB/s, 1089 x 1089 2.6 -> 3.2; seven levels, 729 x 729 2.7 -> 3.5.
+// Whole steps: 38 spin orbitals, solve 53.2 -> 51.2 ms; 54, update 11.2 ->
+// 10.7; 66 23.1 -> 22.4; 114 132.6 -> 129.8.
+constexpr int PC_MAX = 8, PC_SLAB = 512;      // CTAs of a cluster, k of a slab
+constexpr int PC_R = 16;                      // rows of a cluster
+
+__host__ __device__ constexpr size_t pack_slab_smem(int slab) {
+    return (size_t)PC_R * (slab + 1) * 8 + (size_t)(slab + PC_R) * 8;
+}
+
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int D>
+__global__ void __launch_bounds__(256)
+pack_cluster_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast,
+                    int rtiles, int ncta, int slab, int *__restrict__ ex,
+                    uint16_t *__restrict__ out) {
+    extern __shared__ unsigned long long prs[];
+    const int ldv = slab + 1;
+    unsigned long long *val = prs;                                       // [PC_R][ldv]
+    long long *koff = reinterpret_cast<long long *>(prs + PC_R * ldv);   // [slab]
+    long long *roff = koff + slab;                                       // [PC_R]
+    __shared__ int rmax[PC_R];
+    const int tid = threadIdx.x, lane = tid % 32, w = tid / 32;
+    const int t = blockIdx.x / ncta, rank = blockIdx.x - t * ncta;
+    const int b = t / rtiles, r0 = (t - b * rtiles) * PC_R, k0 = rank * slab;
+    const int kn = max(0, min(slab, K - k0));
+    for (int x = tid; x < slab; x += 256) koff[x] = x < kn ? v.c.off(k0 + x) : -1;
+    if (tid < PC_R) roff[tid] = r0 + tid < R ? v.r.off(r0 + tid) : -1;
+    __syncthreads();
+    const double *base = v.base(b);
+    auto load = [&](int r, int k) {
+        const long long ro = roff[r], ko = koff[k];
+        unsigned long long *d = val + r * ldv + k;
+        if (ro >= 0 && ko >= 0)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d)),
+                         "l"(base + ro + ko)
+                         : "memory");
+        else
+            *d = 0ull;
+    };
+    if (rows_fast) {
+#pragma unroll 8
+        for (int k = tid / PC_R; k < slab; k += 256 / PC_R) load(tid % PC_R, k);
+    } else {
+        for (int r = w; r < PC_R; r += 8)
+#pragma unroll 4
+            for (int k = lane; k < slab; k += 32) load(r, k);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PC_R / 8; i++) {
+        const int rr = w + 8 * i;
+        int e = -2000;
+        for (int k = lane; k < slab; k += 32) e = max(e, raw_exp(val[rr * ldv + k]));
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) rmax[rr] = e;
+    }
+    cluster_arrive();
+    cluster_wait();
+    int em[PC_R / 8];
+#pragma unroll
+    for (int i = 0; i < PC_R / 8; i++) {
+        int e = -2000;
+        if (lane < ncta) {
+            uint32_t peer;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(peer)
+                         : "r"(smem_u32(&rmax[w + 8 * i])), "r"(lane));
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(e) : "r"(peer) : "memory");
+        }
+        em[i] = __reduce_max_sync(0xffffffffu, e);
+    }
+    cluster_arrive();                         // the peers' maxima have been read
+    const size_t plane = (size_t)R * ld;
+#pragma unroll
+    for (int i = 0; i < PC_R / 8; i++) {
+        const int rr = w + 8 * i, row = r0 + rr;
+        if (row >= R) break;
+        // the raw exponents of the other paths (0x80808080 for an all-zero row)
+        const int raw = em[i] > -2000 ? em[i] : (int)0x80808080u;
+        if (rank == 0 && lane == 0) ex[(long long)b * R + row] = raw;
+        const int e = exp_of(raw);
+        uint16_t *ob = out + (size_t)b * Dig<D>::S * plane + (size_t)row * ld + k0;
+        // the second value of the last pair is zero beyond K
+        for (int k = 2 * lane; k < kn; k += 64)
+            store_digits<D>(ob + k, plane, val[rr * ldv + k], val[rr * ldv + k + 1], e);
+    }
+    cluster_wait();
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                   const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                   const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1013,6 +1120,41 @@ int launch_pack_digits(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, i
     return KVFT_OK;
 }
 
+template <int D>
+int launch_pack_cluster(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb,
+                        int rows_fast, Packed *out) {
+    static bool attr = false;
+    if (!attr) {
+        KV_CHECK(ctx, cudaFuncSetAttribute(pack_cluster_kernel<D>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)pack_slab_smem(PC_SLAB)));
+        attr = true;
+    }
+    // slabs of at most 256, longer ones only for K > 2048; shorter ones while
+    // the blocks do not fill the SMs
+    const int rtiles = (R + PC_R - 1) / PC_R;
+    const long long tiles = (long long)rtiles * nb;
+    int ncta = std::min(PC_MAX, (K + 255) / 256);
+    while (ncta < PC_MAX && tiles * ncta < 2LL * ctx->sm_count && K > 64 * ncta) ncta++;
+    const int slab = ((K + ncta - 1) / ncta + 31) / 32 * 32;
+    ncta = (K + slab - 1) / slab;
+    if (tiles * ncta > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many row tiles");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * ncta));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = pack_slab_smem(slab);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ncta;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    KV_CHECK(ctx, cudaLaunchKernelEx(&cfg, pack_cluster_kernel<D>, v, R, K, ld, rows_fast,
+                                     rtiles, ncta, slab, out->ex, out->planes));
+    return kv_launch_check(ctx, "pack_cluster");
+}
+
 template <int D, int KT>
 int launch_pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb,
                      int rows_fast, int rtiles, Packed *out) {
@@ -1039,6 +1181,7 @@ int pack_rows_s(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, 
     if (K <= PT_K) return launch_pack_rows<D, 1>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
     if (K <= 2 * PT_K)
         return launch_pack_rows<D, 2>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
+    if (K > PR_KMAX) return launch_pack_cluster<D>(ctx, v, R, K, ld, nb, rows_fast, out);
     return launch_pack_rows<D, 4>(ctx, v, R, K, ld, nb, rows_fast, rtiles, out);
 }
 
@@ -1099,7 +1242,7 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     const int rows_fast = (kidx_fast_stride(v.r) == 1 && kidx_fast_stride(v.c) != 1) ? 1 : 0;
     const long long rtiles = (R + PT_R - 1) / PT_R;
     if (rtiles > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: too many rows");
-    if (K <= PR_KMAX) return pack_rows(ctx, v, R, K, ld, nb, D, rows_fast, (int)rtiles, out);
+    if (K <= PC_MAX * PC_SLAB) return pack_rows(ctx, v, R, K, ld, nb, D, rows_fast, (int)rtiles, out);
     KV_CHECK(ctx, cudaMemsetAsync(out->ex, 0x80, (size_t)nb * R * sizeof(int), ctx->stream));
     const dim3 g((K + PT_K - 1) / PT_K, (unsigned)rtiles, nb);
     // long rows: each exponent block walks up to 16 k tiles, so that about

@@ -77,3 +77,34 @@ def test_split_k_with_few_tiles(ctx, M, N, K, batch, digits, tol):
                               dC.ptr), "kvft_gemm")
     bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
     assert (abs(dC.to_host() - A @ B) <= tol * bound).all()
+
+
+# Rows of 257 to 4096 values are packed by clusters, longer ones in two
+# passes: K at the edges of both, of the cluster sizes and of the slabs (odd
+# K, one value in the last slab), rows at the edges of the 16- and 32-row tiles, an
+# all-zero row on each side, one operand contiguous along its rows and one
+# along K.  A row scaled by a power of two gives exactly the scaled product.
+@pytest.mark.parametrize("digits,tol", [(3, 5e-5), (6, 5e-11), (7, 5e-12)])
+@pytest.mark.parametrize("M,N,K,batch", [(31, 33, 257, 1), (64, 97, 511, 3), (33, 40, 513, 1),
+                                         (777, 130, 777, 1), (65, 32, 2047, 2), (40, 70, 2049, 1),
+                                         (32, 65, 3249, 2), (17, 16, 4095, 1), (64, 33, 4096, 1),
+                                         (33, 64, 4097, 1), (5000, 40, 361, 4)])
+def test_pack_long_rows(ctx, M, N, K, batch, digits, tol):
+    rng = numpy.random.default_rng(M + N + K)
+    A = rng.standard_normal((batch, M, K)) * numpy.exp(3 * rng.standard_normal((batch, M, 1)))
+    B = rng.standard_normal((batch, K, N)) * numpy.exp(3 * rng.standard_normal((batch, 1, N)))
+    A[:, 2] = 0.0
+    B[:, :, 1] = 0.0
+    A[:, 5] = A[:, 4] * 2.0 ** 40
+    A[:, 7] = 0.0
+    A[:, 7, K - 1] = 3.0                          # the last value alone sets the exponent
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, (batch, M, N))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, N, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    C = dC.to_host()
+    bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
+    assert (abs(C - A @ B) <= tol * bound).all()
+    assert not C[:, 2].any() and not C[:, :, 1].any()
+    if digits == 3 and K <= 2048:                 # one K range: one fixed order
+        assert (C[:, 5] == C[:, 4] * 2.0 ** 40).all()
