@@ -49,6 +49,11 @@ constexpr int TMEM_COLS = 512;               // all of an SM's TMEM (one CTA per
 constexpr int KRANGE = 2048;                  // K range of a unit that adds by atomics
 constexpr int GROUP_M = 8;                    // m-tiles per raster group (L2 reuse)
 
+// A converted in the kernel (CV): at most CV_M rows, NCV more warps that turn
+// FP64 values into digits, CV_RING k-blocks of FP64 values in flight.
+constexpr int CV_M = 64, NCV = 8;
+constexpr int CV_RING = 3;
+
 struct TcParams {
     int M, N;             // output extent
     int mt, nt;           // output tiles along M and N
@@ -77,6 +82,13 @@ struct TcParams {
     int *err;
     FastDiv dv_split, dv_perb, dv_gsz, dv_batch;   // nsplit, mt nt, GROUP_M nt, batch
     FastDiv dv_cr2, dv_cr1;               // C's row index: sizes of its fast components
+    // converted A (CV): the FP64 operand, its products' offsets, its K index
+    const double *A;
+    long long ar;                         // stride of its rows
+    KIdx Ac;
+    KIdxDiv dv_ac;
+    long long a_bst, oa[KV_MAXPROD];
+    int K;
 };
 
 // A work unit: one output tile of one batch entry of one block of C over a
@@ -91,10 +103,21 @@ struct Unit {
 // Units are numbered split-fastest, then in raster groups of GROUP_M m-tiles
 // (n-tiles walk inside a group), then by batch entry, then by block of C, so
 // the CTAs that run at the same time share a few A row panels and sweep B
-// once per group.
+// once per group.  With a converted A the batch entries come first: they share
+// B (the integrals), which is then read from memory once.
+template <bool CV>
 __device__ __forceinline__ Unit unit_of(const TcParams &p, int u, int tn) {
     static_assert(GROUP_M == 8, "raster groups of 8 m-tiles (shift and mask below)");
     Unit w;
+    if constexpr (CV) {                   // one m-tile and one n-tile
+        const int t = p.dv_batch.div(u);
+        w.b = u - t * p.batch;
+        w.cb = p.dv_split.div(t);
+        w.m0 = w.n0 = 0;
+        w.kb0 = (t - w.cb * p.nsplit) * p.split_kb;
+        w.kb1 = min(w.kb0 + p.split_kb, p.nkb_total);
+        return w;
+    }
     const int t = p.dv_split.div(u);
     const int split = u - t * p.nsplit;
     const int per_b = p.mt * p.nt;
@@ -127,9 +150,9 @@ __device__ __forceinline__ Unit unit_of(const TcParams &p, int u, int tn) {
 // Shared-memory bytes of the kernel: 1 KB alignment slack, NS pipeline stages
 // (S digit planes of A and of B per stage), the barriers, the epilogue's
 // per-warp column tables and two words (TMEM base, failure flag).
-__host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb) {
-    return 1024 + (size_t)NS * S * (TM + tn) * kb * 2 + 8 * (2 * NS + 5) +
-           (size_t)NEPI * (tn / 2) * 12 + 16;
+__host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb, bool cv = false) {
+    return 1024 + (size_t)NS * S * ((cv ? CV_M : TM) + tn) * kb * 2 + 8 * (2 * NS + 5) +
+           (size_t)NEPI * (tn / 2) * 12 + 16 + (cv ? (size_t)CV_RING * CV_M * kb * 8 + 16 : 0);
 }
 
 // Persistent kernel: each CTA walks the units blockIdx.x, blockIdx.x +
@@ -165,13 +188,20 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb) {
 // DL (the digit levels D) is a template parameter: the MMA issue loop is then
 // straight-line code whose descriptors are per-stage bases plus constant
 // offsets, so the single issuing thread keeps up with the tensor core.
-template <int TN, bool FF, int KBT, int DL>
-__global__ void __launch_bounds__(NTHREADS, 1)
+//
+// CV (a small A that no cache holds, K > 4096; the caller's rule): A is not
+// packed.  Warps 10-17 copy its FP64 values asynchronously into a ring of
+// k-blocks in shared memory, CV_RING - 1 ahead, each warp its own rows and so
+// without barriers, and write their digits into the stage that the TMA
+// producer fills with B.  A's planes then have CV_M rows; the MMA reads 128, and
+// the rows beyond are other planes' bytes, whose products no one reads.
+template <int TN, bool FF, int KBT, int DL, bool CV>
+__global__ void __launch_bounds__(NTHREADS + (CV ? 32 * NCV : 0), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                TcParams p) {
     using G = Dig<DL>;
     constexpr int SD = G::S, nl = G::NL;     // digit planes and levels
-    constexpr int PLANE_BYTES = TM * KBT * 2;    // one digit plane of an A k-block
+    constexpr int PLANE_BYTES = (CV ? CV_M : TM) * KBT * 2;   // a digit plane of an A k-block
     constexpr int BPLANE = TN * KBT * 2;         // one digit plane of a B k-block
     constexpr int WCOLS = TN / 2;            // columns per epilogue warp
     constexpr int LW = FF ? 4 : 16;          // columns per TMEM load (<= 32 registers in flight)
@@ -201,7 +231,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) {
         *s_fail = 0;
         for (int i = 0; i < NS; i++) {
-            mbar_init(smem_u32(&full[i]), 1);
+            mbar_init(smem_u32(&full[i]), CV ? 1 + NCV : 1);
             mbar_init(smem_u32(&empty[i]), 1);
         }
         for (int i = 0; i < NSET; i++) {
@@ -227,12 +257,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == 0) {
         if (lane == 0) {
             // ---- TMA producer ----
-            const uint32_t bytes = (uint32_t)(stage_a + stage_b);
+            const uint32_t bytes = (uint32_t)(CV ? stage_b : stage_a + stage_b);
             int st = 0, issued = 0;
             uint32_t ph = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                const Unit w = unit_of(p, u, TN);
+                const Unit w = unit_of<CV>(p, u, TN);
                 for (int q = p.beg[w.cb]; q < p.beg[w.cb + 1] && ok; q++) {
                     const int ya = p.arow[q] + w.b * p.a_batch_rows + w.m0;
                     const int yb = p.brow[q] + w.b * p.b_batch_rows + w.n0;
@@ -247,8 +277,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         mbar_expect_tx(fb, bytes);
                         const int x = kb * KBT;
                         for (int s = 0; s < S; s++) {
-                            tma_load_2d(smem_u32(sA + st * stage_a + s * PLANE_BYTES), &tmA, x,
-                                        ya + s * p.Mp, fb);
+                            if (!CV)
+                                tma_load_2d(smem_u32(sA + st * stage_a + s * PLANE_BYTES), &tmA, x,
+                                            ya + s * p.Mp, fb);
                             tma_load_2d(smem_u32(sB + st * stage_b + s * BPLANE), &tmB, x,
                                         yb + s * p.Np, fb);
                         }
@@ -282,7 +313,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t ph = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-                const Unit w = unit_of(p, u, TN);
+                const Unit w = unit_of<CV>(p, u, TN);
                 const int nsrc = p.beg[w.cb + 1] - p.beg[w.cb];
                 for (int q = 0; q < nsrc && ok; q++)
                 for (int c0 = w.kb0; c0 < w.kb1 && ok; c0 += p.chunk_kb) {
@@ -343,6 +374,131 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             umma_commit(smem_u32(done));
             if (!mbar_wait(smem_u32(done), 0)) atomicExch(p.err, 5);
         }
+    } else if (CV && warp >= 2 + NEPI) {
+        // ---- A: FP64 values to digits ----
+        // A warp's rows are w0 + y + i STEP, y < RPI, i < ni; it copies a row's
+        // values with neighbouring lanes and converts a pair a lane.  Rows past
+        // the last one repeat it: branches per row would serialise the loads
+        // and the conversions (3800 clocks a k-block of 57 x 64 with them).
+        constexpr int LPR = KBT / 2, RPI = 32 / LPR;   // lanes and rows of a conversion step
+        constexpr int STEP = NCV * RPI, NI = CV_M / STEP, KPL = KBT / 32;
+        const int w0 = (warp - 2 - NEPI) * RPI, r0 = w0 + lane / LPR, kp = 2 * (lane % LPR);
+        const int ni = w0 < p.M ? (p.M - w0 + STEP - 1) / STEP : 0;
+        double *ring = (double *)(((uintptr_t)(tmem_slot + 4) + 15) & ~(uintptr_t)15);
+        // position in the sequence of k-blocks of this CTA's units
+        struct Cursor {
+            Unit w;
+            int u, q, kb;
+            const double *base;
+            __device__ __forceinline__ void unit(const TcParams &p) {
+                if (u >= p.units) return;
+                w = unit_of<CV>(p, u, TN);
+                q = p.beg[w.cb];
+                kb = w.kb0;
+                base = p.A + p.oa[q] + (long long)w.b * p.a_bst;
+            }
+            __device__ __forceinline__ bool next(const TcParams &p) {   // another source or unit
+                if (++kb < w.kb1) return false;
+                kb = w.kb0;
+                if (++q >= p.beg[w.cb + 1]) {
+                    u += gridDim.x;
+                    unit(p);
+                } else {
+                    base = p.A + p.oa[q] + (long long)w.b * p.a_bst;
+                }
+                return true;
+            }
+        };
+        auto fetch = [&](Cursor &c, int slot) {
+            if (c.u < p.units) {
+                const int k0 = c.kb * KBT + lane;
+                const uint32_t d0 = smem_u32(ring + (slot * CV_M + w0) * KBT + lane);
+                const double *g[KPL];
+#pragma unroll
+                for (int j = 0; j < KPL; j++)
+                    g[j] = c.base + p.dv_ac.off(p.Ac, min(k0 + 32 * j, p.K - 1));
+#pragma unroll
+                for (int i = 0; i < NI; i++) {
+                    if (i >= ni) break;
+#pragma unroll
+                    for (int y = 0; y < RPI; y++)
+#pragma unroll
+                        for (int j = 0; j < KPL; j++)
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                             d0 + ((i * STEP + y) * KBT + 32 * j) * 8),
+                                         "l"(g[j] + min(w0 + i * STEP + y, p.M - 1) * p.ar)
+                                         : "memory");
+                }
+                c.next(p);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        Cursor f, c;
+        f.u = c.u = blockIdx.x;
+        f.unit(p);
+        c.unit(p);
+#pragma unroll
+        for (int i = 0; i < CV_RING - 1; i++) fetch(f, i);
+        int st = 0, slot = 0;
+        uint32_t ph = 0;
+        bool fresh = true;
+        int ex[NI];
+        // swizzled byte offset in a plane; rows STEP apart have the same swizzle
+        static_assert(STEP % 8 == 0, "swizzle period");
+        const uint32_t so =
+            (uint32_t)(r0 * KBT * 2 + (((kp >> 3) ^ (KBT == 64 ? r0 & 7 : (r0 >> 1) & 3)) << 4) +
+                       (kp & 7) * 2);
+        while (c.u < p.units) {
+            fetch(f, slot == 0 ? CV_RING - 1 : slot - 1);
+            if (fresh) {
+                const int *ea = p.ea + p.aex[c.q] + c.w.b * p.ea_bst;
+#pragma unroll
+                for (int i = 0; i < NI; i++) ex[i] = exp_of(ea[min(r0 + i * STEP, p.M - 1)]);
+            }
+            const bool tail = c.kb * KBT + KBT > p.K;
+            asm volatile("cp.async.wait_group %0;" ::"n"(CV_RING - 1) : "memory");
+            __syncwarp();                        // the other lanes' copies too
+            const bool got = mbar_wait(smem_u32(&empty[st]), ph ^ 1);
+            if (__any_sync(0xffffffffu, !got || *s_fail)) {
+                if (lane == 0) {
+                    atomicExch(p.err, 11);
+                    *s_fail = 1;
+                }
+                break;
+            }
+            uint8_t *dst = sA + st * stage_a;
+            const double *src = ring + (slot * CV_M + r0) * KBT + kp;
+#pragma unroll
+            for (int i = 0; i < NI; i += 2) {
+                if (i >= ni) break;
+                uint32_t wd[2][S];
+#pragma unroll
+                for (int y = 0; y < 2 && i + y < NI; y++) {
+                    ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(src + (i + y) * STEP * KBT);
+                    if (tail) {                  // beyond K
+                        const int k = c.kb * KBT + kp;
+                        if (k >= p.K) x.x = 0;
+                        if (k + 1 >= p.K) x.y = 0;
+                    }
+                    digit_words<DL>(x.x, x.y, ex[i + y], wd[y]);
+                }
+#pragma unroll
+                for (int y = 0; y < 2 && i + y < NI; y++)
+#pragma unroll
+                    for (int t = 0; t < S; t++)
+                        *reinterpret_cast<uint32_t *>(dst + t * PLANE_BYTES + so + (i + y) * STEP * KBT * 2) = wd[y][t];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&full[st]));
+            if (++st == NS) {
+                st = 0;
+                ph ^= 1;
+            }
+            slot = slot == CV_RING - 1 ? 0 : slot + 1;
+            fresh = c.next(p);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         // ---- epilogue ----
         const int ew = warp - 2, q = warp & 3, h = ew >> 2;
@@ -355,7 +511,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         bool ok = true;
         int cached_n = -1, cached_e = -1;   // the columns coff / cexp hold (warp-uniform)
         for (int u = blockIdx.x; u < p.units && ok; u += gridDim.x) {
-            const Unit w = unit_of(p, u, TN);
+            const Unit w = unit_of<CV>(p, u, TN);
             if (w.kb0 >= w.kb1) continue;
             const int q0 = p.beg[w.cb], q1 = p.beg[w.cb + 1];
             for (int src = q0; src < q1 && ok; src++) {
@@ -394,7 +550,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const int krow = (m < p.M) ? exp_of(p.ea[p.aex[src] + w.b * p.ea_bst + m]) -
                                                  2 * G::C + p.alpha_exp
                                            : 0;
-                if (m < p.M && p.nsplit == 1 && beta != 0.0 && beta != 1.0) {
+                if (!CV && m < p.M && p.nsplit == 1 && beta != 0.0 && beta != 1.0) {
                     for (int i = 0; i < min(WCOLS, nlim); i++)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(Cr + coff[i]));
                 }
@@ -464,7 +620,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (!p.alpha_pow2) v *= p.alpha;
                         return v;
                     };
-                    if (p.nsplit > 1 || beta == 1.0) {
+                    if (CV || p.nsplit > 1 || beta == 1.0) {
                         // C += value: each element gets exactly one addition in
                         // this launch unless K chunks run as separate units, so a
                         // fire-and-forget reduction at L2 gives old + value
@@ -1198,6 +1354,21 @@ int pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb, in
     }
 }
 
+// row exponents of v: cleared, then the maxima of k ranges by atomics
+int launch_pack_exp(kvft_ctx *ctx, const PackView &v, int R, int K, int nb, int *ex) {
+    const int rows_fast = (kidx_fast_stride(v.r) == 1 && kidx_fast_stride(v.c) != 1) ? 1 : 0;
+    KV_CHECK(ctx, cudaMemsetAsync(ex, 0x80, (size_t)nb * R * sizeof(int), ctx->stream));
+    const dim3 g((K + PT_K - 1) / PT_K, (unsigned)((R + PT_R - 1) / PT_R), nb);
+    if (g.y > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: too many rows");
+    // long rows: each exponent block walks up to 16 k tiles, so that about
+    // 32 blocks per SM remain and the atomics per row drop accordingly
+    const long long tiles = (long long)g.x * g.y * g.z;
+    const int ktiles = (int)std::max(1LL, std::min(16LL, tiles / (32LL * ctx->sm_count)));
+    const dim3 ge((g.x + ktiles - 1) / ktiles, g.y, g.z);
+    pack_exp_kernel<<<ge, 256, 0, ctx->stream>>>(v, R, K, rows_fast, ktiles, ex);
+    return kv_launch_check(ctx, "pack_exp");
+}
+
 }  // namespace
 
 int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int D,
@@ -1243,15 +1414,9 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     const long long rtiles = (R + PT_R - 1) / PT_R;
     if (rtiles > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: too many rows");
     if (K <= PC_MAX * PC_SLAB) return pack_rows(ctx, v, R, K, ld, nb, D, rows_fast, (int)rtiles, out);
-    KV_CHECK(ctx, cudaMemsetAsync(out->ex, 0x80, (size_t)nb * R * sizeof(int), ctx->stream));
+    KV_TRY(launch_pack_exp(ctx, v, R, K, nb, out->ex));
     const dim3 g((K + PT_K - 1) / PT_K, (unsigned)rtiles, nb);
-    // long rows: each exponent block walks up to 16 k tiles, so that about
-    // 32 blocks per SM remain and the atomics per row drop accordingly
     const long long tiles = (long long)g.x * g.y * g.z;
-    const int ktiles = (int)std::max(1LL, std::min(16LL, tiles / (32LL * ctx->sm_count)));
-    const dim3 ge((g.x + ktiles - 1) / ktiles, g.y, g.z);
-    pack_exp_kernel<<<ge, 256, 0, ctx->stream>>>(v, R, K, rows_fast, ktiles, out->ex);
-    KV_TRY(kv_launch_check(ctx, "pack_exp"));
     if (tiles > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many tiles");
     switch (D) {
 #define KV_PACK_CASE(s_)                                                                   \
@@ -1265,6 +1430,20 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     }
     KV_TRY(kv_launch_check(ctx, "pack_digits"));
     return KVFT_OK;
+}
+
+int kv_tc_exps(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb,
+               Packed *out) {
+    if (nb > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: batch too large");
+    void *buf = nullptr;
+    KV_TRY(kv_scratch(ctx, key, (size_t)nb * R * sizeof(int), &buf));
+    out->planes = nullptr;
+    out->ex = (int *)buf;
+    out->R = R;
+    out->ld = out->K = K;
+    out->nb = nb;
+    KvProfScope prof(ctx, KV_CAT_PACK, 8.0 * nb * (double)R * K);
+    return launch_pack_exp(ctx, v, R, K, nb, out->ex);
 }
 
 PackView kv_tc_group_view(const double *p, const KIdx &r, const KIdx &c, long long bst, int stable,
@@ -1300,15 +1479,17 @@ constexpr size_t SMEM_CAP = 225 * 1024;
 constexpr size_t SMEM_FLOOR = 120 * 1024;
 
 // Launches the persistent kernel, one CTA per SM.
-template <int TN, bool FF, int KBT, int DL>
+template <int TN, bool FF, int KBT, int DL, bool CV = false>
 int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcParams &p) {
-    auto kern = tc_gemm_kernel<TN, FF, KBT, DL>;
+    if constexpr (!CV && TN <= 64)
+        if (p.A) return launch_tc<TN, FF, KBT, DL, true>(ctx, ma, mb, p);
+    auto kern = tc_gemm_kernel<TN, FF, KBT, DL, CV>;
     int NS = 2;
-    while (NS < 8 && tc_smem(p.S, NS + 1, TN, KBT) <= SMEM_CAP) NS++;
-    if (tc_smem(p.S, NS, TN, KBT) > SMEM_CAP)
+    while (NS < 8 && tc_smem(p.S, NS + 1, TN, KBT, CV) <= SMEM_CAP) NS++;
+    if (tc_smem(p.S, NS, TN, KBT, CV) > SMEM_CAP)
         return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: stages exceed shared memory");
     p.NS = NS;
-    const size_t smem = std::max(tc_smem(p.S, NS, TN, KBT), SMEM_FLOOR);
+    const size_t smem = std::max(tc_smem(p.S, NS, TN, KBT, CV), SMEM_FLOOR);
     static bool attr = false;
     if (!attr) {
         KV_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1317,12 +1498,30 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
     }
     const int grid = std::min(p.units, ctx->sm_count);
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
-    kern<<<grid, NTHREADS, smem, ctx->stream>>>(ma, mb, p);
+    kern<<<grid, NTHREADS + (CV ? 32 * NCV : 0), smem, ctx->stream>>>(ma, mb, p);
     return kv_launch_check(ctx, "tc_gemm");
 }
 
+// Products whose A the kernel converts itself: one tile, K beyond the packing
+// in one pass (so that packing would read A twice, write and read its planes),
+// A not a cached operand, its row a single index and its K contiguous, so that
+// a warp reads a row's neighbouring values.  The K ranges of all products give
+// every SM a unit (a residual of one tau point, 37 virtual and 21 occupied spin
+// orbitals, does not: there packing, which uses all SMs, is 1.5 % faster), and
+// the products are few enough that ranges run as units of their own (C
+// pre-scaled, every write an addition).  Exponents and contraction of the
+// F_ae, F_mi and R1 reductions, before and now: 114 spin orbitals, three tau
+// points a launch, three levels 14.4 -> 12.6 ms a step, six levels 21.8 -> 16.2;
+// 66 and 16, three levels 3.5 -> 3.0; 54 and 10, seven levels 1.6 -> 1.35.
+bool cv_fits(kvft_ctx *ctx, int M, int N, int K, int batch, int nprod, const KMat &A) {
+    return M <= CV_M && N <= 64 && batch < 2 * ctx->sm_count && A.r.size[0] == 1 &&
+           A.r.size[1] == 1 && K > PC_MAX * PC_SLAB && !A.stable &&
+           kidx_fast_stride(A.c) == 1 &&
+           (long long)batch * nprod * ((K + KRANGE - 1) / KRANGE) >= ctx->sm_count;
+}
+
 int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
-                const KMat &B, double beta, const KOut &C, int D, const KvProds &g) {
+                const KMat &B, double beta, const KOut &C, int D, const KvProds &g, bool cv) {
     const int S = dig_planes(D);
     // D >= 4: three to five levels, FP32 pairs, TN = 64 (48 at D = 7, see the
     // kernel) and 32-deep k-blocks (up to five digit
@@ -1330,7 +1529,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     // a full 128-byte line, and TN = 128 unless C has at most 64 columns (then
     // 64-wide tiles keep all eight epilogue warps busy)
     const bool ff = D >= 4;
-    const int tn = D == 7 ? 48 : (ff || N <= 64) ? 64 : 128;
+    const int tn = D == 7 && (!cv || N <= 48) ? 48 : (ff || N <= 64) ? 64 : 128;
     const int kchunk = D == 7 ? Dig<7>::KCHUNK : Dig<6>::KCHUNK;
     const int kb = ff ? 32 : 64;
     const int nbA = A.bst ? batch : 1, nbB = B.bst ? batch : 1;
@@ -1339,13 +1538,14 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const PackView va = kv_tc_group_view(A.p, A.r, A.c, A.bst, A.stable, nbA, g.n, g.oa, wa);
     const PackView vb = kv_tc_group_view(B.p, B.c, B.r, B.bst, B.stable, nbB, g.n, g.ob, wb);
     Packed pa, pb;
-    KV_TRY(kv_tc_pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, D, &pa));
+    if (cv) KV_TRY(kv_tc_exps(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, &pa));
+    else KV_TRY(kv_tc_pack(ctx, "tc_pack_a", va, M, K, va.nsub * nbA, D, &pa));
     KV_TRY(kv_tc_pack(ctx, "tc_pack_b", vb, N, K, vb.nsub * nbB, D, &pb));
     const long long rows_a = (long long)va.nsub * nbA * S * M, rows_b = (long long)vb.nsub * nbB * S * N;
     if (rows_a > 0x7FFFFFFFLL || rows_b > 0x7FFFFFFFLL)
         return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: operand too large");
-    CUtensorMap ma, mb;
-    KV_TRY(kv_tc_map(ctx, &ma, pa.planes, pa.K, pa.ld, rows_a, kb, TM));
+    CUtensorMap ma = {}, mb;
+    if (!cv) KV_TRY(kv_tc_map(ctx, &ma, pa.planes, pa.K, pa.ld, rows_a, kb, TM));
     KV_TRY(kv_tc_map(ctx, &mb, pb.planes, pb.K, pb.ld, rows_b, kb, tn));
     const int mt = (M + TM - 1) / TM, nt = (N + tn - 1) / tn;
     const int nkb_total = (K + kb - 1) / kb;
@@ -1386,14 +1586,18 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         const int x = wa[tab.prod[q]], y = wb[tab.prod[q]];
         p.arow[q] = x * nbA * S * M, p.aex[q] = x * nbA * M;
         p.brow[q] = y * nbB * S * N, p.bex[q] = y * nbB * N;
+        p.oa[q] = g.oa[tab.prod[q]];
     }
+    p.A = cv ? A.p : nullptr;
+    p.ar = A.r.st[2], p.Ac = A.c, p.a_bst = A.bst, p.dv_ac = kidx_div(A.c);
+    p.K = K;
     p.M = M;
     p.N = N;
     p.mt = mt;
     p.nt = nt;
     p.units = (int)units;
     p.nsplit = par ? nranges : 1;
-    p.split_kb = split_kb;
+    p.split_kb = par ? split_kb : nkb_total;
     p.chunk_kb = chunk_kb;
     p.nkb_total = nkb_total;
     p.S = S;
@@ -1428,7 +1632,9 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     case 4: return launch_tc<64, true, 32, 4>(ctx, ma, mb, p);
     case 5: return launch_tc<64, true, 32, 5>(ctx, ma, mb, p);
     case 6: return launch_tc<64, true, 32, 6>(ctx, ma, mb, p);
-    default: return launch_tc<48, true, 32, 7>(ctx, ma, mb, p);
+    default:
+        return tn == 64 ? launch_tc<64, true, 32, 7, true>(ctx, ma, mb, p)
+                        : launch_tc<48, true, 32, 7>(ctx, ma, mb, p);
     }
 }
 
@@ -1455,14 +1661,20 @@ int kv_gemm_tc(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, cons
     // store then covers 32 consecutive doubles) unless that extent is short
     // and K long (the unused TMEM lanes would cost MMA time); otherwise the
     // larger extent goes to the rows.
+    // A long K against few rows (the reductions to F_ae, F_mi and R1): the side
+    // that no cache holds is converted in the kernel.
+    if (cv_fits(ctx, M, N, K, batch, g.n, A))
+        return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g, true);
+    if (cv_fits(ctx, N, M, K, batch, g.n, At))
+        return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt, true);
     bool swap = M < N;
     const bool rc = unit_stride(C.r), cc = unit_stride(C.c);
     if (rc != cc) {
         const int ext = cc ? N : M;
         if (ext >= 64 || K <= 512) swap = cc;
     }
-    if (swap) return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt);
-    return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g);
+    if (swap) return gemm_tc_run(ctx, N, M, K, batch, alpha, At, Bt, beta, Ct, D, gt, false);
+    return gemm_tc_run(ctx, M, N, K, batch, alpha, A, B, beta, C, D, g, false);
 }
 
 int kv_tc_planes(int digits) { return dig_planes(std::min(digits, 7)); }

@@ -310,6 +310,9 @@ struct Packed {
 // the scratch buffer `key`, or into the cache of stable operands.
 int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb, int D,
                Packed *out);
+// The row exponents of v alone, into the scratch buffer `key`.
+int kv_tc_exps(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb,
+               Packed *out);
 // 2D tensor map over digit planes (K x rows, row stride ld elements); one box
 // is a k-block of kb values (swizzled by its 2 kb bytes) by box_rows rows.
 int kv_tc_map(kvft_ctx *ctx, CUtensorMap *map, void *base, int K, int ld, long long rows, int kb,

@@ -108,3 +108,32 @@ def test_pack_long_rows(ctx, M, N, K, batch, digits, tol):
     assert not C[:, 2].any() and not C[:, :, 1].any()
     if digits == 3 and K <= 2048:                 # one K range: one fixed order
         assert (C[:, 5] == C[:, 4] * 2.0 ** 40).all()
+
+
+# A long K against few rows: one operand is converted inside the contraction
+# (not packed).  Rows and columns at the edges (1, 48 / 49, 64, and 65, which
+# packs), K just beyond the packed lengths, odd, at and beside the k-blocks and
+# ranges; either side converted (the other one has more than 64 rows or both
+# fit); products that give every SM a K range and just too few or too many;
+# zero rows.  Tolerances: those of the digit counts.
+@pytest.mark.parametrize("digits,tol", [(2, 2e-3), (3, 5e-5), (5, 5e-9), (6, 5e-11), (7, 5e-12)])
+@pytest.mark.parametrize("M,N,K,batch", [(57, 57, 4097, 60), (1, 64, 4129, 51), (64, 1, 5000, 60),
+                                         (48, 49, 6143, 60), (49, 48, 6144, 51),
+                                         (64, 65, 4999, 52), (65, 64, 5001, 52),
+                                         (19, 19, 6859, 60), (8, 9, 70001, 6),
+                                         (57, 57, 4097, 50), (37, 21, 28749, 1),
+                                         (3, 5, 4200, 303), (3, 5, 4200, 304)])
+def test_converted_operand(ctx, M, N, K, batch, digits, tol):
+    rng = numpy.random.default_rng(M + N + K)
+    A = rng.standard_normal((batch, M, K)) * numpy.exp(3 * rng.standard_normal((batch, M, 1)))
+    B = rng.standard_normal((batch, K, N)) * numpy.exp(3 * rng.standard_normal((batch, 1, N)))
+    A[:, M // 2] = 0.0
+    B[0, :, N // 2] = 0.0
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray.from_host(ctx, numpy.full((batch, M, N), numpy.nan))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, N, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    C = dC.to_host()
+    bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
+    assert (abs(C - A @ B) <= tol * bound).all()
+    assert not C[:, M // 2].any() and not C[0, :, N // 2].any()
