@@ -897,6 +897,15 @@ __device__ __forceinline__ __nv_bfloat162 digit_pair(int d0, int d1) {
     return __floats2bfloat162_rn(f0, f1);
 }
 
+template <int D>
+__device__ __forceinline__ void store_words(uint16_t *ob, size_t plane, unsigned long long x0,
+                                            unsigned long long x1, int e) {
+    uint32_t w[Dig<D>::S];
+    digit_words<D>(x0, x1, e, w);
+#pragma unroll
+    for (int s = 0; s < Dig<D>::S; s++) *reinterpret_cast<uint32_t *>(ob + s * plane) = w[s];
+}
+
 // Base-128 digits here come from the loop above: digit_words, the same values,
 // costs these kernels 1.5 % of a step of 114 spin orbitals.
 template <int D>
@@ -1104,11 +1113,13 @@ pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int r
 // asynchronous copies to shared memory, so a block's whole slab is in flight
 // at once, and three or more blocks an SM overlap loads and conversion (16 rows
 // keep a slab of 416, K = 3249, at 53 KB; 32 rows leave two blocks and cost 15 %).
-// Bound by the copies' issue and the conversion: 3.3 to 3.7 TB/s of 8 + 2 S
-// bytes an element.  Three levels, before and now: 3249 x 3249
-// 2.8 -> 3.3 TB/s, 1089 x 1089 2.6 -> 3.2; seven levels, 729 x 729 2.7 -> 3.5.
-// Whole steps: 38 spin orbitals, solve 53.2 -> 51.2 ms; 54, update 11.2 ->
-// 10.7; 66 23.1 -> 22.4; 114 132.6 -> 129.8.
+// Bound by instruction issue (40 an element, 2.9 a clock, before the maxima came
+// from the high words alone, the copies' predicates from k and the digits from
+// two FP32 additions): 3.3 to 3.9 TB/s of 8 + 2 S bytes an element.  The general
+// path, the first form and now: three levels, 3249 x 3249 2.8, 3.3, 3.3 TB/s,
+// 1089 x 1089 2.6, 3.2, 3.8; seven levels, 729 x 729 2.7, 3.5, 3.9.  Whole cases,
+// general path and first form: 38 spin orbitals, solve 53.2 -> 51.2 ms; 54,
+// update 11.2 -> 10.7; 66 23.1 -> 22.4; 114 132.6 -> 129.8.
 constexpr int PC_MAX = 8, PC_SLAB = 512;      // CTAs of a cluster, k of a slab
 constexpr int PC_R = 16;                      // rows of a cluster
 
@@ -1142,33 +1153,49 @@ pack_cluster_kernel(const __grid_constant__ PackView v, int R, int K, int ld, in
     if (tid < PC_R) roff[tid] = r0 + tid < R ? v.r.off(r0 + tid) : -1;
     __syncthreads();
     const double *base = v.base(b);
-    auto load = [&](int r, int k) {
-        const long long ro = roff[r], ko = koff[k];
-        unsigned long long *d = val + r * ldv + k;
-        if (ro >= 0 && ko >= 0)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d)),
-                         "l"(base + ro + ko)
-                         : "memory");
+    auto load = [&](uint32_t d, const double *g, bool in) {
+        if (in)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(g) : "memory");
         else
-            *d = 0ull;
+            asm volatile("st.shared.b64 [%0], %1;" ::"r"(d), "l"(0ll) : "memory");
     };
     if (rows_fast) {
+        const int r = tid % PC_R;
+        const double *row = base + roff[r];
+        const int lim = roff[r] >= 0 ? kn : 0;
+        uint32_t d = smem_u32(val + r * ldv + tid / PC_R);
 #pragma unroll 8
-        for (int k = tid / PC_R; k < slab; k += 256 / PC_R) load(tid % PC_R, k);
+        for (int k = tid / PC_R; k < slab; k += 256 / PC_R, d += 8 * (256 / PC_R))
+            load(d, row + koff[k], k < lim);
     } else {
-        for (int r = w; r < PC_R; r += 8)
+        const double *row0 = base + roff[w], *row1 = base + roff[w + 8];
+        const int lim0 = roff[w] >= 0 ? kn : 0, lim1 = roff[w + 8] >= 0 ? kn : 0;
+        uint32_t d = smem_u32(val + w * ldv + lane);
 #pragma unroll 4
-            for (int k = lane; k < slab; k += 32) load(r, k);
+        for (int k = lane; k < slab; k += 32, d += 8 * 32) {
+            load(d, row0 + koff[k], k < lim0);
+            load(d + 8 * 8 * ldv, row1 + koff[k], k < lim1);
+        }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < PC_R / 8; i++) {
-        const int rr = w + 8 * i;
-        int e = -2000;
-        for (int k = lane; k < slab; k += 32) e = max(e, raw_exp(val[rr * ldv + k]));
-        e = __reduce_max_sync(0xffffffffu, e);
-        if (lane == 0) rmax[rr] = e;
+    // the largest high word of a row has its exponent (a row of nothing but
+    // subnormals below 2^-1042 counts as zero, as its digits are)
+    static_assert(PC_R == 16, "rows w and w + 8 of a warp");
+    {
+        const uint32_t *h0 = reinterpret_cast<const uint32_t *>(val + w * ldv) + 1;
+        const uint32_t *h1 = h0 + 2 * 8 * ldv;
+        uint32_t m0 = 0, m1 = 0;
+        for (int k = lane; k < slab; k += 32) {
+            m0 = max(m0, h0[2 * k] & 0x7FFFFFFFu);
+            m1 = max(m1, h1[2 * k] & 0x7FFFFFFFu);
+        }
+        m0 = __reduce_max_sync(0xffffffffu, m0);
+        m1 = __reduce_max_sync(0xffffffffu, m1);
+        if (lane == 0) {
+            rmax[w] = m0 ? (int)(m0 >> 20) - 1023 : -2000;
+            rmax[w + 8] = m1 ? (int)(m1 >> 20) - 1023 : -2000;
+        }
     }
     cluster_arrive();
     cluster_wait();
@@ -1198,7 +1225,7 @@ pack_cluster_kernel(const __grid_constant__ PackView v, int R, int K, int ld, in
         uint16_t *ob = out + (size_t)b * Dig<D>::S * plane + (size_t)row * ld + k0;
         // the second value of the last pair is zero beyond K
         for (int k = 2 * lane; k < kn; k += 64)
-            store_digits<D>(ob + k, plane, val[rr * ldv + k], val[rr * ldv + k + 1], e);
+            store_words<D>(ob + k, plane, val[rr * ldv + k], val[rr * ldv + k + 1], e);
     }
     cluster_wait();
 }
