@@ -91,6 +91,7 @@ template <int KIND>
 __global__ void __launch_bounds__(256)
 axpby4_kernel(long long nblk, Dims4 g, double alpha, const double *__restrict__ src,
               double beta, double *__restrict__ dst) {
+    if (!kv_depend()) return;
     const long long n23 = (long long)g.d[2] * g.d[3];
     const long long nch = (n23 + AX_CHUNK - 1) / AX_CHUNK;
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
@@ -123,6 +124,7 @@ axpby4_kernel(long long nblk, Dims4 g, double alpha, const double *__restrict__ 
 __global__ void __launch_bounds__(256)
 make_tau_kernel(long long nblk, int nv, int no, int sh, const double *__restrict__ t1,
                 const double *__restrict__ t2, double c, double *__restrict__ out) {
+    if (!kv_depend()) return;
     extern __shared__ double cab[];                  // [2][no]: c t1[a,:], c t1[b,:]
     const int oo = no * no;
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
@@ -167,6 +169,7 @@ make_tau_kernel(long long nblk, int nv, int no, int sh, const double *__restrict
 __global__ void __launch_bounds__(256)
 wmbej_tmp_kernel(int nv, int no, const double *__restrict__ t1,
                  const double *__restrict__ t2, double *__restrict__ out) {
+    if (!kv_depend()) return;
     __shared__ double tile[32][33];
     const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
     const int ntn = (no + 31) / 32;
@@ -211,6 +214,7 @@ __global__ void __launch_bounds__(256, 3)
 assemble_t2_kernel(int nv, int no, int sh, double fac, const double *__restrict__ Z,
                    const double *__restrict__ Lc, const double *__restrict__ seed,
                    double *__restrict__ T2) {
+    if (!kv_depend()) return;
     const PairOrder ov{nv, sh}, oo_{no, sh};
     __shared__ double qa[32][33], qb[32][33];
     const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
@@ -327,6 +331,7 @@ __device__ __forceinline__ double half_of(double x) {
 __global__ void __launch_bounds__(ST_T)
 wmbej_tmp_spin_kernel(int n, SpinTiles g, const double *__restrict__ t1,
                       const double *__restrict__ t2, double *__restrict__ out) {
+    if (!kv_depend()) return;
     extern __shared__ double tile[];
     const int h = g.h, ld = g.te | 1, nt2 = g.nt * g.nt;
     const int q = blockIdx.x / nt2, tt = blockIdx.x % nt2;
@@ -368,6 +373,7 @@ __global__ void __launch_bounds__(ST_T)
 assemble_t2_spin_kernel(int n, SpinTiles g, double fac, const double *__restrict__ Z,
                         const double *__restrict__ Lc, const double *__restrict__ seed,
                         double *__restrict__ T2) {
+    if (!kv_depend()) return;
     extern __shared__ double tile[];
     const int h = g.h, ld = g.te | 1;
     const PairOrder ov{n, h};
@@ -438,6 +444,7 @@ assemble_t2_spin_kernel(int n, SpinTiles g, double fac, const double *__restrict
 __global__ void bcast_kernel(long long total, long long count,
                              const double *__restrict__ src,
                              double *__restrict__ dst) {
+    if (!kv_depend()) return;
     for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total;
          x += (long long)gridDim.x * blockDim.x)
         dst[x] = src[x % count];
@@ -449,6 +456,7 @@ __global__ void __launch_bounds__(256)
 make_tau_pairs_kernel(long long nblk, int nv, int no, int pv, int po, int sh,
                       const double *__restrict__ t1, const double *__restrict__ t2,
                       double *__restrict__ out) {
+    if (!kv_depend()) return;
     const long long s4 = (long long)nv * nv * no * no;
     const PairOrder ov{nv, sh}, oo_{no, sh};
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
@@ -483,6 +491,7 @@ struct PairGather {
 // one block per (batch, p<q), threads over the (a<b) pairs
 __global__ void __launch_bounds__(256)
 pair_gather_kernel(long long nblk, PairGather g, double *__restrict__ out) {
+    if (!kv_depend()) return;
     for (long long blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
         const long long y = blk / g.P1;
         int p, q;
@@ -539,11 +548,11 @@ int kv_axpby4(kvft_ctx *ctx, int batch, const int dims[4], double alpha,
                            (((long long)dims[2] * dims[3] + AX_CHUNK - 1) / AX_CHUNK);
     const unsigned grid = (unsigned)std::min(nblk, (long long)ctx->sm_count * 16);
     if (beta == 0.0 && (alpha == 1.0 || alpha == -1.0))
-        axpby4_kernel<0><<<grid, 256, 0, ctx->stream>>>(nblk, g, alpha, src, beta, dst);
+        kv_launch(ctx, axpby4_kernel<0>, grid, 256, 0, nblk, g, alpha, src, beta, dst);
     else if (beta == 0.0)
-        axpby4_kernel<1><<<grid, 256, 0, ctx->stream>>>(nblk, g, alpha, src, beta, dst);
+        kv_launch(ctx, axpby4_kernel<1>, grid, 256, 0, nblk, g, alpha, src, beta, dst);
     else
-        axpby4_kernel<2><<<grid, 256, 0, ctx->stream>>>(nblk, g, alpha, src, beta, dst);
+        kv_launch(ctx, axpby4_kernel<2>, grid, 256, 0, nblk, g, alpha, src, beta, dst);
     return kv_launch_check(ctx, "axpby4");
 }
 
@@ -555,8 +564,8 @@ int kv_make_tau(kvft_ctx *ctx, int batch, int nv, int no, const double *t1,
     const long long nblk = (long long)batch * nv * nv;
     if (no > 3072) return kv_fail(ctx, KVFT_EINVAL, "make_tau: more than 3072 occupied orbitals");
     const int sh = (nv == no && nv == 2 * spin_half) ? spin_half : 0;
-    make_tau_kernel<<<(unsigned)std::min(nblk, (long long)ctx->sm_count * 16), 256,
-                      2 * no * sizeof(double), ctx->stream>>>(nblk, nv, no, sh, t1, t2, c, out);
+    kv_launch(ctx, make_tau_kernel, (unsigned)std::min(nblk, (long long)ctx->sm_count * 16), 256,
+              2 * no * sizeof(double), nblk, nv, no, sh, t1, t2, c, out);
     return kv_launch_check(ctx, "make_tau");
 }
 
@@ -570,13 +579,13 @@ int kv_make_wmbej_tmp(kvft_ctx *ctx, int batch, int nv, int no,
         const SpinTiles st(spin_half);
         const size_t smem = sizeof(double) * st.te * (st.te | 1);
         const dim3 gs(2 * st.nt * st.nt, std::min(nv * no, 2048), batch);
-        wmbej_tmp_spin_kernel<<<gs, ST_T, smem, ctx->stream>>>(nv, st, t1, t2, out);
+        kv_launch(ctx, wmbej_tmp_spin_kernel, gs, ST_T, smem, nv, st, t1, t2, out);
         return kv_launch_check(ctx, "wmbej_tmp_spin");
     }
     // each block walks several (b, j): short-lived blocks would leave the SMs
     // waiting for new ones
     const dim3 grid(((nv + 31) / 32) * ((no + 31) / 32), std::min(nv * no, 2048), batch);
-    wmbej_tmp_kernel<<<grid, 256, 0, ctx->stream>>>(nv, no, t1, t2, out);
+    kv_launch(ctx, wmbej_tmp_kernel, grid, 256, 0, nv, no, t1, t2, out);
     return kv_launch_check(ctx, "wmbej_tmp");
 }
 
@@ -599,8 +608,7 @@ int kv_assemble_t2(kvft_ctx *ctx, int batch, int nv, int no, double fac, const d
     const int pv = nv * (nv - 1) / 2;
     const dim3 grid(nt * (nt + 1) / 2, std::min(pv, 65535), batch);
 #define KV_ASM(fs_, seed_)                                                                  \
-    assemble_t2_kernel<fs_, seed_><<<grid, 256, 0, ctx->stream>>>(nv, no, sh, fac, Z, Lc, seed, \
-                                                                  T2)
+    kv_launch(ctx, assemble_t2_kernel<fs_, seed_>, grid, 256, 0, nv, no, sh, fac, Z, Lc, seed, T2)
     const int fs = fac == 1.0 ? 1 : (fac == -1.0 ? 2 : 0);
     if (seed && sh) {
         const SpinTiles st(sh);
@@ -617,11 +625,14 @@ int kv_assemble_t2(kvft_ctx *ctx, int batch, int nv, int no, double fac, const d
             attr = true;
         }
         if (fs == 1)
-            assemble_t2_spin_kernel<1><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
+            kv_launch(ctx, assemble_t2_spin_kernel<1>, gs, ST_T, smem, nv, st, fac, Z, Lc, seed,
+                      T2);
         else if (fs == 2)
-            assemble_t2_spin_kernel<2><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
+            kv_launch(ctx, assemble_t2_spin_kernel<2>, gs, ST_T, smem, nv, st, fac, Z, Lc, seed,
+                      T2);
         else
-            assemble_t2_spin_kernel<0><<<gs, ST_T, smem, ctx->stream>>>(nv, st, fac, Z, Lc, seed, T2);
+            kv_launch(ctx, assemble_t2_spin_kernel<0>, gs, ST_T, smem, nv, st, fac, Z, Lc, seed,
+                      T2);
         return kv_launch_check(ctx, "assemble_t2_spin");
     }
     if (seed) {
@@ -645,8 +656,8 @@ int kv_make_tau_pairs(kvft_ctx *ctx, int batch, int nv, int no, const double *t1
     if (total == 0) return KVFT_OK;
     KvProfScope prof(ctx, KV_CAT_ELEM, 16.0 * total * kv_spin_frac(nv, no, sh));
     const long long nblk = (long long)batch * pv;
-    make_tau_pairs_kernel<<<(unsigned)std::min(nblk, (long long)ctx->sm_count * 16), 256, 0,
-                            ctx->stream>>>(nblk, nv, no, pv, po, sh, t1, t2, out);
+    kv_launch(ctx, make_tau_pairs_kernel, (unsigned)std::min(nblk, (long long)ctx->sm_count * 16),
+              256, 0, nblk, nv, no, pv, po, sh, t1, t2, out);
     return kv_launch_check(ctx, "make_tau_pairs");
 }
 
@@ -676,8 +687,8 @@ int kv_pair_gather(kvft_ctx *ctx, int batch, int n1, int n2, const double *A,
     KvProfScope prof(ctx, KV_CAT_ELEM,
                      8.0 * total * (B ? 3 : 2) * kv_spin_frac(n1, n2, g.sh));
     const long long nblk = (long long)batch * g.P1;
-    pair_gather_kernel<<<(unsigned)std::min(nblk, (long long)ctx->sm_count * 16), 256, 0,
-                         ctx->stream>>>(nblk, g, out);
+    kv_launch(ctx, pair_gather_kernel, (unsigned)std::min(nblk, (long long)ctx->sm_count * 16), 256,
+              0, nblk, g, out);
     return kv_launch_check(ctx, "pair_gather");
 }
 
@@ -686,7 +697,7 @@ int kv_bcast(kvft_ctx *ctx, int batch, size_t count, const double *src,
     long long total = (long long)batch * count;
     if (total == 0) return KVFT_OK;
     KvProfScope prof(ctx, KV_CAT_ELEM, 8.0 * total);
-    bcast_kernel<<<grid_for(ctx, total, 256), 256, 0, ctx->stream>>>(total, (long long)count,
-                                                                     src, dst);
+    kv_launch(ctx, bcast_kernel, grid_for(ctx, total, 256), 256, 0, total, (long long)count, src,
+              dst);
     return kv_launch_check(ctx, "bcast");
 }

@@ -76,6 +76,7 @@ energy2_kernel(int ng, int nv, int no, const double *__restrict__ T1,
                const double *__restrict__ eri, const double *__restrict__ g, int qterm, int sh,
                int gx, int tiles, double *partial, unsigned *count, double inv_beta,
                double *res) {
+    if (!kv_depend()) return;
     __shared__ double E[TILE][TILE + 1];     // [ij][ab]
     __shared__ double red[EN_T];
     __shared__ double gs[WTAB / 4];          // g_y of the chunk
@@ -195,6 +196,7 @@ energy2_spin_kernel(int ng, int n, int h, const double *__restrict__ T1,
                     const double *__restrict__ eri, const double *__restrict__ g, int qterm,
                     long long items, double *partial, unsigned *count, double inv_beta,
                     double *res) {
+    if (!kv_depend()) return;
     extern __shared__ double E[];            // [h][h + 1]: E[j1][b1]
     __shared__ double red[EN_T];
     __shared__ double gs[64], w[64];         // g_y and g_y T1_y[a][i]
@@ -275,12 +277,12 @@ int kv_energy(kvft_ctx *ctx, int ng, int nv, int no, const double *T1, const dou
                                                (int)(sizeof(double) * ESP_HMAX * (ESP_HMAX + 1))));
             attr = true;
         }
-        energy2_spin_kernel<<<grid, EN_T, smem, ctx->stream>>>(ng, nv, sh, T1, T2, f, eri, g, qterm,
-                                                              work, pp, count, 1.0 / beta, dres);
+        kv_launch(ctx, energy2_spin_kernel, grid, EN_T, smem, ng, nv, sh, T1, T2, f, eri, g, qterm,
+                  work, pp, count, 1.0 / beta, dres);
         return kv_launch_check(ctx, "energy2_spin");
     }
-    energy2_kernel<<<grid, EN_T, 0, ctx->stream>>>(ng, nv, no, T1, T2, f, eri, g, qterm, sh, (int)gx,
-                                                   (int)work, pp, count, 1.0 / beta, dres);
+    kv_launch(ctx, energy2_kernel, grid, EN_T, 0, ng, nv, no, T1, T2, f, eri, g, qterm, sh, (int)gx,
+              (int)work, pp, count, 1.0 / beta, dres);
     return kv_launch_check(ctx, "energy2");
 }
 

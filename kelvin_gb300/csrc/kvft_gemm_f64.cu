@@ -82,6 +82,7 @@ __host__ __device__ constexpr size_t f64_smem(int BM, int BN, int BK) {
 // whose threads take K in SL interleaved slices.
 template <int T, int BK, int SL>
 __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F64Params p) {
+    if (!kv_depend()) return;
     extern __shared__ double sm[];
     const int lda = p.BM | 1, ldb = p.BN | 1;
     double *As = sm;                                   // [BK][lda]
@@ -185,6 +186,7 @@ __host__ __device__ constexpr size_t rows_smem(int nthr, int T) {
 // the rows layout: blockDim.x rows, columns n0 .. n0 + T - 1
 template <int T>
 __global__ void __launch_bounds__(NT) gemm_f64_rows_kernel(const __grid_constant__ F64Params p) {
+    if (!kv_depend()) return;
     extern __shared__ __align__(16) double sm[];
     const int nthr = blockDim.x, lda = nthr | 1, tid = threadIdx.x;
     double *Bs = sm;                                   // [RK][T]
@@ -282,6 +284,7 @@ struct ScaleBlocks {
 __global__ void __launch_bounds__(256)
 scale_blocks_kernel(int M, int N, long long items, int batch, double beta, KOut C,
                     const __grid_constant__ ScaleBlocks g, int rows_fast) {
+    if (!kv_depend()) return;
     constexpr int CH = 2048;
     const long long per = (long long)M * N, nch = (per + CH - 1) / CH;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
@@ -319,13 +322,13 @@ void f64_tile(int M, int N, int cap, int *BM, int *BN) {
 template <int T, int BK, int SL = 1>
 int launch_f64_t(kvft_ctx *ctx, const F64Params &p, int grid) {
     const size_t smem = f64_smem(p.BM, p.BN, BK);
-    gemm_f64_kernel<T, BK, SL><<<grid, NT, smem, ctx->stream>>>(p);
+    kv_launch(ctx, gemm_f64_kernel<T, BK, SL>, grid, NT, smem, p);
     return kv_launch_check(ctx, "gemm_f64");
 }
 
 template <int T>
 int launch_rows_t(kvft_ctx *ctx, const F64Params &p, int grid) {
-    gemm_f64_rows_kernel<T><<<grid, p.BM, rows_smem(p.BM, T), ctx->stream>>>(p);
+    kv_launch(ctx, gemm_f64_rows_kernel<T>, grid, p.BM, rows_smem(p.BM, T), p);
     return kv_launch_check(ctx, "gemm_f64_rows");
 }
 
@@ -376,8 +379,9 @@ int kv_scale_blocks(kvft_ctx *ctx, int M, int N, int batch, double beta, const K
         g.n = std::min(64, n - k0);
         for (int k = 0; k < g.n; k++) g.off[k] = off[k0 + k];
         const long long items = (((long long)M * N + 2047) / 2048) * batch * g.n;
-        scale_blocks_kernel<<<(unsigned)std::min(items, (long long)ctx->sm_count * 16), 256, 0,
-                              ctx->stream>>>(M, N, items, batch, beta, C, g, rows_fast);
+        kv_launch(ctx, scale_blocks_kernel, (unsigned)std::min(items,
+                  (long long)ctx->sm_count * 16), 256, 0, M, N, items, batch, beta, C, g,
+                  rows_fast);
         KV_TRY(kv_launch_check(ctx, "scale_view"));
     }
     return KVFT_OK;

@@ -289,6 +289,44 @@ int kv_cuda(kvft_ctx *ctx, cudaError_t e, const char *what);
     } while (0)
 int kv_launch_check(kvft_ctx *ctx, const char *what);
 
+// Launches on the context's stream that may start before their predecessor's
+// last blocks have ended (programmatic dependent launch).  A kernel launched
+// this way begins with `if (!kv_depend()) return;`, which waits until
+// everything before it in the stream is complete and visible: order and
+// results are those of plain launches, and only the launch itself and the start
+// of the blocks overlap the predecessor's tail.  The wait's result is always
+// true, but not to the compiler: loads that it may take for invariant
+// (const __restrict__, __ldg) cannot move above the branch.
+// No kernel triggers its successor early: blocks that start while SMs free up
+// one by one crowd on the first of them, which costs more than the overlap
+// gives (8-site ring 472 -> 509 us, Lambda of 38 spin orbitals 30.9 -> 32.3 ms).
+// They start when the predecessor's last block has left, about 2 us per launch
+// earlier than plain launches: residual of 37 virtual and 21 occupied spin
+// orbitals 919 -> 737 us, solve of 38 49.9 -> 45.9 ms, update of 54 10.4 ->
+// 10.05, 8-site ring (in a graph) 471 -> 453 us.
+#ifdef __CUDACC__
+__device__ __forceinline__ bool kv_depend() {
+    uint32_t blocks;
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nctaid.x;" : "=r"(blocks)::"memory");
+    return blocks != 0;
+}
+
+template <class... P, class... A>
+void kv_launch(kvft_ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);    // errors: kv_launch_check
+}
+#endif
+
 // Device memory of the library.  kv_dev_free keeps a block for the next
 // kv_dev_alloc of about its size instead of returning it to the driver, up to
 // a 32nd of the device per process (kvft_ctx.cu).  kv_mem_info: free bytes

@@ -293,6 +293,7 @@ constexpr int SQ_T = 256;
 __global__ void __launch_bounds__(SQ_T)
 sumsq_kernel(long long total, SQ q, double a, const double *__restrict__ x, double b,
              const double *__restrict__ y, double *__restrict__ part) {
+    if (!kv_depend()) return;
     double acc = 0.0;
     for (long long t = blockIdx.x * (long long)SQ_T + threadIdx.x; t < total;
          t += (long long)gridDim.x * SQ_T) {
@@ -320,6 +321,7 @@ sumsq_kernel(long long total, SQ q, double a, const double *__restrict__ x, doub
 }
 
 __global__ void sum_parts_kernel(const double *__restrict__ part, int n, double *out) {
+    if (!kv_depend()) return;
     __shared__ double red[SQ_T];
     double acc = 0.0;
     for (int k = threadIdx.x; k < n; k += SQ_T) acc += part[k];
@@ -357,9 +359,9 @@ int kv_sumsq4(kvft_ctx *ctx, int batch, const int dims[4], double a, const doubl
     void *part = nullptr;
     KV_TRY(kv_scratch(ctx, "sumsq_part", sizeof(double) * grid, &part));
     KvProfScope prof(ctx, KV_CAT_ELEM, 8.0 * total * (y ? 2 : 1));
-    sumsq_kernel<<<grid, SQ_T, 0, ctx->stream>>>(total, q, a, x, b, y, (double *)part);
+    kv_launch(ctx, sumsq_kernel, grid, SQ_T, 0, total, q, a, x, b, y, (double *)part);
     KV_TRY(kv_launch_check(ctx, "sumsq"));
-    sum_parts_kernel<<<1, SQ_T, 0, ctx->stream>>>((const double *)part, grid, out);
+    kv_launch(ctx, sum_parts_kernel, 1, SQ_T, 0, (const double *)part, grid, out);
     return kv_launch_check(ctx, "sum_parts");
 }
 

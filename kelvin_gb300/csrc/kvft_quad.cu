@@ -149,6 +149,7 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
             const double *__restrict__ G_g, const double *__restrict__ D,
             const double *__restrict__ ev, const double *__restrict__ eo,
             double *out, double *__restrict__ partial) {
+    if (!kv_depend()) return;
     extern __shared__ double sm[];
     const int ng = q.ng;
     double *ti = sm;
@@ -338,6 +339,7 @@ __global__ void quad_tables_kernel(int ng, int rank, int nv, int no, double tc,
                                    const double *__restrict__ ti, const double *__restrict__ ev,
                                    const double *__restrict__ eo, long long NL, long long NR,
                                    double *__restrict__ tab) {
+    if (!kv_depend()) return;
     const long long per = NL + NR;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < ng * per;
          k += (long long)gridDim.x * blockDim.x) {
@@ -412,6 +414,7 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
                   const double *__restrict__ ti_g, const double *__restrict__ G_g,
                   const double *__restrict__ D, const double *__restrict__ ev,
                   const double *__restrict__ eo, double *out, double *__restrict__ partial) {
+    if (!kv_depend()) return;
     extern __shared__ double sm[];
     const int ng = q.ng;
     double *ti = sm;
@@ -563,6 +566,7 @@ __global__ void quad_single_kernel(QuadParams q, int ig, const double *__restric
                                    const double *__restrict__ ev,
                                    const double *__restrict__ eo,
                                    double *__restrict__ out) {
+    if (!kv_depend()) return;
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < q.P;
          p += (long long)gridDim.x * blockDim.x) {
         const int NR = q.rank == 2 ? q.no * q.no : q.no;
@@ -581,6 +585,7 @@ __global__ void quad_single_kernel(QuadParams q, int ig, const double *__restric
 
 __global__ void reduce_pairs_kernel(const double *__restrict__ partial, int n,
                                     double *__restrict__ res) {
+    if (!kv_depend()) return;
     __shared__ double red[2][256];
     double a = 0.0, b = 0.0;
     for (int k = threadIdx.x; k < n; k += 256) {
@@ -682,8 +687,8 @@ int quad_dense_launch(kvft_ctx *ctx, int mode, QuadParams &q, const double *tbar
             const double tc = 0.5 * (hti[0] + hti[ng - 1]);
             const long long work = ng * (NL + NR);
             const int gb = (int)std::max(1LL, std::min((work + 255) / 256, 4096LL));
-            quad_tables_kernel<<<gb, 256, 0, ctx->stream>>>(ng, q.rank, q.nv, q.no, tc, ti, ev,
-                                                            eo, NL, NR, tab);
+            kv_launch(ctx, quad_tables_kernel, gb, 256, 0, ng, q.rank, q.nv, q.no, tc, ti, ev, eo,
+                      NL, NR, tab);
             KV_TRY(kv_launch_check(ctx, "quad_tables"));
             tabs = DenseTabs{tab, tab + ng * NL, tab + 2 * ng * NL, tab + 2 * ng * NL + ng * NR,
                              NL, NR};
@@ -708,16 +713,16 @@ int quad_dense_launch(kvft_ctx *ctx, int mode, QuadParams &q, const double *tbar
     KvProfScope prof(ctx, KV_CAT_QUAD, 8.0 * ng * (double)q.P * (mode == 0 ? 2 : 3) *
                                            kv_spin_frac(q.nv, q.no, q.spin_half));
     if (mode == 0) {
-        quad_dense_kernel<0><<<grid, QT, smem, ctx->stream>>>(q, tabs, tbar, ti, G, D, ev, eo,
-                                                              out, nullptr);
+        kv_launch(ctx, quad_dense_kernel<0>, grid, QT, smem, q, tabs, tbar, ti, G, D, ev, eo, out,
+                  nullptr);
         return kv_launch_check(ctx, "quad_dense_kernel");
     }
     void *part = nullptr;
     KV_TRY(kv_scratch(ctx, "quad_partial", sizeof(double) * 2 * grid, &part));
-    quad_dense_kernel<1><<<grid, QT, smem, ctx->stream>>>(q, tabs, tbar, ti, G, D, ev, eo, out,
-                                                          (double *)part);
+    kv_launch(ctx, quad_dense_kernel<1>, grid, QT, smem, q, tabs, tbar, ti, G, D, ev, eo, out,
+              (double *)part);
     KV_TRY(kv_launch_check(ctx, "quad_dense_update_kernel"));
-    reduce_pairs_kernel<<<1, 256, 0, ctx->stream>>>((const double *)part, grid, res);
+    kv_launch(ctx, reduce_pairs_kernel, 1, 256, 0, (const double *)part, grid, res);
     return kv_launch_check(ctx, "reduce_pairs");
 }
 
@@ -776,23 +781,23 @@ int kv_quad_launch(kvft_ctx *ctx, int mode, int ng, long long P, int rank, int n
                                            kv_spin_frac(nv, no, q.spin_half));
     if (mode == 0) {
         if (q.uniform)
-            quad_kernel<0, true><<<grid, QT, smem, ctx->stream>>>(q, tbar, ti, G, D, ev, eo, out,
-                                                                  nullptr);
+            kv_launch(ctx, quad_kernel<0, true>, grid, QT, smem, q, tbar, ti, G, D, ev, eo, out,
+                      nullptr);
         else
-            quad_kernel<0, false><<<grid, QT, smem, ctx->stream>>>(q, tbar, ti, G, D, ev, eo,
-                                                                   out, nullptr);
+            kv_launch(ctx, quad_kernel<0, false>, grid, QT, smem, q, tbar, ti, G, D, ev, eo, out,
+                      nullptr);
         return kv_launch_check(ctx, "quad_kernel");
     }
     void *part = nullptr;
     KV_TRY(kv_scratch(ctx, "quad_partial", sizeof(double) * 2 * grid, &part));
     if (q.uniform)
-        quad_kernel<1, true><<<grid, QT, smem, ctx->stream>>>(q, tbar, ti, G, D, ev, eo, out,
-                                                              (double *)part);
+        kv_launch(ctx, quad_kernel<1, true>, grid, QT, smem, q, tbar, ti, G, D, ev, eo, out,
+                  (double *)part);
     else
-        quad_kernel<1, false><<<grid, QT, smem, ctx->stream>>>(q, tbar, ti, G, D, ev, eo, out,
-                                                               (double *)part);
+        kv_launch(ctx, quad_kernel<1, false>, grid, QT, smem, q, tbar, ti, G, D, ev, eo, out,
+                  (double *)part);
     KV_TRY(kv_launch_check(ctx, "quad_update_kernel"));
-    reduce_pairs_kernel<<<1, 256, 0, ctx->stream>>>((const double *)part, grid, res);
+    kv_launch(ctx, reduce_pairs_kernel, 1, 256, 0, (const double *)part, grid, res);
     return kv_launch_check(ctx, "reduce_pairs");
 }
 
@@ -828,8 +833,7 @@ int int_tbar_single_entry(kvft_ctx *ctx, int rank, int ng, int ig, int nv, int n
     q.P = (long long)nv * no * (rank == 2 ? (long long)nv * no : 1LL);
     long long blocks = (q.P + 255) / 256;
     int grid = (int)std::min(blocks, (long long)ctx->sm_count * 8);
-    quad_single_kernel<<<grid, 256, 0, ctx->stream>>>(q, ig, tbar, ti, G, D, nullptr, nullptr,
-                                                      out);
+    kv_launch(ctx, quad_single_kernel, grid, 256, 0, q, ig, tbar, ti, G, D, nullptr, nullptr, out);
     return kv_launch_check(ctx, "quad_single");
 }
 
@@ -847,7 +851,7 @@ int kv_quad_single(kvft_ctx *ctx, int ng, int ig, long long P, int rank, int nv,
     q.no = no;
     const int grid = (int)std::min((P + 255) / 256, (long long)ctx->sm_count * 8);
     KvProfScope prof(ctx, KV_CAT_QUAD, 8.0 * (double)P * (ng + 1));
-    quad_single_kernel<<<grid, 256, 0, ctx->stream>>>(q, ig, tbar, ti, G, D, ev, eo, out);
+    kv_launch(ctx, quad_single_kernel, grid, 256, 0, q, ig, tbar, ti, G, D, ev, eo, out);
     return kv_launch_check(ctx, "quad_single");
 }
 

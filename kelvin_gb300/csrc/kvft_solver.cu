@@ -37,6 +37,7 @@ __device__ __forceinline__ void fermi_sqrt(double beta, double e, double mu, dou
 
 __global__ void fermi_kernel(int n, double beta, double mu, const double *__restrict__ eps,
                              double *__restrict__ sfo, double *__restrict__ sfv) {
+    if (!kv_depend()) return;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
         fermi_sqrt(beta, eps[p], mu, &sfo[p], &sfv[p]);
 }
@@ -47,6 +48,7 @@ __global__ void scale_fock_kernel(int n, const double *__restrict__ fock,
                                   const double *__restrict__ sfo,
                                   const double *__restrict__ sfv, double *oo, double *ov,
                                   double *vo, double *vv) {
+    if (!kv_depend()) return;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n * n; k += gridDim.x * blockDim.x) {
         const int p = k / n, q = k % n;
         const double f = fock[k] - (p == q ? eps[p] : 0.0);
@@ -66,6 +68,7 @@ struct Blk9 {
 __global__ void scale_eri_kernel(int n, const double *__restrict__ eri,
                                  const double *__restrict__ sfo,
                                  const double *__restrict__ sfv, Blk9 out) {
+    if (!kv_depend()) return;
     const long long n4 = (long long)n * n * n * n;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n4;
          k += (long long)gridDim.x * blockDim.x) {
@@ -90,6 +93,7 @@ __global__ void scale_eri_kernel(int n, const double *__restrict__ eri,
 }
 
 __global__ void sumsq_kernel(long long n, const double *__restrict__ x, double *__restrict__ part) {
+    if (!kv_depend()) return;
     __shared__ double red[256];
     double a = 0.0;
     for (long long k = blockIdx.x * 256LL + threadIdx.x; k < n; k += (long long)gridDim.x * 256)
@@ -104,6 +108,7 @@ __global__ void sumsq_kernel(long long n, const double *__restrict__ x, double *
 }
 
 __global__ void sum_kernel(const double *__restrict__ part, int n, double *__restrict__ out) {
+    if (!kv_depend()) return;
     __shared__ double red[256];
     double a = 0.0;
     for (int k = threadIdx.x; k < n; k += 256) a += part[k];
@@ -120,15 +125,16 @@ int sumsq(kvft_ctx *ctx, long long n, const double *x, double *dout) {
     int grid = (int)std::max(1LL, std::min((long long)ctx->sm_count * 4, (n + 255) / 256));
     void *part = nullptr;
     KV_TRY(kv_scratch(ctx, "sumsq_partial", sizeof(double) * grid, &part));
-    sumsq_kernel<<<grid, 256, 0, ctx->stream>>>(n, x, (double *)part);
+    kv_launch(ctx, sumsq_kernel, grid, 256, 0, n, x, (double *)part);
     KV_TRY(kv_launch_check(ctx, "sumsq"));
-    sum_kernel<<<1, 256, 0, ctx->stream>>>((double *)part, grid, dout);
+    kv_launch(ctx, sum_kernel, 1, 256, 0, (double *)part, grid, dout);
     return kv_launch_check(ctx, "sum");
 }
 
 // T = alpha T + (1 - alpha) u with a block partial of |u - T_old|^2
 __global__ void damp_norm_kernel(long long n, double alpha, const double *__restrict__ u,
                                  double *__restrict__ T, double *__restrict__ part) {
+    if (!kv_depend()) return;
     __shared__ double red[256];
     double a = 0.0;
     for (long long k = blockIdx.x * 256LL + threadIdx.x; k < n; k += (long long)gridDim.x * 256) {
@@ -152,9 +158,9 @@ int damp_norm(kvft_ctx *ctx, long long n, double alpha, const double *u, double 
     void *part = nullptr;
     KV_TRY(kv_scratch(ctx, "damp_norm_partial", sizeof(double) * grid, &part));
     KvProfScope prof(ctx, KV_CAT_ELEM, 24.0 * n);
-    damp_norm_kernel<<<grid, 256, 0, ctx->stream>>>(n, alpha, u, T, (double *)part);
+    kv_launch(ctx, damp_norm_kernel, grid, 256, 0, n, alpha, u, T, (double *)part);
     KV_TRY(kv_launch_check(ctx, "damp_norm"));
-    sum_kernel<<<1, 256, 0, ctx->stream>>>((double *)part, grid, dout);
+    kv_launch(ctx, sum_kernel, 1, 256, 0, (double *)part, grid, dout);
     return kv_launch_check(ctx, "sum");
 }
 
@@ -358,6 +364,7 @@ int refresh_norms(kvft_solver *s) {
 // over the remaining (r, s) with 32-bit index arithmetic.
 __global__ void spin_check_kernel(const double *__restrict__ x, int n, int h, int rank,
                                   long long rows, int *__restrict__ bad) {
+    if (!kv_depend()) return;
     const int inner = rank == 4 ? n * n : n;
     for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
         int lead = 0;
@@ -384,8 +391,7 @@ int spin_blocked(kvft_ctx *ctx, int n, int h, int count, const double *const *ar
     for (int k = 0; k < count; k++) {
         const long long rows = batch[k] * (rank[k] == 4 ? (long long)n * n : n);
         const int grid = (int)std::min<long long>(rows, (long long)ctx->sm_count * 16);
-        spin_check_kernel<<<grid, 256, 0, ctx->stream>>>(arr[k], n, h, rank[k], rows,
-                                                         (int *)flag);
+        kv_launch(ctx, spin_check_kernel, grid, 256, 0, arr[k], n, h, rank[k], rows, (int *)flag);
         KV_TRY(kv_launch_check(ctx, "spin_check"));
     }
     int h_bad = 0;
@@ -540,6 +546,7 @@ struct AaHist {
 template <int NV>
 __global__ void __launch_bounds__(AA_T, AA_BLOCKS)
 aa_stats_kernel(AaSeg g, AaHist hs, double *part) {
+    if (!kv_depend()) return;
     float v[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const bool has_new = hs.dRnew != nullptr;
     aa_visit(g, [&](long long base, const int (&o)[AA_U], long long cb, int cs, int cnt) {
@@ -585,6 +592,7 @@ template <int NV>
 __global__ void __launch_bounds__(AA_T, AA_BLOCKS)
 aa_update_kernel(AaSeg g, AaHist hs, double beta, float g0, float g1, float g2,
                  double *part) {
+    if (!kv_depend()) return;
     float v[2] = {0.f, 0.f};
     const float gam[3] = {g0, g1, g2};
     const float bf = (float)beta;
@@ -623,6 +631,7 @@ aa_update_kernel(AaSeg g, AaHist hs, double beta, float g0, float g1, float g2,
 // out[k] = sum over blocks of part[b K + k] (fixed order)
 __global__ void aa_reduce_kernel(const double *__restrict__ part, int nb, int K,
                                  double *__restrict__ out) {
+    if (!kv_depend()) return;
     __shared__ double red[256];
     for (int k = 0; k < K; k++) {
         double a = 0.0;
@@ -665,6 +674,7 @@ __host__ __device__ __forceinline__ long long spin_item_base(long long it, long 
 __global__ void __launch_bounds__(256)
 amp_gather_kernel(const double *__restrict__ T2, long long P, int n, int h, long long it0,
                   long long nit, double *__restrict__ out) {
+    if (!kv_depend()) return;
     const int hh = h * h;
     const long long tot = nit * hh;
     for (long long t = blockIdx.x * 256LL + threadIdx.x; t < tot; t += (long long)gridDim.x * 256) {
@@ -990,14 +1000,14 @@ int aa_step_begin(kvft_solver *s, double damp) {
             hs.dRnew = has_new ? g[q].dR[slots[0]] : nullptr;
             double *pq = part + (q ? 7 * gridA[0] : 0);
             switch (nvalid) {
-            case 0: aa_stats_kernel<0><<<gridA[q], AA_T, 0, ctx->stream>>>(g[q], hs, pq); break;
-            case 1: aa_stats_kernel<1><<<gridA[q], AA_T, 0, ctx->stream>>>(g[q], hs, pq); break;
-            case 2: aa_stats_kernel<2><<<gridA[q], AA_T, 0, ctx->stream>>>(g[q], hs, pq); break;
-            default: aa_stats_kernel<3><<<gridA[q], AA_T, 0, ctx->stream>>>(g[q], hs, pq); break;
+            case 0: kv_launch(ctx, aa_stats_kernel<0>, gridA[q], AA_T, 0, g[q], hs, pq); break;
+            case 1: kv_launch(ctx, aa_stats_kernel<1>, gridA[q], AA_T, 0, g[q], hs, pq); break;
+            case 2: kv_launch(ctx, aa_stats_kernel<2>, gridA[q], AA_T, 0, g[q], hs, pq); break;
+            default: kv_launch(ctx, aa_stats_kernel<3>, gridA[q], AA_T, 0, g[q], hs, pq); break;
             }
             KV_TRY(kv_launch_check(ctx, "aa_stats"));
-            aa_reduce_kernel<<<1, 256, 0, ctx->stream>>>(part + (q ? 7 * gridA[0] : 0),
-                                                         gridA[q], 7, s->dsc + 8 + 7 * q);
+            kv_launch(ctx, aa_reduce_kernel, 1, 256, 0, part + (q ? 7 * gridA[0] : 0), gridA[q], 7,
+                      s->dsc + 8 + 7 * q);
             KV_TRY(kv_launch_check(ctx, "aa_reduce"));
         }
     }
@@ -1078,25 +1088,25 @@ int aa_step_finish(kvft_solver *s) {
             double *pq = part + (q ? 2 * gridB[0] : 0);
             switch (nvalid) {
             case 0:
-                aa_update_kernel<0><<<gridB[q], AA_T, 0, ctx->stream>>>(g[q], hs, beta, gf[0],
-                                                                       gf[1], gf[2], pq);
+                kv_launch(ctx, aa_update_kernel<0>, gridB[q], AA_T, 0, g[q], hs, beta, gf[0], gf[1],
+                          gf[2], pq);
                 break;
             case 1:
-                aa_update_kernel<1><<<gridB[q], AA_T, 0, ctx->stream>>>(g[q], hs, beta, gf[0],
-                                                                       gf[1], gf[2], pq);
+                kv_launch(ctx, aa_update_kernel<1>, gridB[q], AA_T, 0, g[q], hs, beta, gf[0], gf[1],
+                          gf[2], pq);
                 break;
             case 2:
-                aa_update_kernel<2><<<gridB[q], AA_T, 0, ctx->stream>>>(g[q], hs, beta, gf[0],
-                                                                       gf[1], gf[2], pq);
+                kv_launch(ctx, aa_update_kernel<2>, gridB[q], AA_T, 0, g[q], hs, beta, gf[0], gf[1],
+                          gf[2], pq);
                 break;
             default:
-                aa_update_kernel<3><<<gridB[q], AA_T, 0, ctx->stream>>>(g[q], hs, beta, gf[0],
-                                                                       gf[1], gf[2], pq);
+                kv_launch(ctx, aa_update_kernel<3>, gridB[q], AA_T, 0, g[q], hs, beta, gf[0], gf[1],
+                          gf[2], pq);
                 break;
             }
             KV_TRY(kv_launch_check(ctx, "aa_update"));
-            aa_reduce_kernel<<<1, 256, 0, ctx->stream>>>(part + (q ? 2 * gridB[0] : 0),
-                                                         gridB[q], 2, s->dsc + 2 * q);
+            kv_launch(ctx, aa_reduce_kernel, 1, 256, 0, part + (q ? 2 * gridB[0] : 0), gridB[q], 2,
+                      s->dsc + 2 * q);
             KV_TRY(kv_launch_check(ctx, "aa_reduce"));
         }
     }
@@ -1416,7 +1426,7 @@ int kvft_solver_read_amplitudes(kvft_solver *s, double *T1h, double *T2h, int ds
         if (sparse) {
             const long long el = cnt * hh;
             const int grid = (int)std::min<long long>((el + 255) / 256, (long long)ctx->sm_count * 8);
-            amp_gather_kernel<<<grid, 256, 0, ctx->stream>>>(s->T2, P, (int)n, h, c0, cnt, dst);
+            kv_launch(ctx, amp_gather_kernel, grid, 256, 0, s->T2, P, (int)n, h, c0, cnt, dst);
             KV_TRY(kv_launch_check(ctx, "amp_gather"));
         } else {
             KV_CHECK(ctx, cudaMemcpyAsync(dst, s->T2 + c0, sizeof(double) * cnt,
@@ -1623,16 +1633,15 @@ int kvft_ft_integrals(kvft_ctx *ctx, int n, const double *eps, const double *foc
     void *sf = nullptr;
     KV_TRY(kv_scratch(ctx, "fermi_sqrt", sizeof(double) * 2 * n, &sf));
     double *sfo = (double *)sf, *sfv = sfo + n;
-    fermi_kernel<<<1, 256, 0, ctx->stream>>>(n, beta, mu, eps, sfo, sfv);
+    kv_launch(ctx, fermi_kernel, 1, 256, 0, n, beta, mu, eps, sfo, sfv);
     KV_TRY(kv_launch_check(ctx, "fermi"));
     const size_t n2 = (size_t)n * n;
     int gb = (int)std::max<size_t>(1, std::min<size_t>((n2 + 255) / 256, 1024));
-    scale_fock_kernel<<<gb, 256, 0, ctx->stream>>>(n, fock, eps, sfo, sfv, F[0], F[1], F[2],
-                                                   F[3]);
+    kv_launch(ctx, scale_fock_kernel, gb, 256, 0, n, fock, eps, sfo, sfv, F[0], F[1], F[2], F[3]);
     KV_TRY(kv_launch_check(ctx, "scale_fock"));
     Blk9 b;
     for (int k = 0; k < 9; k++) b.p[k] = I[k];
-    scale_eri_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(n, eri, sfo, sfv, b);
+    kv_launch(ctx, scale_eri_kernel, ctx->sm_count * 8, 256, 0, n, eri, sfo, sfv, b);
     return kv_launch_check(ctx, "scale_eri");
 }
 

@@ -199,6 +199,7 @@ template <int TN, bool FF, int KBT, int DL, bool CV>
 __global__ void __launch_bounds__(NTHREADS + (CV ? 32 * NCV : 0), 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                TcParams p) {
+    if (!kv_depend()) return;
     using G = Dig<DL>;
     constexpr int SD = G::S, nl = G::NL;     // digit planes and levels
     constexpr int PLANE_BYTES = (CV ? CV_M : TM) * KBT * 2;   // a digit plane of an A k-block
@@ -776,6 +777,7 @@ __device__ __forceinline__ void tile_fetch(const double *base, const long long *
 // loads are issued before the current tile's values are used.
 __global__ void __launch_bounds__(256)
 pack_exp_kernel(const __grid_constant__ PackView v, int R, int K, int rows_fast, int ktiles, int *__restrict__ ex) {
+    if (!kv_depend()) return;
     __shared__ long long off[PT_R + PT_K];
     __shared__ int rmax[8][PT_R];
     const int b = blockIdx.z, r0 = blockIdx.y * PT_R;
@@ -941,6 +943,7 @@ template <int D>
 __global__ void __launch_bounds__(256)
 pack_digits_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int ktn, int rtn,
                    int ntiles, const int *__restrict__ ex, uint16_t *__restrict__ out) {
+    if (!kv_depend()) return;
     __shared__ unsigned long long val[PT_R][PT_K + 1];
     __shared__ long long off[PT_R + PT_K];
     const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
@@ -1014,6 +1017,7 @@ template <int D, int KT>
 __global__ void __launch_bounds__(256, 2)
 pack_rows_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast, int rtiles, int ntiles,
                  int *__restrict__ ex, uint16_t *__restrict__ out) {
+    if (!kv_depend()) return;
     constexpr int NK = KT * PT_K, LDV = NK + 1, PER = NK / 8;   // values per thread
     extern __shared__ unsigned long long prs[];
     unsigned long long *val = prs;                                      // [PT_R][LDV]
@@ -1139,6 +1143,7 @@ __global__ void __launch_bounds__(256)
 pack_cluster_kernel(const __grid_constant__ PackView v, int R, int K, int ld, int rows_fast,
                     int rtiles, int ncta, int slab, int *__restrict__ ex,
                     uint16_t *__restrict__ out) {
+    if (!kv_depend()) return;
     extern __shared__ unsigned long long prs[];
     const int ldv = slab + 1;
     unsigned long long *val = prs;                                       // [PC_R][ldv]
@@ -1298,8 +1303,8 @@ int launch_pack_digits(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, i
         per_sm = std::max(per_sm, 1);
     }
     const int grid = (int)std::min(tiles, (long long)per_sm * ctx->sm_count);
-    pack_digits_kernel<D><<<grid, 256, 0, ctx->stream>>>(v, R, K, ld, rows_fast, ktn, rtn,
-                                                        (int)tiles, out->ex, out->planes);
+    kv_launch(ctx, pack_digits_kernel<D>, grid, 256, 0, v, R, K, ld, rows_fast, ktn, rtn,
+              (int)tiles, out->ex, out->planes);
     return KVFT_OK;
 }
 
@@ -1327,12 +1332,14 @@ int launch_pack_cluster(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, 
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = pack_slab_smem(slab);
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)ncta;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     KV_CHECK(ctx, cudaLaunchKernelEx(&cfg, pack_cluster_kernel<D>, v, R, K, ld, rows_fast,
                                      rtiles, ncta, slab, out->ex, out->planes));
     return kv_launch_check(ctx, "pack_cluster");
@@ -1353,8 +1360,8 @@ int launch_pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int
     const long long ntiles = (long long)rtiles * nb;
     if (ntiles > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many row tiles");
     const int grid = (int)std::min(ntiles, (long long)per_sm * ctx->sm_count);
-    pack_rows_kernel<D, KT><<<grid, 256, smem, ctx->stream>>>(
-        v, R, K, ld, rows_fast, rtiles, (int)ntiles, out->ex, out->planes);
+    kv_launch(ctx, pack_rows_kernel<D, KT>, grid, 256, smem, v, R, K, ld, rows_fast, rtiles,
+              (int)ntiles, out->ex, out->planes);
     return kv_launch_check(ctx, "pack_rows");
 }
 
@@ -1392,7 +1399,7 @@ int launch_pack_exp(kvft_ctx *ctx, const PackView &v, int R, int K, int nb, int 
     const long long tiles = (long long)g.x * g.y * g.z;
     const int ktiles = (int)std::max(1LL, std::min(16LL, tiles / (32LL * ctx->sm_count)));
     const dim3 ge((g.x + ktiles - 1) / ktiles, g.y, g.z);
-    pack_exp_kernel<<<ge, 256, 0, ctx->stream>>>(v, R, K, rows_fast, ktiles, ex);
+    kv_launch(ctx, pack_exp_kernel, ge, 256, 0, v, R, K, rows_fast, ktiles, ex);
     return kv_launch_check(ctx, "pack_exp");
 }
 
@@ -1525,7 +1532,7 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
     }
     const int grid = std::min(p.units, ctx->sm_count);
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
-    kern<<<grid, NTHREADS + (CV ? 32 * NCV : 0), smem, ctx->stream>>>(ma, mb, p);
+    kv_launch(ctx, kern, grid, NTHREADS + (CV ? 32 * NCV : 0), smem, ma, mb, p);
     return kv_launch_check(ctx, "tc_gemm");
 }
 

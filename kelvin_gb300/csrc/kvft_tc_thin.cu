@@ -133,6 +133,7 @@ __host__ __device__ constexpr int thin_threads(int kbt, int D) {
 template <int KBT, int DL>
 __global__ void __launch_bounds__(thin_threads(KBT, DL), thin_threads(KBT, DL) == 512 ? 1 : 2)
 tc_thin_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ThinParams p) {
+    if (!kv_depend()) return;
     constexpr int NT = thin_threads(KBT, DL);
     using G = Dig<DL>;
     constexpr int S = G::S, nl = G::NL;
@@ -500,7 +501,7 @@ int launch_thin(kvft_ctx *ctx, const CUtensorMap &mb, ThinParams &p) {
     }
     const int grid = std::min(p.items, per * ctx->sm_count);
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
-    kern<<<grid, NT, smem, ctx->stream>>>(mb, p);
+    kv_launch(ctx, kern, grid, NT, smem, mb, p);
     return kv_launch_check(ctx, "tc_thin");
 }
 
