@@ -455,7 +455,7 @@ def run_gpu(args, w):
         return 0
     peaks, peak_src = load_peaks()
     kernels = {"gemm6": "tc_gemm_kernel, n^6-class contractions",
-               "gemm": "tc_gemm_kernel, n^5-class contractions", "quad": "quad_kernel",
+               "gemm": "tc_thin_kernel and tc_gemm_kernel, n^5-class contractions", "quad": "quad_kernel",
                "energy": "energy2_kernel", "elem": "element-wise passes",
                "pack": "digit packing (pack_rows/pack_exp/pack_digits)"}
     if args.precision == "fp64":

@@ -183,7 +183,7 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb, bool
 // residual of 21 occupied and 37 virtual spin orbitals; at D = 6 the narrower
 // tile costs 4.5 % of a sweep of 114 spin orbitals and 3 tau points instead).
 // Seven levels in whole: 12.4 -> 11.2 ms for that update (nine-bit digits, 15
-// products for 21), 34.2 -> 32.2 ms for a Lambda sweep of 38 and 8 points.
+// products for 21), 34.2 -> 32.2 ms for two Lambda iterations of 38 and 10 points.
 //
 // DL (the digit levels D) is a template parameter: the MMA issue loop is then
 // straight-line code whose descriptors are per-stage bases plus constant
@@ -475,7 +475,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 uint32_t wd[2][S];
 #pragma unroll
                 for (int y = 0; y < 2 && i + y < NI; y++) {
-                    ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(src + (i + y) * STEP * KBT);
+                    ulonglong2 x =
+                        *reinterpret_cast<const ulonglong2 *>(src + (i + y) * STEP * KBT);
                     if (tail) {                  // beyond K
                         const int k = c.kb * KBT + kp;
                         if (k >= p.K) x.x = 0;
@@ -487,7 +488,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int y = 0; y < 2 && i + y < NI; y++)
 #pragma unroll
                     for (int t = 0; t < S; t++)
-                        *reinterpret_cast<uint32_t *>(dst + t * PLANE_BYTES + so + (i + y) * STEP * KBT * 2) = wd[y][t];
+                        *reinterpret_cast<uint32_t *>(dst + t * PLANE_BYTES + so +
+                                                      (i + y) * STEP * KBT * 2) = wd[y][t];
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -1623,6 +1625,9 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         p.oa[q] = g.oa[tab.prod[q]];
     }
     p.A = cv ? A.p : nullptr;
+    if (cv)                               // bytes it must move: A as FP64, B's planes, C
+        ctx->gemm_work = g.n * (8.0 * M * (double)K * nbA + 2.0 * S * N * (double)K * nbB) +
+                         8.0 * M * N * (double)batch * tab.ncb * (beta != 0.0 ? 2 : 1);
     p.ar = A.r.st[2], p.Ac = A.c, p.a_bst = A.bst, p.dv_ac = kidx_div(A.c);
     p.K = K;
     p.M = M;

@@ -39,9 +39,9 @@
 // accumulations, about 250 clocks each).  Memory traffic would allow 3-4x.
 // Measured, ten contractions of one update, packing included, before (digit
 // planes through memory, general tiles) and now: 54 spin orbitals, 10 tau
-// points, seven levels 8.9 -> 2.7 ms; 66, 16 points, three levels 11.8 -> 6.3;
+// points, seven levels 8.9 -> 2.3 ms; 66, 16 points, three levels 11.8 -> 5.9;
 // 38, 16 points, six levels 5.4 -> 1.3; 114, 3 points, three levels 12.7 ->
-// 8.9, six levels 22 -> 15.5.
+// 8.4, six levels 22 -> 13.8.
 #include "kvft_tc.h"
 
 namespace {
