@@ -17,6 +17,8 @@ namespace {
 //          thread owns one row and all N columns, its A value comes from shared
 //          memory once per k and B's by broadcast; no FMA is padding but those
 //          of the last, partial row block.
+//   square many full 64 x 64 tiles: 256 threads with 4 x 4 outputs each, so an
+//          operand value serves four FMAs and the k-blocks have two barriers.
 //   flat   everything else: a BM x BN tile of any extents (chosen by the host
 //          to divide M and N), its outputs flat over the threads -- o = t + 128
 //          i, i < T, along C's contiguous index -- and both operands of every
@@ -171,6 +173,76 @@ __global__ void __launch_bounds__(NT) gemm_f64_kernel(const __grid_constant__ F6
 #pragma unroll
     for (int i = 0; i < T; i++)
         if (ok >> i & 1) f64_out(p, C + cr[mn[i] & 0xFFFF] + cc[mn[i] >> 16], acc[i]);
+}
+
+// the square layout: 64 x 64 tiles, thread (tx, ty) owns rows ty + 16 i and
+// columns tx + 16 j
+constexpr int SQ = 64, SQ_K = 16, SQ_T = 256;
+
+__global__ void __launch_bounds__(SQ_T)
+gemm_f64_square_kernel(const __grid_constant__ F64Params p) {
+    if (!kv_depend()) return;
+    __shared__ double As[SQ_K][SQ + 1], Bs[SQ_K][SQ + 1];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const F64Tile t(p, blockIdx.x);
+    const int m0 = t.tm * SQ, n0 = t.tn * SQ;
+    const int kbeg = t.ks * p.klen, kend = min(p.K, kbeg + p.klen);
+    // a thread loads rows and columns ty + 16 r at k = tid % 16 where k is
+    // contiguous, else row or column tid % 64 at k = tid / 64 + 4 r
+    long long ao[4], bo[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const int m = m0 + (p.a_kfast ? ty + 16 * r : tid % SQ);
+        const int n = n0 + (p.b_kfast ? ty + 16 * r : tid % SQ);
+        ao[r] = m < p.M ? p.dar.off(p.Ar, m) : -1;
+        bo[r] = n < p.N ? p.dbc.off(p.Bc, n) : -1;
+    }
+    double acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
+    for (int s = p.beg[t.cb]; s < p.beg[t.cb + 1]; s++) {
+        const double *A = p.A + (long long)t.b * p.a_bst + p.oa[s];
+        const double *B = p.B + (long long)t.b * p.b_bst + p.ob[s];
+        for (int k0 = kbeg; k0 < kend; k0 += SQ_K) {
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int ka = p.a_kfast ? tx : tid / SQ + 4 * r;
+                const int kb = p.b_kfast ? tx : tid / SQ + 4 * r;
+                As[ka][p.a_kfast ? ty + 16 * r : tid % SQ] =
+                    ao[r] >= 0 && k0 + ka < kend ? A[ao[r] + p.dac.off(p.Ac, k0 + ka)] : 0.0;
+                Bs[kb][p.b_kfast ? ty + 16 * r : tid % SQ] =
+                    bo[r] >= 0 && k0 + kb < kend ? B[bo[r] + p.dbr.off(p.Br, k0 + kb)] : 0.0;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < SQ_K; k++) {
+                double a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) a[i] = As[k][ty + 16 * i];
+#pragma unroll
+                for (int j = 0; j < 4; j++) b[j] = Bs[k][tx + 16 * j];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+            }
+            __syncthreads();
+        }
+    }
+    double *C = p.C.p + (long long)t.b * p.C.bst + p.oc[t.cb];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int m = m0 + ty + 16 * i;
+        if (m >= p.M) continue;
+        const long long ro = p.dcr.off(p.C.r, m);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int n = n0 + tx + 16 * j;
+            if (n < p.N) f64_out(p, C + ro + p.dcc.off(p.C.c, n), acc[i][j]);
+        }
+    }
 }
 
 constexpr int RK = 16;           // k values per shared-memory block of the rows layout
@@ -423,25 +495,50 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
             break;
         }
     }
-    p.mt = rows ? ceil_div(M, p.BM) : 0;
+    // The square layout where its tiles are full (at most 2 % of their FMAs on
+    // padding) and enough to balance the SMs (six each): 3249^3 61.6 ms in flat
+    // tiles, 59.3 here; with 625 tiles (1596^3) flat ones are as fast.  Also
+    // where one tile holds C (at most 30 % padding) and a long K gives every SM
+    // ranges of 256: 57 x 57, K = 57^3, two products, 2.85 ms in flat tiles,
+    // 2.66 here; 40 x 40 (61 % padding) is better off flat.
+    const long long sq = (long long)ceil_div(M, SQ) * ceil_div(N, SQ);
+    const long long sqk = (long long)batch * g.n * (K / 256);
+    const bool square_k = !rows && sq == 1 && M * N >= 0.7 * SQ * SQ && K >= 1024 &&
+                          sqk >= want && nprod < 2 * want;
+    const bool square = square_k || (!rows && sq * nprod >= 6LL * ctx->sm_count &&
+                                     (double)sq * SQ * SQ <= 1.02 * M * (double)N);
+    if (square) p.BM = p.BN = SQ, p.nt = ceil_div(N, SQ);
+    p.mt = rows || square ? ceil_div(M, p.BM) : 0;
     int T = TMAX;
     long long tiles = (long long)p.mt * p.nt * batch;
-    if (!rows) {
+    if (!rows && !square) {
         // The largest tile (16 outputs per thread) that leaves four blocks per
-        // SM to balance the SMs, down to two outputs per thread; then K is
-        // split into chunks of at least 32 while fewer than two blocks per SM
-        // remain.
+        // SM to balance the SMs, where K ranges of 256 of a long K count as
+        // blocks (every product's, since they then add by atomics) when neither
+        // extent is short; smaller tiles, down to two outputs per thread, else.  Shrinking first reads a long operand once per tile: 57 x 57
+        // outputs, K = 57^3, two products, 5.7 ms in tiles of 57 x 4, 2.85 so.
+        const bool longk = K >= 1024 && std::min(M, N) > 32;
         for (;; T /= 2) {
             f64_tile(M, N, NT * T, &p.BM, &p.BN);
             p.mt = ceil_div(M, p.BM);
             p.nt = ceil_div(N, p.BN);
             tiles = (long long)p.mt * p.nt * batch;
-            if (T == 2 || tiles * tab.ncb >= 2 * want) break;
+            if (T == 2 || tiles * tab.ncb >= 2 * want ||
+                (longk && tiles * g.n * (K / 256) >= 2 * want))
+                break;
         }
+        while (T > 2 && p.BM * p.BN <= NT * T / 2) T /= 2;
         const int bk = T <= 4 ? 32 : 16;
-        if (tiles * tab.ncb < want && K > 32)
+        if (longk && tiles * tab.ncb < 2 * want)
+            p.nsplit = (int)std::min<long long>(ceil_div(4 * want, tiles * g.n), K / 256);
+        else if (tiles * tab.ncb < want && K > 32)
             p.nsplit = (int)std::min<long long>(ceil_div(want, tiles * tab.ncb), ceil_div(K, 32));
         p.klen = ceil_div(ceil_div(K, p.nsplit), bk) * bk;
+        p.nsplit = ceil_div(K, p.klen);
+    }
+    if (square_k) {
+        p.nsplit = (int)std::min<long long>(ceil_div(want, (long long)batch * g.n), K / 256);
+        p.klen = ceil_div(ceil_div(K, p.nsplit), SQ_K) * SQ_K;
         p.nsplit = ceil_div(K, p.klen);
     }
     p.store = beta == 0.0 ? 1 : beta == 1.0 ? 2 : 3;
@@ -477,6 +574,10 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         if (p.BN <= 8) return launch_rows_t<8>(ctx, p, (int)grid);
         if (p.BN <= 16) return launch_rows_t<16>(ctx, p, (int)grid);
         return launch_rows_t<24>(ctx, p, (int)grid);
+    }
+    if (square) {
+        kv_launch(ctx, gemm_f64_square_kernel, (unsigned)grid, SQ_T, 0, p);
+        return kv_launch_check(ctx, "gemm_f64_square");
     }
     switch (T) {
     case 16: return launch_f64_t<16, 16>(ctx, p, (int)grid);

@@ -26,7 +26,12 @@ pytestmark = pytest.mark.gpu
     # K in two or four slices of a block: 32, 33, 64 and 65 outputs a tile, K
     # below the slice count and around the block of 32
     (4, 8, 1, 2), (4, 8, 3, 2), (8, 4, 33, 2), (3, 11, 31, 1), (8, 8, 5, 3), (8, 8, 65, 3),
-    (5, 13, 34, 1)])
+    (5, 13, 34, 1),
+    # 64 x 64 tiles: full ones, ragged by one and two in each direction, K
+    # around its block of 16, a batch; just too few tiles; a long K whose ranges
+    # count as blocks
+    (2048, 2048, 17, 1), (2047, 2046, 31, 1), (1024, 1023, 48, 4), (1920, 1920, 20, 1),
+    (57, 57, 9000, 2), (300, 57, 1024, 2), (200, 130, 1023, 1)])
 def test_gemm_fp64_tiles(ctx, M, N, K, batch):
     rng = numpy.random.default_rng(M + 3 * N + 7 * K + batch)
     A = rng.standard_normal((batch, M, K))
