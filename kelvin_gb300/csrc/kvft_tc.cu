@@ -13,7 +13,7 @@
 //     level s + t have one weight; levels up to NL + 1 are kept.  A base-128
 //     product is an integer below 2^12 (times a power of two), so an FP32
 //     accumulator over K <= 2048 terms and two pairs is exact; nine-bit digits
-//     are read out after 512 terms.
+//     are read out after 128 terms (kvft_tc.h: which levels that keeps exact).
 //     Every level l = s + t has its own TMEM accumulator, at column
 //     (l - 2) TN of the set, and the digit planes of a B tile lie one after
 //     another in shared memory, so a single tcgen05.mma of A plane s against
@@ -162,7 +162,7 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb, bool
 //   warp 0      TMA producer: all S digit planes of A and B of one k-block per
 //               stage.
 //   warp 1      TMEM owner and MMA issuer: the level products of K chunk c
-//               (at most KCHUNK deep, so each level sum is exact in FP32) go
+//               (at most KCHUNK deep, so the leading level sums are exact) go
 //               to accumulator set c % NSET; a commit marks the set full.
 //   warps 2-9   epilogue: warp w reads TMEM lanes 32 (w % 4).. of column half
 //               (w - 2) / 4, frees the set, and carries the sum over the
@@ -177,13 +177,12 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb, bool
 // of one chunk run while the epilogue drains the other.  D >= 4: TN = 64, three
 // to five levels, two sets up to D = 5; at D = 6 there is room for one, which
 // the epilogue frees as soon as the levels are in registers (a few percent of
-// a 2048-deep chunk's MMA time).  D = 7 reads out four times as often and so
+// a 2048-deep chunk's MMA time).  D = 7 reads out sixteen times as often and so
 // takes TN = 48, where two sets of five levels fit (against 64 columns and one
-// set: 1 % of an update of 54 spin orbitals and 10 tau points, 5 % of a
-// residual of 21 occupied and 37 virtual spin orbitals; at D = 6 the narrower
-// tile costs 4.5 % of a sweep of 114 spin orbitals and 3 tau points instead).
-// Seven levels in whole: 12.4 -> 11.2 ms for that update (nine-bit digits, 15
-// products for 21), 34.2 -> 32.2 ms for two Lambda iterations of 38 and 10 points.
+// set, both with read-outs every 512 terms: 1 % of an update of 54 spin
+// orbitals and 10 tau points, 5 % of a residual of 21 occupied and 37 virtual
+// spin orbitals; at D = 6 the narrower tile costs 4.5 % of a sweep of 114 spin
+// orbitals and 3 tau points instead).
 //
 // DL (the digit levels D) is a template parameter: the MMA issue loop is then
 // straight-line code whose descriptors are per-stage bases plus constant
@@ -588,7 +587,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 if (nl > 1) hi += __uint_as_float(r[nl > 1 ? 1 : 0][j]);
                                 rhi[i] = first ? hi : rhi[i] + hi;
                             } else {
-                                // exact level sums, leading first: an FP32 pair
+                                // level sums, leading first: an FP32 pair
                                 float lo = 0.f, e;
     #pragma unroll
                                 for (int l = 1; l < nl; l++) {
@@ -1588,8 +1587,8 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const long long tiles = (long long)mt * nt * batch;
     // K ranges.  Fewer output tiles than two waves of SMs and several ranges of
     // 2048: every range of every product becomes a unit of its own and adds
-    // into C with FP64 atomics (C pre-scaled by beta).  With error-free level
-    // sums (D >= 4) the ranges may be shorter: while there are fewer units than
+    // into C with FP64 atomics (C pre-scaled by beta).  At D >= 4 the
+    // ranges may be shorter (the exact sums stay so): while there are fewer units than
     // SMs, down to 256 deep (below that the pipeline's start and the atomics
     // cost what the other SMs would save).  D <= 3 keeps 2048, which is part
     // of its rounding.  37 x 37 outputs against K = 16317, one product, seven

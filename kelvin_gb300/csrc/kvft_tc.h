@@ -24,19 +24,33 @@ constexpr int TM = 128;
 //           digits need 21 for six planes.
 // BF16 holds balanced nine-bit digits, so the wide ones spend no product on
 // bits that the type leaves empty.  What bounds the width is the rounding of
-// the FP32 sums, hence the narrower leading digit and the shorter KCHUNK.
-// Error against seven-bit digits in an exact emulation with round-to-nearest
-// and with truncating FP32 sums (K = 57 to 3249; normal, uniform, constant,
-// few-valued and wide-range operands, A A^T): 0.1 to 0.8 of it, in the 2-norm
-// and for the largest element.  At D = 6 the digits stay as they are: results
-// there are only good to ~1e-9, and any other digits would move them by that.
+// the FP32 sums: they are exact up to 2^24, and a level's weight falls by 2^-9
+// (2^-7) from one level to the next.  KCHUNK keeps exact by the digits' bounds
+// what weighs enough to show beside the planes' own rounding (2^-45, seven-bit
+// planes at D = 7 2^-43):
+//   D = 7   128 terms of level 3 (two products of at most 2^7 2^8) reach 2^23,
+//           of level 4 (2^7 2^8 twice and 2^8 2^8) 2^24; level 5 may round at
+//           weight 2^-43.  With 512 terms level 3 could reach 2^25, and rows
+//           of close-by values (1.9605 (1 + 1e-4 x)) came out 10^5 times less
+//           accurate than with seven-bit digits; with 256 terms level 4 could,
+//           up to 180 times (rows that agree in three digits).
+//   D <= 6  2048 terms of level 3 (two products of at most 2^12) reach 2^24.
+// Reading out every 128 terms costs an update of 54 spin orbitals and 10 tau
+// points 10.0 -> 10.9 ms against 512, two Lambda iterations of 38 and 10
+// 29.3 -> 30.75, a residual of 37 virtual and 21 occupied 0.724 -> 0.753;
+// seven-bit digits cost the first two 1.2 and 2.0 ms.
+// Error against seven-bit digits with exact sums (K = 33 to 4129; normal,
+// constant, few-valued and wide-range operands, A A^T, rows of close-by
+// values): 0.2 to 0.8 of it, in the 2-norm and for the largest element.  At D =
+// 6 the digits stay as they are: results there are only good to ~1e-9, and any
+// other digits would move them by that.
 template <int D>
 struct Dig {
     static_assert(D >= 2 && D <= 7, "digit count");
     static constexpr bool WIDE = D == 7;
     static constexpr int S = WIDE ? 5 : D - 1;
     static constexpr int NL = S;                       // levels (accumulators)
-    static constexpr int KCHUNK = WIDE ? 512 : 2048;
+    static constexpr int KCHUNK = WIDE ? 128 : 2048;
     static constexpr int C = WIDE ? 8 : 7;
     // bits after the point down to and including digit s = 1 .. S
     __host__ __device__ static constexpr int pos(int s) { return WIDE ? 9 * s - 1 : 7 * s; }

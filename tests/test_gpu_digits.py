@@ -1,4 +1,4 @@
-"""The wide digits of seven levels (nine-bit, read out every 512 terms) are at
+"""The wide digits of seven levels (nine-bit, read out every 128 terms) are at
 least as accurate as seven-bit digits of the same level count: the error of the device product is at most that of seven-bit
 digits with exact sums, computed here, in the 2-norm and for the largest
 element.  Operands: normal, A A^T (equal signs in every square), few-valued,
@@ -137,3 +137,50 @@ def test_converted_operand(ctx, M, N, K, batch, digits, tol):
     bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
     assert (abs(C - A @ B) <= tol * bound).all()
     assert not C[:, M // 2].any() and not C[0, :, N // 2].any()
+
+
+# Rows whose values lie close together: their leading digits agree, so the
+# products of a level all have one sign and a level's sum grows with K times
+# the largest product.  Kinds by the digits that agree: two, three and four of
+# the wide ones, and values of a few close-by numbers.  K at and beside the
+# read-out length, in one range and several, packed and (the batch)
+# converted inside the contraction.  The bound is the one of the test above.
+def close_operands(kind, K, batch, M):
+    rng = numpy.random.default_rng(K + batch)
+
+    def draw(shape):
+        n, u = rng.standard_normal(shape), rng.random(shape)
+        return {"rel 1e-4": lambda: 1.9605 * (1 + 1e-4 * n), "rel 1e-6": lambda: 1.9605 * (1 + 1e-6 * n),
+                "half": lambda: 0.49 + 2e-4 * u, "one": lambda: 0.98 + 5e-4 * n,
+                "pi": lambda: numpy.pi * (1 + 1e-3 * u),
+                "three": lambda: numpy.array([1.9591, 1.9602, 1.9608])[rng.integers(0, 3, shape)],
+                # leading digits 127, 255, 255
+                "top": lambda: 127 * 2.0 ** -8 + 255 * 2.0 ** -17 + 255 * 2.0 ** -26 + 2.0 ** -35 * u,
+                }[kind]()
+
+    return draw((batch, M, K)), draw((batch, K, M))
+
+
+@pytest.mark.parametrize("kind", ["rel 1e-4", "rel 1e-6", "half", "one", "pi", "three", "top"])
+@pytest.mark.parametrize("K,batch,M", [(128, 1, 48), (129, 1, 48), (257, 1, 48), (361, 1, 48),
+                                       (512, 1, 48), (1024, 1, 48), (3249, 1, 24), (4129, 60, 8)])
+def test_wide_digits_of_close_values(ctx, K, batch, M, kind, digits=7):
+    A, B = close_operands(kind, K, batch, M)
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, (batch, M, M))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, M, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    C = dC.to_host()
+    s = s7 = m = m7 = 0.0
+    for b in range(batch):
+        ref = A[b].astype(numpy.longdouble) @ B[b].astype(numpy.longdouble)
+        (x, ex), (y, ey) = seven_bit(A[b], digits), seven_bit(B[b].T, digits)
+        old = sum((x[i - 1] @ y[j - 1].T).astype(numpy.longdouble)
+                  for i in range(1, digits) for j in range(1, digits) if i + j <= digits)
+        old = old * numpy.longdouble(2) ** (ex[:, None] + ey[None, :])
+        bound = abs(A[b]).max(1)[:, None] * abs(B[b]).max(0)[None, :]
+        err, err7 = abs(C[b] - ref) / bound, abs(old - ref) / bound
+        s, s7 = s + (err ** 2).sum(), s7 + (err7 ** 2).sum()
+        m, m7 = max(m, err.max()), max(m7, err7.max())
+    assert s <= s7
+    assert m <= m7
