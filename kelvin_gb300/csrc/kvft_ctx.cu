@@ -26,9 +26,11 @@ int kv_cuda(kvft_ctx *ctx, cudaError_t e, const char *what) {
 // 5.1 ms); a solve of 38 spin orbitals makes 65 of each (6 of 57 ms).  Freed
 // blocks are kept, per device and shared by all contexts of the process, and
 // handed out again to requests of at least 7/8 of their size.
-//   * A block becomes free only after a device-wide synchronisation, as with
+//   * A block becomes free only once all work of the device has ended, as with
 //     cudaFree, so no stream -- a caller's included -- still uses it when it is
-//     handed out again.
+//     handed out again.  The wait is that of a cudaFree (of a small block, 1.7
+//     us with its cudaMalloc on an idle device), which leaves stream captures
+//     of other threads alone; cudaDeviceSynchronize would invalidate them.
 //   * At most a 32nd of the device is kept, the oldest blocks going first; all
 //     of it is returned when an allocation fails and when the device's last
 //     context is destroyed.
@@ -51,6 +53,19 @@ void pool_release(DevPool &d) {
     for (auto &k : d.kept) cudaFree(k.second);
     d.kept.clear();
     d.kept_bytes = 0;
+}
+
+}  // namespace
+
+namespace {
+
+// Waits for all work of the current device, on every stream.
+cudaError_t device_wait() {
+    void *p = nullptr;
+    cudaError_t e = cudaMalloc(&p, 512);
+    if (e == cudaSuccess) e = cudaFree(p);
+    if (e != cudaSuccess) cudaGetLastError();       // the caller deals with it
+    return e;
 }
 
 }  // namespace
@@ -88,19 +103,14 @@ int kv_dev_alloc(kvft_ctx *ctx, size_t bytes, void **p) {
 int kv_dev_free(kvft_ctx *ctx, void *p) {
     if (!p) return KVFT_OK;
     DevPool &d = pool_of(ctx->device);
-    const cudaError_t sync = cudaDeviceSynchronize();
+    const bool idle = device_wait() == cudaSuccess;
     std::lock_guard<std::mutex> lock(d.mu);
     auto it = d.live.find(p);
-    if (it == d.live.end()) {
-        // not the library's: another allocator's block, or one already freed
+    if (it == d.live.end())          // another allocator's block, or one already freed
         for (auto &k : d.kept)
             if (k.second == p) return kv_fail(ctx, KVFT_EINVAL, "kvft_free: already freed");
-        KV_CHECK(ctx, cudaFree(p));
-        return KVFT_OK;
-    }
-    const size_t bytes = it->second;
-    d.live.erase(it);
-    if (sync == cudaSuccess && bytes <= d.cap) {
+    const size_t bytes = it == d.live.end() ? 0 : it->second;
+    if (bytes && idle && bytes <= d.cap) {
         while (d.kept_bytes + bytes > d.cap) {
             d.kept_bytes -= d.kept.front().first;
             cudaFree(d.kept.front().second);
@@ -108,9 +118,14 @@ int kv_dev_free(kvft_ctx *ctx, void *p) {
         }
         d.kept.emplace_back(bytes, p);
         d.kept_bytes += bytes;
-        return KVFT_OK;
+    } else {
+        const cudaError_t e = cudaFree(p);
+        if (e != cudaSuccess) {      // still the caller's
+            cudaGetLastError();
+            return kv_cuda(ctx, e, "cudaFree");
+        }
     }
-    KV_CHECK(ctx, cudaFree(p));
+    if (bytes) d.live.erase(it);
     return KVFT_OK;
 }
 

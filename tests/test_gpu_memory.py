@@ -1,5 +1,6 @@
 """Device blocks kept for reuse: sizes, contents, limits, misuse."""
 import ctypes
+import threading
 
 import numpy
 import pytest
@@ -57,5 +58,66 @@ def test_a_kept_block_is_not_larger_than_the_limit():
         x = _lib.DeviceArray.from_host(ctx, numpy.arange(5.0))
         assert numpy.array_equal(x.to_host(), numpy.arange(5.0))
         x.free()
+    finally:
+        ctx.close()
+
+
+def test_free_leaves_another_threads_capture_alone():
+    """A block freed while another thread captures a graph: the capture goes
+    on, the block is kept, and the freeing thread's next launch is fine."""
+    torch = pytest.importorskip("torch")
+    ctx = _lib.Context(0)
+    try:
+        a = alloc(ctx, 48 << 20)
+        y = _lib.DeviceArray.from_host(ctx, numpy.arange(4096.0).reshape(64, 64))
+        z = _lib.DeviceArray(ctx, (64, 64))
+        x = torch.zeros(8, device="cuda")
+        side = torch.cuda.Stream()
+        x.add_(1)
+        torch.cuda.synchronize()
+        status = []
+
+        def free():
+            status.append(ctx.L.kvft_free(ctx.h, a))
+            status.append(ctx.L.kvft_gemm(ctx.h, 64, 64, 64, 1, _lib.PREC_FP64, 7, y.ptr, y.ptr,
+                                          z.ptr))
+
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side, capture_error_mode="relaxed"):
+            x.add_(1)
+            t = threading.Thread(target=free)
+            t.start()
+            t.join()
+            x.add_(1)
+        assert status == [0, 0]
+        g.replay()
+        torch.cuda.synchronize()
+        assert (x == 3).all()
+        h = numpy.arange(4096.0).reshape(64, 64)
+        assert numpy.allclose(z.to_host(), h @ h, rtol=1e-13)
+        b = alloc(ctx, 48 << 20)
+        assert b == a
+        assert ctx.L.kvft_free(ctx.h, b) == 0
+        y.free()
+        z.free()
+    finally:
+        ctx.close()
+
+
+def test_free_waits_for_every_stream():
+    """A freed block is not handed out while a stream of the caller's own may
+    still use it."""
+    torch = pytest.importorskip("torch")
+    ctx = _lib.Context(0)
+    try:
+        a = alloc(ctx, 8 << 20)
+        side = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(40 * 1000 * 1000)          # clocks: about 20 ms
+        done = side.record_event()
+        assert not done.query()
+        assert ctx.L.kvft_free(ctx.h, a) == 0
+        assert done.query()
     finally:
         ctx.close()
