@@ -150,6 +150,25 @@ int kv_launch_check(kvft_ctx *ctx, const char *what) {
     return KVFT_OK;
 }
 
+int kv_smem_optin_ptr(kvft_ctx *ctx, const void *kern, size_t bytes) {
+    size_t &have = ctx->smem_optin[kern];
+    if (have >= bytes) return KVFT_OK;
+    KV_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    have = bytes;
+    return KVFT_OK;
+}
+
+int kv_blocks_per_sm_ptr(kvft_ctx *ctx, const void *kern, int threads, size_t smem, int *n) {
+    int &have = ctx->blocks_per_sm[kern];
+    if (!have) {
+        int b = 0;
+        KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, threads, smem));
+        have = std::max(b, 1);
+    }
+    *n = have;
+    return KVFT_OK;
+}
+
 int kv_scratch(kvft_ctx *ctx, const char *key, size_t bytes, void **p) {
     auto it = ctx->scratch.find(key);
     if (it != ctx->scratch.end() && it->second.second >= bytes) {

@@ -614,16 +614,10 @@ int kv_assemble_t2(kvft_ctx *ctx, int batch, int nv, int no, double fac, const d
         const SpinTiles st(sh);
         const size_t smem = 2 * sizeof(double) * st.te * (st.te | 1);
         const dim3 gs(st.nt * st.nt, std::min(pv, 65535), batch);
-        static bool attr = false;
-        if (!attr) {
-            const void *k[3] = {(const void *)assemble_t2_spin_kernel<0>,
-                                (const void *)assemble_t2_spin_kernel<1>,
-                                (const void *)assemble_t2_spin_kernel<2>};
-            for (const void *f : k)
-                KV_CHECK(ctx, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   2 * 8 * 64 * 65));
-            attr = true;
-        }
+        KV_TRY(kv_smem_optin(ctx, fs == 1   ? assemble_t2_spin_kernel<1>
+                                  : fs == 2 ? assemble_t2_spin_kernel<2>
+                                            : assemble_t2_spin_kernel<0>,
+                             2 * sizeof(double) * 64 * 65));
         if (fs == 1)
             kv_launch(ctx, assemble_t2_spin_kernel<1>, gs, ST_T, smem, nv, st, fac, Z, Lc, seed,
                       T2);

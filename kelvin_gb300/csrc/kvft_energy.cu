@@ -270,13 +270,7 @@ int kv_energy(kvft_ctx *ctx, int ng, int nv, int no, const double *T1, const dou
                             (double)ng * nv * no));
     if (spin) {
         const size_t smem = sizeof(double) * (size_t)sh * (sh + 1);
-        static bool attr = false;
-        if (!attr) {
-            KV_CHECK(ctx, cudaFuncSetAttribute(energy2_spin_kernel,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(sizeof(double) * ESP_HMAX * (ESP_HMAX + 1))));
-            attr = true;
-        }
+        KV_TRY(kv_smem_optin(ctx, energy2_spin_kernel, sizeof(double) * ESP_HMAX * (ESP_HMAX + 1)));
         kv_launch(ctx, energy2_spin_kernel, grid, EN_T, smem, ng, nv, sh, T1, T2, f, eri, g, qterm,
                   work, pp, count, 1.0 / beta, dres);
         return kv_launch_check(ctx, "energy2_spin");

@@ -175,6 +175,10 @@ struct kvft_ctx {
     // halves), kept for the context's lifetime.
     void *hstage = nullptr;
     size_t hstage_bytes = 0;
+    // kernels by the dynamic shared memory they were allowed and by the
+    // blocks an SM holds (kv_smem_optin, kv_blocks_per_sm)
+    std::map<const void *, size_t> smem_optin;
+    std::map<const void *, int> blocks_per_sm;
 };
 // FP64 <-> FP32 by integer operations on the bit patterns, for values that
 // only steer the iteration (norms, the Anderson history): GB300's FP64 pipe
@@ -324,6 +328,20 @@ void kv_launch(kvft_ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t 
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);    // errors: kv_launch_check
+}
+
+// Lets launches of a kernel take `bytes` of dynamic shared memory (the same for
+// all its launches), and the blocks an SM holds at one launch shape per kernel.
+// Both belong to a device, so each context asks for itself, once.
+int kv_smem_optin_ptr(kvft_ctx *ctx, const void *kern, size_t bytes);
+int kv_blocks_per_sm_ptr(kvft_ctx *ctx, const void *kern, int threads, size_t smem, int *n);
+template <class... P>
+int kv_smem_optin(kvft_ctx *ctx, void (*kern)(P...), size_t bytes) {
+    return kv_smem_optin_ptr(ctx, (const void *)kern, bytes);
+}
+template <class... P>
+int kv_blocks_per_sm(kvft_ctx *ctx, void (*kern)(P...), int threads, size_t smem, int *n) {
+    return kv_blocks_per_sm_ptr(ctx, (const void *)kern, threads, smem, n);
 }
 #endif
 

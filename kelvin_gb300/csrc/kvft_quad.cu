@@ -695,13 +695,8 @@ int quad_dense_launch(kvft_ctx *ctx, int mode, QuadParams &q, const double *tbar
         }
     }
     const size_t smem = dense_smem(ng);
-    static bool attr_done = false;
-    if (!attr_done) {
-        const int mx = (int)dense_smem(MAXNG);
-        cudaFuncSetAttribute(quad_dense_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        cudaFuncSetAttribute(quad_dense_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        attr_done = true;
-    }
+    KV_TRY(kv_smem_optin(ctx, mode == 0 ? quad_dense_kernel<0> : quad_dense_kernel<1>,
+                         dense_smem(MAXNG)));
     int per_sm = 1;
     KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                       &per_sm, mode == 0 ? (const void *)quad_dense_kernel<0>
@@ -766,15 +761,9 @@ int kv_quad_launch(kvft_ctx *ctx, int mode, int ng, long long P, int rank, int n
     long long blocks = (P + QT - 1) / QT;
     long long cap = (long long)ctx->sm_count * 16;
     int grid = (int)std::min(blocks, cap);
-    static bool attr_done = false;
-    if (!attr_done) {
-        const int mx = (int)quad_smem(MAXNG, 0, 0, 1);
-        cudaFuncSetAttribute(quad_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        cudaFuncSetAttribute(quad_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        cudaFuncSetAttribute(quad_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        cudaFuncSetAttribute(quad_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        attr_done = true;
-    }
+    KV_TRY(kv_smem_optin(ctx, mode == 0 ? (q.uniform ? quad_kernel<0, true> : quad_kernel<0, false>)
+                                        : (q.uniform ? quad_kernel<1, true> : quad_kernel<1, false>),
+                         quad_smem(MAXNG, 0, 0, 1)));
     // algorithmic bytes: tbar in, T out (mode 0); tbar + T_old in, T_old out
     // (mode 1); with spin blocks, of the spin-conserving elements
     KvProfScope prof(ctx, KV_CAT_QUAD, 8.0 * ng * (double)P * (mode == 0 ? 2 : 3) *

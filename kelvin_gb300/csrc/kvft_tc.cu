@@ -1297,12 +1297,8 @@ std::string pack_key(const PackView &v, int R, int K, int nb, int D) {
 template <int D>
 int launch_pack_digits(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int rows_fast,
                        int ktn, int rtn, long long tiles, Packed *out) {
-    static int per_sm = 0;
-    if (!per_sm) {
-        KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                          &per_sm, pack_digits_kernel<D>, 256, 0));
-        per_sm = std::max(per_sm, 1);
-    }
+    int per_sm = 1;
+    KV_TRY(kv_blocks_per_sm(ctx, pack_digits_kernel<D>, 256, 0, &per_sm));
     const int grid = (int)std::min(tiles, (long long)per_sm * ctx->sm_count);
     kv_launch(ctx, pack_digits_kernel<D>, grid, 256, 0, v, R, K, ld, rows_fast, ktn, rtn,
               (int)tiles, out->ex, out->planes);
@@ -1312,13 +1308,7 @@ int launch_pack_digits(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, i
 template <int D>
 int launch_pack_cluster(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb,
                         int rows_fast, Packed *out) {
-    static bool attr = false;
-    if (!attr) {
-        KV_CHECK(ctx, cudaFuncSetAttribute(pack_cluster_kernel<D>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)pack_slab_smem(PC_SLAB)));
-        attr = true;
-    }
+    KV_TRY(kv_smem_optin(ctx, pack_cluster_kernel<D>, pack_slab_smem(PC_SLAB)));
     // slabs of at most 256, longer ones only for K > 2048; shorter ones while
     // the blocks do not fill the SMs
     const int rtiles = (R + PC_R - 1) / PC_R;
@@ -1350,14 +1340,9 @@ template <int D, int KT>
 int launch_pack_rows(kvft_ctx *ctx, const PackView &v, int R, int K, int ld, int nb,
                      int rows_fast, int rtiles, Packed *out) {
     constexpr size_t smem = pack_rows_smem(KT);
-    static int per_sm = 0;
-    if (!per_sm) {
-        KV_CHECK(ctx, cudaFuncSetAttribute(pack_rows_kernel<D, KT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        KV_CHECK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                          &per_sm, pack_rows_kernel<D, KT>, 256, smem));
-        per_sm = std::max(per_sm, 1);
-    }
+    int per_sm = 1;
+    KV_TRY(kv_smem_optin(ctx, pack_rows_kernel<D, KT>, smem));
+    KV_TRY(kv_blocks_per_sm(ctx, pack_rows_kernel<D, KT>, 256, smem, &per_sm));
     const long long ntiles = (long long)rtiles * nb;
     if (ntiles > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "pack: too many row tiles");
     const int grid = (int)std::min(ntiles, (long long)per_sm * ctx->sm_count);
@@ -1525,12 +1510,7 @@ int launch_tc(kvft_ctx *ctx, const CUtensorMap &ma, const CUtensorMap &mb, TcPar
         return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: stages exceed shared memory");
     p.NS = NS;
     const size_t smem = std::max(tc_smem(p.S, NS, TN, KBT, CV), SMEM_FLOOR);
-    static bool attr = false;
-    if (!attr) {
-        KV_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)SMEM_CAP));
-        attr = true;
-    }
+    KV_TRY(kv_smem_optin(ctx, kern, SMEM_CAP));
     const int grid = std::min(p.units, ctx->sm_count);
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
     kv_launch(ctx, kern, grid, NTHREADS + (CV ? 32 * NCV : 0), smem, ma, mb, p);

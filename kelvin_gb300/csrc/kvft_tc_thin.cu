@@ -493,12 +493,7 @@ int launch_thin(kvft_ctx *ctx, const CUtensorMap &mb, ThinParams &p) {
     int per = NT == 512 || cols > 256 ? 1 : 2;
     if (per == 1) smem = std::max(smem, (size_t)118 * 1024);
     else if (2 * smem > THIN_SMEM_CAP) per = 1;
-    static bool attr = false;
-    if (!attr) {
-        KV_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)THIN_SMEM_CAP));
-        attr = true;
-    }
+    KV_TRY(kv_smem_optin(ctx, kern, THIN_SMEM_CAP));
     const int grid = std::min(p.items, per * ctx->sm_count);
     KvProfScope prof(ctx, ctx->gemm_cat, ctx->gemm_work);
     kv_launch(ctx, kern, grid, NT, smem, mb, p);
