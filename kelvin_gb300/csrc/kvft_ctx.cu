@@ -1,6 +1,7 @@
 // Context, memory, timing and error plumbing of libkvft.
 #include "kvft_internal.h"
 
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -72,6 +73,7 @@ cudaError_t device_wait() {
 
 int kv_dev_alloc(kvft_ctx *ctx, size_t bytes, void **p) {
     *p = nullptr;
+    if (bytes > SIZE_MAX - 511) return kv_fail(ctx, KVFT_ENOMEM, "cudaMalloc: size out of range");
     const size_t need = (std::max(bytes, (size_t)16) + 511) / 512 * 512;
     DevPool &d = pool_of(ctx->device);
     std::lock_guard<std::mutex> lock(d.mu);

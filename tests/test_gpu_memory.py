@@ -121,3 +121,15 @@ def test_free_waits_for_every_stream():
         assert done.query()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("nbytes", [2 ** 64 - 1, 2 ** 64 - 511, 2 ** 64 - 512, 2 ** 63, 2 ** 48 + 1])
+def test_sizes_beyond_the_address_space_are_refused(nbytes):
+    """Sizes that rounding up to whole blocks would wrap, and beside them."""
+    ctx = _lib.Context(0)
+    try:
+        p = _lib.vp()
+        assert ctx.L.kvft_alloc(ctx.h, nbytes, ctypes.byref(p)) != 0
+        assert not p.value
+    finally:
+        ctx.close()
