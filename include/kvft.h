@@ -37,7 +37,12 @@ typedef enum {
 } kvft_status;
 
 /* Arithmetic used for the n^6/n^5 contractions.  Quadrature, energy,
- * damping and norms are FP64 in every mode. */
+ * damping and norms are FP64 in every mode.
+ * Long sums with few outputs (a tensor-core product with K > 2048 and fewer
+ * than two output tiles per SM; an FP64 one with K > 64 and fewer than two tiles
+ * of 64 x 64 per SM) are cut into ranges that add into the result in any order:
+ * its last bits may differ from run to run.  Everything else repeats to the
+ * bit. */
 typedef enum {
     KVFT_PREC_FP64 = 0,      /* FP64 FMA (SIMT) contractions */
     KVFT_PREC_FP64_TC = 1,   /* FP64-accurate: digit-sliced BF16 tcgen05 GEMM */

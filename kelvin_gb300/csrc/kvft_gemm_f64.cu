@@ -502,8 +502,11 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     // ranges of 256: 57 x 57, K = 57^3, two products, 2.85 ms in flat tiles,
     // 2.66 here; 40 x 40 (61 % padding) is better off flat.
     const long long sq = (long long)ceil_div(M, SQ) * ceil_div(N, SQ);
+    // Sums that are never cut, and so repeatable to the bit: K up to 64, and
+    // products that fill the SMs twice with 64 x 64 tiles.
+    const bool cut = K > 64 && sq * batch < want;
     const long long sqk = (long long)batch * g.n * (K / 256);
-    const bool square_k = !rows && sq == 1 && M * N >= 0.7 * SQ * SQ && K >= 1024 &&
+    const bool square_k = cut && !rows && sq == 1 && M * N >= 0.7 * SQ * SQ && K >= 1024 &&
                           sqk >= want && nprod < 2 * want;
     const bool square = square_k || (!rows && sq * nprod >= 6LL * ctx->sm_count &&
                                      (double)sq * SQ * SQ <= 1.02 * M * (double)N);
@@ -517,7 +520,7 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         // blocks (every product's, since they then add by atomics) when neither
         // extent is short; smaller tiles, down to two outputs per thread, else.  Shrinking first reads a long operand once per tile: 57 x 57
         // outputs, K = 57^3, two products, 5.7 ms in tiles of 57 x 4, 2.85 so.
-        const bool longk = K >= 1024 && std::min(M, N) > 32;
+        const bool longk = cut && K >= 1024 && std::min(M, N) > 32;
         for (;; T /= 2) {
             f64_tile(M, N, NT * T, &p.BM, &p.BN);
             p.mt = ceil_div(M, p.BM);
@@ -531,7 +534,7 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
         const int bk = T <= 4 ? 32 : 16;
         if (longk && tiles * tab.ncb < 2 * want)
             p.nsplit = (int)std::min<long long>(ceil_div(4 * want, tiles * g.n), K / 256);
-        else if (tiles * tab.ncb < want && K > 32)
+        else if (cut && tiles * tab.ncb < want)
             p.nsplit = (int)std::min<long long>(ceil_div(want, tiles * tab.ncb), ceil_div(K, 32));
         p.klen = ceil_div(ceil_div(K, p.nsplit), bk) * bk;
         p.nsplit = ceil_div(K, p.klen);

@@ -59,6 +59,7 @@ struct TcParams {
     int mt, nt;           // output tiles along M and N
     int units;            // work units: C blocks * mt * nt * batch * nsplit
     int nsplit;           // >1: each K range is its own unit, added into C by FP64 atomics
+    long long c_split;    // or stored to its own copy of C, this far from the range before (0: added)
     int split_kb;         // k-blocks per K range
     int chunk_kb;         // k-blocks per K chunk (exactness bound)
     int nkb_total;        // k-blocks of the padded K extent
@@ -549,6 +550,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                            (long long)i2 * p.C.r.st[2];
                 }
                 double *Cr = p.C.p + (long long)w.b * p.C.bst + p.coff[w.cb] + roff;
+                if (p.c_split) Cr += w.kb0 / p.split_kb * p.c_split;
                 const int krow = (m < p.M) ? exp_of(p.ea[p.aex[src] + w.b * p.ea_bst + m]) -
                                                  2 * G::C + p.alpha_exp
                                            : 0;
@@ -622,7 +624,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (!p.alpha_pow2) v *= p.alpha;
                         return v;
                     };
-                    if (CV || p.nsplit > 1 || beta == 1.0) {
+                    if (CV || (p.nsplit > 1 && !p.c_split) || beta == 1.0) {
                         // C += value: each element gets exactly one addition in
                         // this launch unless K chunks run as separate units, so a
                         // fire-and-forget reduction at L2 gives old + value
@@ -1486,6 +1488,31 @@ bool kv_tc_pow2(double alpha, int *exp, unsigned *sign) {
 
 namespace {
 
+// C = beta C + the copies of its K ranges, product after product and range
+// after range: one thread per element (rows fastest, as the copies are), y = block
+// of C, z = batch entry.
+struct SumRanges {
+    int beg[KV_MAXPROD + 1], prod[KV_MAXPROD];
+    long long coff[KV_MAXPROD];
+};
+
+__global__ void __launch_bounds__(256)
+sum_ranges_kernel(int M, int MN, int nranges, double beta, KOut C, const double *__restrict__ parts,
+                  long long c_split, const __grid_constant__ SumRanges s) {
+    if (!kv_depend()) return;
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= MN) return;
+    const double *part = parts + (long long)blockIdx.z * MN + e;
+    double acc = 0.0;
+    for (int q = s.beg[blockIdx.y]; q < s.beg[blockIdx.y + 1]; q++) {
+        const double *x = part + s.prod[q] * nranges * c_split;
+        for (int r = 0; r < nranges; r++) acc += x[r * c_split];
+    }
+    const int n = e / M, m = e - n * M;
+    double *d = C.p + (long long)blockIdx.z * C.bst + s.coff[blockIdx.y] + C.r.off(m) + C.c.off(n);
+    *d = beta == 0.0 ? acc : fma(beta, *d, acc);
+}
+
 // The stride-1 index of a view: its fastest dimension of extent > 1 has
 // element stride 1 (or the index has a single value).
 bool unit_stride(const KIdx &x) {
@@ -1567,20 +1594,26 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const long long tiles = (long long)mt * nt * batch;
     // K ranges.  Fewer output tiles than two waves of SMs and several ranges of
     // 2048: every range of every product becomes a unit of its own and adds
-    // into C with FP64 atomics (C pre-scaled by beta).  At D >= 4 the
-    // ranges may be shorter (the exact sums stay so): while there are fewer units than
-    // SMs, down to 256 deep (below that the pipeline's start and the atomics
-    // cost what the other SMs would save).  D <= 3 keeps 2048, which is part
+    // into C with FP64 atomics (C pre-scaled by beta).  At D >= 4 the ranges
+    // may be shorter (the exact sums stay so): while there are fewer units than
+    // SMs, down to 256 deep (below that the pipeline's start and the additions
+    // cost what the other SMs would save).  Where only that cuts K, the ranges
+    // go to copies of C, at most two tiles per SM, which one more launch (in
+    // place of the scaling) adds in a fixed order: a sum of up to 2048 terms
+    // is repeatable to the bit, as it is uncut.  D <= 3 keeps 2048, which is part
     // of its rounding.  37 x 37 outputs against K = 16317, one product, seven
     // levels: 40 us on 8 SMs; the residual of 37 virtual and 21 occupied spin
     // orbitals 1067 -> 962 us, a solve of 38 and 10 points 53.6 -> 52.8 ms.
     int nranges = (nkb_total + KRANGE / kb - 1) / (KRANGE / kb);
     bool par = nranges > 1 && tiles < 2LL * ctx->sm_count;
     const long long now = tiles * (par ? (long long)nranges * g.n : kv_group_tab(g, false).ncb);
+    bool ordered = false;
     if (ff && now < ctx->sm_count) {
+        ordered = nranges == 1;
         const long long want = (ctx->sm_count + tiles * g.n - 1) / (tiles * g.n);
         nranges = (int)std::max<long long>(nranges, std::min<long long>(want, K / 256));
         par = nranges > 1;
+        ordered = ordered && par;
     }
     const int split_kb = (nkb_total + nranges - 1) / nranges;     // balanced ranges
     nranges = (nkb_total + split_kb - 1) / split_kb;
@@ -1589,10 +1622,9 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     const KvGroupTab tab = kv_group_tab(g, par);
     const long long units = tiles * (par ? nranges : 1) * tab.ncb;
     if (units > 0x7FFFFFFFLL) return kv_fail(ctx, KVFT_EINVAL, "tensor-core gemm: too many tiles");
-    if (par && beta != 1.0) {
-        const KvGroupTab t = kv_group_tab(g, false);
-        KV_TRY(kv_scale_blocks(ctx, M, N, batch, beta, C, t.ncb, t.coff));
-    }
+    const KvGroupTab blocks = kv_group_tab(g, false);
+    if (par && !ordered && beta != 1.0)
+        KV_TRY(kv_scale_blocks(ctx, M, N, batch, beta, C, blocks.ncb, blocks.coff));
     TcParams p;
     p.batch = batch;
     for (int c = 0; c <= tab.ncb; c++) p.beg[c] = tab.beg[c];
@@ -1630,30 +1662,52 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     p.ea_bst = (nbA > 1) ? pa.R : 0;
     p.eb_bst = (nbB > 1) ? pb.R : 0;
     p.alpha = alpha;
-    p.beta = par ? 1.0 : beta;
+    p.beta = ordered ? 0.0 : par ? 1.0 : beta;
     p.alpha_pow2 = kv_tc_pow2(alpha, &p.alpha_exp, &p.alpha_sign);
     p.C = C;
+    p.c_split = 0;
+    if (ordered) {
+        // copies [product][range][batch][n][m]
+        const long long mn = (long long)M * N;
+        void *parts = nullptr;
+        KV_TRY(kv_scratch(ctx, "tc_ranges", sizeof(double) * mn * batch * nranges * g.n, &parts));
+        p.C = KOut{(double *)parts, kidx1(M, 1), kidx1(N, M), mn};
+        p.c_split = mn * batch;
+        for (int c = 0; c < tab.ncb; c++) p.coff[c] = tab.prod[c] * nranges * p.c_split;
+    }
     p.err = ctx->dflag;
     p.dv_split = fastdiv(p.nsplit);
     p.dv_perb = fastdiv(p.mt * p.nt);
     p.dv_gsz = fastdiv(GROUP_M * p.nt);
     p.dv_batch = fastdiv(batch);
-    p.dv_cr2 = fastdiv(C.r.size[2]);
-    p.dv_cr1 = fastdiv(C.r.size[1]);
-    switch (D) {
-    case 2:
-        return tn == 64 ? launch_tc<64, false, 64, 2>(ctx, ma, mb, p)
-                        : launch_tc<128, false, 64, 2>(ctx, ma, mb, p);
-    case 3:
-        return tn == 64 ? launch_tc<64, false, 64, 3>(ctx, ma, mb, p)
-                        : launch_tc<128, false, 64, 3>(ctx, ma, mb, p);
-    case 4: return launch_tc<64, true, 32, 4>(ctx, ma, mb, p);
-    case 5: return launch_tc<64, true, 32, 5>(ctx, ma, mb, p);
-    case 6: return launch_tc<64, true, 32, 6>(ctx, ma, mb, p);
-    default:
-        return tn == 64 ? launch_tc<64, true, 32, 7, true>(ctx, ma, mb, p)
-                        : launch_tc<48, true, 32, 7>(ctx, ma, mb, p);
-    }
+    p.dv_cr2 = fastdiv(p.C.r.size[2]);
+    p.dv_cr1 = fastdiv(p.C.r.size[1]);
+    const auto run = [&]() -> int {
+        switch (D) {
+        case 2:
+            return tn == 64 ? launch_tc<64, false, 64, 2>(ctx, ma, mb, p)
+                            : launch_tc<128, false, 64, 2>(ctx, ma, mb, p);
+        case 3:
+            return tn == 64 ? launch_tc<64, false, 64, 3>(ctx, ma, mb, p)
+                            : launch_tc<128, false, 64, 3>(ctx, ma, mb, p);
+        case 4: return launch_tc<64, true, 32, 4>(ctx, ma, mb, p);
+        case 5: return launch_tc<64, true, 32, 5>(ctx, ma, mb, p);
+        case 6: return launch_tc<64, true, 32, 6>(ctx, ma, mb, p);
+        default:
+            return tn == 64 ? launch_tc<64, true, 32, 7, true>(ctx, ma, mb, p)
+                            : launch_tc<48, true, 32, 7>(ctx, ma, mb, p);
+        }
+    };
+    KV_TRY(run());
+    if (!ordered) return KVFT_OK;
+    SumRanges sr;
+    for (int c = 0; c <= blocks.ncb; c++) sr.beg[c] = blocks.beg[c];
+    for (int c = 0; c < blocks.ncb; c++) sr.coff[c] = blocks.coff[c];
+    for (int q = 0; q < g.n; q++) sr.prod[q] = blocks.prod[q];
+    kv_launch(ctx, sum_ranges_kernel,
+              dim3((unsigned)(((long long)M * N + 255) / 256), blocks.ncb, batch), 256, 0, M,
+              M * N, nranges, beta, C, (const double *)p.C.p, p.c_split, sr);
+    return kv_launch_check(ctx, "sum_ranges");
 }
 
 }  // namespace
