@@ -70,8 +70,10 @@ int kvft_launch_count(kvft_ctx *ctx, uint64_t *count);     /* own kernels */
 int kvft_flush_l2(kvft_ctx *ctx);                          /* writes 256 MB */
 /* Memory from kvft_alloc comes with arbitrary contents.  kvft_free waits for the
  * whole device, as cudaFree does, and keeps the block for a later kvft_alloc of
- * the process: at most a 32nd of the device in all, returned to the driver
- * when an allocation fails and when the device's last context is destroyed. */
+ * the process: at most a 32nd of the device in all, returned to the driver by
+ * kvft_mem_release, when an allocation fails and when the device's last context
+ * is destroyed.  Until then only this library can use it. */
+int kvft_mem_release(kvft_ctx *ctx);
 /* Free (the driver's and the kept blocks) and total memory of the context's
  * device. */
 int kvft_mem_info(kvft_ctx *ctx, size_t *free_bytes, size_t *total_bytes);

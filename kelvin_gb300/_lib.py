@@ -117,6 +117,7 @@ _SIGS = {
     "kvft_solver_set_acceleration": (ctypes.c_int, [vp, ctypes.c_int]),
     "kvft_solver_set_graph": (ctypes.c_int, [vp, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
     "kvft_solver_step_end": (ctypes.c_int, [vp, c_double_p, c_double_p]),
+    "kvft_mem_release": (ctypes.c_int, [vp]),
     "kvft_mem_info": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_size_t),
                                      ctypes.POINTER(ctypes.c_size_t)]),
     "kvft_lambda_guess": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int,
@@ -243,8 +244,14 @@ class Context(object):
     def flush_l2(self):
         self.check(self.L.kvft_flush_l2(self.h), "kvft_flush_l2")
 
+    def release_memory(self):
+        """Give the device blocks that the library keeps for reuse back to the
+        driver, for other users of the device (torch, another process)."""
+        self.check(self.L.kvft_mem_release(self.h), "kvft_mem_release")
+
     def mem_info(self):
-        """(free, total) bytes of the context's device."""
+        """(free, total) bytes of the context's device; free includes the blocks
+        kept for reuse."""
         f, t = ctypes.c_size_t(), ctypes.c_size_t()
         self.check(self.L.kvft_mem_info(self.h, ctypes.byref(f), ctypes.byref(t)),
                    "kvft_mem_info")

@@ -33,8 +33,8 @@ int kv_cuda(kvft_ctx *ctx, cudaError_t e, const char *what) {
 //     us with its cudaMalloc on an idle device), which leaves stream captures
 //     of other threads alone; cudaDeviceSynchronize would invalidate them.
 //   * At most a 32nd of the device is kept, the oldest blocks going first; all
-//     of it is returned when an allocation fails and when the device's last
-//     context is destroyed.
+//     of it is returned by kvft_mem_release, when an allocation fails and when
+//     the device's last context is destroyed.
 namespace {
 
 struct DevPool {
@@ -534,6 +534,16 @@ extern "C" int kvft_flush_l2(kvft_ctx *c) {
     static unsigned salt = 1;
     kv_flush_kernel<<<c->sm_count * 4, 512, 0, c->stream>>>((uint4 *)c->l2buf, bytes / 16, salt++);
     return kv_launch_check(c, "flush_l2");
+}
+
+extern "C" int kvft_mem_release(kvft_ctx *c) {
+    if (c && c->dry) return kv_fail(c, KVFT_EINVAL, "kvft_mem_release: not on a dry-run context");
+    if (!c) return KVFT_EINVAL;
+    cudaSetDevice(c->device);
+    DevPool &d = pool_of(c->device);
+    std::lock_guard<std::mutex> lock(d.mu);
+    pool_release(d);
+    return KVFT_OK;
 }
 
 extern "C" int kvft_mem_info(kvft_ctx *c, size_t *free_bytes, size_t *total_bytes) {

@@ -133,3 +133,22 @@ def test_sizes_beyond_the_address_space_are_refused(nbytes):
         assert not p.value
     finally:
         ctx.close()
+
+
+def test_kept_blocks_are_given_back_on_request():
+    """What is kept for reuse returns to the driver, where others find it."""
+    torch = pytest.importorskip("torch")
+    ctx, other = _lib.Context(0), _lib.Context(0)
+    try:
+        a = alloc(ctx, 640 << 20)
+        assert ctx.L.kvft_free(ctx.h, a) == 0
+        free = torch.cuda.mem_get_info()[0]
+        other.release_memory()                          # any context of the device
+        assert torch.cuda.mem_get_info()[0] >= free + (640 << 20)
+        ctx.release_memory()                            # nothing kept: nothing happens
+        x = _lib.DeviceArray.from_host(ctx, numpy.arange(5.0))
+        assert numpy.array_equal(x.to_host(), numpy.arange(5.0))
+        x.free()
+    finally:
+        other.close()
+        ctx.close()
