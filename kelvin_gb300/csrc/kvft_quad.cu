@@ -14,8 +14,9 @@
 //     chained: T_y = w(y,y-s) (T_{y-s} - G[y-s,y-s] tbar_{y-s})
 //                    + sum_{x=y-s}^{y} G[y,x] w(y,x) tbar_x,
 //     which is O(ng) per element instead of O(ng^2).
-// The product of <= ng correctly rounded factors differs from a direct exp
-// by at most ~ng ulp (relative), far inside the 1e-10 parity tolerance.
+// The product of <= ng factors, each within a unit in the last place, differs
+// from a direct exp by at most ~2 ng ulp (relative), far inside the 1e-10
+// parity tolerance.
 #include "kvft_internal.h"
 
 #include <cmath>
@@ -35,7 +36,7 @@ struct QuadParams {
     int full;
     int same;                // first chained row from which gd, g1 and cs are constant
     int symmetric;           // ti[x] + ti[ng-1-x] the same for every x
-    int mirror;              // the same to the last bits
+    int mirror;              // ti[x] - tc and ti[ng-1-x] - tc differ in sign alone
     double alpha;            // damping (fused update only)
     int spin_half;           // fused update over the spin-conserving elements only (0: all)
 };
@@ -653,12 +654,22 @@ size_t quad_smem(int ng, int uniform, int step, int full) {
                              (step > 0 ? 0 : ng * QT) + (full ? ng * QT : 0));
 }
 
-// ti[x] + ti[ng-1-x] equal for every x (to `rel` of the range)
-int grid_symmetric(int ng, const double *ti, double rel) {
+// ti[x] + ti[ng-1-x] equal for every x (to rounding)
+int grid_symmetric(int ng, const double *ti) {
     const double c = ti[0] + ti[ng - 1];
-    const double tol = rel * std::max(std::fabs(ti[ng - 1] - ti[0]), 1e-300);
+    const double tol = 1e-13 * std::max(std::fabs(ti[ng - 1] - ti[0]), 1e-300);
     for (int x = 0; x < ng; x++)
         if (std::fabs(ti[x] + ti[ng - 1 - x] - c) > tol) return 0;
+    return 1;
+}
+
+// ti[x] - tc = -(ti[ng-1-x] - tc) to the bit, as the tables form them: then the
+// entries for x are the inverse ones for ng-1-x to the bit, too.  (A grid off
+// by a last place in its nodes would put that times beta |d| into the factors.)
+int grid_mirrored(int ng, const double *ti) {
+    const double tc = 0.5 * (ti[0] + ti[ng - 1]);
+    for (int x = 0; x < ng; x++)
+        if (ti[x] - tc != -(ti[ng - 1 - x] - tc)) return 0;
     return 1;
 }
 
@@ -754,8 +765,8 @@ int kv_quad_launch(kvft_ctx *ctx, int mode, int ng, long long P, int rank, int n
     // solver's passes, which read no other; callers pass 0 otherwise)
     q.spin_half = (rank == 2 && nv == no && nv == 2 * spin_half) ? spin_half : 0;
     analyse_grid(ng, hti, hG, full, &q.step, &q.uniform, &q.same);
-    q.symmetric = grid_symmetric(ng, hti, 1e-13);
-    q.mirror = grid_symmetric(ng, hti, 1e-15);
+    q.symmetric = grid_symmetric(ng, hti);
+    q.mirror = grid_mirrored(ng, hti);
     if (full) return quad_dense_launch(ctx, mode, q, tbar, ti, hti, G, D, ev, eo, out, res);
     size_t smem = quad_smem(ng, q.uniform, q.step, q.full);
     long long blocks = (P + QT - 1) / QT;

@@ -96,3 +96,36 @@ def test_energy_rectangular(ctx, nv, no, ng, qterm):
     # both sums lie within a roundoff per term of the sum of magnitudes
     mag = oft.ft_cc_energy(abs(T1), abs(T2), abs(f), abs(eri), g, 2.0, qterm)
     assert abs(E - ref) <= 4.0 * 2.0 ** -53 * (ng + 4) * mag + 1e-15 * mag
+
+
+@pytest.mark.parametrize("shift", [0.0, 8e-16, -8e-16])
+def test_dense_integral_on_a_grid_off_by_last_places(ctx, shift):
+    """Nodes that are symmetric about the centre only to 8e-16 of the range, and
+    a large beta |d|: exp((t_x - t_y) d) keeps their actual distances.  One
+    sweep from zero amplitudes with a Fock matrix alone integrates a constant;
+    its values at two nodes are compared by their ratio.  Tolerance at a node:
+    half a unit of the arguments (at most beta |d| / 2) of two exponentials, four
+    units for these and the products, 1e-14 for the compensated FP32 sum."""
+    E, ng = 80.0, 8
+    ti, g, G = ft_quad(ng, 1.0, "gl")
+    ti = ti.copy()
+    ti[1] += shift
+    fock = numpy.array([[0.0, 0.01, 0.0, 0.0], [0.01, E, 0.0, 0.0],
+                        [0.0, 0.0, 0.0, 0.01], [0.0, 0.0, 0.01, E]])
+    en = numpy.array([0.0, E, 0.0, E])
+    sv = DeviceSolver.from_system(ctx, en, fock, numpy.zeros((4,) * 4), 1.0, -60.0, ti, g, G)
+    try:
+        sv.full = True
+        sv.guess(0)
+        sv.step(0.0)
+        T1, _ = sv.amplitudes()
+    finally:
+        sv.close()
+    t = ti.astype(numpy.longdouble)
+    for a, i, d in ((0, 1, -E), (1, 0, E)):
+        w = G * numpy.exp((t[None, :] - t[:, None]) * d)
+        ref, size = w.sum(1), abs(w).sum(1)
+        tol = (1e-14 + (E + 8) * 2.0 ** -53) * size / abs(ref)
+        for y in range(ng):
+            r = numpy.longdouble(T1[y, a, i]) / T1[3, a, i] * ref[3] / ref[y]
+            assert abs(r - 1) <= tol[y] + tol[3]
