@@ -1382,6 +1382,7 @@ int launch_pack_exp(kvft_ctx *ctx, const PackView &v, int R, int K, int nb, int 
     KV_CHECK(ctx, cudaMemsetAsync(ex, 0x80, (size_t)nb * R * sizeof(int), ctx->stream));
     const dim3 g((K + PT_K - 1) / PT_K, (unsigned)((R + PT_R - 1) / PT_R), nb);
     if (g.y > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: too many rows");
+    if (g.z > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: batch too large");
     // long rows: each exponent block walks up to 16 k tiles, so that about
     // 32 blocks per SM remain and the atomics per row drop accordingly
     const long long tiles = (long long)g.x * g.y * g.z;
@@ -1404,7 +1405,7 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
     out->ld = ld;
     out->K = K;
     out->nb = nb;
-    if (nb > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: batch too large");
+    if (v.nb > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: batch too large");
     void *buf = nullptr;
     std::string ckey;
     if (v.stable && ctx->pack_cache_on) {
@@ -1456,7 +1457,6 @@ int kv_tc_pack(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, 
 
 int kv_tc_exps(kvft_ctx *ctx, const char *key, const PackView &v, int R, int K, int nb,
                Packed *out) {
-    if (nb > 65535) return kv_fail(ctx, KVFT_EINVAL, "pack: batch too large");
     void *buf = nullptr;
     KV_TRY(kv_scratch(ctx, key, (size_t)nb * R * sizeof(int), &buf));
     out->planes = nullptr;

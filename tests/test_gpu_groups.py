@@ -3,8 +3,9 @@ FP64 kernel's free tile extents."""
 import numpy
 import pytest
 
+from conftest import random_system, random_T
 from kelvin_gb300 import _lib, ft_cc_equations, systems
-from kelvin_gb300.cc_utils import DeviceSolver
+from kelvin_gb300.cc_utils import F_ORDER, I_ORDER, DeviceSolver
 from kelvin_gb300.quadrature import ft_quad
 from oracle import ft_ccsd as oft
 from oracle import ft_utils
@@ -122,3 +123,42 @@ def test_thin_contraction(ctx, M, N, K, batch, digits, big_left):
     tol = {2: 2e-3, 3: 5e-5, 4: 5e-7, 5: 5e-9, 6: 5e-11, 7: 5e-12}[digits]
     bound = abs(A).max(2)[:, :, None] * abs(B).max(1)[:, None, :] * K
     assert (abs(C - A @ B) <= tol * (256 / K) ** 0.5 * bound).all()
+
+
+def test_group_of_a_large_batch(ctx, n=8, nb=11000, digits=7):
+    """The sub-blocks of a group times its batch exceed 65535, a single
+    product's batch does not: each entry is what it is in a batch of three.
+    The tolerance is the rounding of FP64 additions in another order."""
+    rng = numpy.random.default_rng(3)
+    h = n // 2
+    s = numpy.arange(n) >= h
+    F, I = random_system(rng, n, n)
+    for b in ("oo", "ov", "vo", "vv"):
+        getattr(F, b)[s[:, None] != s] = 0.0
+    cons = (s[:, None, None, None].astype(int) + s[:, None, None]) == (s[:, None].astype(int) + s)
+    for b in ("vvvv", "vvvo", "vovv", "vvoo", "vovo", "oovv", "vooo", "ooov", "oooo"):
+        getattr(I, b)[~cons] = 0.0
+    t1, t2 = random_T(rng, 3, n, n)
+    t1[:, s[:, None] != s] = 0.0
+    t2[:, ~cons] = 0.0
+    dF = [_lib.DeviceArray.from_host(ctx, getattr(F, k)) for k in F_ORDER]
+    dI = [_lib.DeviceArray.from_host(ctx, getattr(I, k)) for k in I_ORDER]
+    out = []
+    ctx.set_precision(_lib.PREC_FP64_TC, digits)
+    ctx.set_residual_spin_blocks(h)
+    try:
+        for idx in (numpy.arange(3), numpy.arange(nb) % 3):
+            d1, d2 = _lib.DeviceArray.from_host(ctx, t1[idx]), _lib.DeviceArray.from_host(ctx, t2[idx])
+            o1 = _lib.DeviceArray.from_host(ctx, numpy.zeros((len(idx), n, n)))
+            o2 = _lib.DeviceArray.from_host(ctx, numpy.zeros((len(idx),) + (n,) * 4))
+            ctx.check(ctx.L.kvft_stanton_residual(ctx.h, len(idx), n, n, _lib.ptr_array(dF),
+                                                  _lib.ptr_array(dI), d1.ptr, d2.ptr, 1.0, o1.ptr,
+                                                  o2.ptr), "kvft_stanton_residual")
+            out.append((o1.to_host(), o2.to_host()))
+    finally:
+        ctx.set_residual_spin_blocks(0)
+        ctx.set_precision(_lib.PREC_FP64, 7)
+    (a1, a2), (b1, b2) = out
+    for y in (0, 1, 2, 5461, 10921, 10922, 10923, nb - 1):
+        assert abs(b1[y] - a1[y % 3]).max() <= 1e-11 * abs(a1).max()
+        assert abs(b2[y] - a2[y % 3]).max() <= 1e-11 * abs(a2).max()
