@@ -53,17 +53,58 @@ __device__ __forceinline__ double denom(const QuadParams &q, long long p, int l,
 
 // e^x by table lookup (P. T. P. Tang, ACM TOMS 15, 144 (1989)): x = n ln2/64 +
 // r, |r| <= ln2/128, e^x = 2^(n / 64) (1 + (e^r - 1)) with the 64 values of
-// 2^(j/64) in shared memory and a fifth-order Taylor polynomial (its remainder
-// is below 4e-17): ten FP64 operations, and two of them more for e^-x, where
-// the library function takes about 17 and the reciprocal ten -- the FP64 pipe
-// is what these kernels wait for.  Within one unit in the last place of the
-// exact value; |x| >= 700 and NaN go to the library function.
+// 2^(j/64) in shared memory, each as a rounded value and the rest, and a
+// sixth-order Taylor polynomial (its remainder is below 3e-20): twelve FP64
+// operations, and three of them more for e^-x, where the library function takes
+// about 17 and the reciprocal ten -- the FP64 pipe is what these kernels wait
+// for.  As accurate as the library function, 0.51 units in the last place:
+// step factors are raised to the ng-th power, and without the rests and the
+// sixth order (two operations less, 1.25 units) the tau integral of 66 spin
+// orbitals and 16 points came out with 1.3 times the error.  |x| >= 700 and NaN
+// go to the library function.
 constexpr int ETAB = 64;
+// 2^(j/64): rounded to FP64, and the difference from it
+__device__ const double EXP2_TAB[ETAB][2] = {
+    {1.0, 0.0}, {1.0108892860517005, -1.523477860e-17},
+    {1.0218971486541166, 5.109225029e-17}, {1.0330248790212284, 7.600838874e-18},
+    {1.0442737824274138, 8.551889706e-17}, {1.0556451783605572, 1.759325739e-18},
+    {1.0671404006768237, -7.899853967e-17}, {1.0787607977571199, -6.656660436e-17},
+    {1.0905077326652577, -3.046782080e-17}, {1.102382583307841, 5.266036872e-17},
+    {1.1143867425958924, 1.041027846e-16}, {1.1265216186082418, 5.165856759e-17},
+    {1.1387886347566916, 8.912812676e-17}, {1.1511892299529827, 3.250710219e-17},
+    {1.1637248587775775, 3.829204837e-17}, {1.1763969916502812, 5.554203254e-17},
+    {1.189207115002721, 3.982015231e-17}, {1.202156731452703, 6.644981499e-17},
+    {1.215247359980469, -7.712630693e-17}, {1.22848053610687, -1.898781631e-17},
+    {1.241857812073484, 4.658027592e-17}, {1.255380757024691, -6.711389821e-18},
+    {1.2690509571917332, 2.667932131e-18}, {1.2828700160787783, 1.713594918e-17},
+    {1.2968395546510096, 2.538250279e-17}, {1.3109612115247644, -7.181536136e-17},
+    {1.3252366431597413, -2.858731210e-17}, {1.339667524053303, 8.927282595e-17},
+    {1.3542555469368927, 7.700948380e-17}, {1.3690024229745905, 9.593797919e-17},
+    {1.383909881963832, -6.770511659e-17}, {1.3989796725383112, -9.614213209e-17},
+    {1.4142135623730951, -9.667293313e-17}, {1.42961333839197, -1.203164249e-17},
+    {1.4451808069770467, -3.023758135e-17}, {1.460917794180647, -5.600377186e-17},
+    {1.4768261459394993, -3.483994557e-17}, {1.4929077282912648, 1.419292015e-17},
+    {1.5091644275934228, -1.016455328e-16}, {1.5255981507445384, -1.102494171e-16},
+    {1.5422108254079407, 7.949834810e-17}, {1.559004400237837, 3.781207053e-17},
+    {1.5759808451078865, -1.013691647e-17}, {1.593142151342267, -1.009440654e-16},
+    {1.6104903319492543, 2.470719257e-17}, {1.6280274218573478, -6.712955085e-17},
+    {1.645755478153965, -1.012567991e-16}, {1.6636765803267364, 5.890992697e-17},
+    {1.681792830507429, 8.199010021e-17}, {1.7001063537185235, -8.023719370e-18},
+    {1.718619298122478, -1.851380418e-17}, {1.7373338352737062, 3.164389299e-17},
+    {1.7562521603732995, 2.960140695e-17}, {1.7753764925265212, 6.429731797e-17},
+    {1.7947090750031072, 1.822745843e-17}, {1.8142521755003989, -9.969531539e-17},
+    {1.8340080864093424, 3.283107224e-17}, {1.8539791250833855, 9.761887491e-17},
+    {1.8741676341103, -6.122763413e-17}, {1.8945759815869656, 3.403403535e-17},
+    {1.9152065613971474, -1.061994606e-16}, {1.9360617934922943, 1.033238596e-16},
+    {1.9571441241754002, 8.960767791e-17}, {1.978456026387951, 4.038875311e-17},
+};
+// shared-memory copy: the rounded values, then the rests
 __device__ __forceinline__ void exp_table(double *T) {       // caller synchronises
-    for (int j = threadIdx.x; j < ETAB; j += blockDim.x) T[j] = exp2(j * (1.0 / ETAB));
+    for (int j = threadIdx.x; j < 2 * ETAB; j += blockDim.x) T[j] = EXP2_TAB[j % ETAB][j / ETAB];
 }
 __device__ __forceinline__ double exp_scaled(const double *T, int n, double p) {
-    const double t = T[n & (ETAB - 1)], y = fma(t, p, t);
+    const double t = T[n & (ETAB - 1)];
+    const double y = t + fma(t, p, T[ETAB + (n & (ETAB - 1))]);
     return __hiloint2double(__double2hiint(y) + (n >> 6) * (1 << 20), __double2loint(y));
 }
 __device__ __forceinline__ bool exp_reduce(double x, int &n, double &r) {
@@ -79,7 +120,7 @@ __device__ __forceinline__ double exp_tab(double x, const double *T) {
     int n;
     double r;
     if (!exp_reduce(x, n, r)) return exp(x);
-    const double q = fma(fma(fma(r, 1.0 / 120.0, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+    const double q = fma(fma(fma(fma(r, 1.0 / 720.0, 1.0 / 120.0), r, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
     return exp_scaled(T, n, fma(q * r, r, r));
 }
 // e^x and e^-x: the polynomial's even and odd parts
@@ -92,7 +133,7 @@ __device__ __forceinline__ void exp_tab2(double x, const double *T, double &ep, 
         return;
     }
     const double r2 = r * r;
-    const double ev = r2 * fma(r2, 1.0 / 24.0, 0.5);
+    const double ev = r2 * fma(r2, fma(r2, 1.0 / 720.0, 1.0 / 24.0), 0.5);
     const double od = fma(r * r2, fma(r2, 1.0 / 120.0, 1.0 / 6.0), r);
     ep = exp_scaled(T, n, ev + od);
     em = exp_scaled(T, -n, ev - od);
@@ -157,7 +198,7 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
     double *G = ti + ng;
     double *cs = G + ng * ng, *g1 = cs + ng, *gd = g1 + ng;
     double *et = gd + ng;                                  // 2^(j/64)
-    double *rk = et + ETAB;                                // [ng][QT]
+    double *rk = et + 2 * ETAB;                              // [ng][QT]
     double *tb = rk + (q.uniform ? 0 : ng * QT);           // [ng][QT]
     for (int k = threadIdx.x; k < ng; k += QT) ti[k] = ti_g[k];
     for (int k = threadIdx.x; k < ng * ng; k += QT) G[k] = G_g[k];
@@ -423,7 +464,7 @@ quad_dense_kernel(QuadParams q, DenseTabs tb_, const double *__restrict__ tbar,
     float *Gh = reinterpret_cast<float *>(G + ng * ng);    // [ng][ng] FP32 high part
     float *Gl = Gh + ng * ng;                              //          low part
     double *et = G + ng * ng + ng * ng;                    // 2^(j/64)
-    double *c0 = et + ETAB;                                // [ng][QT]: u (FP64 or FP32 pair)
+    double *c0 = et + 2 * ETAB;                              // [ng][QT]: u (FP64 or FP32 pair)
     double *c1 = c0 + ng * QT;                             // [ng][QT]: E (FP64 path)
     for (int k = threadIdx.x; k < ng; k += QT) ti[k] = ti_g[k];
     for (int k = threadIdx.x; k < ng * ng; k += QT) {
@@ -650,7 +691,7 @@ void analyse_grid(int ng, const double *ti, const double *G, int full, int *step
 // lower-triangular path on a non-uniform grid), inputs (general and dense
 // paths), and the dense path's scale factors
 size_t quad_smem(int ng, int uniform, int step, int full) {
-    return sizeof(double) * (4 * ng + ng * ng + ETAB + ((uniform || full) ? 0 : ng * QT) +
+    return sizeof(double) * (4 * ng + ng * ng + 2 * ETAB + ((uniform || full) ? 0 : ng * QT) +
                              (step > 0 ? 0 : ng * QT) + (full ? ng * QT : 0));
 }
 
@@ -678,7 +719,7 @@ int grid_mirrored(int ng, const double *ti) {
 namespace {
 
 size_t dense_smem(int ng) {
-    return sizeof(double) * ((size_t)ng + 2 * (size_t)ng * ng + ETAB + 2 * (size_t)ng * QT);
+    return sizeof(double) * ((size_t)ng + 2 * (size_t)ng * ng + 2 * ETAB + 2 * (size_t)ng * QT);
 }
 
 // The dense-G integral: pair tables of the orbital energies (when given),

@@ -129,3 +129,20 @@ def test_dense_integral_on_a_grid_off_by_last_places(ctx, shift):
         for y in range(ng):
             r = numpy.longdouble(T1[y, a, i]) / T1[3, a, i] * ref[3] / ref[y]
             assert abs(r - 1) <= tol[y] + tol[3]
+
+
+def test_exponentials_are_as_accurate_as_the_library_function(ctx):
+    """Step factors are powers of one exponential, so its last bit counts.  The
+    same single weight as above, here against 64 bits: a nearly correctly
+    rounded value, half a unit in the last place and a fiftieth."""
+    rng = numpy.random.default_rng(8)
+    x = numpy.concatenate((rng.uniform(-3.0, 3.0, 40000), rng.uniform(-600.0, 600.0, 20000),
+                           rng.uniform(-0.02, 0.02, 5000)))
+    n = x.shape[0]
+    ti, g, G = quadrature.ft_quad(2, 1.0, "lin")
+    t = numpy.zeros((2, 1, n))
+    t[0] = 1.0
+    out = quadrature.int_tbar1(2, t, ti, -x.reshape(1, n), G)[1, 0]
+    ref = numpy.exp(x.astype(numpy.longdouble)) / 2
+    ulp = numpy.spacing(ref.astype(float))
+    assert (abs(out - ref) <= 0.52 * ulp).all()
