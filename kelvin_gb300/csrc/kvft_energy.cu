@@ -311,9 +311,10 @@ extern "C" int kvft_ft_cc_energy(kvft_ctx *ctx, int ng, int nv, int no, const do
 // libkvft holds (256 KiB) until the process exits.  Its device address is
 // looked up with cudaGetSymbolAddress once per device, on that device's first
 // call, so that first call should come before any stream capture.  All calls
-// on a device share the array and every call overwrites the slots it reads,
-// so nothing has to be cleared between calls; two calls that overlap on the
-// GPU (different streams, no ordering) race on it.
+// on a device share the array; every call overwrites the partial sums it
+// reads and clears the arrival count before its launch, so nothing is left to
+// the caller between calls.  Two calls that overlap on the GPU (different
+// streams, no ordering) race on both.
 // ---------------------------------------------------------------------------
 #include <mutex>
 

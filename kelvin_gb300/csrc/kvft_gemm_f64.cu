@@ -12,7 +12,7 @@ namespace {
 // GB300 issues about 2 FP64 FMAs per clock per SM: a warp's FMA occupies the
 // pipe for 16 clocks, in which the SM can issue 64 other instructions and
 // serve 16 shared-memory wavefronts.  So FMAs spent on padding are what costs,
-// and operand reuse in registers buys little.  Two layouts:
+// and operand reuse in registers buys little.  Three layouts:
 //   rows   a big tensor times a small matrix (N columns at a time, N <= 24): a
 //          thread owns one row and all N columns, its A value comes from shared
 //          memory once per k and B's by broadcast; no FMA is padding but those
@@ -27,8 +27,9 @@ namespace {
 // Measured, the whole update of 19 plane waves (38 spin orbitals, ng = 10,
 // 26.4 GFLOP; 21 ms at the FP64 peak): 64.7 ms with 64 x 64 tiles (19-wide
 // outputs padded to 64) and one launch per product, 29.1 ms with flat tiles
-// and one launch per group; an 8-site ring's iteration (8-wide outputs)
-// 4.5 -> 0.6 ms.
+// and one launch per group (27.9 with the rows layout); an 8-site ring's
+// iteration (8-wide outputs) 4.5 -> 0.6 ms (0.47 with K slices and dependent
+// launches).
 constexpr int NT = 128, TMAX = 16, BDIM_MAX = 128;
 
 struct F64Params {
@@ -516,10 +517,11 @@ int kv_gemm_f64(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     long long tiles = (long long)p.mt * p.nt * batch;
     if (!rows && !square) {
         // The largest tile (16 outputs per thread) that leaves four blocks per
-        // SM to balance the SMs, where K ranges of 256 of a long K count as
-        // blocks (every product's, since they then add by atomics) when neither
-        // extent is short; smaller tiles, down to two outputs per thread, else.  Shrinking first reads a long operand once per tile: 57 x 57
-        // outputs, K = 57^3, two products, 5.7 ms in tiles of 57 x 4, 2.85 so.
+        // SM to balance the SMs; where neither extent is short, K ranges of 256
+        // of a long K count as blocks (every product's, since they then add by
+        // atomics).  Else smaller tiles, down to two outputs per thread.
+        // Shrinking first reads a long operand once per tile: 57 x 57 outputs,
+        // K = 57^3, two products, 5.7 ms in tiles of 57 x 4, 2.85 so.
         const bool longk = cut && K >= 1024 && std::min(M, N) > 32;
         for (;; T /= 2) {
             f64_tile(M, N, NT * T, &p.BM, &p.BN);
