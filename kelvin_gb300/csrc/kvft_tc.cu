@@ -24,9 +24,9 @@
 //   * epilogue: the accumulators are read from TMEM (tcgen05.ld), the K
 //     chunks (K > KCHUNK) are summed in registers, and the tile is scaled by
 //     2^(e_m + e_n - 2 C) alpha and written to the FP64 output view once.
-// With D = 7 (15 pair products, five digits) the norm-wise relative error is
-// ~1e-11, far inside the 1e-8 amplitude / 1e-10 Ha parity bounds; D = 3..5 is
-// the mixed-precision form.
+// With D = 7 (15 pair products, five digits) the error is ~1e-13 of K max|A|
+// max|B|, far inside the 1e-8 amplitude / 1e-10 Ha parity bounds; D = 3..5 is the
+// mixed-precision form.
 //
 // Kernel: persistent, one CTA per SM walking output tiles; warp 0 = TMA
 // producer, warp 1 = MMA issuer (and TMEM owner), warps 2..9 = epilogue; the
@@ -48,6 +48,9 @@ constexpr int NTHREADS = 64 + 32 * NEPI;      // + TMA producer warp + MMA warp
 constexpr int TMEM_COLS = 512;               // all of an SM's TMEM (one CTA per SM)
 constexpr int KRANGE = 2048;                  // K range of a unit that adds by atomics
 constexpr int GROUP_M = 8;                    // m-tiles per raster group (L2 reuse)
+// Wide digits: unit 2^-WUNIT of the integer sums (level 2 has weight one), and
+// the terms after which a sum (at most 2^14 a term) goes to C, below 2^63.
+constexpr int WUNIT = 30, WFLUSH = 1 << 18;
 
 // A converted in the kernel (CV): at most CV_M rows, NCV more warps that turn
 // FP64 values into digits, CV_RING k-blocks of FP64 values in flight.
@@ -62,6 +65,7 @@ struct TcParams {
     long long c_split;    // or stored to its own copy of C, this far from the range before (0: added)
     int split_kb;         // k-blocks per K range
     int chunk_kb;         // k-blocks per K chunk (exactness bound)
+    int flush_kb;         // wide digits: k-blocks after which the running sum goes to C
     int nkb_total;        // k-blocks of the padded K extent
     int S, D, NS;         // digit planes, levels, pipeline stages
     int Mp, Np;           // rows per digit plane of A / B
@@ -169,7 +173,8 @@ __host__ __device__ constexpr size_t tc_smem(int S, int NS, int tn, int kb, bool
 //               (w - 2) / 4, frees the set, and carries the sum over the
 //               unit's K chunks in registers -- one FP32 value per element
 //               when D <= 3 (the few-digit form), an unevaluated FP32 pair
-//               (error-free two-sums) otherwise.  After the last chunk the
+//               (error-free two-sums) at D = 4 to 6, a 64-bit integer at D = 7
+//               (the level sums are integers).  After the last chunk the
 //               tile goes to C once: FP64 built from bit patterns with the
 //               scale 2^(e_m + e_n - 2 C) (and a power-of-two alpha) in the
 //               exponent field, old values of C loaded 8 at a time.
@@ -204,6 +209,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int SD = G::S, nl = G::NL;     // digit planes and levels
     constexpr int PLANE_BYTES = (CV ? CV_M : TM) * KBT * 2;   // a digit plane of an A k-block
     constexpr int BPLANE = TN * KBT * 2;         // one digit plane of a B k-block
+    constexpr bool WD = G::WIDE;             // running sums are 64-bit integers
     constexpr int WCOLS = TN / 2;            // columns per epilogue warp
     constexpr int LW = FF ? 4 : 16;          // columns per TMEM load (<= 32 registers in flight)
     constexpr int NG = WCOLS / LW;           // TMEM loads per level
@@ -508,8 +514,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int row = q * 32 + lane;
         long long *coff = s_coff + ew * WCOLS;
         int *cexp = s_cexp + ew * WCOLS;
-        float rhi[WCOLS];
-        float rlo[FF ? WCOLS : 1];
+        float rhi[WD ? 1 : WCOLS];
+        float rlo[FF && !WD ? WCOLS : 1];
+        unsigned long long sum[WD ? WCOLS : 1];      // in units of 2^-WUNIT
         int gc = 0;
         bool ok = true;
         int cached_n = -1, cached_e = -1;   // the columns coff / cexp hold (warp-uniform)
@@ -558,7 +565,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int i = 0; i < min(WCOLS, nlim); i++)
                         asm volatile("prefetch.global.L2 [%0];" ::"l"(Cr + coff[i]));
                 }
-                for (int c0 = w.kb0; c0 < w.kb1; c0 += p.chunk_kb) {
+                for (int f0 = w.kb0, f1; f0 < w.kb1 && ok; f0 = f1) {
+                f1 = WD ? min(f0 + p.flush_kb, w.kb1) : w.kb1;
+                const double be = f0 == w.kb0 ? beta : 1.0;
+                for (int c0 = f0; c0 < f1; c0 += p.chunk_kb) {
                     const int set = gc % NSET;
                     const bool got = mbar_wait(smem_u32(&accf[set]), (gc / NSET) & 1);
                     // one verdict per warp: tcgen05.ld below needs every lane
@@ -571,7 +581,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         break;
                     }
                     fence_after();
-                    const bool first = (c0 == w.kb0);
+                    const bool first = (c0 == f0);
                     const uint32_t tb =
                         tmem + ((uint32_t)(q * 32) << 16) + set * SET_COLS + h * WCOLS;
     #pragma unroll
@@ -588,8 +598,22 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             if constexpr (!FF) {
                                 if (nl > 1) hi += __uint_as_float(r[nl > 1 ? 1 : 0][j]);
                                 rhi[i] = first ? hi : rhi[i] + hi;
+                            } else if constexpr (WD) {
+                                // level l holds an integer times 2^(18 - 9 l): the
+                                // sum of all as one integer, exact but for the
+                                // rounding of the last two levels' sum
+                                const int i2 = __float2int_rn(hi);
+                                const int i3 = __float2int_rn(__uint_as_float(r[1][j]) * 512.f);
+                                const int i4 = __float2int_rn(__uint_as_float(r[2][j]) * 262144.f);
+                                const int i5 = __float2int_rn(
+                                    (__uint_as_float(r[3][j]) + __uint_as_float(r[nl > 4 ? 4 : 0][j])) *
+                                    (float)(1 << WUNIT));
+                                sum[i] = (first ? 0ull : sum[i]) +
+                                         (unsigned long long)((i2 * 512 + i3) * (1ll << (WUNIT - 9))) +
+                                         (unsigned long long)(i4 * (1ll << (WUNIT - 18))) +
+                                         (unsigned long long)(long long)i5;
                             } else {
-                                // level sums, leading first: an FP32 pair
+                                // exact level sums, leading first: an FP32 pair
                                 float lo = 0.f, e;
     #pragma unroll
                                 for (int l = 1; l < nl; l++) {
@@ -619,12 +643,17 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     // value of column i of this thread's row
                     auto value = [&](int i) -> double {
                         const int k = krow + cexp[i];
-                        double v = f32_scaled(rhi[i], k, p.alpha_sign);
-                        if constexpr (FF) v += f32_scaled(rlo[i], k, p.alpha_sign);
+                        double v;
+                        if constexpr (WD) {
+                            v = i64_scaled((long long)sum[i], k - WUNIT, p.alpha_sign);
+                        } else {
+                            v = f32_scaled(rhi[i], k, p.alpha_sign);
+                            if constexpr (FF) v += f32_scaled(rlo[i], k, p.alpha_sign);
+                        }
                         if (!p.alpha_pow2) v *= p.alpha;
                         return v;
                     };
-                    if (CV || (p.nsplit > 1 && !p.c_split) || beta == 1.0) {
+                    if (CV || (p.nsplit > 1 && !p.c_split) || be == 1.0) {
                         // C += value: each element gets exactly one addition in
                         // this launch unless K chunks run as separate units, so a
                         // fire-and-forget reduction at L2 gives old + value
@@ -632,7 +661,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         // thread waiting for the old value (measured on the
                         // 114-spin-orbital n^5 class: 82 ms per iteration
                         // against 120 ms for the load-add-store ring below)
-                        if constexpr (FF) {
+                        if constexpr (FF && !WD) {
                             if (p.alpha_pow2) {
                                 // the FP32 pair as two reductions at L2: no FP64
                                 // add on the SM (GB300's FP64 pipe bounded this
@@ -655,16 +684,16 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             for (int i = 0; i < WCOLS; i++)
                                 if (i < nlim) atomicAdd(Cr + coff[i], value(i));
                         }
-                    } else if (beta == 0.0) {
-                        if (FF && p.alpha_pow2) {
+                    } else if (be == 0.0) {
+                        if (FF && !WD && p.alpha_pow2) {
                             // hi stored, lo added at L2: hi + lo rounded once,
                             // as the FP64 add gave, without it on the SM
     #pragma unroll
                             for (int i = 0; i < WCOLS; i++) {
                                 if (i < nlim) {
                                     const int k = krow + cexp[i];
-                                    Cr[coff[i]] = f32_scaled(rhi[i], k, p.alpha_sign);
-                                    if constexpr (FF)
+                                    Cr[coff[i]] = f32_scaled(rhi[WD ? 0 : i], k, p.alpha_sign);
+                                    if constexpr (FF && !WD)
                                         atomicAdd(Cr + coff[i], f32_scaled(rlo[i], k, p.alpha_sign));
                                 }
                             }
@@ -690,7 +719,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     #pragma unroll
                             for (int j = 0; j < WG; j++) {
                                 const int i = g * WG + j;
-                                const double v = fma(beta, old[q][j], value(i));
+                                const double v = fma(be, old[q][j], value(i));
                                 if (i < nlim) Cr[coff[i]] = v;
                             }
                             if (g + RING < NGW) {
@@ -704,6 +733,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                 }
                 __syncwarp();
+                }
             }
         }
     }
@@ -1565,7 +1595,7 @@ bool cv_fits(kvft_ctx *ctx, int M, int N, int K, int batch, int nprod, const KMa
 int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, const KMat &A,
                 const KMat &B, double beta, const KOut &C, int D, const KvProds &g, bool cv) {
     const int S = dig_planes(D);
-    // D >= 4: three to five levels, FP32 pairs, TN = 64 (48 at D = 7, see the
+    // D >= 4: three to five levels, FP32 pairs or integers, TN = 64 (48 at D = 7, see the
     // kernel) and 32-deep k-blocks (up to five digit
     // planes per stage); D <= 3: 64-deep k-blocks, so that every TMA box row is
     // a full 128-byte line, and TN = 128 unless C has at most 64 columns (then
@@ -1649,6 +1679,7 @@ int gemm_tc_run(kvft_ctx *ctx, int M, int N, int K, int batch, double alpha, con
     p.nsplit = par ? nranges : 1;
     p.split_kb = par ? split_kb : nkb_total;
     p.chunk_kb = chunk_kb;
+    p.flush_kb = std::max(1, WFLUSH / kb / chunk_kb) * chunk_kb;
     p.nkb_total = nkb_total;
     p.S = S;
     p.D = D;

@@ -35,10 +35,12 @@ constexpr int TM = 128;
 //           accurate than with seven-bit digits; with 256 terms level 4 could,
 //           up to 180 times (rows that agree in three digits).
 //   D <= 6  2048 terms of level 3 (two products of at most 2^12) reach 2^24.
-// Reading out every 128 terms costs an update of 54 spin orbitals and 10 tau
-// points 10.0 -> 10.9 ms against 512, two Lambda iterations of 38 and 10
-// 29.3 -> 30.75, a residual of 37 virtual and 21 occupied 0.724 -> 0.753;
-// seven-bit digits cost the first two 1.2 and 2.0 ms.
+// So many read-outs want a short epilogue: the running sums of D = 7 are 64-bit
+// integers (the levels are integers: half the instructions of an FP32 pair
+// and no rounding).  8192^3: 15.6 ms with pairs, 12.6 so; 11.8 read out every
+// 512 terms, 12.9 with seven-bit digits.  3249^3 4 times 4.35, 3.51; 3.35; 3.71.
+// 361^3 60 times 0.237, 0.231; 0.216; 0.316.  Update of 54 spin orbitals and 10
+// tau points 11.0, 10.3; 10.0; two Lambda iterations of 38 and 10 31.0, 29.6; 29.3.
 // Error against seven-bit digits with exact sums (K = 33 to 4129; normal,
 // constant, few-valued and wide-range operands, A A^T, rows of close-by
 // values): 0.2 to 0.8 of it, in the 2-norm and for the largest element.  At D =
@@ -80,6 +82,29 @@ __device__ __forceinline__ double f32_scaled(float x, int k, unsigned sgn) {
     if (E == 0 || e64 <= 0) return 0.0;
     const uint32_t hi = ((u & 0x80000000u) ^ sgn) | ((uint32_t)e64 << 20) | ((u >> 3) & 0xFFFFFu);
     return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// FP64 value of the integer r times 2^k, rounded to nearest, with sign flipped
+// by `sgn`, by integer operations (GB300's FP64 pipe would take 16 clocks a
+// warp for the conversion alone).  Below 2^-1022 zero, above the FP64 range
+// infinite.
+__device__ __forceinline__ double i64_scaled(long long r, int k, unsigned sgn) {
+    if (r == 0) return 0.0;
+    const unsigned neg = (unsigned)(r >> 63);
+    unsigned long long a = r < 0 ? 0ull - (unsigned long long)r : (unsigned long long)r;
+    const int z = __clzll((long long)a);
+    a <<= z;                                        // 2^63 <= a
+    const int E = 63 - z + k + 1023;
+    if (E <= 0) return 0.0;
+    const unsigned s = (neg & 0x80000000u) ^ sgn;
+    if (E >= 0x7FF) return __hiloint2double((int)(s | 0x7FF00000u), 0);
+    // 53 bits, ties to even; the leading bit adds one to the exponent field
+    // and a carry out of the rounding another
+    unsigned long long m = a >> 11;
+    const unsigned rest = (unsigned)a & 0x7FFu;
+    m += rest > 0x400u || (rest == 0x400u && (m & 1));
+    m += (unsigned long long)(E - 1) << 52;
+    return __hiloint2double((int)((unsigned)(m >> 32) | s), (int)(unsigned)m);
 }
 
 // Raw row exponents are reduced with atomicMax into an array preset to

@@ -184,3 +184,52 @@ def test_wide_digits_of_close_values(ctx, K, batch, M, kind, digits=7):
         m, m7 = max(m, err.max()), max(m7, err7.max())
     assert s <= s7
     assert m <= m7
+
+
+# Integers whose digits and products the kept levels hold in full: the running
+# sums are integers, so the product is exact, up to the last bit of a rounding
+# to FP64 that does not happen.  K at and beside the read-out length, in one range
+# and several; rows and columns scaled by powers of two, whose product is then
+# exactly the scaled one, or zero or not finite where FP64 ends.
+@pytest.mark.parametrize("M,N,K,batch", [(48, 48, 65, 1), (48, 33, 128, 1), (130, 50, 129, 2),
+                                         (48, 48, 361, 1), (300, 200, 1025, 1), (64, 64, 2049, 60),
+                                         (33, 17, 4097, 60), (2000, 700, 600, 1)])
+def test_wide_digits_of_integers(ctx, M, N, K, batch, digits=7):
+    rng = numpy.random.default_rng(M + N + K)
+    A = rng.integers(-2 ** 20 + 1, 2 ** 20, (batch, M, K)).astype(float)
+    B = rng.integers(-2 ** 20 + 1, 2 ** 20, (batch, K, N)).astype(float)
+    B[:, :, 0] = abs(B[:, :, 0])
+    A[:, 0] = abs(A[:, 0])                           # the largest sums
+    ref = A @ B                                      # below 2^53: exact
+    a = rng.integers(-300, 300, (batch, M, 1)).astype(float)
+    b = rng.integers(-300, 300, (batch, 1, N)).astype(float)
+    a[:, 1], b[:, :, 1], a[:, 2], b[:, :, 2] = -560, -560, 560, 560
+    A, B = A * 2.0 ** a, B * 2.0 ** b
+    dA, dB = _lib.DeviceArray.from_host(ctx, A), _lib.DeviceArray.from_host(ctx, B)
+    dC = _lib.DeviceArray(ctx, (batch, M, N))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, M, N, K, batch, _lib.PREC_FP64_TC, digits, dA.ptr, dB.ptr,
+                              dC.ptr), "kvft_gemm")
+    with numpy.errstate(over="ignore", under="ignore"):
+        ref = numpy.ldexp(ref, (a + b).astype(int))
+    ref[abs(ref) < 2.0 ** -1022] = 0.0
+    C, fin = dC.to_host(), numpy.isfinite(ref)
+    assert (C[fin] == ref[fin]).all()
+    # sums of K ranges that each end beyond FP64 may have both signs
+    assert not numpy.isfinite(C[~fin]).any()
+
+
+def test_wide_digits_of_a_long_sum(ctx, K=600001, batch=304):
+    """A sum that runs through every read-out of a K no unit shares, with the
+    largest terms of one sign.  Tolerance: that of the digit count."""
+    torch = pytest.importorskip("torch")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    A, B = (0.49 + 0.0099 * torch.rand((batch, K), generator=g, device="cuda", dtype=torch.float64)
+            for _ in range(2))
+    C = torch.full((batch,), float("nan"), device="cuda", dtype=torch.float64)
+    torch.cuda.synchronize()
+    a, b, c = (_lib.DeviceArray(ctx, t.shape, ptr=t.data_ptr(), owner=t) for t in (A, B, C))
+    ctx.check(ctx.L.kvft_gemm(ctx.h, 1, 1, K, batch, _lib.PREC_FP64_TC, 7, a.ptr, b.ptr, c.ptr),
+              "kvft_gemm")
+    ref = (A * B).sum(1)
+    assert (abs(C - ref) <= 5e-12 * 0.25 * K).all()
