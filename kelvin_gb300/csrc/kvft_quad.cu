@@ -14,9 +14,9 @@
 //     chained: T_y = w(y,y-s) (T_{y-s} - G[y-s,y-s] tbar_{y-s})
 //                    + sum_{x=y-s}^{y} G[y,x] w(y,x) tbar_x,
 //     which is O(ng) per element instead of O(ng^2).
-// The product of <= ng factors, each within a unit in the last place, differs
-// from a direct exp by at most ~2 ng ulp (relative), far inside the 1e-10
-// parity tolerance.
+// The product of <= ng factors, each within 1.25 units in the last place,
+// differs from a direct exp by at most ~2 ng ulp (relative), far inside the
+// 1e-10 parity tolerance.
 #include "kvft_internal.h"
 
 #include <cmath>
@@ -53,15 +53,22 @@ __device__ __forceinline__ double denom(const QuadParams &q, long long p, int l,
 
 // e^x by table lookup (P. T. P. Tang, ACM TOMS 15, 144 (1989)): x = n ln2/64 +
 // r, |r| <= ln2/128, e^x = 2^(n / 64) (1 + (e^r - 1)) with the 64 values of
-// 2^(j/64) in shared memory, each as a rounded value and the rest, and a
-// sixth-order Taylor polynomial (its remainder is below 3e-20): twelve FP64
-// operations, and three of them more for e^-x, where the library function takes
-// about 17 and the reciprocal ten -- the FP64 pipe is what these kernels wait
-// for.  As accurate as the library function, 0.51 units in the last place:
-// step factors are raised to the ng-th power, and without the rests and the
-// sixth order (two operations less, 1.25 units) the tau integral of 66 spin
-// orbitals and 16 points came out with 1.3 times the error.  |x| >= 700 and NaN
-// go to the library function.
+// 2^(j/64) in shared memory and a Taylor polynomial -- the FP64 pipe is what
+// these kernels wait for.
+//   exp_tab   fifth order: ten FP64 operations, where the library function
+//             takes about 17, and three of them more for e^-x (exp_tab2), where
+//             a reciprocal takes ten; 1.25 units in the last place.
+//   exp_acc   sixth order, and the table's rounding added: twelve operations,
+//             0.51 units, as the library function.  For the one step factor of
+//             a uniform grid, which the rows raise to powers of up to ng: the
+//             integral of 66 spin orbitals and 16 points has an error of
+//             7.8e-16 with it (8.0e-16 with the library function), 1.0e-15
+//             with exp_tab, for 2.71 -> 2.78 ms.  Factors of their own
+//             for every step or node do not add up so (17 logarithmic points
+//             4.4e-16 with exp_tab, 5.0e-16 with the library function; 16
+//             Gauss-Legendre points 3.5e-16, 3.9e-16), and there exp_acc would
+//             cost 2 to 7 %.
+// |x| >= 700 and NaN go to the library function.
 constexpr int ETAB = 64;
 // 2^(j/64): rounded to FP64, and the difference from it
 __device__ const double EXP2_TAB[ETAB][2] = {
@@ -102,9 +109,10 @@ __device__ const double EXP2_TAB[ETAB][2] = {
 __device__ __forceinline__ void exp_table(double *T) {       // caller synchronises
     for (int j = threadIdx.x; j < 2 * ETAB; j += blockDim.x) T[j] = EXP2_TAB[j % ETAB][j / ETAB];
 }
+template <bool ACC = false>
 __device__ __forceinline__ double exp_scaled(const double *T, int n, double p) {
     const double t = T[n & (ETAB - 1)];
-    const double y = t + fma(t, p, T[ETAB + (n & (ETAB - 1))]);
+    const double y = ACC ? t + fma(t, p, T[ETAB + (n & (ETAB - 1))]) : fma(t, p, t);
     return __hiloint2double(__double2hiint(y) + (n >> 6) * (1 << 20), __double2loint(y));
 }
 __device__ __forceinline__ bool exp_reduce(double x, int &n, double &r) {
@@ -120,8 +128,15 @@ __device__ __forceinline__ double exp_tab(double x, const double *T) {
     int n;
     double r;
     if (!exp_reduce(x, n, r)) return exp(x);
-    const double q = fma(fma(fma(fma(r, 1.0 / 720.0, 1.0 / 120.0), r, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+    const double q = fma(fma(fma(r, 1.0 / 120.0, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
     return exp_scaled(T, n, fma(q * r, r, r));
+}
+__device__ __forceinline__ double exp_acc(double x, const double *T) {
+    int n;
+    double r;
+    if (!exp_reduce(x, n, r)) return exp(x);
+    const double q = fma(fma(fma(fma(r, 1.0 / 720.0, 1.0 / 120.0), r, 1.0 / 24.0), r, 1.0 / 6.0), r, 0.5);
+    return exp_scaled<true>(T, n, fma(q * r, r, r));
 }
 // e^x and e^-x: the polynomial's even and odd parts
 __device__ __forceinline__ void exp_tab2(double x, const double *T, double &ep, double &em) {
@@ -133,7 +148,7 @@ __device__ __forceinline__ void exp_tab2(double x, const double *T, double &ep, 
         return;
     }
     const double r2 = r * r;
-    const double ev = r2 * fma(r2, fma(r2, 1.0 / 720.0, 1.0 / 24.0), 0.5);
+    const double ev = r2 * fma(r2, 1.0 / 24.0, 0.5);
     const double od = fma(r * r2, fma(r2, 1.0 / 120.0, 1.0 / 6.0), r);
     ep = exp_scaled(T, n, ev + od);
     em = exp_scaled(T, -n, ev - od);
@@ -219,7 +234,7 @@ quad_kernel(QuadParams q, const double *__restrict__ tbar, const double *__restr
         // step factors r_k = exp((ti[k]-ti[k+1]) d)
         double r0 = 1.0;
         if (UNI) {
-            r0 = (ng > 1) ? exp_tab((ti[0] - ti[1]) * d, et) : 1.0;
+            r0 = (ng > 1) ? exp_acc((ti[0] - ti[1]) * d, et) : 1.0;
         } else {
             for (int k = 0; k + 1 < ng; k++) rk[k * QT + t] = exp_tab((ti[k] - ti[k + 1]) * d, et);
         }
