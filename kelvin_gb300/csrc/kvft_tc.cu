@@ -48,9 +48,11 @@ constexpr int NTHREADS = 64 + 32 * NEPI;      // + TMA producer warp + MMA warp
 constexpr int TMEM_COLS = 512;               // all of an SM's TMEM (one CTA per SM)
 constexpr int KRANGE = 2048;                  // K range of a unit that adds by atomics
 constexpr int GROUP_M = 8;                    // m-tiles per raster group (L2 reuse)
-// Wide digits: unit 2^-WUNIT of the integer sums (level 2 has weight one), and
-// the terms after which a sum (at most 2^14 a term) goes to C, below 2^63.
-constexpr int WUNIT = 30, WFLUSH = 1 << 18;
+// Wide digits: unit 2^-WUNIT of the integer sums (level 2 has weight one; the
+// last two levels are rounded to it, a sixteenth of their planes' own rounding
+// over 128 terms), and the terms after which a sum (at most 2^14 a term) goes to
+// C, below 2^63.
+constexpr int WUNIT = 32, WFLUSH = 1 << 16;
 
 // A converted in the kernel (CV): at most CV_M rows, NCV more warps that turn
 // FP64 values into digits, CV_RING k-blocks of FP64 values in flight.
@@ -607,7 +609,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 const int i4 = __float2int_rn(__uint_as_float(r[2][j]) * 262144.f);
                                 const int i5 = __float2int_rn(
                                     (__uint_as_float(r[3][j]) + __uint_as_float(r[nl > 4 ? 4 : 0][j])) *
-                                    (float)(1 << WUNIT));
+                                    (float)(1ll << WUNIT));
                                 sum[i] = (first ? 0ull : sum[i]) +
                                          (unsigned long long)((i2 * 512 + i3) * (1ll << (WUNIT - 9))) +
                                          (unsigned long long)(i4 * (1ll << (WUNIT - 18))) +
